@@ -206,9 +206,12 @@ int vfs_batch_solve_host(vfs_batch* b, const uint8_t* const* i0, const uint8_t* 
  * returns after enqueueing. */
 int vfs_batch_solve_device(vfs_batch* b, const uint8_t* const* d_i0, const uint8_t* const* d_i1,
                            float* const* d_u_out, int masked);
-/* The fused path picks the tile height of its iteration kernel per pyramid level by timing
- * the variants on the first solve of each batch composition (on by default); the timing
- * launches do not change results.  Off: the default 31 x 8 tiles everywhere. */
+/* A one-pair solve (and each pair of a concurrent batch) runs every pyramid level whose state fits
+ * the GPU's registers and shared memory (up to about 600,000 solved pixels with half storage,
+ * 560,000 with float) in one cooperative launch per warp, all iterations in it.  For the other levels the fused path
+ * picks the tile height of its iteration kernel by timing the variants on the first solve of
+ * each batch composition (on by default); the timing launches do not change results.  Off: the
+ * default 31 x 8 tiles there. */
 int vfs_batch_set_autotune(vfs_batch* b, int on);
 /* How a batch runs its pairs:
  *   VFS_BATCH_CONCURRENT (default): each pair replays its own CUDA graph of one-pair fused
@@ -258,7 +261,8 @@ int vfs_set_iteration_variant(vfs_stereo* s, int variant);
 int vfs_set_iteration_variants(vfs_stereo* s, const int* variants, int n_levels);
 int vfs_batch_set_iteration_variants(vfs_batch* b, const int* variants, int n_levels);
 /* The variant each pyramid level (finest first) used in the handle's last fused solve
- * (tuned, default or forced); *count receives the number of levels. */
+ * (tuned, default or forced); *count receives the number of levels.  A level held on the chip by
+ * the whole GPU (unforced, see vfs_batch_set_autotune) is reported as 14. */
 int vfs_get_iteration_variants(vfs_stereo* s, int* variants, int max_levels, int* count);
 int vfs_batch_set_iteration_variant(vfs_batch* b, int variant);
 
@@ -295,8 +299,10 @@ int vfs_equalize_hist_u8_noalloc(const uint8_t* d_src, uint8_t* d_dst, size_t n,
 long long vfs_launch_count(void);
 
 /* Device-side status of the current device (no counterpart in the reference): *status = 1 if
- * a kernel of the TMA-staged iteration variant gave up a bounded wait for its copies since the
- * last call (its block then wrote nothing), else 0; the flag is cleared.  Synchronous. */
+ * a kernel of the TMA-staged iteration variant gave up a bounded wait for its copies (its block
+ * then wrote nothing), or one of the whole-level launches a wait for a neighbour's values (the
+ * solve's results are then undefined), since the last call, else 0; the flag is cleared.
+ * Synchronous. */
 int vfs_device_status(int* status);
 /* Process-wide: launch the fused iteration kernels with programmatic dependent launch
  * (on = 1, the default), so that each launch is scheduled while the previous one drains;

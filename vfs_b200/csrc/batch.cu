@@ -379,12 +379,15 @@ void fused_solve_direct(std::vector<StereoTgvImpl*>& pairs, bool masked, bool ha
           level_variant[level] = kIterDefaultVariant;
         }
       }
-      const int variant = level_variant[level] < 0 ? kIterDefaultVariant : level_variant[level];
+      const ResPlan* res = level_variant[level] == kIterResident ? act[0]->residentPlan(masked, half, level) : nullptr;
+      const int variant = level_variant[level] < 0 || level_variant[level] == kIterResident ? kIterDefaultVariant
+                                                                                         : level_variant[level];
       // K iterations per launch where the variant is a multi-iteration one and it applies
       // here; the remaining iterations (and the fallback) use the default one-iteration form
       // (the cluster-resident kernel: all iterations, in launches of up to kCLMaxIters)
       const bool cl_here = tb_here && iter_variant_cluster(variant) && cluster_fits(variant, masked, half, lw, lh);
-      const int K = cl_here ? kCLMaxIters : tb_here ? tb_iterations(variant) : 1;
+      const int n_it = P0.nSolverIters;
+      const int K = res ? n_it : cl_here ? kCLMaxIters : tb_here ? tb_iterations(variant) : 1;
       const int v1 = (tb_iterations(variant) > 1 || iter_variant_cluster(variant) ||
                       (iter_variant_single_pair(variant) && na != 1) ||
                       (variant == kIterTmaVariant && !tma_here))
@@ -392,12 +395,33 @@ void fused_solve_direct(std::vector<StereoTgvImpl*>& pairs, bool masked, bool ha
                          : variant;
       float tau = 1.0f;
       float sigma = 1.0f / tau;
-      const int n_it = P0.nSolverIters;
       prof->profBeginPx(kProfFused, px_level, n_it, st,
-                        cl_here ? (n_it + K - 1) / K : K > 1 ? n_it / K + n_it % K : n_it);
+                        res ? 1 : cl_here ? (n_it + K - 1) / K : K > 1 ? n_it / K + n_it % K : n_it);
       for (int iter = 0; iter < n_it;) {
-        const int k = cl_here ? std::min(K, n_it - iter) : (K > 1 && iter + K <= n_it) ? K : 1;
-        if (cl_here) {
+        const int k = res ? n_it : cl_here ? std::min(K, n_it - iter) : (K > 1 && iter + K <= n_it) ? K : 1;
+        if (res) {
+          ResArgs A{};
+          A.P = iter_args(kIterDefaultVariant, sigma, tau, 1.0f, 0).pr[0];
+          A.exch = res->exch;
+          A.ctl = res->ctl;
+          A.tiles = res->tiles;
+          A.ntiles = res->ntiles;
+          A.fill = res->fill;
+          A.nfill = res->nfill;
+          A.n = n_it;
+          A.p_planes = 1;
+          A.rows = res->rows;
+          A.blocks = res->blocks;
+          A.minus_zero = make_float2(-0.0f, -0.0f);
+          for (int j = 0; j < n_it; j++) {
+            const float mu = sigma < 1000.0f ? 1.0f / std::sqrt(1 + 0.7f * tau * P0.timestep_lambda) : 1.0f;
+            const float sp = act[0]->P.alpha1 * sigma / 3.0f, sq = act[0]->P.alpha0 * sigma / 2.0f;
+            A.step[j] = ResStep{make_float2(sp, sp), make_float2(sq, sq), make_float2(tau, tau), make_float2(mu, mu)};
+            sigma = sigma / mu;
+            tau = tau * mu;
+          }
+          launch_resident(A, masked, half, st);
+        } else if (cl_here) {
           IterCLArgs C = cl_args(variant, sigma, tau, iter, k);
           C.write_tp = iter + k == n_it;
           launch_fused_iteration_cluster(C, masked, half, st, variant);
@@ -542,7 +566,9 @@ std::mutex& shared_tuned_mutex() {
 
 FusedEngine::~FusedEngine() { clear(); }
 
-void FusedEngine::note_variants(const std::vector<int>& v, int part) {
+void FusedEngine::note_variants(std::vector<int> v, int part) {
+  for (int& x : v)
+    if (x == kIterResident) x = kIterFirstClusterVariant;
   if (part == 0) {
     last_variants = v;
     return;
@@ -594,105 +620,127 @@ void FusedEngine::prepare(std::vector<StereoTgvImpl*>& pairs, bool masked) {
   for (auto* s : pairs) {
     if (!s->initialized()) throw ArgError{"fused solve: pair not initialized"};
     s->ensureFused();
+    if (!masked && s->host_code[0].empty()) {
+      s->host_code[0].resize(s->levels());
+      for (int l = 0; l < s->levels(); l++) {
+        s->host_code[0][l].resize((size_t)s->pW[l] * s->pH[l]);
+        VFS_CUDA(cudaMemcpy2DAsync(s->host_code[0][l].data(), s->pW[l], s->code_plain[l], s->pS[l], s->pW[l], s->pH[l],
+                                   cudaMemcpyDeviceToHost, s->stream()));
+      }
+      VFS_CUDA(cudaStreamSynchronize(s->stream()));
+    }
     if (masked && !s->codes_valid) {
+      s->dropResident(true);
+      s->host_code[1].assign(s->levels(), {});
       for (int l = 0; l < s->levels(); l++)
         launch_edge_codes(s->pMask[l], s->code_masked[l], s->pW[l], s->pH[l], s->pS[l], s->stream());
-      // a level without row padding reads the previous row's last pixel west of column 0;
-      // the multi-iteration kernel cannot follow that pixel, so it is used there only when
-      // no pixel of column 0 is on
-      s->tb_ok.assign(s->levels(), 1);
-      s->tma_ok.assign(s->levels(), 1);
-      for (int v = 0; v < kIterSpanSlots; v++) {
-        s->span_lo[v].assign(s->levels(), {});
-        s->span_hi[v].assign(s->levels(), {});
-        s->inner_lo[v].assign(s->levels(), {});
-        s->inner_hi[v].assign(s->levels(), {});
-      }
       for (int l = 0; l < s->levels(); l++) {
         const int w = s->pW[l], h = s->pH[l];
-        std::vector<uint8_t> code((size_t)w * h);
+        std::vector<uint8_t>& code = s->host_code[1][l];
+        code.resize((size_t)w * h);
         VFS_CUDA(cudaMemcpy2DAsync(code.data(), w, s->code_masked[l], s->pS[l], w, h, cudaMemcpyDeviceToHost,
                                    s->stream()));
-        VFS_CUDA(cudaStreamSynchronize(s->stream()));
-        for (int y = 0; y < h; y++)
-          if (code[(size_t)y * w] & kOn) {
-            s->tma_ok[l] = 0;
-            if (w == s->pS[l]) s->tb_ok[l] = 0;
-          }
-        // first and last on column of every image row
-        std::vector<int> xmin(h, w), xmax(h, -1);
-        for (int y = 0; y < h; y++)
-          for (int x = 0; x < w; x++)
-            if (code[(size_t)y * w + x] & kOn) {
-              xmin[y] = std::min(xmin[y], x);
-              xmax[y] = std::max(xmax[y], x);
-            }
-        const int tiles_x = iter_tiles_x_of(w);
-        // per row, the number of pixels left of x that are not interior (edge code 0x1F: on,
-        // with the four neighbours in the image and on)
-        const uint8_t kInterior = kOn | kR | kL | kD | kU;
-        std::vector<int> notin((size_t)h * (w + 1), 0);
-        for (int y = 0; y < h; y++)
-          for (int x = 0; x < w; x++)
-            notin[(size_t)y * (w + 1) + x + 1] = notin[(size_t)y * (w + 1) + x] + (code[(size_t)y * w + x] != kInterior);
-        for (int v = 0; v < kIterVariants; v++) {
-          const int slot = iter_span_slot(v);
-          if (slot < 0 || !iter_variant_tiled(v)) continue;
-          const int TH = kIterVariantRows[v];
-          const int rows = (h + TH - 1) / TH;
-          std::vector<uint16_t> lo(rows), hi(rows);
-          for (int r = 0; r < rows; r++) {
-            // tile row r covers image rows TH r - 1 (north halo) .. TH r + TH - 1; a column x
-            // lies in tile x / 31 and, when x % 31 == 30, in the west halo of the next tile
-            int a = w, b = -1;
-            for (int y = std::max(0, TH * r - 1); y <= std::min(h - 1, TH * r + TH - 1); y++) {
-              a = std::min(a, xmin[y]);
-              b = std::max(b, xmax[y]);
-            }
-            if (b < 0) {
-              lo[r] = 1;
-              hi[r] = 0;
-              continue;
-            }
-            lo[r] = (uint16_t)(a / 31);
-            hi[r] = (uint16_t)std::min(tiles_x - 1, b / 31 + (b % 31 == 30 ? 1 : 0));
-          }
-          s->span_lo[slot][l] = lo;
-          s->span_hi[slot][l] = hi;
-          // the longest run of tiles whose region (rows TH r - 1 .. TH r + TH - 1, columns
-          // 31 tx - 1 .. 31 tx + 30) lies in the image and holds interior pixels only
-          std::vector<uint16_t> ilo(rows, 1), ihi(rows, 0);
-          for (int r = 0; r < rows; r++) {
-            const int y_lo = TH * r - 1, y_hi = TH * r + TH - 1;
-            if (y_lo < 0 || y_hi >= h) continue;
-            int run0 = -1, best_len = 0;
-            for (int tx = 0; tx <= tiles_x; tx++) {
-              bool ok = false;
-              const int x_lo = 31 * tx - 1, x_hi = 31 * tx + 30;
-              if (tx < tiles_x && x_lo >= 0 && x_hi < w) {
-                ok = true;
-                for (int y = y_lo; ok && y <= y_hi; y++)
-                  ok = notin[(size_t)y * (w + 1) + x_hi + 1] == notin[(size_t)y * (w + 1) + x_lo];
-              }
-              if (ok && run0 < 0) run0 = tx;
-              if (!ok && run0 >= 0) {
-                if (tx - run0 > best_len) {
-                  best_len = tx - run0;
-                  ilo[r] = (uint16_t)run0;
-                  ihi[r] = (uint16_t)(tx - 1);
-                }
-                run0 = -1;
-              }
-            }
-          }
-          s->inner_lo[slot][l] = ilo;
-          s->inner_hi[slot][l] = ihi;
-        }
       }
+      VFS_CUDA(cudaStreamSynchronize(s->stream()));
+      s->spans_valid = false;
       s->codes_valid = true;
       s->generation = next_generation();  // graphs captured under the old mask are not reused
     }
   }
+}
+
+void StereoTgvImpl::ensureSpans() {
+  if (spans_valid) return;
+  // a level without row padding reads the previous row's last pixel west of column 0;
+  // the multi-iteration kernel cannot follow that pixel, so it is used there only when
+  // no pixel of column 0 is on
+  tb_ok.assign(levels(), 1);
+  tma_ok.assign(levels(), 1);
+  for (int v = 0; v < kIterSpanSlots; v++) {
+    span_lo[v].assign(levels(), {});
+    span_hi[v].assign(levels(), {});
+    inner_lo[v].assign(levels(), {});
+    inner_hi[v].assign(levels(), {});
+  }
+  for (int l = 0; l < levels(); l++) {
+    const int w = pW[l], h = pH[l];
+    const std::vector<uint8_t>& code = host_code[1][l];
+    for (int y = 0; y < h; y++)
+      if (code[(size_t)y * w] & kOn) {
+        tma_ok[l] = 0;
+        if (w == pS[l]) tb_ok[l] = 0;
+      }
+    // first and last on column of every image row
+    std::vector<int> xmin(h, w), xmax(h, -1);
+    for (int y = 0; y < h; y++)
+      for (int x = 0; x < w; x++)
+        if (code[(size_t)y * w + x] & kOn) {
+          xmin[y] = std::min(xmin[y], x);
+          xmax[y] = std::max(xmax[y], x);
+        }
+    const int tiles_x = iter_tiles_x_of(w);
+    // per row, the number of pixels left of x that are not interior (edge code 0x1F: on,
+    // with the four neighbours in the image and on)
+    const uint8_t kInterior = kOn | kR | kL | kD | kU;
+    std::vector<int> notin((size_t)h * (w + 1), 0);
+    for (int y = 0; y < h; y++)
+      for (int x = 0; x < w; x++)
+        notin[(size_t)y * (w + 1) + x + 1] = notin[(size_t)y * (w + 1) + x] + (code[(size_t)y * w + x] != kInterior);
+    for (int v = 0; v < kIterVariants; v++) {
+      const int slot = iter_span_slot(v);
+      if (slot < 0 || !iter_variant_tiled(v)) continue;
+      const int TH = kIterVariantRows[v];
+      const int rows = (h + TH - 1) / TH;
+      std::vector<uint16_t> lo(rows), hi(rows);
+      for (int r = 0; r < rows; r++) {
+        // tile row r covers image rows TH r - 1 (north halo) .. TH r + TH - 1; a column x
+        // lies in tile x / 31 and, when x % 31 == 30, in the west halo of the next tile
+        int a = w, b = -1;
+        for (int y = std::max(0, TH * r - 1); y <= std::min(h - 1, TH * r + TH - 1); y++) {
+          a = std::min(a, xmin[y]);
+          b = std::max(b, xmax[y]);
+        }
+        if (b < 0) {
+          lo[r] = 1;
+          hi[r] = 0;
+          continue;
+        }
+        lo[r] = (uint16_t)(a / 31);
+        hi[r] = (uint16_t)std::min(tiles_x - 1, b / 31 + (b % 31 == 30 ? 1 : 0));
+      }
+      span_lo[slot][l] = lo;
+      span_hi[slot][l] = hi;
+      // the longest run of tiles whose region (rows TH r - 1 .. TH r + TH - 1, columns
+      // 31 tx - 1 .. 31 tx + 30) lies in the image and holds interior pixels only
+      std::vector<uint16_t> ilo(rows, 1), ihi(rows, 0);
+      for (int r = 0; r < rows; r++) {
+        const int y_lo = TH * r - 1, y_hi = TH * r + TH - 1;
+        if (y_lo < 0 || y_hi >= h) continue;
+        int run0 = -1, best_len = 0;
+        for (int tx = 0; tx <= tiles_x; tx++) {
+          bool ok = false;
+          const int x_lo = 31 * tx - 1, x_hi = 31 * tx + 30;
+          if (tx < tiles_x && x_lo >= 0 && x_hi < w) {
+            ok = true;
+            for (int y = y_lo; ok && y <= y_hi; y++)
+              ok = notin[(size_t)y * (w + 1) + x_hi + 1] == notin[(size_t)y * (w + 1) + x_lo];
+          }
+          if (ok && run0 < 0) run0 = tx;
+          if (!ok && run0 >= 0) {
+            if (tx - run0 > best_len) {
+              best_len = tx - run0;
+              ilo[r] = (uint16_t)run0;
+              ihi[r] = (uint16_t)(tx - 1);
+            }
+            run0 = -1;
+          }
+        }
+      }
+      inner_lo[slot][l] = ilo;
+      inner_hi[slot][l] = ihi;
+    }
+  }
+  spans_valid = true;
 }
 
 void FusedEngine::solve(std::vector<StereoTgvImpl*>& pairs, bool masked, bool half, cudaStream_t st, int part) {
@@ -727,9 +775,18 @@ void FusedEngine::solve_parts(std::vector<StereoTgvImpl*>& pairs, bool masked, b
   auto in_part = [&](int l) { return !((part == 1 && l == 0) || (part == 2 && l > 0)) && l <= max_top; };
   bool need_tune = false;
   const bool one_pair = pairs.size() == 1;
+  // levels that fit the chip run the register-resident form; it is never timed against the others
+  auto resident = [&](int l) { return one_pair && !forced && pairs[0]->residentPlan(masked, half, l) != nullptr; };
+  if (one_pair && !forced) pairs[0]->ensureResident(masked, half, st);
   auto level_key = [&](int l) {
     return std::array<int, 5>{(int)masked, (int)half, concurrency > 1 ? 2 : 1, pairs[0]->pW[l], pairs[0]->pH[l]};
   };
+  if (masked) {
+    bool all = true;
+    for (int l = 0; l < maxL; l++) all = all && (!in_part(l) || resident(l));
+    if (!all)
+      for (auto* s : pairs) s->ensureSpans();
+  }
   if (autotune && !forced) {
     // a composition tuned before (by any engine of the process) is reused, so that every
     // pair of a batch runs the same choice and only the first tunes; a one-pair solve also
@@ -738,7 +795,7 @@ void FusedEngine::solve_parts(std::vector<StereoTgvImpl*>& pairs, bool masked, b
     auto& shared = shared_tuned();
     auto sit = shared.find(comp);
     for (int l = 0; l < maxL; l++) {
-      if (!in_part(l) || tit->second[l] >= 0) continue;
+      if (!in_part(l) || tit->second[l] >= 0 || resident(l)) continue;
       if (sit != shared.end() && l < (int)sit->second.size() && sit->second[l] >= 0) {
         tit->second[l] = sit->second[l];
         continue;
@@ -765,7 +822,12 @@ void FusedEngine::solve_parts(std::vector<StereoTgvImpl*>& pairs, bool masked, b
     // first solve of this composition (and part): run it directly and tune while it runs
     tuning_solves().fetch_add(1, std::memory_order_relaxed);
     std::vector<int> lv = tit->second;
+    for (int l = 0; l < maxL; l++)
+      if (resident(l)) lv[l] = kIterResident;
     fused_solve_direct(pairs, masked, half, st, lv, true, concurrency, part);
+    std::vector<int> ran = lv;
+    for (int l = 0; l < maxL; l++)
+      if (resident(l)) lv[l] = tit->second[l];
     tit->second = lv;
     {
       std::lock_guard<std::mutex> lk(shared_tuned_mutex());
@@ -777,10 +839,12 @@ void FusedEngine::solve_parts(std::vector<StereoTgvImpl*>& pairs, bool masked, b
           if (one_pair && l < pairs[0]->levels()) shared_level_tuned().emplace(level_key(l), lv[l]);
         }
     }
-    note_variants(lv, part);
+    note_variants(ran, part);
     return;
   }
   std::vector<int> variants = tit->second;
+  for (int l = 0; l < maxL; l++)
+    if (resident(l)) variants[l] = kIterResident;
   if (forced_variant >= 0) variants.assign(maxL, forced_variant);
   if (!forced_levels.empty()) {
     variants.assign(maxL, kIterDefaultVariant);

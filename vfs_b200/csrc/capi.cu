@@ -706,7 +706,8 @@ long long vfs_launch_count(void) { return vfs::launch_counter().load(); }
 
 int vfs_device_status(int* status) {
   try {
-    int v = vfs::tma_status_take();
+    const int tma = vfs::tma_status_take(), res = vfs::resident_status_take();
+    const int v = tma || res ? 1 : 0;
     if (status) *status = v;
     return VFS_OK;
   } catch (const vfs::CudaError& e) {

@@ -324,6 +324,10 @@ constexpr int kIterFirstDeepTBVariant = 12;
 constexpr int kIterFirstClusterVariant = 14;
 inline bool iter_variant_cluster(int v) { return v == kIterFirstClusterVariant || v == kIterFirstClusterVariant + 1; }
 constexpr int kIterDefaultVariant = 1;
+// Not a numbered variant: the register-resident form (resident.cuh), taken by every unforced
+// one-pair solve at the levels that have a plan.  vfs_get_iteration_variants reports it as 14,
+// the other form that holds a whole level on the chip.
+constexpr int kIterResident = 100;
 inline int iter_tiles_x_of(int w) { return (w + 30) / 31; }
 inline int iter_tiles_of(int w, int h, int rows) { return iter_tiles_x_of(w) * ((h + rows - 1) / rows); }
 

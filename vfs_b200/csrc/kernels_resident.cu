@@ -1,0 +1,1067 @@
+// Kernels of the register-resident iteration (resident.cuh).
+#include "resident.cuh"
+
+#include <algorithm>
+#include <map>
+#include <mutex>
+#include <tuple>
+#include <type_traits>
+
+#include "tgv_exact_pairs.cuh"
+#include "tgv_pixel.cuh"
+#include "tgv_pixel_fast.cuh"
+
+namespace vfs {
+
+namespace x2 = fast::x2;
+
+namespace {
+
+constexpr unsigned kFull = 0xffffffffu;
+constexpr int kResMaxPolls = 1 << 20;
+
+__device__ int g_res_status;  // 1 = a wait for a neighbour's words ran out
+
+// one exchange word as a single 128-bit memory operation at L2
+__device__ __forceinline__ void st_word(uint4* p, uint4 v) {
+  const unsigned long long lo = v.x | ((unsigned long long)v.y << 32), hi = v.z | ((unsigned long long)v.w << 32);
+  asm volatile("{\n .reg .b128 t;\n mov.b128 t, {%1, %2};\n st.relaxed.gpu.global.b128 [%0], t;\n}" ::"l"(p), "l"(lo),
+               "l"(hi)
+               : "memory");
+}
+__device__ __forceinline__ uint4 ld_word(const uint4* p) {
+  unsigned long long lo, hi;
+  asm volatile("{\n .reg .b128 t;\n ld.relaxed.gpu.global.b128 t, [%2];\n mov.b128 {%0, %1}, t;\n}"
+               : "=l"(lo), "=l"(hi)
+               : "l"(p)
+               : "memory");
+  return make_uint4((unsigned)lo, (unsigned)(lo >> 32), (unsigned)hi, (unsigned)(hi >> 32));
+}
+
+__device__ __forceinline__ unsigned bits(__half2 h) { return *reinterpret_cast<unsigned*>(&h); }
+__device__ __forceinline__ __half2 as_half2(unsigned b) { return *reinterpret_cast<__half2*>(&b); }
+
+// Per-warp shared memory: the coefficients (rows -1 .. R-1) and edge codes, and a place to hand
+// the halo columns to lanes 0 and 31.  At a masked-out pixel a and b hold its stale T p instead
+// (its tensor is not used).
+// Beside them each lane's exchange offsets and pixel masks, read back at every iteration.
+// half storage: rows in pairs, each coefficient's two rows side by side for the packed
+// instructions: (a, b), (c, 1 / eta_u), (Iu, Iz), (1 / eta_v1, 1 / eta_v2), 1 / Iu
+// float storage: (a, b), (c, Iu), Iz, and p, (q.x, q.y), (q.z, q.w) in the same pairs
+// What a lane's edge rules need, bit r + 1 for row r: x (y): the pixel is on and takes its right
+// (lower) neighbour; on: the pixel is on.
+struct ResEdge {
+  unsigned x, y, on;
+};
+// What a warp reads back at every iteration.
+struct ResLinks {
+  uint4 at[32];    // per lane: exchange words of ring slot 0 read from above, below and beside; e.x
+  uint2 edge[32];  // e.y, e.on
+  int kind;        // ResKind of the tile
+  int t;           // tile
+  int pad[2];
+};
+template <class ST, int R>
+struct ResShared;
+template <int R>
+struct ResShared<__half, R> {
+  float4 top[32];
+  float4 cf[R / 2][4][32];
+  float2 riu[R / 2][32];
+  uint2 col[2][R];
+  ResLinks k;
+};
+template <int R>
+struct ResShared<float, R> {
+  float4 top[32];
+  float4 ab[R / 2][32], ci[R / 2][32];
+  float4 p[R / 2][32], qxy[R / 2][32], qzw[R / 2][32];
+  float4 qtop[32];
+  float2 iz[R / 2][32];
+  float2 ptop[32];
+  uint4 col[2][R];
+  ResLinks k;
+};
+
+__device__ __forceinline__ float lo(x2::f2 v) { return x2::upk(v).x; }
+__device__ __forceinline__ x2::f2 both(float v) { return x2::pk(v, v); }
+__device__ __forceinline__ float hi(x2::f2 v) { return x2::upk(v).y; }
+__device__ __forceinline__ float2 unpack(unsigned h) { return __half22float2(as_half2(h)); }
+__device__ __forceinline__ unsigned pack(float x, float y) { return bits(__float22half2_rn(make_float2(x, y))); }
+
+// A tile's state and its iteration.
+template <bool MASKED, class ST, int R>
+struct ResState;
+
+// Half storage.  Rows are taken two at a time, a row's value in each half of the packed FP32
+// instructions, so that nearly every operation of the dual, threshold and primal steps serves
+// two pixels; only the differences along a column, whose operands straddle the pairs, the
+// comparisons and the conversions are per pixel.
+template <bool MASKED, int R>
+struct ResState<MASKED, __half, R> {
+  typedef ResShared<__half, R> Sh;
+  typedef x2::f2 f2;
+  f2 u[R / 2], ub[R / 2];
+  unsigned v[R];                                 // v-bar
+  unsigned p[R + 1], q0[R + 1], q1[R + 1];       // rows -1 .. R-1: p, (q.x, q.y), (q.z, q.w)
+
+  __device__ __forceinline__ void clear(Sh&, int) {
+#pragma unroll
+    for (int i = 0; i <= R; i++) p[i] = q0[i] = q1[i] = 0u;
+  }
+  // east / south: edge codes of the pixel's right and lower neighbour
+  __device__ __forceinline__ bool set_row(Sh& sh, int lane, const IterPair& P, int r, bool in, int pos, unsigned code,
+                                          unsigned east, unsigned south) {
+    float4 ca = make_float4(0.f, 0.f, 0.f, 1.f);
+    if (in) ca = P.abce[pos];
+    if (MASKED && in && !(code & kOn)) {
+      // read by the right / lower neighbour only where that one's other side is off too
+      const float2 tp = P.Tp[pos];
+      ca.x = (east & kOn) && !(east & kR) ? tp.x : 0.f;
+      ca.y = (south & kOn) && !(south & kD) ? tp.y : 0.f;
+    }
+    if (r < 0) {
+      sh.top[lane] = ca;
+      return false;
+    }
+    const int i = r >> 1, k = r & 1;
+    float2 rv = in ? P.rv[pos] : make_float2(1.f, 1.f);
+    // eta_v2 = 0 (updatePrimalVariables.cu:103-105): .x takes tau itself, .y keeps its value
+    if (fast::etav2_zero(rv.y)) rv = make_float2(1.f, 0.f);
+    const float iu = in ? P.Iu[pos] : 0.f;
+    const float c[8] = {ca.x, ca.y, ca.z, ca.w, iu, in ? P.Iz[pos] : 0.f, rv.x, rv.y};
+#pragma unroll
+    for (int j = 0; j < 8; j++) reinterpret_cast<float*>(&sh.cf[i][j >> 1][lane])[2 * (j & 1) + k] = c[j];
+    // the Newton step -rho / Iu of the threshold; 0 where Iu = 0 (no step there)
+    reinterpret_cast<float*>(&sh.riu[i][lane])[k] = iu == 0.0f ? 0.0f : fast::rcp(iu);
+    float un = in ? P.u[pos] : 0.f, ubn = in ? P.u_[pos] : 0.f;
+    v[r] = 0u;
+    if (MASKED && in && !(code & kOn)) {  // the other ping-pong values of a masked-out pixel
+      un = P.u_s[pos];
+      p[r + 1] = bits(((const __half2*)P.v_s)[pos]);
+    }
+    u[i] = k ? x2::pk(lo(u[i]), un) : x2::pk(un, 0.f);
+    ub[i] = k ? x2::pk(lo(ub[i]), ubn) : x2::pk(ubn, 0.f);
+    return false;
+  }
+  __device__ __forceinline__ float u_of(int r) const { return r & 1 ? hi(u[r >> 1]) : lo(u[r >> 1]); }
+  __device__ __forceinline__ float ub_of(int r) const { return r & 1 ? hi(ub[r >> 1]) : lo(ub[r >> 1]); }
+  __device__ __forceinline__ __half2 v_of(int r) const { return as_half2(v[r]); }
+  __device__ __forceinline__ uint4 word(int r, unsigned tag) const {
+    return make_uint4(__float_as_uint(ub_of(r)), v[r], 0u, tag);
+  }
+  static __device__ __forceinline__ void put_col(Sh& sh, int side, int r, uint4 w) { sh.col[side][r] = make_uint2(w.x, w.y); }
+  __device__ __forceinline__ void take_col(Sh& sh, int side) {
+#pragma unroll
+    for (int i = 0; i < R / 2; i++) {
+      const uint4 w = *reinterpret_cast<const uint4*>(&sh.col[side][2 * i]);
+      ub[i] = x2::pk(__uint_as_float(w.x), __uint_as_float(w.z));
+      v[2 * i] = w.y;
+      v[2 * i + 1] = w.w;
+    }
+  }
+  __device__ __forceinline__ void store_pq(const Sh&, int, int r, void* po, void* qo, int pos) const {
+    reinterpret_cast<unsigned*>(po)[pos] = p[r + 1];
+    reinterpret_cast<uint2*>(qo)[pos] = make_uint2(q0[r + 1], q1[r + 1]);
+  }
+
+  // One iteration.  wn / ws: the words of the row above / below the tile.  KIND: ResKind of the
+  // tile.  E: what the edge rules need (bit r + 1 of each mask: row r).
+  //
+  // Edge rules.  The x difference of an on pixel takes its right neighbour where that is on, else
+  // its left one; either is the difference to the east of a lane, its own or its west lane's.
+  // The threshold and primal steps take T p.x, q.x and q.w of the pixel and of its left
+  // neighbour; the pixel's own count where its right neighbour is on, the left one's where that is
+  // on, which is the same condition seen from the left pixel (it is on, and so is its right
+  // neighbour).  So those values are replaced by zero once, at the pixel, where it is off or
+  // its right neighbour is; likewise along y.  (-0 in T p, so that 0 - x is -x.)
+  template <int KIND>
+  __device__ __forceinline__ void iterate(Sh& sh, const ResArgs& A, int lane, const ResStep& S, const ResEdge& E,
+                                          uint4 wn, uint4 ws, float2* tp_out, int s, unsigned tp_rows) {
+    using namespace x2;
+    constexpr bool EDGE = KIND != kResInner;
+    constexpr bool KEEP = MASKED && KIND == kResKeep;
+    const f2 sp = pk(S.sp.x, S.sp.y), sq = pk(S.sq.x, S.sq.y), tau = pk(S.tau.x, S.tau.y), mu = pk(S.mu.x, S.mu.y);
+    const f2 lam = both(A.P.lambda), al0 = both(A.P.alpha0), al1 = both(A.P.alpha1);
+    auto bit = [](unsigned m, int r) { return (m >> (r + 1)) & 1u; };
+    // row -1: its dual step, for T p and q of the row above row 0
+    float tpy_n, qz_n, qy_n;       // T p.y, q.z and q.y of the row above
+    float du_n;                    // u-bar and v-bar less those of the row above
+    float2 dv_n;
+    float2 vc = unpack(v[0]);      // v-bar of the pair's first row
+    {
+      const float4 ca = sh.top[lane];
+      const float ubc = __uint_as_float(wn.x);
+      const float2 vp = unpack(wn.y), ve = unpack(__shfl_down_sync(kFull, wn.y, 1));
+      float dux = __shfl_down_sync(kFull, ubc, 1) - ubc;
+      float2 dvx = make_float2(ve.x - vp.x, ve.y - vp.y);
+      du_n = lo(ub[0]) - ubc;
+      dv_n = make_float2(vc.x - vp.x, vc.y - vp.y);
+      if (EDGE) {
+        const float wu = __shfl_up_sync(kFull, dux, 1);
+        const float2 wv = make_float2(__shfl_up_sync(kFull, dvx.x, 1), __shfl_up_sync(kFull, dvx.y, 1));
+        const bool r0 = bit(E.x, -1);
+        dux = r0 ? dux : wu;
+        dvx = make_float2(r0 ? dvx.x : wv.x, r0 ? dvx.y : wv.y);
+      }
+      const float gx = dux - vp.x, gy = du_n - vp.y;
+      const float2 h0 = unpack(p[0]), h1 = unpack(q0[0]), h2 = unpack(q1[0]);
+      float px = __fmaf_rn(S.sp.x, __fmaf_rn(ca.x, gx, ca.z * gy), h0.x);
+      float py = __fmaf_rn(S.sp.x, __fmaf_rn(ca.z, gx, ca.y * gy), h0.y);
+      const float rp = fast::unit_scale(__fmaf_rn(px, px, py * py));
+      px *= rp;
+      py *= rp;
+      float qx = __fmaf_rn(S.sq.x, dvx.x, h1.x), qy = __fmaf_rn(S.sq.x, dv_n.y, h1.y);
+      float qz = __fmaf_rn(S.sq.x, dv_n.x, h2.x), qw = __fmaf_rn(S.sq.x, dvx.y, h2.y);
+      const float rq = fast::unit_scale(__fmaf_rn(qx, qx, __fmaf_rn(qy, qy, __fmaf_rn(qz, qz, qw * qw))));
+      qx *= rq;
+      qy *= rq;
+      qz *= rq;
+      qw *= rq;
+      p[0] = pack(px, py);
+      q0[0] = pack(qx, qy);
+      q1[0] = pack(qz, qw);
+      tpy_n = __fmaf_rn(ca.z, px, ca.y * py);
+      qz_n = qz;
+      qy_n = qy;
+      if (EDGE) {
+        const bool d0 = bit(E.y, -1);
+        const bool o0 = MASKED ? d0 : bit(E.on, -1);
+        tpy_n = o0 ? tpy_n : KEEP && !bit(E.on, -1) ? ca.y : -0.0f;
+        qz_n = d0 ? qz : 0.f;
+        qy_n = d0 ? qy : 0.f;
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < R / 2; i++) {
+      const int r = 2 * i;
+      const f2 UB = ub[i];
+      const float ub0 = lo(UB), ub1 = hi(UB);
+      const float2 v1 = unpack(v[r + 1]);
+      const float ubd = i + 1 < R / 2 ? lo(ub[i + 1 < R / 2 ? i + 1 : 0]) : __uint_as_float(ws.x);
+      const float2 vd = unpack(i + 1 < R / 2 ? v[r + 2 < R ? r + 2 : 0] : ws.y);
+      const f2 VX = pk(vc.x, v1.x), VY = pk(vc.y, v1.y);
+      const ulonglong2 ab = *reinterpret_cast<const ulonglong2*>(&sh.cf[i][0][lane]);
+      const ulonglong2 ce = *reinterpret_cast<const ulonglong2*>(&sh.cf[i][1][lane]);
+      const ulonglong2 uz = *reinterpret_cast<const ulonglong2*>(&sh.cf[i][2][lane]);
+      const ulonglong2 rr = *reinterpret_cast<const ulonglong2*>(&sh.cf[i][3][lane]);
+      const f2 riu = *reinterpret_cast<const f2*>(&sh.riu[i][lane]);
+      // ---- differences of u-bar and v-bar to the east and to the south -----------------
+      const float2 e0 = unpack(__shfl_down_sync(kFull, v[r], 1)), e1 = unpack(__shfl_down_sync(kFull, v[r + 1], 1));
+      f2 dux = sub(pk(__shfl_down_sync(kFull, ub0, 1), __shfl_down_sync(kFull, ub1, 1)), UB);
+      f2 dxx = sub(pk(e0.x, e1.x), VX), dxy = sub(pk(e0.y, e1.y), VY);
+      const float du0 = ub1 - ub0, du1 = ubd - ub1;
+      const float2 dv0 = make_float2(v1.x - vc.x, v1.y - vc.y), dv1 = make_float2(vd.x - v1.x, vd.y - v1.y);
+      f2 duy = pk(du0, du1), dyx = pk(dv0.x, dv1.x), dyy = pk(dv0.y, dv1.y);
+      bool r0 = true, r1 = true, d0 = true, d1 = true;
+      if (EDGE) {
+        r0 = bit(E.x, r);
+        r1 = bit(E.x, r + 1);
+        d0 = bit(E.y, r);
+        d1 = bit(E.y, r + 1);
+        const float wu0 = __shfl_up_sync(kFull, lo(dux), 1), wu1 = __shfl_up_sync(kFull, hi(dux), 1);
+        const float wx0 = __shfl_up_sync(kFull, lo(dxx), 1), wx1 = __shfl_up_sync(kFull, hi(dxx), 1);
+        const float wy0 = __shfl_up_sync(kFull, lo(dxy), 1), wy1 = __shfl_up_sync(kFull, hi(dxy), 1);
+        dux = pk(r0 ? lo(dux) : wu0, r1 ? hi(dux) : wu1);
+        dxx = pk(r0 ? lo(dxx) : wx0, r1 ? hi(dxx) : wx1);
+        dxy = pk(r0 ? lo(dxy) : wy0, r1 ? hi(dxy) : wy1);
+        duy = pk(d0 ? du0 : du_n, d1 ? du1 : du0);
+        dyx = pk(d0 ? dv0.x : dv_n.x, d1 ? dv1.x : dv0.x);
+        dyy = pk(d0 ? dv0.y : dv_n.y, d1 ? dv1.y : dv0.y);
+        du_n = du1;
+        dv_n = dv1;
+      }
+      // ---- dual step ------------------------------------------------------------------
+      const f2 a = ab.x, b = ab.y, c = ce.x;
+      const f2 ux = sub(dux, VX), uy = sub(duy, VY);
+      const float2 p0 = unpack(p[r + 1]), p1 = unpack(p[r + 2]);
+      const float2 qa0 = unpack(q0[r + 1]), qa1 = unpack(q0[r + 2]), qb0 = unpack(q1[r + 1]), qb1 = unpack(q1[r + 2]);
+      f2 px = fma(sp, fma(a, ux, mul(c, uy)), pk(p0.x, p1.x));
+      f2 py = fma(sp, fma(c, ux, mul(b, uy)), pk(p0.y, p1.y));
+      const f2 n2 = fma(px, px, mul(py, py));
+      const f2 rp = pk(fast::unit_scale(lo(n2)), fast::unit_scale(hi(n2)));
+      px = mul(px, rp);
+      py = mul(py, rp);
+      f2 qx = fma(sq, dxx, pk(qa0.x, qa1.x));
+      f2 qy = fma(sq, dyy, pk(qa0.y, qa1.y));
+      f2 qz = fma(sq, dyx, pk(qb0.x, qb1.x));
+      f2 qw = fma(sq, dxy, pk(qb0.y, qb1.y));
+      const f2 m2 = fma(qx, qx, fma(qy, qy, fma(qz, qz, mul(qw, qw))));
+      const f2 rq = pk(fast::unit_scale(lo(m2)), fast::unit_scale(hi(m2)));
+      qx = mul(qx, rq);
+      qy = mul(qy, rq);
+      qz = mul(qz, rq);
+      qw = mul(qw, rq);
+      f2 tpx = fma(a, px, mul(c, py)), tpy = fma(c, px, mul(b, py));
+      unsigned pn0 = pack(lo(px), lo(py)), pn1 = pack(hi(px), hi(py));
+      q0[r + 1] = pack(lo(qx), lo(qy));
+      q1[r + 1] = pack(lo(qz), lo(qw));
+      q0[r + 2] = pack(hi(qx), hi(qy));
+      q1[r + 2] = pack(hi(qz), hi(qw));
+      if (!MASKED && EDGE) {  // outside the circle p = 0: T p = T 0
+        const float2 z = make_float2(0.f, 0.f);
+        if ((tp_rows >> r) & 1u) tp_out[r * s] = bit(E.on, r) ? make_float2(lo(tpx), lo(tpy)) : tp_math(lo(a), lo(b), lo(c), z);
+        if ((tp_rows >> (r + 1)) & 1u)
+          tp_out[(r + 1) * s] = bit(E.on, r + 1) ? make_float2(hi(tpx), hi(tpy)) : tp_math(hi(a), hi(b), hi(c), z);
+      } else {
+        if ((tp_rows >> r) & 1u) tp_out[r * s] = make_float2(lo(tpx), lo(tpy));
+        if ((tp_rows >> (r + 1)) & 1u) tp_out[(r + 1) * s] = make_float2(hi(tpx), hi(tpy));
+      }
+      // ---- threshold step -----------------------------------------------------------
+      f2 txo = tpx, tyo = tpy;  // as counted for this pixel and its right / lower neighbour
+      bool o0 = true, o1 = true;
+      if (EDGE) {
+        if (KEEP || !MASKED) {
+          o0 = bit(E.on, r);
+          o1 = bit(E.on, r + 1);
+        }
+        const float zx0 = KEEP && !o0 ? lo(a) : -0.0f, zx1 = KEEP && !o1 ? hi(a) : -0.0f;
+        const float zy0 = KEEP && !o0 ? lo(b) : -0.0f, zy1 = KEEP && !o1 ? hi(b) : -0.0f;
+        // the plain form takes the difference at the last row and column too
+        txo = pk((MASKED ? r0 : o0) ? lo(tpx) : zx0, (MASKED ? r1 : o1) ? hi(tpx) : zx1);
+        tyo = pk((MASKED ? d0 : o0) ? lo(tpy) : zy0, (MASKED ? d1 : o1) ? hi(tpy) : zy1);
+        qx = pk(r0 ? lo(qx) : 0.f, r1 ? hi(qx) : 0.f);
+        qw = pk(r0 ? lo(qw) : 0.f, r1 ? hi(qw) : 0.f);
+        qz = pk(d0 ? lo(qz) : 0.f, d1 ? hi(qz) : 0.f);
+        qy = pk(d0 ? lo(qy) : 0.f, d1 ? hi(qy) : 0.f);
+      }
+      const f2 tpw = pk(__shfl_up_sync(kFull, lo(txo), 1), __shfl_up_sync(kFull, hi(txo), 1));
+      const f2 qxw = pk(__shfl_up_sync(kFull, lo(qx), 1), __shfl_up_sync(kFull, hi(qx), 1));
+      const f2 qww = pk(__shfl_up_sync(kFull, lo(qw), 1), __shfl_up_sync(kFull, hi(qw), 1));
+      const f2 dy = pk(lo(tyo) - tpy_n, hi(tyo) - lo(tyo));
+      const f2 dqz = pk(lo(qz) - qz_n, hi(qz) - lo(qz)), dqy = pk(lo(qy) - qy_n, hi(qy) - lo(qy));
+      const f2 U = u[i], iu = uz.x;
+      const f2 teu = mul(tau, ce.y);
+      const f2 dun = sub(fma(teu, add(sub(txo, tpw), dy), UB), U);
+      const f2 rho = fma(iu, dun, uz.y);
+      const f2 lt = mul(lam, teu);
+      const f2 up = mul(lt, mul(iu, iu));
+      f2 un;
+      {
+        // |rho| <= upper: the Newton step; beyond it a step of lambda tau / eta_u against the sign of
+        // rho (lambda >= 0); a NaN residual leaves u
+        float x[2], y[2];
+        bool num[2];
+#pragma unroll
+        for (int k = 0; k < 2; k++) {
+          const float rh = k ? hi(rho) : lo(rho), upk_ = k ? hi(up) : lo(up), ltk = k ? hi(lt) : lo(lt);
+          const bool in = fabsf(rh) <= upk_;
+          num[k] = in || fabsf(rh) > upk_;
+          const float away = __uint_as_float(__float_as_uint(ltk) ^ (~__float_as_uint(rh) & 0x80000000u));
+          x[k] = in ? -rh : away;
+          y[k] = in ? (k ? hi(riu) : lo(riu)) : (k ? hi(iu) : lo(iu));
+        }
+        const f2 d = fma(pk(x[0], x[1]), pk(y[0], y[1]), dun);
+        un = add(U, pk(num[0] ? lo(d) : 0.0f, num[1] ? hi(d) : 0.0f));
+      }
+      // ---- primal step --------------------------------------------------------------
+      const f2 gx = fma(al1, tpx, mul(al0, add(sub(qx, qxw), dqz)));
+      const f2 gy = fma(al1, tpy, mul(al0, add(sub(qw, qww), dqy)));
+      const f2 vx = fma(mul(tau, rr.x), gx, VX);
+      const f2 vy = fma(mul(tau, rr.y), gy, VY);
+      f2 us = fma(mu, sub(un, UB), un);
+      const f2 vsx = fma(mu, sub(vx, VX), vx), vsy = fma(mu, sub(vy, VY), vy);
+      unsigned vn0 = pack(lo(vsx), lo(vsy)), vn1 = pack(hi(vsx), hi(vsy));
+      if (KEEP) {  // unwritten pixels alternate between the two ping-pong buffers' values
+        un = pk(o0 ? lo(un) : ub0, o1 ? hi(un) : ub1);
+        us = pk(o0 ? lo(us) : lo(U), o1 ? hi(us) : hi(U));
+        vn0 = o0 ? vn0 : p[r + 1];
+        vn1 = o1 ? vn1 : p[r + 2];
+        pn0 = o0 ? pn0 : v[r];
+        pn1 = o1 ? pn1 : v[r + 1];
+      } else if (EDGE && !MASKED) {  // outside the circle
+        un = pk(o0 ? lo(un) : 0.f, o1 ? hi(un) : 0.f);
+        us = pk(o0 ? lo(us) : 0.f, o1 ? hi(us) : 0.f);
+        vn0 = o0 ? vn0 : 0u;
+        vn1 = o1 ? vn1 : 0u;
+      }
+      u[i] = un;
+      ub[i] = us;
+      v[r] = vn0;
+      v[r + 1] = vn1;
+      p[r + 1] = pn0;
+      p[r + 2] = pn1;
+      tpy_n = hi(tyo);
+      qz_n = hi(qz);
+      qy_n = hi(qy);
+      vc = vd;
+    }
+  }
+};
+
+// Float storage: the operations of the drop-in kernels in their order, rows in pairs as above.
+// PLAIN: quotients and roots by the plain operators.
+template <bool MASKED, int R>
+struct ResState<MASKED, float, R> {
+  typedef ResShared<float, R> Sh;
+  typedef x2::f2 f2;
+  f2 u[R / 2], ub[R / 2], vx[R / 2], vy[R / 2];
+
+  static __device__ __forceinline__ float& el(float4& v, int j) { return reinterpret_cast<float*>(&v)[j]; }
+  static __device__ __forceinline__ float el(const float4& v, int j) { return reinterpret_cast<const float*>(&v)[j]; }
+
+  __device__ __forceinline__ void clear(Sh& sh, int lane) {
+    const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int i = 0; i < R / 2; i++) sh.p[i][lane] = sh.qxy[i][lane] = sh.qzw[i][lane] = z;
+    sh.qtop[lane] = z;
+    sh.ptop[lane] = make_float2(0.f, 0.f);
+  }
+  // in the range of the exact quotients
+  static __device__ __forceinline__ bool ranged(float b) { return fabsf(b) >= 0x1p-100f && fabsf(b) <= 0x1p100f; }
+  // returns whether the pixel asks for the plain operators
+  __device__ __forceinline__ bool set_row(Sh& sh, int lane, const IterPair& P, int r, bool in, int pos, unsigned code,
+                                          unsigned east, unsigned south) {
+    float a = 0.f, b = 0.f, c = 0.f;
+    if (in) {
+      a = P.a[pos];
+      b = P.b[pos];
+      c = P.c[pos];
+    }
+    bool plain = false;
+    if (in && r >= 0 && (code & kOn)) {
+      const float eu = etau_math(a, b, c, P.alpha1), iu = P.Iu[pos];
+      plain = !((eu == 0.0f || ranged(eu)) && ranged(etav1_math(b, c, P.alpha0, P.alpha1)) && ranged(etav2_math(a, c, P.alpha0, P.alpha1)) &&
+                (iu == 0.0f || ranged(iu)));
+    }
+    if (MASKED && in && !(code & kOn)) {
+      // read by the right / lower neighbour only where that one's other side is off too
+      const float2 tp = P.Tp[pos];
+      a = (east & kOn) && !(east & kR) ? tp.x : 0.f;
+      b = (south & kOn) && !(south & kD) ? tp.y : 0.f;
+    }
+    if (r < 0) {
+      sh.top[lane] = make_float4(a, b, c, 0.f);
+      return plain;
+    }
+    const int i = r >> 1, k = r & 1;
+    el(sh.ab[i][lane], k) = a;
+    el(sh.ab[i][lane], 2 + k) = b;
+    el(sh.ci[i][lane], k) = c;
+    el(sh.ci[i][lane], 2 + k) = in ? P.Iu[pos] : 0.f;
+    reinterpret_cast<float*>(&sh.iz[i][lane])[k] = in ? P.Iz[pos] : 0.f;
+    float un = in ? P.u[pos] : 0.f, ubn = in ? P.u_[pos] : 0.f;
+    if (MASKED && in && !(code & kOn)) {  // the other ping-pong values of a masked-out pixel
+      un = P.u_s[pos];
+      const float2 o = ((const float2*)P.v_s)[pos];
+      el(sh.p[i][lane], k) = o.x;
+      el(sh.p[i][lane], 2 + k) = o.y;
+    }
+    u[i] = k ? x2::pk(lo(u[i]), un) : x2::pk(un, 0.f);
+    ub[i] = k ? x2::pk(lo(ub[i]), ubn) : x2::pk(ubn, 0.f);
+    vx[i] = vy[i] = x2::pk(0.f, 0.f);
+    return plain;
+  }
+  static __device__ __forceinline__ float of(f2 v, int r) { return r & 1 ? hi(v) : lo(v); }
+  __device__ __forceinline__ float u_of(int r) const { return of(u[r >> 1], r); }
+  __device__ __forceinline__ float ub_of(int r) const { return of(ub[r >> 1], r); }
+  __device__ __forceinline__ float2 v_of(int r) const { return make_float2(of(vx[r >> 1], r), of(vy[r >> 1], r)); }
+  __device__ __forceinline__ uint4 word(int r, unsigned tag) const {
+    const float2 v = v_of(r);
+    return make_uint4(__float_as_uint(ub_of(r)), __float_as_uint(v.x), __float_as_uint(v.y), tag);
+  }
+  static __device__ __forceinline__ void put_col(Sh& sh, int side, int r, uint4 w) { sh.col[side][r] = w; }
+  __device__ __forceinline__ void take_col(Sh& sh, int side) {
+#pragma unroll
+    for (int i = 0; i < R / 2; i++) {
+      const uint4 w0 = sh.col[side][2 * i], w1 = sh.col[side][2 * i + 1];
+      ub[i] = x2::pk(__uint_as_float(w0.x), __uint_as_float(w1.x));
+      vx[i] = x2::pk(__uint_as_float(w0.y), __uint_as_float(w1.y));
+      vy[i] = x2::pk(__uint_as_float(w0.z), __uint_as_float(w1.z));
+    }
+  }
+  __device__ __forceinline__ void store_pq(const Sh& sh, int lane, int r, void* po, void* qo, int pos) const {
+    const int i = r >> 1, k = r & 1;
+    ((float2*)po)[pos] = make_float2(el(sh.p[i][lane], k), el(sh.p[i][lane], 2 + k));
+    ((float4*)qo)[pos] = make_float4(el(sh.qxy[i][lane], k), el(sh.qxy[i][lane], 2 + k), el(sh.qzw[i][lane], k),
+                                     el(sh.qzw[i][lane], 2 + k));
+  }
+
+  // p and q projected: |.| is divided out where it is above 1
+  template <bool PLAIN>
+  static __device__ __forceinline__ void project(f2 n2, f2& a, f2& b) {
+    using namespace x2;
+    if (PLAIN) {
+      const float r0 = sqrtf(lo(n2)), r1 = sqrtf(hi(n2));
+      const bool k0 = r0 <= 1.0f, k1 = r1 <= 1.0f;
+      a = pk(k0 ? lo(a) : lo(a) / r0, k1 ? hi(a) : hi(a) / r1);
+      b = pk(k0 ? lo(b) : lo(b) / r0, k1 ? hi(b) : hi(b) / r1);
+    } else {
+      f2 s, y;
+      exact::root(pk(max1(lo(n2)), max1(hi(n2))), s, y);
+      a = exact::quot(a, s, y);
+      b = exact::quot(b, s, y);
+    }
+  }
+  // max(v, 1); a NaN stays
+  static __device__ __forceinline__ float max1(float v) {
+    float r;
+    asm("max.NaN.f32 %0, %1, 0f3F800000;" : "=f"(r) : "f"(v));
+    return r;
+  }
+  template <bool PLAIN>
+  static __device__ __forceinline__ void project4(f2 m2, f2& x, f2& y_, f2& z, f2& w) {
+    using namespace x2;
+    if (PLAIN) {
+      f2 a = x, b = y_;
+      project<true>(m2, a, b);
+      x = a;
+      y_ = b;
+      a = z;
+      b = w;
+      project<true>(m2, a, b);
+      z = a;
+      w = b;
+    } else {
+      f2 s, y;
+      exact::root(pk(max1(lo(m2)), max1(hi(m2))), s, y);
+      x = exact::quot(x, s, y);
+      y_ = exact::quot(y_, s, y);
+      z = exact::quot(z, s, y);
+      w = exact::quot(w, s, y);
+    }
+  }
+  // tau / eta; eta = 0 takes tau itself
+  template <bool PLAIN>
+  static __device__ __forceinline__ f2 step_of(f2 tau, f2 eta) {
+    if (PLAIN)
+      return x2::pk(lo(eta) == 0.0f ? lo(tau) : lo(tau) / lo(eta), hi(eta) == 0.0f ? hi(tau) : hi(tau) / hi(eta));
+    return exact::quot(tau, eta, exact::recip(eta));
+  }
+
+  template <int KIND>
+  __device__ __forceinline__ void iterate(Sh& sh, const ResArgs& A, int lane, const ResStep& S, const ResEdge& E,
+                                          uint4 wn, uint4 ws, float2* tp_out, int s, unsigned tp_rows) {
+    using namespace x2;
+    constexpr bool PLAIN = KIND == kResPlain;
+    constexpr bool EDGE = KIND != kResInner;
+    constexpr bool KEEP = MASKED && (KIND == kResKeep || PLAIN);
+    const f2 sp = pk(S.sp.x, S.sp.y), sq = pk(S.sq.x, S.sq.y), tau = pk(S.tau.x, S.tau.y), mu = pk(S.mu.x, S.mu.y);
+    const f2 lam = both(A.P.lambda), al0 = both(A.P.alpha0), al1 = both(A.P.alpha1);
+    const f2 a1s = both(A.P.alpha1 * A.P.alpha1), a0s4 = both(4 * A.P.alpha0 * A.P.alpha0);
+    // A product that is added to something else.  ptxas contracts mul.rn.f32x2 and add.rn.f32x2 into
+    // one fma (CUDA 12.9, -fmad=false notwithstanding); a fused multiply-add of -0, which it
+    // cannot see, rounds the product alone.
+    const f2 nz = pk(A.minus_zero.x, A.minus_zero.y);
+    auto prod = [nz](f2 x, f2 y) { return fma(x, y, nz); };
+    auto bit = [](unsigned m, int r) { return (m >> (r + 1)) & 1u; };
+    auto pair = [](const float4& v) { return *reinterpret_cast<const ulonglong2*>(&v); };
+    float tpy_n, qz_n, qy_n, du_n;
+    float2 dv_n;
+    {
+      const float4 ca = sh.top[lane];
+      const float ubc = __uint_as_float(wn.x);
+      const float2 vp = make_float2(__uint_as_float(wn.y), __uint_as_float(wn.z));
+      float dux = __shfl_down_sync(kFull, ubc, 1) - ubc;
+      float2 dvx = make_float2(__shfl_down_sync(kFull, vp.x, 1) - vp.x, __shfl_down_sync(kFull, vp.y, 1) - vp.y);
+      du_n = lo(ub[0]) - ubc;
+      dv_n = make_float2(lo(vx[0]) - vp.x, lo(vy[0]) - vp.y);
+      if (EDGE) {
+        const float wu = __shfl_up_sync(kFull, dux, 1);
+        const float2 wv = make_float2(__shfl_up_sync(kFull, dvx.x, 1), __shfl_up_sync(kFull, dvx.y, 1));
+        const bool r0 = bit(E.x, -1);
+        dux = r0 ? dux : wu;
+        dvx = make_float2(r0 ? dvx.x : wv.x, r0 ? dvx.y : wv.y);
+      }
+      const float gx = dux - vp.x, gy = du_n - vp.y;
+      float2 p = sh.ptop[lane];
+      float4 q = sh.qtop[lane];
+      const float dtx = ca.x * gx + ca.z * gy, dty = ca.z * gx + ca.y * gy;
+      // both p lanes and the norms of p and q side by side
+      f2 pp = pk(p.x + S.sp.x * dtx, p.y + S.sp.x * dty);
+      f2 qa = pk(q.x + S.sq.x * dvx.x, q.y + S.sq.x * dv_n.y), qb = pk(q.z + S.sq.x * dv_n.x, q.w + S.sq.x * dvx.y);
+      const f2 p2 = prod(pp, pp), qa2 = prod(qa, qa), qb2 = prod(qb, qb);
+      const float n2 = lo(p2) + hi(p2), m2 = lo(qa2) + hi(qa2) + lo(qb2) + hi(qb2);
+      if (PLAIN) {
+        const float rp = sqrtf(n2), rq = sqrtf(m2);
+        if (!(rp <= 1.0f)) pp = pk(lo(pp) / rp, hi(pp) / rp);
+        if (!(rq <= 1.0f)) {
+          qa = pk(lo(qa) / rq, hi(qa) / rq);
+          qb = pk(lo(qb) / rq, hi(qb) / rq);
+        }
+      } else {
+        f2 sr, y;
+        exact::root(pk(max1(n2), max1(m2)), sr, y);
+        pp = exact::quot(pp, both(lo(sr)), both(lo(y)));
+        qa = exact::quot(qa, both(hi(sr)), both(hi(y)));
+        qb = exact::quot(qb, both(hi(sr)), both(hi(y)));
+      }
+      p = upk(pp);
+      sh.ptop[lane] = p;
+      sh.qtop[lane] = make_float4(lo(qa), hi(qa), lo(qb), hi(qb));
+      tpy_n = ca.z * p.x + ca.y * p.y;
+      qz_n = lo(qb);
+      qy_n = hi(qa);
+      if (EDGE) {
+        const bool d0 = bit(E.y, -1);
+        const bool o0 = MASKED ? d0 : bit(E.on, -1);
+        tpy_n = o0 ? tpy_n : KEEP && !bit(E.on, -1) ? ca.y : -0.0f;
+        qz_n = d0 ? qz_n : 0.f;
+        qy_n = d0 ? qy_n : 0.f;
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < R / 2; i++) {
+      const int r = 2 * i;
+      const int in_ = i + 1 < R / 2 ? i + 1 : 0;
+      const f2 UB = ub[i], VX = vx[i], VY = vy[i];
+      const float ub0 = lo(UB), ub1 = hi(UB);
+      const float ubd = i + 1 < R / 2 ? lo(ub[in_]) : __uint_as_float(ws.x);
+      const float vxd = i + 1 < R / 2 ? lo(vx[in_]) : __uint_as_float(ws.y);
+      const float vyd = i + 1 < R / 2 ? lo(vy[in_]) : __uint_as_float(ws.z);
+      const ulonglong2 ab = pair(sh.ab[i][lane]), ci = pair(sh.ci[i][lane]);
+      // ---- differences of u-bar and v-bar to the east and to the south -----------------
+      f2 dux = sub(pk(__shfl_down_sync(kFull, ub0, 1), __shfl_down_sync(kFull, ub1, 1)), UB);
+      f2 dxx = sub(pk(__shfl_down_sync(kFull, lo(VX), 1), __shfl_down_sync(kFull, hi(VX), 1)), VX);
+      f2 dxy = sub(pk(__shfl_down_sync(kFull, lo(VY), 1), __shfl_down_sync(kFull, hi(VY), 1)), VY);
+      const float du0 = ub1 - ub0, du1 = ubd - ub1;
+      const float2 dv0 = make_float2(hi(VX) - lo(VX), hi(VY) - lo(VY)), dv1 = make_float2(vxd - hi(VX), vyd - hi(VY));
+      f2 duy = pk(du0, du1), dyx = pk(dv0.x, dv1.x), dyy = pk(dv0.y, dv1.y);
+      bool r0 = true, r1 = true, d0 = true, d1 = true;
+      if (EDGE) {
+        r0 = bit(E.x, r);
+        r1 = bit(E.x, r + 1);
+        d0 = bit(E.y, r);
+        d1 = bit(E.y, r + 1);
+        const float wu0 = __shfl_up_sync(kFull, lo(dux), 1), wu1 = __shfl_up_sync(kFull, hi(dux), 1);
+        const float wx0 = __shfl_up_sync(kFull, lo(dxx), 1), wx1 = __shfl_up_sync(kFull, hi(dxx), 1);
+        const float wy0 = __shfl_up_sync(kFull, lo(dxy), 1), wy1 = __shfl_up_sync(kFull, hi(dxy), 1);
+        dux = pk(r0 ? lo(dux) : wu0, r1 ? hi(dux) : wu1);
+        dxx = pk(r0 ? lo(dxx) : wx0, r1 ? hi(dxx) : wx1);
+        dxy = pk(r0 ? lo(dxy) : wy0, r1 ? hi(dxy) : wy1);
+        duy = pk(d0 ? du0 : du_n, d1 ? du1 : du0);
+        dyx = pk(d0 ? dv0.x : dv_n.x, d1 ? dv1.x : dv0.x);
+        dyy = pk(d0 ? dv0.y : dv_n.y, d1 ? dv1.y : dv0.y);
+        du_n = du1;
+        dv_n = dv1;
+      }
+      // ---- dual step ------------------------------------------------------------------
+      const f2 a = ab.x, b = ab.y, c = ci.x, iu = ci.y;
+      const f2 ux = sub(dux, VX), uy = sub(duy, VY);
+      const ulonglong2 p0 = pair(sh.p[i][lane]), qa = pair(sh.qxy[i][lane]), qb = pair(sh.qzw[i][lane]);
+      f2 px = add(p0.x, prod(sp, add(prod(a, ux), prod(c, uy))));
+      f2 py = add(p0.y, prod(sp, add(prod(c, ux), prod(b, uy))));
+      project<PLAIN>(add(prod(px, px), prod(py, py)), px, py);
+      f2 qx = add(qa.x, prod(sq, dxx));
+      f2 qy = add(qa.y, prod(sq, dyy));
+      f2 qz = add(qb.x, prod(sq, dyx));
+      f2 qw = add(qb.y, prod(sq, dxy));
+      project4<PLAIN>(add(add(add(prod(qx, qx), prod(qy, qy)), prod(qz, qz)), prod(qw, qw)), qx, qy, qz, qw);
+      const f2 tpx = add(prod(a, px), prod(c, py)), tpy = add(prod(c, px), prod(b, py));
+      f2 pnx = px, pny = py;
+      *reinterpret_cast<ulonglong2*>(&sh.qxy[i][lane]) = make_ulonglong2(qx, qy);
+      *reinterpret_cast<ulonglong2*>(&sh.qzw[i][lane]) = make_ulonglong2(qz, qw);
+      if (!MASKED && EDGE) {  // outside the circle p = 0: T p = T 0
+        const float2 z = make_float2(0.f, 0.f);
+        if ((tp_rows >> r) & 1u) tp_out[r * s] = bit(E.on, r) ? make_float2(lo(tpx), lo(tpy)) : tp_math(lo(a), lo(b), lo(c), z);
+        if ((tp_rows >> (r + 1)) & 1u)
+          tp_out[(r + 1) * s] = bit(E.on, r + 1) ? make_float2(hi(tpx), hi(tpy)) : tp_math(hi(a), hi(b), hi(c), z);
+      } else {
+        if ((tp_rows >> r) & 1u) tp_out[r * s] = make_float2(lo(tpx), lo(tpy));
+        if ((tp_rows >> (r + 1)) & 1u) tp_out[(r + 1) * s] = make_float2(hi(tpx), hi(tpy));
+      }
+      // ---- threshold step -----------------------------------------------------------
+      f2 txo = tpx, tyo = tpy;  // as counted for this pixel and its right / lower neighbour
+      bool o0 = true, o1 = true;
+      if (EDGE) {
+        if (KEEP || !MASKED) {
+          o0 = bit(E.on, r);
+          o1 = bit(E.on, r + 1);
+        }
+        const float zx0 = KEEP && !o0 ? lo(a) : -0.0f, zx1 = KEEP && !o1 ? hi(a) : -0.0f;
+        const float zy0 = KEEP && !o0 ? lo(b) : -0.0f, zy1 = KEEP && !o1 ? hi(b) : -0.0f;
+        // the plain form takes the difference at the last row and column too
+        txo = pk((MASKED ? r0 : o0) ? lo(tpx) : zx0, (MASKED ? r1 : o1) ? hi(tpx) : zx1);
+        tyo = pk((MASKED ? d0 : o0) ? lo(tpy) : zy0, (MASKED ? d1 : o1) ? hi(tpy) : zy1);
+        qx = pk(r0 ? lo(qx) : 0.f, r1 ? hi(qx) : 0.f);
+        qw = pk(r0 ? lo(qw) : 0.f, r1 ? hi(qw) : 0.f);
+        qz = pk(d0 ? lo(qz) : 0.f, d1 ? hi(qz) : 0.f);
+        qy = pk(d0 ? lo(qy) : 0.f, d1 ? hi(qy) : 0.f);
+      }
+      const f2 tpw = pk(__shfl_up_sync(kFull, lo(txo), 1), __shfl_up_sync(kFull, hi(txo), 1));
+      const f2 qxw = pk(__shfl_up_sync(kFull, lo(qx), 1), __shfl_up_sync(kFull, hi(qx), 1));
+      const f2 qww = pk(__shfl_up_sync(kFull, lo(qw), 1), __shfl_up_sync(kFull, hi(qw), 1));
+      const f2 dy = pk(lo(tyo) - tpy_n, hi(tyo) - lo(tyo));
+      const f2 dqz = pk(lo(qz) - qz_n, hi(qz) - lo(qz)), dqy = pk(lo(qy) - qy_n, hi(qy) - lo(qy));
+      const f2 aa = prod(a, a), bb = prod(b, b), cc = prod(c, c), ac = add(a, c), bc = add(b, c);
+      const f2 eu = prod(add(add(add(add(aa, bb), add(cc, cc)), prod(ac, ac)), prod(bc, bc)), a1s);
+      // (the reference leaves the tensor zero beyond its launch grid: eta_u = 0 there, tau / 1 = tau)
+      const f2 te = step_of<PLAIN>(tau, PLAIN ? eu : pk(lo(eu) == 0.0f ? 1.0f : lo(eu), hi(eu) == 0.0f ? 1.0f : hi(eu)));
+      const f2 U = u[i];
+      const f2 dun = sub(add(UB, prod(te, add(sub(txo, tpw), dy))), U);
+      const f2 rho = add(prod(iu, dun), *reinterpret_cast<const f2*>(&sh.iz[i][lane]));
+      const f2 lt = prod(lam, te);
+      const f2 up = prod(lt, prod(iu, iu)), far = prod(lt, iu);
+      f2 newton;
+      if (PLAIN) newton = pk(lo(rho) / lo(iu), hi(rho) / hi(iu));
+      else newton = exact::quot(rho, iu, exact::recip(iu));
+      f2 un;
+      {
+        // |rho| <= upper: the Newton step (none where Iu = 0); beyond it a step of lambda tau Iu / eta_u
+        // against the sign of rho (lambda >= 0); a NaN residual leaves u
+        float t[2];
+        bool num[2];
+#pragma unroll
+        for (int k = 0; k < 2; k++) {
+          const float rh = k ? hi(rho) : lo(rho), upk_ = k ? hi(up) : lo(up);
+          const bool in = fabsf(rh) <= upk_;
+          num[k] = in || fabsf(rh) > upk_;
+          const float away = __uint_as_float(__float_as_uint(k ? hi(far) : lo(far)) ^ (__float_as_uint(rh) & 0x80000000u));
+          const float nk = (k ? hi(iu) : lo(iu)) == 0.0f ? 0.0f : k ? hi(newton) : lo(newton);
+          t[k] = in ? nk : away;
+        }
+        const f2 d = sub(dun, pk(t[0], t[1]));
+        un = add(U, pk(num[0] ? lo(d) : 0.0f, num[1] ? hi(d) : 0.0f));
+      }
+      // ---- primal step --------------------------------------------------------------
+      const f2 e1 = add(prod(a1s, add(bb, cc)), a0s4), e2 = add(prod(a1s, add(aa, cc)), a0s4);
+      const f2 gx = add(prod(al1, tpx), prod(al0, add(sub(qx, qxw), dqz)));
+      const f2 gy = add(prod(al1, tpy), prod(al0, add(sub(qw, qww), dqy)));
+      f2 t1 = step_of<PLAIN>(tau, e1);
+      if (PLAIN)  // eta_v2 = 0: updatePrimalVariables.cu:103-105 writes .x again, .y keeps its value
+        t1 = pk(lo(e2) == 0.0f ? lo(tau) : lo(t1), hi(e2) == 0.0f ? hi(tau) : hi(t1));
+      const f2 wx = add(VX, prod(t1, gx));
+      f2 wy = add(VY, prod(step_of<PLAIN>(tau, e2), gy));
+      if (PLAIN) wy = pk(lo(e2) == 0.0f ? lo(VY) : lo(wy), hi(e2) == 0.0f ? hi(VY) : hi(wy));
+      f2 us = add(un, prod(mu, sub(un, UB)));
+      f2 vsx = add(wx, prod(mu, sub(wx, VX))), vsy = add(wy, prod(mu, sub(wy, VY)));
+      if (KEEP) {  // unwritten pixels alternate between the two ping-pong buffers' values
+        un = pk(o0 ? lo(un) : ub0, o1 ? hi(un) : ub1);
+        us = pk(o0 ? lo(us) : lo(U), o1 ? hi(us) : hi(U));
+        vsx = pk(o0 ? lo(vsx) : lo(p0.x), o1 ? hi(vsx) : hi(p0.x));
+        vsy = pk(o0 ? lo(vsy) : lo(p0.y), o1 ? hi(vsy) : hi(p0.y));
+        pnx = pk(o0 ? lo(px) : lo(VX), o1 ? hi(px) : hi(VX));
+        pny = pk(o0 ? lo(py) : lo(VY), o1 ? hi(py) : hi(VY));
+      } else if (EDGE && !MASKED) {  // outside the circle
+        un = pk(o0 ? lo(un) : 0.f, o1 ? hi(un) : 0.f);
+        us = pk(o0 ? lo(us) : 0.f, o1 ? hi(us) : 0.f);
+        vsx = pk(o0 ? lo(vsx) : 0.f, o1 ? hi(vsx) : 0.f);
+        vsy = pk(o0 ? lo(vsy) : 0.f, o1 ? hi(vsy) : 0.f);
+      }
+      *reinterpret_cast<ulonglong2*>(&sh.p[i][lane]) = make_ulonglong2(pnx, pny);
+      u[i] = un;
+      ub[i] = us;
+      vx[i] = vsx;
+      vy[i] = vsy;
+      tpy_n = hi(tyo);
+      qz_n = hi(qz);
+      qy_n = hi(qy);
+    }
+  }
+};
+
+// Publishes a tile's border u-bar and v-bar as tag `tag` to its words `out`.
+template <int R, class State>
+__device__ __forceinline__ void publish(const State& st, uint4* out, int lane, unsigned tag) {
+  if (lane >= 1 && lane <= kResCols) {
+    st_word(out + lane, st.word(0, tag));
+    st_word(out + 32 + lane, st.word(R - 1, tag));
+  }
+  if (lane == 1 || lane == kResCols) {
+    uint4* c = out + 64 + (lane == 1 ? 0 : R);
+#pragma unroll
+    for (int r = 0; r < R; r++) st_word(c + r, st.word(r, tag));
+  }
+}
+
+}  // namespace
+
+// One warp's tile.
+template <bool MASKED, class ST, int R>
+struct ResWarp {
+  typedef ResShared<ST, R> Sh;
+  typedef typename Store2<ST>::T2 T2;
+  typedef typename Store2<ST>::T4 T4;
+  static constexpr int kSlots = 64 + 2 * R;
+  static constexpr bool kPlain = std::is_same<ST, float>::value;
+  ResState<MASKED, ST, R> s;
+
+  // Loads tile t: its coefficients, codes and state before the first iteration.
+  __device__ __forceinline__ void load(Sh& sh, const ResArgs& A, int lane, int t) {
+    const IterPair& P = A.P;
+    const ResTile& T = A.tiles[t];
+    const int x = T.x0 - 1 + lane, y0 = T.y0;
+    const bool x_in = x >= 0 && x < P.w;
+    ResEdge e{0u, 0u, 0u};
+    bool plain = false;
+    s.clear(sh, lane);
+#pragma unroll
+    for (int r = -1; r < R; r++) {
+      const int y = y0 + r, pos = x + y * P.s;
+      const bool in = x_in && y >= 0 && y < P.h;
+      unsigned code = 0, east = 0, south = 0;
+      if (in) {
+        code = P.code[pos];
+        if (!MASKED) {
+          code &= kOn;
+          code |= (x + 1 < P.w ? kR : 0) | (x >= 1 ? kL : 0) | (y + 1 < P.h ? kD : 0) | (y >= 1 ? kU : 0);
+        } else if (!(code & kOn)) {
+          if (code & kR) east = P.code[pos + 1];
+          if (code & kD) south = P.code[pos + P.s];
+        }
+      }
+      plain = s.set_row(sh, lane, P, r, in, pos, code, east, south) || plain;
+      const unsigned b = 1u << (r + 1);
+      if (code & kOn) {
+        e.on |= b;
+        if (code & kR) e.x |= b;
+        if (code & kD) e.y |= b;
+      }
+    }
+    // exchange words; a missing neighbour is replaced by this tile itself: the tags come, the
+    // values are not used.  Lanes 0 .. R-1 fetch the west column, lanes 16 .. 16 + R-1 the east one.
+    const int tn = lane == 0 ? T.nb[4] : lane == 31 ? T.nb[5] : T.nb[0];
+    const int ts = lane == 0 ? T.nb[6] : lane == 31 ? T.nb[7] : T.nb[1];
+    const int col = lane == 0 ? kResCols : lane == 31 ? 1 : lane;
+    const int side = lane >> 4, row = lane & 15;
+    sh.k.at[lane] = make_uint4((unsigned)(tn * kSlots + 32 + col), (unsigned)(ts * kSlots + col),
+                               (unsigned)(T.nb[side ? 3 : 2] * kSlots + 64 + (side ? 0 : R) + (row < R ? row : 0)), e.x);
+    sh.k.edge[lane] = make_uint2(e.y, e.on);
+    plain = __any_sync(kFull, plain);
+    if (lane == 0) {
+      sh.k.kind = plain ? kResPlain : T.kind;
+      sh.k.t = t;
+    }
+    __syncwarp();
+  }
+
+  // One iteration.  Returns false once a wait ran out.
+  __device__ __forceinline__ bool step(Sh& sh, const ResArgs& A, int lane, int j,
+                                       unsigned epoch, bool waiting) {
+    const IterPair& P = A.P;
+    const uint4 o = sh.k.at[lane];
+    const unsigned ring = (unsigned)A.ntiles * kSlots;
+    const uint4* const base = A.exch + (size_t)(j & (kResRing - 1)) * ring;
+    const unsigned tag = epoch | (unsigned)j;
+    uint4 wn, ws, wc;
+    for (int polls = 0;; polls++) {
+      wn = ld_word(base + o.x);
+      ws = ld_word(base + o.y);
+      wc = ld_word(base + o.z);
+      if (__all_sync(kFull, wn.w == tag && ws.w == tag && wc.w == tag) || !waiting) break;
+      if (polls >= kResMaxPolls) {
+        waiting = false;
+        if (lane == 0) g_res_status = 1;
+        break;
+      }
+    }
+    const int side = lane >> 4, row = lane & 15;
+    if (row < R) s.put_col(sh, side, row, wc);
+    __syncwarp();
+    if (lane == 0 || lane == 31) s.take_col(sh, side);
+    __syncwarp();
+    const bool last = j + 1 == A.n;
+    const uint2 ek = sh.k.edge[lane];
+    const ResEdge E{o.w, ek.x, ek.y};
+    const int kind = sh.k.kind;
+    float2* tp_out = nullptr;
+    unsigned tp_rows = 0u;
+    if (last) {
+      int pos0;
+      tp_rows = owned(sh, A, lane, pos0);
+      tp_out = P.Tp + pos0;
+    }
+    if (kind == kResInner) s.template iterate<kResInner>(sh, A, lane, A.step[j], E, wn, ws, tp_out, P.s, tp_rows);
+    else if (kind == kResEdge) s.template iterate<kResEdge>(sh, A, lane, A.step[j], E, wn, ws, tp_out, P.s, tp_rows);
+    else if (kPlain && kind == kResPlain)
+      s.template iterate<kPlain ? kResPlain : kResEdge>(sh, A, lane, A.step[j], E, wn, ws, tp_out, P.s, tp_rows);
+    else if constexpr (MASKED) s.template iterate<kResKeep>(sh, A, lane, A.step[j], E, wn, ws, tp_out, P.s, tp_rows);
+    if (!last)
+      publish<R>(s, A.exch + (size_t)((j + 1) & (kResRing - 1)) * ring + (unsigned)(sh.k.t * kSlots), lane, tag + 1);
+    return waiting;
+  }
+
+  // The rows of this lane's column that the tile owns and the iterations write (bit r), and the
+  // flat position of row 0.
+  __device__ __forceinline__ unsigned owned(const Sh& sh, const ResArgs& A, int lane, int& pos0) const {
+    const ResTile& T = A.tiles[sh.k.t];
+    const int x = T.x0 - 1 + lane;
+    pos0 = x + T.y0 * A.P.s;
+    const int rows = lane >= 1 && lane <= kResCols && x < A.P.w ? min(R, A.P.h - T.y0) : 0;
+    const unsigned in = (1u << rows) - 1u;
+    return MASKED ? in & (sh.k.edge[lane].y >> 1) : in;
+  }
+
+  // Writes the tile's u, u-bar and v-bar: the state current after n iterations (fin), or the one
+  // before the last iteration into the other ping-pong buffers.
+  __device__ __forceinline__ void store(const Sh& sh, const ResArgs& A, int lane,
+                                        bool fin) {
+    const IterPair& P = A.P;
+    const bool first = (A.n & 1) ^ (fin ? 1 : 0);  // into the launch's input buffers
+    float* uo = first ? const_cast<float*>(P.u) : P.us;
+    float* ubo = first ? const_cast<float*>(P.u_) : P.u_s;
+    T2* vo = (T2*)(first ? const_cast<void*>(P.v_) : P.v_s);
+    int pos0;
+    const unsigned own = owned(sh, A, lane, pos0);
+#pragma unroll
+    for (int r = 0; r < R; r++) {
+      if (!((own >> r) & 1u)) continue;
+      const int pos = pos0 + r * P.s;
+      uo[pos] = s.u_of(r);
+      ubo[pos] = s.ub_of(r);
+      vo[pos] = s.v_of(r);
+    }
+    if (fin) {
+      const int plane = A.p_planes ? (A.n & 1) * P.s * P.h : 0;
+      const unsigned on = own & (sh.k.edge[lane].y >> 1);
+#pragma unroll
+      for (int r = 0; r < R; r++)
+        if ((on >> r) & 1u) s.store_pq(sh, lane, r, (T2*)P.p + plane, (T4*)P.q + plane, pos0 + r * P.s);
+    }
+  }
+};
+
+// Warps per block (one block per SM): what the registers of R rows leave.
+template <class ST>
+constexpr int res_warps(int rows) {
+  return rows <= 8 ? 16 : 12;
+}
+
+template <bool MASKED, class ST, int R>
+__global__ void __launch_bounds__(32 * res_warps<ST>(R), 1) k_resident(const __grid_constant__ ResArgs A) {
+  typedef typename Store2<ST>::T2 T2;
+  extern __shared__ __align__(16) unsigned char smem[];
+  const IterPair& P = A.P;
+  const int warp = (int)threadIdx.x >> 5, lane = (int)threadIdx.x & 31;
+  ResShared<ST, R>& sh = reinterpret_cast<ResShared<ST, R>*>(smem)[warp];
+  // Tiles go round the blocks first, then the warps of a block: every SM, and every scheduler of an
+  // SM, has the same number of tiles but for one.
+  const int t = (int)blockIdx.x + (int)gridDim.x * warp;
+  const unsigned epoch = (*(volatile unsigned*)&A.ctl->epoch + 1u) << 8;
+
+  if (t < A.ntiles) {
+    ResWarp<MASKED, ST, R> W;
+    W.load(sh, A, lane, t);
+    publish<R>(W.s, A.exch + (size_t)t * (64 + 2 * R), lane, epoch);  // iteration 0's input
+    __syncwarp();
+    bool waiting = true;
+#pragma unroll 1
+    for (int j = 0; j < A.n; j++) {
+      waiting = W.step(sh, A, lane, j, epoch, waiting);
+      if (j + 2 >= A.n) W.store(sh, A, lane, j + 1 == A.n);
+    }
+  }
+  // ---- plain form: pixels outside the circle in tiles without a pixel to solve --------------
+  if (!MASKED) {
+    const int warps = (int)blockDim.x >> 5, nw = (int)gridDim.x * warps;
+    const float2 z = make_float2(0.f, 0.f);
+    for (int k = (int)blockIdx.x * warps + warp; k < A.nfill; k += nw) {
+      const int2 f = A.fill[k];
+      const int x = f.x - 1 + lane;
+      if (lane < 1 || lane > kResCols || x >= P.w) continue;
+      for (int y = f.y; y < min(f.y + R, P.h); y++) {
+        const int pos = x + y * P.s;
+        // the buffers current after n iterations and, from two iterations on, the others
+        if ((A.n & 1) == 0 || A.n >= 2) {
+          const_cast<float*>(P.u)[pos] = 0.f;
+          const_cast<float*>(P.u_)[pos] = 0.f;
+          Store2<ST>::st2((T2*)const_cast<void*>(P.v_), pos, z);
+        }
+        P.us[pos] = 0.f;
+        P.u_s[pos] = 0.f;
+        Store2<ST>::st2((T2*)P.v_s, pos, z);
+        P.Tp[pos] = tp_math(P.a[pos], P.b[pos], P.c[pos], z);
+      }
+    }
+  }
+  // ---- the last block to end renews the epoch: every block has read it by then --------------
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    if (atomicAdd(&A.ctl->done, 1u) == gridDim.x - 1) {
+      A.ctl->done = 0;
+      A.ctl->epoch += 1;
+    }
+  }
+}
+
+namespace {
+
+template <bool MASKED, class ST, int R>
+struct Res {
+  static constexpr int kThreads = 32 * res_warps<ST>(R);
+  static constexpr size_t kSmem = sizeof(ResShared<ST, R>) * res_warps<ST>(R);
+  // tiles that a grid of one block per SM holds, all of it resident
+  static int capacity() {
+    int dev = 0, sms = 0, per = 0, coop = 0, smem = 0;
+    VFS_CUDA(cudaGetDevice(&dev));
+    VFS_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    VFS_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
+    VFS_CUDA(cudaDeviceGetAttribute(&smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+    if (!coop || kSmem > (size_t)smem) return 0;
+    VFS_CUDA(cudaFuncSetAttribute(k_resident<MASKED, ST, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem));
+    VFS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_resident<MASKED, ST, R>, kThreads, kSmem));
+    return per >= 1 ? sms * res_warps<ST>(R) : 0;
+  }
+  static int launch(const ResArgs& A, cudaStream_t st) {
+    // only the warps that have a tile: blocks of other pairs' levels share the SM
+    const int warps = (A.ntiles + A.blocks - 1) / A.blocks;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(A.blocks);
+    cfg.blockDim = dim3(32 * warps);
+    cfg.dynamicSmemBytes = sizeof(ResShared<ST, R>) * warps;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeCooperative;
+    at[0].val.cooperative = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    VFS_CUDA(cudaLaunchKernelEx(&cfg, k_resident<MASKED, ST, R>, A));
+    return 0;
+  }
+};
+
+// f(Res<...>()) for the instance of `rows` rows (kResRows)
+template <bool MASKED, class ST, class F>
+int res_rows(int rows, F&& f) {
+  if (rows == 2) return f(Res<MASKED, ST, 2>());
+  if (rows == 4) return f(Res<MASKED, ST, 4>());
+  if (rows == 6) return f(Res<MASKED, ST, 6>());
+  if (rows == 8) return f(Res<MASKED, ST, 8>());
+  if constexpr (!std::is_same<ST, float>::value) {
+    if (rows == 12) return f(Res<MASKED, ST, 12>());
+  }
+  return 0;
+}
+template <class F>
+int res_dispatch(bool masked, bool half, int rows, F&& f) {
+  if (masked) return half ? res_rows<true, __half>(rows, f) : res_rows<true, float>(rows, f);
+  return half ? res_rows<false, __half>(rows, f) : res_rows<false, float>(rows, f);
+}
+
+}  // namespace
+
+int res_capacity(bool masked, bool half, int rows) {
+  int dev = 0;
+  VFS_CUDA(cudaGetDevice(&dev));
+  static std::mutex mu;
+  static std::map<std::tuple<int, bool, bool, int>, int> known;
+  std::lock_guard<std::mutex> lk(mu);
+  const auto key = std::make_tuple(dev, masked, half, rows);
+  auto it = known.find(key);
+  if (it != known.end()) return it->second;
+  return known[key] = res_dispatch(masked, half, rows, [](auto k) { return decltype(k)::capacity(); });
+}
+
+void launch_resident(const ResArgs& A, bool masked, bool half, cudaStream_t st) {
+  if (A.ntiles <= 0 || A.blocks <= 0 || A.n < 1 || A.n > kResMaxIters) throw ArgError{"resident iteration: bad launch"};
+  int dev = 0, sms = 0;
+  VFS_CUDA(cudaGetDevice(&dev));
+  VFS_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  const int per_sm = res_capacity(masked, half, A.rows) / sms;  // warps of a block
+  if (A.blocks > sms || A.ntiles > A.blocks * per_sm) throw ArgError{"resident iteration: more tiles than can be resident"};
+  res_dispatch(masked, half, A.rows, [&](auto k) { return decltype(k)::launch(A, st); });
+  VFS_LAUNCH_CHECK();
+}
+
+int resident_status_take() {
+  int v = 0;
+  VFS_CUDA(cudaMemcpyFromSymbol(&v, g_res_status, sizeof(v)));
+  if (v) {
+    const int z = 0;
+    VFS_CUDA(cudaMemcpyToSymbol(g_res_status, &z, sizeof(z)));
+  }
+  return v;
+}
+
+}  // namespace vfs

@@ -1,0 +1,136 @@
+// Register-resident form of the fused primal-dual iteration: all iterations of one warp of a
+// pyramid level in one cooperative launch, the level's state held in registers and shared
+// memory of the whole GPU (one pair per launch).
+//
+// A level is cut into tiles of 30 x R pixels, one warp each; only tiles that hold a pixel that
+// is on (or that such a pixel reads) exist.  Lane k of a warp is image column x0 - 1 + k: lanes
+// 1..30 own their column, lanes 0 and 31 hold the west and east halo.  A warp keeps u, u-bar,
+// v-bar, p and q of its rows in registers (float storage: p and q in shared memory) and the
+// level's coefficients in shared memory.  One iteration streams down the rows: the dual step of
+// row r needs u-bar and v-bar of row r + 1 (still the old values) and of the east lane; the
+// threshold and primal steps of row r need T p and q of the west lane and of row r - 1.  The
+// dual step of the west column and of the row above the tile is recomputed by the warp, so an
+// iteration needs one exchange: u-bar and v-bar of the pixels around the tile.
+//
+// Exchange.  Every tile publishes the u-bar and v-bar of its border pixels as 16-byte words
+// that carry a tag (launch epoch and iteration) beside the values, and reads the words of its
+// eight neighbours until their tags are the ones it waits for.  A word is written and read by
+// single 128-bit memory operations, so a reader that sees the tag has the values: no fence, no
+// barrier, no grid-wide synchronisation; one store and one load through L2 are the whole
+// latency.  Words live in a ring of two iterations: a tile that has the words of iteration k of
+// all its neighbours knows that each of them has finished k - 1, and so has read this tile's
+// words of k - 1, before it overwrites them with those of k + 1.
+//
+// The grid is launched cooperatively, so that all its blocks are resident and every wait ends;
+// a wait is bounded all the same (a warp that gives up records it, stops waiting and runs on).
+//
+// The arithmetic is that of k_fused_iter (tgv_pixel.cuh, tgv_pixel_fast.cuh) with the same
+// storage rounding, so the results are bit-identical to one launch per iteration, the values
+// that the other ping-pong buffers hold included (the state before the last iteration is
+// written there).
+//
+// What bounds it, on B200 (FP16 storage, 848 x 800, 2037 tiles of 8 rows, 4.2 us per iteration):
+// about half of an iteration is instruction issue (1060 instructions per tile, 3.4 warps per
+// scheduler, close to one per cycle), the rest the exchange: about 1500 cycles from a
+// store to the load that sees it, and the wait for the slowest neighbour.  One launch per iteration
+// (k_fused_iter) takes 8.0 us there alone, bound by its loads; float storage 7.9 against 10.3 us.
+// Small levels are all latency: 53 x 50 takes 1.33 us (one launch per iteration 3.2 us, the
+// cluster-resident form 1.54 us).
+#pragma once
+#include <vector>
+
+#include "common.cuh"
+#include "fused.cuh"
+
+namespace vfs {
+
+constexpr int kResCols = 30;       // owned columns per tile
+constexpr int kResRing = 2;        // iterations of exchange words kept
+constexpr int kResMaxIters = 128;  // iterations per launch
+// tile heights the kernel is built for (float storage: those up to 8)
+constexpr int kResRows[] = {2, 4, 6, 8, 12};
+constexpr int kResNumRows = 5;
+constexpr int kResMostTiles = 148 * 16;  // a bound on the tiles of a plan (one warp each)
+inline int res_slots(int rows) { return 64 + 2 * rows; }  // words per tile: top, bottom, left, right
+
+// What a tile's pixels ask of its iterations: none of the edge rules; the edge rules; or
+// also the values that masked-out pixels keep (an on pixel reads one of them: it has neither its
+// right nor its left, or neither its lower nor its upper, neighbour).
+// kResPlain (found by the kernel): as kResKeep, with the plain division and square root.
+enum ResKind { kResInner = 0, kResEdge = 1, kResKeep = 2, kResPlain = 3 };
+
+struct ResTile {
+  int x0, y0;   // first owned column and row
+  int nb[8];    // tile index of the N, S, W, E, NW, NE, SW, SE neighbour (own index: none)
+  int kind;     // ResKind
+  int pad;
+};
+
+struct ResCtl {   // per level plan, in device memory
+  unsigned epoch; // launches completed
+  unsigned done;  // blocks of the running launch that have ended
+};
+
+// One iteration's step sizes (evaluated on the host), each twice for the packed instructions.
+struct ResStep {
+  float2 sp, sq, tau, mu;
+};
+
+struct ResArgs {
+  IterPair P;            // pointers of the first iteration (u, u-bar current; v-bar, p, q are zero)
+  uint4* exch;           // [kResRing][ntiles][res_slots]
+  ResCtl* ctl;
+  const ResTile* tiles;
+  int ntiles;
+  const int2* fill;      // plain form: (x0, y0) of the tiles without a pixel to solve
+  int nfill;
+  int n;                 // iterations (1 .. kResMaxIters)
+  int p_planes;          // p and q have two planes (result in plane n & 1); else one
+  int rows, blocks;      // tile height, blocks of the grid
+  float2 minus_zero;     // -0, where the compiler does not see it
+  ResStep step[kResMaxIters];
+};
+
+// A level's tiles (host side).
+struct ResTiles {
+  int rows = 0, blocks = 0;
+  std::vector<ResTile> tiles;
+  std::vector<int2> fill;
+};
+// What the tiles of any height need of a w x h level with edge codes `code` (tight rows; masked form:
+// k_edge_codes of the mask, plain form: kOn inside the circle), found in one pass over it.
+struct ResLevel {
+  int w = 0, h = 0, tx = 0;
+  bool masked = false;
+  std::vector<uint8_t> need;          // per tile column and two rows: holds a pixel to solve
+  std::vector<uint8_t> inner, keep;   // per row and tile column (ResKind)
+  // False where the form does not apply: a masked-in pixel of column 0 (row 0) without its right
+  // (lower) neighbour reads outside the image, a one-pixel-wide or -high plain level has no
+  // neighbour to take, or no pixel is on.
+  bool scan(const uint8_t* code, int w, int h, bool masked);
+  int count(int rows) const;                   // tiles of `rows` rows
+  void tiles(int rows, ResTiles& out) const;
+};
+// Picks the tile height for the level among the instances whose grid can be resident;
+// false: no instance fits (or the form does not apply).
+bool res_choose(const uint8_t* code, int w, int h, bool masked, bool half, ResTiles& out);
+
+// Device bytes a level's plan takes at most.
+size_t res_bytes_bound(int w, int h);
+
+// A level's plan on the device.
+struct ResPlan {
+  int rows = 0, blocks = 0, ntiles = 0, nfill = 0;  // ntiles = 0: the level has no plan
+  const ResTile* tiles = nullptr;
+  const int2* fill = nullptr;
+  uint4* exch = nullptr;
+  ResCtl* ctl = nullptr;
+};
+
+// most tiles an instance holds with its whole grid resident (0: not available)
+int res_capacity(bool masked, bool half, int rows);
+void launch_resident(const ResArgs& A, bool masked, bool half, cudaStream_t st);
+// reads and clears the device status (1: a bounded wait ran out)
+int resident_status_take();
+
+}  // namespace vfs

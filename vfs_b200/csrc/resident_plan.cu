@@ -1,0 +1,159 @@
+// Host side of the register-resident iteration: the tiles of a level (resident.cuh).
+#include <algorithm>
+
+#include "resident.cuh"
+
+namespace vfs {
+
+bool ResLevel::scan(const uint8_t* code, int w_, int h_, bool masked_) {
+  w = w_;
+  h = h_;
+  masked = masked_;
+  tx = (w + kResCols - 1) / kResCols;
+  const int ty = (h + kResRows[0] - 1) / kResRows[0];
+  need.assign((size_t)tx * ty, 0);
+  inner.assign((size_t)tx * h, 0);
+  keep.assign((size_t)tx * h, 0);
+  if (w < 2 || h < 2) return false;
+  const uint8_t kAll = kOn | kR | kL | kD | kU;
+  // per pixel: 1 on, 2 interior, 4 takes part in a read of a masked-out pixel
+  std::vector<uint8_t> f(w);
+  bool any = false;
+  for (int y = 0; y < h; y++) {
+    const uint8_t* c = code + (size_t)y * w;
+    auto mark = [&](int x, int yy) { need[(size_t)(yy / kResRows[0]) * tx + x / kResCols] = 1; };
+    for (int x = 0; x < w; x++) {
+      const uint8_t k = c[x];
+      f[x] = 0;
+      if (!(k & kOn)) continue;
+      f[x] = 1;
+      if (masked) {
+        if (k == kAll) {
+          f[x] = 3;
+          continue;
+        }
+        // the neighbours an edge rule falls back to, which may be masked out
+        if (!(k & kR)) {
+          if (x == 0) return false;
+          mark(x - 1, y);
+        }
+        if (!(k & kD)) {
+          if (y == 0) return false;
+          mark(x, y - 1);
+        }
+        if (!(k & (kR | kL)) || !(k & (kD | kU))) f[x] = 5;
+      } else {
+        if (x >= 1 && y >= 1 && x + 1 < w && y + 1 < h) f[x] = 3;
+        // a pixel outside the circle that the first iteration reads
+        if (x + 1 < w && !(c[x + 1] & kOn)) mark(x + 1, y);
+        if (y + 1 < h && !(c[x + w] & kOn)) mark(x, y + 1);
+      }
+    }
+    for (int i = 0; i < tx; i++) {
+      const int x0 = i * kResCols, x1 = std::min(w, x0 + kResCols);
+      uint8_t all = 7, some = 0;
+      for (int x = x0; x < x1; x++) {
+        all &= f[x];
+        some |= f[x];
+      }
+      if (some & 1) {
+        any = true;
+        need[(size_t)(y / kResRows[0]) * tx + i] = 1;
+      }
+      inner[(size_t)y * tx + i] = x0 >= 1 && x0 + kResCols <= w && (all & 2) && (f[x0 - 1] & 2);
+      if (x0 >= 1) some |= f[x0 - 1];
+      if (x1 < w) some |= f[x1];
+      keep[(size_t)y * tx + i] = some & 4;
+    }
+  }
+  return any;
+}
+
+int ResLevel::count(int rows) const {
+  const int per = rows / kResRows[0], ty2 = (int)(need.size() / tx);
+  int n = 0;
+  for (int j = 0; j < ty2; j += per)
+    for (int i = 0; i < tx; i++) {
+      uint8_t v = 0;
+      for (int k = j; k < std::min(ty2, j + per); k++) v |= need[(size_t)k * tx + i];
+      n += v;
+    }
+  return n;
+}
+
+void ResLevel::tiles(int rows, ResTiles& out) const {
+  out.rows = rows;
+  out.tiles.clear();
+  out.fill.clear();
+  const int per = rows / kResRows[0], ty2 = (int)(need.size() / tx), ty = (h + rows - 1) / rows;
+  std::vector<int> id((size_t)tx * ty, -1);
+  for (int j = 0; j < ty; j++)
+    for (int i = 0; i < tx; i++) {
+      uint8_t v = 0;
+      for (int k = j * per; k < std::min(ty2, (j + 1) * per); k++) v |= need[(size_t)k * tx + i];
+      if (!v) {
+        if (!masked) out.fill.push_back(make_int2(i * kResCols, j * rows));
+        continue;
+      }
+      id[(size_t)j * tx + i] = (int)out.tiles.size();
+      ResTile t{};
+      t.x0 = i * kResCols;
+      t.y0 = j * rows;
+      out.tiles.push_back(t);
+    }
+  for (int j = 0; j < ty; j++)
+    for (int i = 0; i < tx; i++) {
+      const int k = id[(size_t)j * tx + i];
+      if (k < 0) continue;
+      ResTile& t = out.tiles[k];
+      auto at = [&](int a, int b) {
+        if (a < 0 || b < 0 || a >= tx || b >= ty) return k;
+        const int n = id[(size_t)b * tx + a];
+        return n < 0 ? k : n;
+      };
+      const int nb[8] = {at(i, j - 1),     at(i, j + 1),     at(i - 1, j),     at(i + 1, j),
+                         at(i - 1, j - 1), at(i + 1, j - 1), at(i - 1, j + 1), at(i + 1, j + 1)};
+      std::copy(nb, nb + 8, t.nb);
+      // interior: the owned pixels, the column west of them and the row above, whose steps the
+      // tile evaluates, are on with all four neighbours in the image (and, masked, on)
+      bool in = t.y0 >= 1 && t.y0 + rows <= h, kept = false;
+      for (int y = t.y0 - 1; in && y < t.y0 + rows; y++) in = inner[(size_t)y * tx + i];
+      for (int y = std::max(0, t.y0 - 1); !in && y <= std::min(h - 1, t.y0 + rows); y++) kept |= keep[(size_t)y * tx + i] != 0;
+      t.kind = in ? kResInner : kept ? kResKeep : kResEdge;
+    }
+}
+
+// The smallest tile height whose tiles fit, since more warps with less to do each hide more of one
+// another's latency and shorten an iteration (B200, us per iteration, FP16 / float storage: 848 x 800
+// disc 8 rows 4.2 / 7.9; 640 x 480 4 rows 2.45 / 3.5, 6 rows 2.75 / 3.9, 8 rows 3.1 / 5.3; 212 x 200
+// 2 rows 1.40 / 1.73, 4 rows 1.60 / 2.15).  Two rows are left to levels that fill at most three
+// quarters of the warps: fuller, the row above each tile, which two rows pay for as much as four,
+// costs more than it gives (424 x 400, 91 %: 2 rows 2.0, 4 rows 1.87).
+bool res_choose(const uint8_t* code, int w, int h, bool masked, bool half, ResTiles& out) {
+  int dev = 0, sms = 0;
+  VFS_CUDA(cudaGetDevice(&dev));
+  VFS_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  ResLevel L;
+  if (!L.scan(code, w, h, masked)) return false;
+  for (int k = 0; k < kResNumRows; k++) {
+    const int rows = kResRows[k];
+    const int cap = res_capacity(masked, half, rows), n = L.count(rows);
+    if (n > cap || (rows == kResRows[0] && 4 * (long long)n > 3 * (long long)cap)) continue;
+    L.tiles(rows, out);
+    out.blocks = std::min(sms, n);
+    return true;
+  }
+  return false;
+}
+
+size_t res_bytes_bound(int w, int h) {
+  size_t most = 0;
+  for (int k = 0; k < kResNumRows; k++) {
+    const int rows = kResRows[k];
+    const size_t tiles = std::min<size_t>((size_t)((w + kResCols - 1) / kResCols) * ((h + rows - 1) / rows), kResMostTiles);
+    most = std::max(most, tiles * (kResRing * res_slots(rows) * sizeof(uint4) + sizeof(ResTile) + sizeof(int2)));
+  }
+  return most + 4 * 256 + sizeof(ResCtl);
+}
+
+}  // namespace vfs

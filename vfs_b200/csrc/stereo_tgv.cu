@@ -129,6 +129,10 @@ static cudaError_t pool_malloc(void** p, size_t bytes) {
 void StereoTgvImpl::release() {
   engine.clear();
   tex.clear();
+  dropResident(false);
+  dropResident(true);
+  host_code[0].clear();
+  host_code[1].clear();
   if (pool_) cudaFree(pool_);
   pool_ = nullptr;
   if (fpool_) cudaFree(fpool_);
@@ -138,8 +142,9 @@ void StereoTgvImpl::release() {
   f_rv = nullptr;
   code_masked.clear();
   code_plain.clear();
-  codes_valid = false;
-  pool_bytes_ = pool_used_ = 0;
+  codes_valid = spans_valid = false;
+  pool_bytes_ = pool_used_ = res_room_ = 0;
+  res_room_used_ = false;
   guards_.clear();
   initialized_ = false;
 }
@@ -197,12 +202,20 @@ static size_t fused_bytes_for(const std::vector<int>& pS, const std::vector<int>
   return bytes;
 }
 
+// room for the plans of the register-resident iteration behind the pool's planes
+static size_t resident_bytes_for(const std::vector<int>& pW, const std::vector<int>& pH) {
+  size_t bytes = 0;
+  for (size_t l = 0; l < pW.size(); l++) bytes += res_bytes_bound(pW[l], pH[l]);
+  return bytes;
+}
+
 size_t estimate_device_bytes(int width, int height, int nLevels, float fScale, int sa, bool fused) {
   if (width <= 0 || height <= 0 || nLevels <= 0 || sa <= 0 || !(fScale > 0.0f)) return 0;
-  std::vector<int> pS, pH;
+  std::vector<int> pS, pH, pW;
   int nh = height, nw = width;
   for (int l = 0; l < nLevels; l++) {
     if (nw <= 0 || nh <= 0) return 0;
+    pW.push_back(nw);
     pS.push_back(align_up(nw, sa));
     pH.push_back(nh);
     nh = (int)((float)nh / fScale);
@@ -210,7 +223,7 @@ size_t estimate_device_bytes(int width, int height, int nLevels, float fScale, i
   }
   size_t full = (size_t)pS[0] * pH[0];
   if (full * 8 >= ((size_t)1 << 31)) return 0;  // initialize refuses this geometry
-  return pool_bytes_for(pS, pH, full) + (fused ? fused_bytes_for(pS, pH, full) : 0);
+  return pool_bytes_for(pS, pH, full) + 256 + resident_bytes_for(pW, pH) + (fused ? fused_bytes_for(pS, pH, full) : 0);
 }
 
 // stereotgv.cu:44-168
@@ -252,7 +265,9 @@ void StereoTgvImpl::initialize(const SolverParams& p) {
     throw ArgError{"initialize: image too large (row pitch x height x 8 must stay below 2^31)"};
   size_t f = full_ * sizeof(float);
   pool_bytes_ = pool_bytes_for(pS, pH, full_);
-  cudaError_t e = pool_malloc((void**)&pool_, pool_bytes_);
+  res_room_ = resident_bytes_for(pW, pH);
+  res_room_used_ = false;
+  cudaError_t e = pool_malloc((void**)&pool_, resRoomAt() + res_room_);
   if (e != cudaSuccess) {
     pool_ = nullptr;
     (void)cudaGetLastError();
@@ -449,6 +464,82 @@ void StereoTgvImpl::ensureFused() {
   fillGuards(guards_before, stream_);
   for (int l = 0; l < levels(); l++) launch_edge_codes(nullptr, code_plain[l], pW[l], pH[l], pS[l], stream_);
   codes_valid = false;
+}
+
+void StereoTgvImpl::dropResident(bool masked) {
+  for (int half = 0; half < 2; half++) {
+    res_plans_[masked][half].clear();
+    char*& m = res_mem_[masked][half];
+    if (m && m == pool_ + resRoomAt()) res_room_used_ = false;
+    else if (m) cudaFree(m);
+    m = nullptr;
+  }
+}
+
+// Needs the host copies of the form's edge codes.  Without memory for the plans the levels
+// simply have none (the solve then launches one iteration at a time).
+void StereoTgvImpl::ensureResident(bool masked, bool half, cudaStream_t st) {
+  std::vector<ResPlan>& plans = res_plans_[masked][half];
+  if (!plans.empty()) return;
+  plans.assign(levels(), ResPlan{});
+  if (P.nSolverIters < 1 || P.nSolverIters > kResMaxIters || !(P.lambda >= 0.0f)) return;
+  // its quotients take step sizes in a range that no sane schedule leaves
+  float tau = 1.0f, sigma = 1.0f;
+  for (int j = 0; j < P.nSolverIters; j++) {
+    const float mu = sigma < 1000.0f ? 1.0f / std::sqrt(1 + 0.7f * tau * P.timestep_lambda) : 1.0f;
+    if (!(tau >= 0x1p-60f && tau <= 0x1p60f)) return;
+    sigma = sigma / mu;
+    tau = tau * mu;
+  }
+  std::vector<ResTiles> cut(levels());
+  size_t bytes = 0;
+  auto take = [&](size_t b) {
+    const size_t off = bytes;
+    bytes += (b + 255) & ~(size_t)255;
+    return off;
+  };
+  struct Off {
+    size_t tiles, fill, exch, ctl;
+  };
+  std::vector<Off> off(levels());
+  for (int l = 0; l < levels(); l++) {
+    if (!res_choose(host_code[masked][l].data(), pW[l], pH[l], masked, half, cut[l])) continue;
+    plans[l].rows = cut[l].rows;
+    plans[l].blocks = cut[l].blocks;
+    plans[l].ntiles = (int)cut[l].tiles.size();
+    plans[l].nfill = (int)cut[l].fill.size();
+    off[l].ctl = take(sizeof(ResCtl));
+    off[l].tiles = take(cut[l].tiles.size() * sizeof(ResTile));
+    off[l].fill = take(cut[l].fill.size() * sizeof(int2));
+    off[l].exch = take((size_t)kResRing * plans[l].ntiles * res_slots(plans[l].rows) * sizeof(uint4));
+  }
+  if (bytes == 0) return;
+  char* m = nullptr;
+  if (!res_room_used_ && bytes <= res_room_) {
+    m = pool_ + resRoomAt();
+    res_room_used_ = true;
+  } else if (cudaMalloc((void**)&m, bytes) != cudaSuccess) {
+    (void)cudaGetLastError();
+    plans.assign(levels(), ResPlan{});
+    return;
+  }
+  res_mem_[masked][half] = m;
+  // the words' tags start at 0, which no launch waits for (epochs count from 1); the uploads are from
+  // pageable memory, staged before the calls return
+  VFS_CUDA(cudaMemsetAsync(m, 0, bytes, st));
+  for (int l = 0; l < levels(); l++) {
+    ResPlan& p = plans[l];
+    if (p.ntiles == 0) continue;
+    p.ctl = (ResCtl*)(m + off[l].ctl);
+    p.tiles = (const ResTile*)(m + off[l].tiles);
+    p.fill = (const int2*)(m + off[l].fill);
+    p.exch = (uint4*)(m + off[l].exch);
+    VFS_CUDA(cudaMemcpyAsync(m + off[l].tiles, cut[l].tiles.data(), cut[l].tiles.size() * sizeof(ResTile),
+                             cudaMemcpyHostToDevice, st));
+    if (p.nfill)
+      VFS_CUDA(cudaMemcpyAsync(m + off[l].fill, cut[l].fill.data(), cut[l].fill.size() * sizeof(int2),
+                               cudaMemcpyHostToDevice, st));
+  }
 }
 
 // stereotgv.cu:389-515 (masked) and 256-387 (plain).  Pointer swaps are the

@@ -12,6 +12,7 @@
 #include "common.cuh"
 #include "fused.cuh"
 #include "kernels.cuh"
+#include "resident.cuh"
 
 namespace vfs {
 
@@ -62,7 +63,7 @@ class FusedEngine {
   size_t graphs() const { return cache_.size(); }
   // iteration-kernel variant per pyramid level (finest first) of the last solve
   std::vector<int> last_variants;
-  void note_variants(const std::vector<int>& v, int part);
+  void note_variants(std::vector<int> v, int part);
 
  private:
   struct Entry {
@@ -176,6 +177,23 @@ class StereoTgvImpl {
   float2* f_rv = nullptr;
   std::vector<uint8_t*> code_masked, code_plain;
   bool codes_valid = false;
+  // host copies of the edge codes per level (tight rows), [0] plain and [1] masked
+  std::vector<std::vector<uint8_t>> host_code[2];
+  // ---- register-resident iteration (resident.cuh): a plan per level, for the plain [0] and
+  // masked [1] form and for float [0] and half [1] storage, made on the first solve of that
+  // form with the current mask, on the solve's stream.  Its device memory (tiles and exchange words)
+  // is not part of the handle's state: a solve starts from none of it.  The first plans take
+  // the room kept for them at the end of the pool, those of another form an allocation of their own.
+  void ensureResident(bool masked, bool half, cudaStream_t st);
+  void dropResident(bool masked);
+  const ResPlan* residentPlan(bool masked, bool half, int level) const {
+    const std::vector<ResPlan>& v = res_plans_[masked][half];
+    return level < (int)v.size() && v[level].ntiles > 0 ? &v[level] : nullptr;
+  }
+  // What the kernels that launch one or a few iterations at a time ask of the mask, derived when
+  // a masked solve first runs one of them.
+  void ensureSpans();
+  bool spans_valid = false;
   // per level: the K-iterations-per-launch kernel reproduces the masked form exactly (false
   // only when the row has no padding and a pixel of column 0 is on; kernels_tb.cu)
   std::vector<uint8_t> tb_ok;
@@ -267,6 +285,12 @@ class StereoTgvImpl {
   std::vector<ProfRec> prof_;
   std::vector<cudaEvent_t> evpool_;
   size_t evused_ = 0;
+
+  std::vector<ResPlan> res_plans_[2][2];
+  char* res_mem_[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};
+  size_t res_room_ = 0;       // bytes kept for plans behind the pool's planes
+  bool res_room_used_ = false;
+  size_t resRoomAt() const { return (pool_bytes_ + 255) & ~(size_t)255; }
 
   cudaStream_t own_stream();
   bool initialized_ = false;
