@@ -175,3 +175,76 @@ int main() {
     assert r.returncode == 0, r.stderr
     r = subprocess.run([str(exe)], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0, r.stdout + r.stderr
+
+
+def _dropin(case, p, stream=None):
+    from vfs_b200.stereotgv import StereoTgv
+    i0, i1, mask, tv, cv = case
+    s = StereoTgv()
+    h, w = i0.shape
+    s.limitRange = p["limit_range"]
+    s.initialize(w, h, p["beta"], p["gamma"], p["alpha0"], p["alpha1"], p["tsl"], p["lam"], p["n_levels"],
+                 p["f_scale"], p["n_warp"], p["n_iter"])
+    s.copyMaskToDevice(mask)
+    s.loadVectorFields(tv, cv)
+    if stream is not None:
+        s.set_stream(stream)
+    return s
+
+
+@pytest.mark.parametrize("masked", [True, False], ids=["masked", "plain"])
+def test_dropin_path_buffers(gpu, masked):
+    """The drop-in path on the register-resident iteration (128 iterations) and on a kernel per
+    operation (129, more than one launch holds): the fused path's one-iteration kernels' buffers, and
+    p and q that are zero where nothing is solved."""
+    case = random_case(64, 48, seed=21)
+    i0, i1 = case[:2]
+    for n_iter in (128, 129):
+        p = params(n_levels=2, n_warp=1, n_iter=n_iter)
+        s = _dropin(case, p)
+        f, _ = _solve(case, p, False, masked, variant=1)
+        for _ in range(2):
+            s.copyImagesToDevice(i0, i1)
+            (s.solveStereoForwardMasked if masked else s.solveStereoForward)()
+        for n, c in OUT:
+            assert np.array_equal(s.debug_buffer(n, c), f[n], equal_nan=True), (n_iter, n)
+        on = case[2] > 0 if masked else None
+        for n, c in (("p", 2), ("q", 4)):  # zero where nothing is solved
+            v = s.debug_buffer(n, c)
+            assert np.isfinite(v).all()
+            if masked:
+                assert not v[~on].any(), n
+        assert s.check_guards() == 0
+
+
+def test_dropin_solve_in_a_captured_stream(gpu):
+    """The drop-in solve inside a caller's stream capture, after solves that made its texture objects:
+    its launches go into the caller's graph."""
+    import torch
+    case = random_case(150, 110, seed=3)
+    p = params(n_levels=2, n_warp=2, n_iter=6)
+    i0, i1 = (torch.from_numpy(x).cuda() for x in case[:2])
+    want = _dropin(case, p)
+    want.copyImagesToDevice(*case[:2])
+    want.solveStereoForwardMasked()
+    u = want.copy1DDisparityToHost()
+    st = torch.cuda.Stream()
+    s = _dropin(case, p, st)
+    out = torch.zeros((110, 150), device="cuda")
+    torch.cuda.synchronize()
+
+    def frame():
+        s.copy_images_from_device(i0, i1)
+        s.solveStereoForwardMasked()
+        s.copy_1d_disparity_to_device(out)
+
+    for _ in range(2):
+        frame()
+    torch.cuda.synchronize()
+    out.zero_()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=st):
+        frame()
+    g.replay()
+    torch.cuda.synchronize()
+    assert np.array_equal(out.cpu().numpy(), u)

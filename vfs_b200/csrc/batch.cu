@@ -43,8 +43,10 @@ void set_iter_tiles(IterArgs& A, int k, int w, int h, int rows) {
 // part: 0 the whole solve; 1 the calibration warp, the pyramid and the levels above full
 // resolution (ending with the upscale to it); 2 the full-resolution level alone.  Running part 1
 // then part 2 enqueues exactly what part 0 does.
+// dropin: the drop-in path (one pair, float storage, every level register-resident): p and q in the
+// pool's single planes, and the preconditioners and the last change of u left where its own kernels do.
 void fused_solve_direct(std::vector<StereoTgvImpl*>& pairs, bool masked, bool half, cudaStream_t st,
-                        std::vector<int>& level_variant, bool can_tune, int concurrency, int part) {
+                        std::vector<int>& level_variant, bool can_tune, int concurrency, int part, bool dropin = false) {
   const int n = (int)pairs.size();
   if (n == 0) return;
   if (n > kMaxPairs) throw ArgError{"batch larger than " + std::to_string(kMaxPairs) + " pairs"};
@@ -55,7 +57,7 @@ void fused_solve_direct(std::vector<StereoTgvImpl*>& pairs, bool masked, bool ha
     if (s->P.nWarpIters != P0.nWarpIters || s->P.nSolverIters != P0.nSolverIters ||
         s->P.timestep_lambda != P0.timestep_lambda)
       throw ArgError{"fused solve: pairs of one batch need equal warp / iteration counts and timestep_lambda"};
-    s->ensureFused();
+    if (!dropin) s->ensureFused();
     maxL = std::max(maxL, s->levels());
   }
   StereoTgvImpl* prof = pairs[0];
@@ -132,6 +134,9 @@ void fused_solve_direct(std::vector<StereoTgvImpl*>& pairs, bool masked, bool ha
         d.cuda_math = s->tensor_cuda_math;
         d.abce = half ? s->f_abce : nullptr;
         d.rv = half ? s->f_rv : nullptr;
+        d.etau = dropin ? s->d_etau : nullptr;
+        d.etav1 = s->d_etav1;
+        d.etav2 = s->d_etav2;
         d.alpha0 = s->P.alpha0;
         d.alpha1 = s->P.alpha1;
         set_tiles(L, k, d.w, d.h);
@@ -142,7 +147,10 @@ void fused_solve_direct(std::vector<StereoTgvImpl*>& pairs, bool masked, bool ha
     }
     // the per-warp prologue's arguments (the current v-bar buffer is the one the iterations
     // left current, so the same call serves a warp's start and the previous warp's epilogue)
-    auto warp_start_args = [&]() {
+    // (the register-resident iteration starts from p = q = 0 by itself; the drop-in path's last
+    // iterations leave zeros at the masked-out pixels)
+    const bool resident = level_variant[level] == kIterResident && act[0]->residentPlan(masked, half, level);
+    auto warp_start_args = [&](int warp) {
       WarpStartArgs W{};
       for (int k = 0; k < na; k++) {
         StereoTgvImpl* s = act[k];
@@ -152,8 +160,9 @@ void fused_solve_direct(std::vector<StereoTgvImpl*>& pairs, bool masked, bool ha
         d.warpUV = s->d_warpUV;
         d.tv2 = s->d_tv2;
         d.i1warp = s->d_i1warp;
-        d.p = s->f_p;
-        d.q = s->f_q;
+        d.p = dropin ? (void*)s->d_p : s->f_p;
+        d.q = dropin ? (void*)s->d_q : s->f_q;
+        d.pq_planes = !resident ? 2 : dropin && level == 0 && warp == P0.nWarpIters - 1 ? 1 : 0;
         d.v_ = half ? s->f_vh : (void*)s->d_v_;
         d.w = s->pW[level];
         d.h = s->pH[level];
@@ -166,7 +175,7 @@ void fused_solve_direct(std::vector<StereoTgvImpl*>& pairs, bool masked, bool ha
     for (int warpIter = 0; warpIter < P0.nWarpIters; warpIter++) {
       prof->profBeginPx(kProfPrologue, px_level, 1, st);
       // later warps' prologues run in the previous warp's epilogue launch
-      if (warpIter == 0) launch_warp_start(warp_start_args(), half, st);
+      if (warpIter == 0) launch_warp_start(warp_start_args(0), half, st);
       {
         DerivArgs Dv{};
         for (int k = 0; k < na; k++) {
@@ -201,8 +210,8 @@ void fused_solve_direct(std::vector<StereoTgvImpl*>& pairs, bool masked, bool ha
           d.u_ = s->d_u_;
           d.u = s->d_u;
           d.v_ = half ? s->f_vh : (const void*)s->d_v_;
-          d.p = s->f_p;
-          d.q = s->f_q;
+          d.p = dropin ? (void*)s->d_p : s->f_p;
+          d.q = dropin ? (void*)s->d_q : s->f_q;
           d.Tp = s->d_Tp;
           d.a = s->d_a;
           d.b = s->d_b;
@@ -395,7 +404,7 @@ void fused_solve_direct(std::vector<StereoTgvImpl*>& pairs, bool masked, bool ha
                          : variant;
       float tau = 1.0f;
       float sigma = 1.0f / tau;
-      prof->profBeginPx(kProfFused, px_level, n_it, st,
+      prof->profBeginPx(dropin ? kProfInner : kProfFused, px_level, n_it, st,
                         res ? 1 : cl_here ? (n_it + K - 1) / K : K > 1 ? n_it / K + n_it % K : n_it);
       for (int iter = 0; iter < n_it;) {
         const int k = res ? n_it : cl_here ? std::min(K, n_it - iter) : (K > 1 && iter + K <= n_it) ? K : 1;
@@ -409,7 +418,7 @@ void fused_solve_direct(std::vector<StereoTgvImpl*>& pairs, bool masked, bool ha
           A.fill = res->fill;
           A.nfill = res->nfill;
           A.n = n_it;
-          A.p_planes = 1;
+          A.p_planes = dropin ? 0 : 1;
           A.rows = res->rows;
           A.blocks = res->blocks;
           A.minus_zero = make_float2(-0.0f, -0.0f);
@@ -470,6 +479,7 @@ void fused_solve_direct(std::vector<StereoTgvImpl*>& pairs, bool masked, bool ha
           d.u_out = masked ? s->d_us : s->d_u;
           d.u_bar = s->d_u_;
           d.u_last = s->d_u_last;
+          d.du = dropin ? s->d_du : nullptr;
           d.tv2 = s->d_tv2;
           d.warpUV = s->d_warpUV;
           d.w = s->pW[level];
@@ -479,7 +489,7 @@ void fused_solve_direct(std::vector<StereoTgvImpl*>& pairs, bool masked, bool ha
           set_tiles(E, k, d.w, d.h);
         }
         E.npairs = na;
-        if (warpIter + 1 < P0.nWarpIters) launch_epilogue_warp_start(E, warp_start_args(), half, st);
+        if (warpIter + 1 < P0.nWarpIters) launch_epilogue_warp_start(E, warp_start_args(warpIter + 1), half, st);
         else launch_warp_epilogue_batched(E, st);
         if (masked)
           for (auto* s : act) std::swap(s->d_u, s->d_us);
@@ -620,32 +630,7 @@ void FusedEngine::prepare(std::vector<StereoTgvImpl*>& pairs, bool masked) {
   for (auto* s : pairs) {
     if (!s->initialized()) throw ArgError{"fused solve: pair not initialized"};
     s->ensureFused();
-    if (!masked && s->host_code[0].empty()) {
-      s->host_code[0].resize(s->levels());
-      for (int l = 0; l < s->levels(); l++) {
-        s->host_code[0][l].resize((size_t)s->pW[l] * s->pH[l]);
-        VFS_CUDA(cudaMemcpy2DAsync(s->host_code[0][l].data(), s->pW[l], s->code_plain[l], s->pS[l], s->pW[l], s->pH[l],
-                                   cudaMemcpyDeviceToHost, s->stream()));
-      }
-      VFS_CUDA(cudaStreamSynchronize(s->stream()));
-    }
-    if (masked && !s->codes_valid) {
-      s->dropResident(true);
-      s->host_code[1].assign(s->levels(), {});
-      for (int l = 0; l < s->levels(); l++)
-        launch_edge_codes(s->pMask[l], s->code_masked[l], s->pW[l], s->pH[l], s->pS[l], s->stream());
-      for (int l = 0; l < s->levels(); l++) {
-        const int w = s->pW[l], h = s->pH[l];
-        std::vector<uint8_t>& code = s->host_code[1][l];
-        code.resize((size_t)w * h);
-        VFS_CUDA(cudaMemcpy2DAsync(code.data(), w, s->code_masked[l], s->pS[l], w, h, cudaMemcpyDeviceToHost,
-                                   s->stream()));
-      }
-      VFS_CUDA(cudaStreamSynchronize(s->stream()));
-      s->spans_valid = false;
-      s->codes_valid = true;
-      s->generation = next_generation();  // graphs captured under the old mask are not reused
-    }
+    s->ensureCodes(masked);
   }
 }
 
@@ -851,12 +836,31 @@ void FusedEngine::solve_parts(std::vector<StereoTgvImpl*>& pairs, bool masked, b
     for (int l = 0; l < maxL && l < (int)forced_levels.size(); l++) variants[l] = forced_levels[l];
   }
   note_variants(variants, part);
-  if (!use_graph) {
-    fused_solve_direct(pairs, masked, half, st, variants, false, concurrency, part);
+  run(pairs, masked, half, st, part, variants, false);
+}
+
+void FusedEngine::solve_dropin(StereoTgvImpl* pair, bool masked, cudaStream_t st) {
+  std::vector<StereoTgvImpl*> one{pair};
+  std::vector<int> variants(pair->levels(), kIterResident);
+  run(one, masked, false, st, 0, variants, true);
+  pair->i1warp_half = false;
+}
+
+// The solve with the variants settled: from a graph captured in the same state, or directly.
+void FusedEngine::run(std::vector<StereoTgvImpl*>& pairs, bool masked, bool half, cudaStream_t st, int part,
+                      std::vector<int>& variants, bool dropin) {
+  bool direct = !use_graph;
+  if (dropin && !direct) {  // a stream under capture takes the launches themselves
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    VFS_CUDA(cudaStreamIsCapturing(st, &cap));
+    direct = cap != cudaStreamCaptureStatusNone;
+  }
+  if (direct) {
+    fused_solve_direct(pairs, masked, half, st, variants, false, concurrency, part, dropin);
     return;
   }
   StereoTgvImpl* prof = pairs[0];
-  std::vector<uintptr_t> key{(uintptr_t)masked, (uintptr_t)half, (uintptr_t)prof->profiling, (uintptr_t)part,
+  std::vector<uintptr_t> key{(uintptr_t)masked, (uintptr_t)half, (uintptr_t)dropin, (uintptr_t)prof->profiling, (uintptr_t)part,
                              (uintptr_t)(intptr_t)launch_priority()};
   for (int v : variants) key.push_back((uintptr_t)v);
   std::vector<PairPtrs> before;
@@ -885,7 +889,7 @@ void FusedEngine::solve_parts(std::vector<StereoTgvImpl*>& pairs, bool masked, b
     long long launches0 = launch_counter().load();
     VFS_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeRelaxed));
     try {
-      fused_solve_direct(pairs, masked, half, st, variants, false, concurrency, part);
+      fused_solve_direct(pairs, masked, half, st, variants, false, concurrency, part, dropin);
     } catch (...) {
       prof->capture_events = nullptr;
       cudaGraph_t junk = nullptr;

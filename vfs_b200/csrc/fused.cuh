@@ -182,7 +182,8 @@ struct WarpStartPair {
   const float2* warpUV;
   float2* tv2;
   void* i1warp;  // warped image: float, or half with half_storage
-  void *p, *q, *v_;  // zeroed (px < w); storage type by half_storage
+  void *p, *q, *v_;  // zeroed (px < w), the first pq_planes planes of p and q; storage type by half_storage
+  int pq_planes;
   int w, h, s, tiles_x, tile0;
 };
 struct WarpStartArgs {
@@ -214,6 +215,7 @@ struct EpiPair {
   const float* u_last;
   const float2* tv2;
   float2* warpUV;      // += du * tv2
+  float* du;           // receives min(median - u_last, limit); null: not kept
   int w, h, s, tiles_x, tile0;
   float limitRange;
 };
@@ -243,6 +245,7 @@ struct LevelPair {
   // whose reciprocal preconditioners take alpha0 and alpha1; null otherwise
   float4* abce;
   float2* rv;
+  float *etau, *etav1, *etav2;  // the preconditioners themselves (drop-in path); etau null: not kept
   float alpha0, alpha1;
 };
 struct LevelArgs {

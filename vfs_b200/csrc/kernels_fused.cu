@@ -409,10 +409,14 @@ __device__ __forceinline__ void warp_start_at(const WarpStartPair& P, int ix, in
   long long plane = (long long)P.s * P.h;
   typename S::T2* p = (typename S::T2*)P.p;
   typename S::T4* q = (typename S::T4*)P.q;
-  S::st2(p, pos, make_float2(0.f, 0.f));
-  S::st2(p, pos + plane, make_float2(0.f, 0.f));
-  S::st4(q, pos, make_float4(0.f, 0.f, 0.f, 0.f));
-  S::st4(q, pos + plane, make_float4(0.f, 0.f, 0.f, 0.f));
+  if (P.pq_planes > 0) {
+    S::st2(p, pos, make_float2(0.f, 0.f));
+    S::st4(q, pos, make_float4(0.f, 0.f, 0.f, 0.f));
+  }
+  if (P.pq_planes > 1) {
+    S::st2(p, pos + plane, make_float2(0.f, 0.f));
+    S::st4(q, pos + plane, make_float4(0.f, 0.f, 0.f, 0.f));
+  }
   S::st2((typename S::T2*)P.v_, pos, make_float2(0.f, 0.f));
   float x = ((float)ix + wv.x + 0.5f) / (float)P.w;
   float y = ((float)iy + wv.y + 0.5f) / (float)P.h;
@@ -477,6 +481,7 @@ __device__ __forceinline__ float2 epilogue_at(const EpiPair& P, bool median, int
   float ul = P.u_last[pos];
   float d = m - ul;
   d = d > P.limitRange ? P.limitRange : d;
+  if (P.du) P.du[pos] = d;
   float un = ul + d;
   P.u_out[pos] = un;
   P.u_bar[pos] = un;
@@ -564,6 +569,13 @@ __device__ __forceinline__ void level_records(const LevelPair& P, long long pos,
   P.rv[pos] = fast::etav_rcp(fast::etav(b, c, a1s, a0s4), fast::etav(a, c, a1s, a0s4));
 }
 
+// preconditioning.cu:18-20 (zero at masked-out pixels)
+__device__ __forceinline__ void level_etas(const LevelPair& P, long long pos, float a, float b, float c, bool off) {
+  P.etau[pos] = off ? 0.0f : etau_math(a, b, c, P.alpha1);
+  P.etav1[pos] = off ? 0.0f : etav1_math(b, c, P.alpha0, P.alpha1);
+  P.etav2[pos] = off ? 0.0f : etav2_math(a, c, P.alpha0, P.alpha1);
+}
+
 // calcTensor.cu:8-73 / 155-219; a = b = c = 0 where the reference does not compute
 // (masked out, or columns >= xmax of its launch grid)
 __global__ void __launch_bounds__(kFTW* kFTH) k_level_tensor(const __grid_constant__ LevelArgs A) {
@@ -575,6 +587,7 @@ __global__ void __launch_bounds__(kFTW* kFTH) k_level_tensor(const __grid_consta
     P.b[pos] = 0.0f;
     P.c[pos] = 0.0f;
     if (P.abce) level_records(P, pos, 0.0f, 0.0f, 0.0f);
+    if (P.etau) level_etas(P, pos, 0.0f, 0.0f, 0.0f, P.mask && P.mask[pos] == 0.0f);
     return;
   }
   float dx = 1.0f / (float)P.w, dy = 1.0f / (float)P.h;
@@ -597,6 +610,7 @@ __global__ void __launch_bounds__(kFTW* kFTH) k_level_tensor(const __grid_consta
   P.c[pos] = c;
   P.b[pos] = b;
   if (P.abce) level_records(P, pos, a, b, c);
+  if (P.etau) level_etas(P, pos, a, b, c, false);
 }
 
 void launch_level_gaussian(const LevelArgs& A, cudaStream_t st) {

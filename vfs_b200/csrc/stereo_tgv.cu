@@ -193,8 +193,9 @@ static size_t pool_bytes_for(const std::vector<int>& pS, const std::vector<int>&
   return bytes + full * sizeof(float) * planes + full * (2 + 2 * 3) + 64 * 512 + 40 * StereoTgvImpl::kGuardBytes;
 }
 
-// p, q two planes each (float: 8 + 16 bytes per pixel and plane), half v-bar pair, and
-// two edge-code bytes per pixel and level.
+// p, q two planes each (float: 8 + 16 bytes per pixel and plane), half v-bar pair, the
+// coefficient records, and two bytes per pixel and level that exported states carry (the edge
+// codes' former place).
 static size_t fused_bytes_for(const std::vector<int>& pS, const std::vector<int>& pH, size_t full) {
   size_t bytes = full * 2 * 8 + full * 2 * 16 + full * 4 * 2 + full * 16 + full * 8 + 8 * 512 +
                  8 * StereoTgvImpl::kGuardBytes;
@@ -202,7 +203,13 @@ static size_t fused_bytes_for(const std::vector<int>& pS, const std::vector<int>
   return bytes;
 }
 
-// room for the plans of the register-resident iteration behind the pool's planes
+// behind the pool's planes, outside the exported state: two edge-code bytes per pixel and level, and
+// room for the plans of the register-resident iteration
+static size_t code_bytes_for(const std::vector<int>& pS, const std::vector<int>& pH) {
+  size_t bytes = 0;
+  for (size_t l = 0; l < pS.size(); l++) bytes += 2 * ((size_t)pS[l] * pH[l] + 512 + StereoTgvImpl::kGuardBytes);
+  return bytes;
+}
 static size_t resident_bytes_for(const std::vector<int>& pW, const std::vector<int>& pH) {
   size_t bytes = 0;
   for (size_t l = 0; l < pW.size(); l++) bytes += res_bytes_bound(pW[l], pH[l]);
@@ -223,7 +230,7 @@ size_t estimate_device_bytes(int width, int height, int nLevels, float fScale, i
   }
   size_t full = (size_t)pS[0] * pH[0];
   if (full * 8 >= ((size_t)1 << 31)) return 0;  // initialize refuses this geometry
-  return pool_bytes_for(pS, pH, full) + 256 + resident_bytes_for(pW, pH) + (fused ? fused_bytes_for(pS, pH, full) : 0);
+  return pool_bytes_for(pS, pH, full) + 512 + code_bytes_for(pS, pH) + resident_bytes_for(pW, pH) + (fused ? fused_bytes_for(pS, pH, full) : 0);
 }
 
 // stereotgv.cu:44-168
@@ -267,6 +274,8 @@ void StereoTgvImpl::initialize(const SolverParams& p) {
   pool_bytes_ = pool_bytes_for(pS, pH, full_);
   res_room_ = resident_bytes_for(pW, pH);
   res_room_used_ = false;
+  const size_t code_bytes = code_bytes_for(pS, pH);
+  code_bytes_ = code_bytes;
   cudaError_t e = pool_malloc((void**)&pool_, resRoomAt() + res_room_);
   if (e != cudaSuccess) {
     pool_ = nullptr;
@@ -323,7 +332,18 @@ void StereoTgvImpl::initialize(const SolverParams& p) {
   d_pack = alloc(4 * f);
   // The reference leaves its buffers uninitialised after cudaMalloc; this
   // implementation starts from all-zero state so that results are deterministic.
-  VFS_CUDA(cudaMemsetAsync(pool_, 0, pool_bytes_, stream_));
+  code_masked.assign(levels(), nullptr);
+  code_plain.assign(levels(), nullptr);
+  size_t at = pool_bytes_;
+  for (int l = 0; l < levels(); l++)
+    for (uint8_t** c : {&code_masked[l], &code_plain[l]}) {
+      at = (at + 511) & ~(size_t)511;
+      *c = (uint8_t*)pool_ + at;
+      at += (size_t)pS[l] * pH[l];
+      guards_.push_back(pool_ + at);
+      at += kGuardBytes;
+    }
+  VFS_CUDA(cudaMemsetAsync(pool_, 0, at, stream_));
   fillGuards(0, stream_);
   VFS_CUDA(cudaStreamSynchronize(stream_));
   initialized_ = true;
@@ -404,7 +424,8 @@ void StereoTgvImpl::solve(bool masked) {
     std::vector<StereoTgvImpl*> one{this};
     engine.solve(one, masked, half_storage, stream_);
   } else {
-    solveReference(masked);
+    if (dropinResident(masked)) engine.solve_dropin(this, masked, stream_);
+    else solveReference(masked);
     have_prev = true;
   }
 }
@@ -426,7 +447,7 @@ void StereoTgvImpl::startState(int top, cudaStream_t st) {
 }
 
 // Fused-path buffers: p and q in two planes each (float: 8 + 16 bytes per pixel per
-// plane; half: 4 + 8), half v-bar ping-pong pair (4 + 4), and per-level edge codes.
+// plane; half: 4 + 8), half v-bar ping-pong pair (4 + 4), and the coefficient records.
 void StereoTgvImpl::ensureFused() {
   if (fpool_) return;
   size_t n = full_;
@@ -454,16 +475,43 @@ void StereoTgvImpl::ensureFused() {
   f_vhs = take(n * 4);
   f_abce = (float4*)take(n * 16);
   f_rv = (float2*)take(n * 8);
-  code_masked.assign(levels(), nullptr);
-  code_plain.assign(levels(), nullptr);
-  for (int l = 0; l < levels(); l++) {
-    code_masked[l] = (uint8_t*)take((size_t)pS[l] * pH[l]);
-    code_plain[l] = (uint8_t*)take((size_t)pS[l] * pH[l]);
-  }
   VFS_CUDA(cudaMemsetAsync(fpool_, 0, bytes, stream_));
   fillGuards(guards_before, stream_);
-  for (int l = 0; l < levels(); l++) launch_edge_codes(nullptr, code_plain[l], pW[l], pH[l], pS[l], stream_);
-  codes_valid = false;
+}
+
+void StereoTgvImpl::ensureCodes(bool masked) {
+  if (masked ? codes_valid : !host_code[0].empty()) return;
+  if (masked) dropResident(true);
+  std::vector<std::vector<uint8_t>>& host = host_code[masked];
+  host.assign(levels(), {});
+  for (int l = 0; l < levels(); l++) {
+    uint8_t* dev = masked ? code_masked[l] : code_plain[l];
+    launch_edge_codes(masked ? pMask[l] : nullptr, dev, pW[l], pH[l], pS[l], stream_);
+    host[l].resize((size_t)pW[l] * pH[l]);
+    VFS_CUDA(cudaMemcpy2DAsync(host[l].data(), pW[l], dev, pS[l], pW[l], pH[l], cudaMemcpyDeviceToHost, stream_));
+  }
+  VFS_CUDA(cudaStreamSynchronize(stream_));
+  if (masked) {
+    spans_valid = false;
+    codes_valid = true;
+    generation = next_generation();  // graphs captured under the old mask are not reused
+  }
+}
+
+// Whether every level of the next solve has a plan; while the stream is being captured, whether they
+// are all there already (making one synchronises the stream).
+bool StereoTgvImpl::dropinResident(bool masked) {
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  VFS_CUDA(cudaStreamIsCapturing(stream_, &cap));
+  if (cap == cudaStreamCaptureStatusNone) {
+    ensureCodes(masked);
+    ensureResident(masked, false, stream_);
+  } else if (masked && !codes_valid) {
+    return false;
+  }
+  for (int l = 0; l <= topLevel(); l++)
+    if (!residentPlan(masked, false, l)) return false;
+  return true;
 }
 
 void StereoTgvImpl::dropResident(bool masked) {

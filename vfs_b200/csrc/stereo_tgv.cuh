@@ -27,7 +27,7 @@ struct SolverParams {
 
 // Which implementation runs the solve.
 enum class SolvePath {
-  kReference = 0,  // one kernel per reference kernel (drop-in form)
+  kReference = 0,  // the reference's buffers to the bit (drop-in form)
   kFused = 1,      // fused kernels (one or several iterations per launch), CUDA graphs
 };
 
@@ -55,8 +55,12 @@ class FusedEngine {
   void clear();
   // part: 0 whole solve; 1 everything before the full-resolution level; 2 that level alone
   void solve(std::vector<StereoTgvImpl*>& pairs, bool masked, bool half, cudaStream_t st, int part = 0);
+  // the drop-in path of one pair whose every level has a plan (StereoTgvImpl::dropinResident)
+  void solve_dropin(StereoTgvImpl* pair, bool masked, cudaStream_t st);
  private:
   void solve_parts(std::vector<StereoTgvImpl*>& pairs, bool masked, bool half, cudaStream_t st, int part);
+  void run(std::vector<StereoTgvImpl*>& pairs, bool masked, bool half, cudaStream_t st, int part, std::vector<int>& variants,
+           bool dropin);
  public:
   // allocate fused buffers and refresh edge codes, each on the pair's own stream
   static void prepare(std::vector<StereoTgvImpl*>& pairs, bool masked);
@@ -177,6 +181,9 @@ class StereoTgvImpl {
   float2* f_rv = nullptr;
   std::vector<uint8_t*> code_masked, code_plain;
   bool codes_valid = false;
+  // the form's edge codes on the device and the host, on the handle's stream (which it synchronises
+  // when they are not there yet)
+  void ensureCodes(bool masked);
   // host copies of the edge codes per level (tight rows), [0] plain and [1] masked
   std::vector<std::vector<uint8_t>> host_code[2];
   // ---- register-resident iteration (resident.cuh): a plan per level, for the plain [0] and
@@ -272,6 +279,8 @@ class StereoTgvImpl {
     return tex.get(p, pW[level], pH[level], (size_t)pS[level] * sizeof(float2), 2, true);
   }
   void solveReference(bool masked);
+  // the drop-in path can run on the register-resident iteration: every level it solves has a plan
+  bool dropinResident(bool masked);
 
  public:
   cudaEvent_t profEvent();
@@ -290,7 +299,8 @@ class StereoTgvImpl {
   char* res_mem_[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};
   size_t res_room_ = 0;       // bytes kept for plans behind the pool's planes
   bool res_room_used_ = false;
-  size_t resRoomAt() const { return (pool_bytes_ + 255) & ~(size_t)255; }
+  size_t code_bytes_ = 0;     // of the edge codes before them
+  size_t resRoomAt() const { return (pool_bytes_ + code_bytes_ + 511) & ~(size_t)255; }
 
   cudaStream_t own_stream();
   bool initialized_ = false;
