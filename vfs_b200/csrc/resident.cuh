@@ -94,6 +94,9 @@ struct ResArgs {
 // A level's tiles (host side).
 struct ResTiles {
   int rows = 0, blocks = 0;
+  // Renumbers the tiles for a grid of `blocks` (tile t: warp t / blocks of block t % blocks) so that
+  // those with edge rules sit on the schedulers (warp % 4) that have the fewest tiles.
+  void place(int blocks);
   std::vector<ResTile> tiles;
   std::vector<int2> fill;
 };
@@ -108,7 +111,7 @@ struct ResLevel {
   // (lower) neighbour reads outside the image, a one-pixel-wide or -high plain level has no
   // neighbour to take, or no pixel is on.
   bool scan(const uint8_t* code, int w, int h, bool masked);
-  int count(int rows) const;                   // tiles of `rows` rows
+  int count(int rows) const;  // tiles of `rows` rows
   void tiles(int rows, ResTiles& out) const;
 };
 // Picks the tile height for the level among the instances whose grid can be resident;

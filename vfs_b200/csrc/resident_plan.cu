@@ -123,6 +123,28 @@ void ResLevel::tiles(int rows, ResTiles& out) const {
     }
 }
 
+void ResTiles::place(int grid) {
+  blocks = grid;
+  const int n = (int)tiles.size();
+  // tiles per scheduler of a block that has all its warps, or one less
+  auto load = [&](int t) {
+    const int b = t % grid, warps = (n - b + grid - 1) / grid, w = t / grid;
+    return (warps - w % 4 + 3) / 4;
+  };
+  std::vector<int> slot(n), tile(n), to(n);
+  for (int t = 0; t < n; t++) slot[t] = tile[t] = t;
+  std::stable_sort(slot.begin(), slot.end(), [&](int a, int b) { return load(a) < load(b); });
+  std::stable_sort(tile.begin(), tile.end(), [&](int a, int b) { return tiles[a].kind > tiles[b].kind; });
+  for (int k = 0; k < n; k++) to[tile[k]] = slot[k];
+  std::vector<ResTile> placed(n);
+  for (int t = 0; t < n; t++) {
+    ResTile r = tiles[t];
+    for (int& k : r.nb) k = to[k];
+    placed[to[t]] = r;
+  }
+  tiles.swap(placed);
+}
+
 // The smallest tile height whose tiles fit, since more warps with less to do each hide more of one
 // another's latency and shorten an iteration (B200, us per iteration, FP16 / float storage: 848 x 800
 // disc 8 rows 4.2 / 7.9; 640 x 480 4 rows 2.45 / 3.5, 6 rows 2.75 / 3.9, 8 rows 3.1 / 5.3; 212 x 200
@@ -140,7 +162,7 @@ bool res_choose(const uint8_t* code, int w, int h, bool masked, bool half, ResTi
     const int cap = res_capacity(masked, half, rows), n = L.count(rows);
     if (n > cap || (rows == kResRows[0] && 4 * (long long)n > 3 * (long long)cap)) continue;
     L.tiles(rows, out);
-    out.blocks = std::min(sms, n);
+    out.place(std::min(sms, n));
     return true;
   }
   return false;
