@@ -248,3 +248,18 @@ def test_dropin_solve_in_a_captured_stream(gpu):
     g.replay()
     torch.cuda.synchronize()
     assert np.array_equal(out.cpu().numpy(), u)
+
+
+@pytest.mark.parametrize("half", [False, True], ids=["fp32", "fp16"])
+@pytest.mark.parametrize("masked", [True, False], ids=["masked", "plain"])
+def test_cluster_sizes(gpu, masked, half):
+    """Levels about the size where the tiles of one cluster give way to the whole GPU (208 tiles of two
+    rows with half storage, 128 with float), one tile, and fewer tiles than blocks."""
+    for w, h in ((28, 2), (30, 18), (61, 130), (115, 64), (118, 66), (118, 104), (119, 106)):
+        case = random_case(w, h, seed=w * h)
+        m = np.ones((h, w), np.float32)
+        if h > 2:
+            m[0] = m[:, 0] = 0
+        case = case[:2] + (m,) + case[3:]
+        for n_iter in (1, 2, 7):
+            _same(case, params(n_levels=1, n_warp=2, n_iter=n_iter), half, masked, resident=None)

@@ -421,6 +421,7 @@ void fused_solve_direct(std::vector<StereoTgvImpl*>& pairs, bool masked, bool ha
           A.p_planes = dropin ? 0 : 1;
           A.rows = res->rows;
           A.blocks = res->blocks;
+          A.cluster = res->cluster;
           A.minus_zero = make_float2(-0.0f, -0.0f);
           for (int j = 0; j < n_it; j++) {
             const float mu = sigma < 1000.0f ? 1.0f / std::sqrt(1 + 0.7f * tau * P0.timestep_lambda) : 1.0f;

@@ -151,10 +151,10 @@ struct ResState<MASKED, __half, R> {
     return make_uint4(__float_as_uint(ub_of(r)), v[r], 0u, tag);
   }
   static __device__ __forceinline__ void put_col(Sh& sh, int side, int r, uint4 w) { sh.col[side][r] = make_uint2(w.x, w.y); }
-  __device__ __forceinline__ void take_col(Sh& sh, int side) {
+  __device__ __forceinline__ void take_col(const uint2* col) {
 #pragma unroll
     for (int i = 0; i < R / 2; i++) {
-      const uint4 w = *reinterpret_cast<const uint4*>(&sh.col[side][2 * i]);
+      const uint4 w = *reinterpret_cast<const uint4*>(col + 2 * i);
       ub[i] = x2::pk(__uint_as_float(w.x), __uint_as_float(w.z));
       v[2 * i] = w.y;
       v[2 * i + 1] = w.w;
@@ -461,10 +461,10 @@ struct ResState<MASKED, float, R> {
     return make_uint4(__float_as_uint(ub_of(r)), __float_as_uint(v.x), __float_as_uint(v.y), tag);
   }
   static __device__ __forceinline__ void put_col(Sh& sh, int side, int r, uint4 w) { sh.col[side][r] = w; }
-  __device__ __forceinline__ void take_col(Sh& sh, int side) {
+  __device__ __forceinline__ void take_col(const uint4* col) {
 #pragma unroll
     for (int i = 0; i < R / 2; i++) {
-      const uint4 w0 = sh.col[side][2 * i], w1 = sh.col[side][2 * i + 1];
+      const uint4 w0 = col[2 * i], w1 = col[2 * i + 1];
       ub[i] = x2::pk(__uint_as_float(w0.x), __uint_as_float(w1.x));
       vx[i] = x2::pk(__uint_as_float(w0.y), __uint_as_float(w1.y));
       vy[i] = x2::pk(__uint_as_float(w0.z), __uint_as_float(w1.z));
@@ -781,7 +781,7 @@ struct ResWarp {
   ResState<MASKED, ST, R> s;
 
   // Loads tile t: its coefficients, codes and state before the first iteration.
-  __device__ __forceinline__ void load(Sh& sh, const ResArgs& A, int lane, int t) {
+  __device__ __forceinline__ ResEdge load(Sh& sh, const ResArgs& A, int lane, int t) {
     const IterPair& P = A.P;
     const ResTile& T = A.tiles[t];
     const int x = T.x0 - 1 + lane, y0 = T.y0;
@@ -812,27 +812,32 @@ struct ResWarp {
         if (code & kD) e.y |= b;
       }
     }
-    // exchange words; a missing neighbour is replaced by this tile itself: the tags come, the
-    // values are not used.  Lanes 0 .. R-1 fetch the west column, lanes 16 .. 16 + R-1 the east one.
-    const int tn = lane == 0 ? T.nb[4] : lane == 31 ? T.nb[5] : T.nb[0];
-    const int ts = lane == 0 ? T.nb[6] : lane == 31 ? T.nb[7] : T.nb[1];
-    const int col = lane == 0 ? kResCols : lane == 31 ? 1 : lane;
-    const int side = lane >> 4, row = lane & 15;
-    sh.k.at[lane] = make_uint4((unsigned)(tn * kSlots + 32 + col), (unsigned)(ts * kSlots + col),
-                               (unsigned)(T.nb[side ? 3 : 2] * kSlots + 64 + (side ? 0 : R) + (row < R ? row : 0)), e.x);
     sh.k.edge[lane] = make_uint2(e.y, e.on);
     plain = __any_sync(kFull, plain);
     if (lane == 0) {
       sh.k.kind = plain ? kResPlain : T.kind;
       sh.k.t = t;
     }
+    return e;
+  }
+
+  // Where this lane finds its neighbours' words.  A missing neighbour is replaced by this tile itself:
+  // the tags come, the values are not used.  Lanes 0 .. R-1 fetch the west column, lanes 16 .. 16 + R-1
+  // the east one.
+  __device__ __forceinline__ void link(Sh& sh, const ResArgs& A, int lane, int t, const ResEdge& e) {
+    const ResTile& T = A.tiles[t];
+    const int tn = lane == 0 ? T.nb[4] : lane == 31 ? T.nb[5] : T.nb[0];
+    const int ts = lane == 0 ? T.nb[6] : lane == 31 ? T.nb[7] : T.nb[1];
+    const int col = lane == 0 ? kResCols : lane == 31 ? 1 : lane;
+    const int side = lane >> 4, row = lane & 15;
+    sh.k.at[lane] = make_uint4((unsigned)(tn * kSlots + 32 + col), (unsigned)(ts * kSlots + col),
+                               (unsigned)(T.nb[side ? 3 : 2] * kSlots + 64 + (side ? 0 : R) + (row < R ? row : 0)), e.x);
     __syncwarp();
   }
 
   // One iteration.  Returns false once a wait ran out.
   __device__ __forceinline__ bool step(Sh& sh, const ResArgs& A, int lane, int j,
                                        unsigned epoch, bool waiting) {
-    const IterPair& P = A.P;
     const uint4 o = sh.k.at[lane];
     const unsigned ring = (unsigned)A.ntiles * kSlots;
     const uint4* const base = A.exch + (size_t)(j & (kResRing - 1)) * ring;
@@ -857,11 +862,20 @@ struct ResWarp {
     const int side = lane >> 4, row = lane & 15;
     if (row < R) s.put_col(sh, side, row, wc);
     __syncwarp();
-    if (lane == 0 || lane == 31) s.take_col(sh, side);
+    if (lane == 0 || lane == 31) s.take_col(sh.col[side]);
     __syncwarp();
+    iterate(sh, A, lane, j, o.w, wn, ws);
+    if (j + 1 < A.n)
+      publish<R>(s, A.exch + (size_t)((j + 1) & (kResRing - 1)) * ring + (unsigned)(sh.k.t * kSlots), lane, tag + 1);
+    return waiting;
+  }
+
+  // The state's iteration j for the tile's kind; the halo columns are in place.
+  __device__ __forceinline__ void iterate(Sh& sh, const ResArgs& A, int lane, int j, unsigned ex, uint4 wn, uint4 ws) {
+    const IterPair& P = A.P;
     const bool last = j + 1 == A.n;
     const uint2 ek = sh.k.edge[lane];
-    const ResEdge E{o.w, ek.x, ek.y};
+    const ResEdge E{ex, ek.x, ek.y};
     const int kind = sh.k.kind;
     float2* tp_out = nullptr;
     unsigned tp_rows = 0u;
@@ -875,9 +889,6 @@ struct ResWarp {
     else if (kPlain && kind == kResPlain)
       s.template iterate<kPlain ? kResPlain : kResEdge>(sh, A, lane, A.step[j], E, wn, ws, tp_out, P.s, tp_rows);
     else if constexpr (MASKED) s.template iterate<kResKeep>(sh, A, lane, A.step[j], E, wn, ws, tp_out, P.s, tp_rows);
-    if (!last)
-      publish<R>(s, A.exch + (size_t)((j + 1) & (kResRing - 1)) * ring + (unsigned)(sh.k.t * kSlots), lane, tag + 1);
-    return waiting;
   }
 
   // The rows of this lane's column that the tile owns and the iterations write (bit r), and the
@@ -926,11 +937,36 @@ constexpr int res_warps(int rows) {
   return rows <= 8 ? 16 : 12;
 }
 
+// The plain form's pixels outside the circle in tiles without a pixel to solve.
+template <class ST, int R>
+__device__ __forceinline__ void res_fill(const ResArgs& A, int warp, int lane) {
+  typedef typename Store2<ST>::T2 T2;
+  const IterPair& P = A.P;
+  const int warps = (int)blockDim.x >> 5, nw = (int)gridDim.x * warps;
+  const float2 z = make_float2(0.f, 0.f);
+  for (int k = (int)blockIdx.x * warps + warp; k < A.nfill; k += nw) {
+    const int2 f = A.fill[k];
+    const int x = f.x - 1 + lane;
+    if (lane < 1 || lane > kResCols || x >= P.w) continue;
+    for (int y = f.y; y < min(f.y + R, P.h); y++) {
+      const int pos = x + y * P.s;
+      // the buffers current after n iterations and, from two iterations on, the others
+      if ((A.n & 1) == 0 || A.n >= 2) {
+        const_cast<float*>(P.u)[pos] = 0.f;
+        const_cast<float*>(P.u_)[pos] = 0.f;
+        Store2<ST>::st2((T2*)const_cast<void*>(P.v_), pos, z);
+      }
+      P.us[pos] = 0.f;
+      P.u_s[pos] = 0.f;
+      Store2<ST>::st2((T2*)P.v_s, pos, z);
+      P.Tp[pos] = tp_math(P.a[pos], P.b[pos], P.c[pos], z);
+    }
+  }
+}
+
 template <bool MASKED, class ST, int R>
 __global__ void __launch_bounds__(32 * res_warps<ST>(R), 1) k_resident(const __grid_constant__ ResArgs A) {
-  typedef typename Store2<ST>::T2 T2;
   extern __shared__ __align__(16) unsigned char smem[];
-  const IterPair& P = A.P;
   const int warp = (int)threadIdx.x >> 5, lane = (int)threadIdx.x & 31;
   ResShared<ST, R>& sh = reinterpret_cast<ResShared<ST, R>*>(smem)[warp];
   // Tiles go round the blocks first, then the warps of a block: every SM, and every scheduler of an
@@ -940,7 +976,7 @@ __global__ void __launch_bounds__(32 * res_warps<ST>(R), 1) k_resident(const __g
 
   if (t < A.ntiles) {
     ResWarp<MASKED, ST, R> W;
-    W.load(sh, A, lane, t);
+    W.link(sh, A, lane, t, W.load(sh, A, lane, t));
     publish<R>(W.s, A.exch + (size_t)t * (64 + 2 * R), lane, epoch);  // iteration 0's input
     __syncwarp();
     bool waiting = true;
@@ -950,29 +986,7 @@ __global__ void __launch_bounds__(32 * res_warps<ST>(R), 1) k_resident(const __g
       if (j + 2 >= A.n) W.store(sh, A, lane, j + 1 == A.n);
     }
   }
-  // ---- plain form: pixels outside the circle in tiles without a pixel to solve --------------
-  if (!MASKED) {
-    const int warps = (int)blockDim.x >> 5, nw = (int)gridDim.x * warps;
-    const float2 z = make_float2(0.f, 0.f);
-    for (int k = (int)blockIdx.x * warps + warp; k < A.nfill; k += nw) {
-      const int2 f = A.fill[k];
-      const int x = f.x - 1 + lane;
-      if (lane < 1 || lane > kResCols || x >= P.w) continue;
-      for (int y = f.y; y < min(f.y + R, P.h); y++) {
-        const int pos = x + y * P.s;
-        // the buffers current after n iterations and, from two iterations on, the others
-        if ((A.n & 1) == 0 || A.n >= 2) {
-          const_cast<float*>(P.u)[pos] = 0.f;
-          const_cast<float*>(P.u_)[pos] = 0.f;
-          Store2<ST>::st2((T2*)const_cast<void*>(P.v_), pos, z);
-        }
-        P.us[pos] = 0.f;
-        P.u_s[pos] = 0.f;
-        Store2<ST>::st2((T2*)P.v_s, pos, z);
-        P.Tp[pos] = tp_math(P.a[pos], P.b[pos], P.c[pos], z);
-      }
-    }
-  }
+  if (!MASKED) res_fill<ST, R>(A, warp, lane);
   // ---- the last block to end renews the epoch: every block has read it by then --------------
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -982,6 +996,181 @@ __global__ void __launch_bounds__(32 * res_warps<ST>(R), 1) k_resident(const __g
       A.ctl->epoch += 1;
     }
   }
+}
+
+// ---- small levels: the tiles of one cluster ---------------------------------------------------
+// A level of few tiles (res_cluster_tiles) runs on the blocks of one thread-block cluster, whose
+// warps store their border straight into their neighbours' shared memory (st.async through
+// distributed shared memory, counted on the neighbour's mbarrier).  A level that small is all
+// latency: a tile computes for 650 cycles, the way through L2 takes another 1100 to 1500, this one
+// about half of that (53 x 50: 1.39 -> 0.90 us per iteration).  Two inboxes, by parity of the
+// iteration, for the reason the ring has two.
+namespace {
+
+constexpr int kResMaxWaits = 1 << 20;
+
+template <class ST>
+struct ResWord;  // u-bar and v-bar of a border pixel
+template <>
+struct ResWord<__half> {
+  typedef uint2 T;
+  static __device__ __forceinline__ uint2 of(uint4 w) { return make_uint2(w.x, w.y); }
+  static __device__ __forceinline__ uint4 wide(uint2 w) { return make_uint4(w.x, w.y, 0u, 0u); }
+};
+template <>
+struct ResWord<float> {
+  typedef uint4 T;
+  static __device__ __forceinline__ uint4 of(uint4 w) { return w; }
+  static __device__ __forceinline__ uint4 wide(uint4 w) { return w; }
+};
+
+template <class ST, int R>
+struct ResInbox {
+  typename ResWord<ST>::T n[32], s[32], c[2][R];  // the rows above and below, the west and east column
+};
+template <class ST, int R>
+struct ResClusterTile {
+  ResShared<ST, R> sh;
+  ResInbox<ST, R> in[2];
+  // per lane, for slot 0, address and barrier of (its words in the tile below, in the tile above),
+  // (in the two diagonal tiles of its side below, above), (in the tile beside); 0: no such tile
+  uint4 row[32], diag[32];
+  uint2 side[32];
+  unsigned long long bar[2];
+  int bytes;  // that arrive in an inbox per iteration
+  int pad[3];
+};
+
+__device__ __forceinline__ unsigned cl_rank() {
+  unsigned r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void cl_barrier() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ unsigned cl_addr(unsigned local, unsigned rank) {
+  unsigned r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(local), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ void st_async(unsigned to, unsigned bar, uint2 v) {
+  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.b32 [%0], {%1, %2}, [%3];" ::"r"(to), "r"(v.x),
+               "r"(v.y), "r"(bar)
+               : "memory");
+}
+__device__ __forceinline__ void st_async(unsigned to, unsigned bar, uint4 v) {
+  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(to),
+               "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w), "r"(bar)
+               : "memory");
+}
+__device__ __forceinline__ void bar_arm(unsigned bar, int bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.release.cta.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ bool bar_wait(unsigned bar, unsigned parity) {
+  unsigned ok;
+  asm volatile(
+      "{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2, %3;\n selp.u32 %0, 1, 0, p;\n}\n"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity), "r"(1000)  // suspended for a microsecond at most
+      : "memory");
+  return ok != 0;
+}
+
+// A tile's border after k iterations into its neighbours' inboxes.
+template <class ST, int R, class State>
+__device__ __forceinline__ void push(const State& s, const ResClusterTile<ST, R>& C, int lane, int k) {
+  typedef ResWord<ST> Word;
+  const unsigned in = (k & 1) * (unsigned)sizeof(ResInbox<ST, R>), bar = (k & 1) * 8u;
+  const auto top = Word::of(s.word(0, 0u)), bottom = Word::of(s.word(R - 1, 0u));
+  const uint4 row = C.row[lane], diag = C.diag[lane];
+  const uint2 side = C.side[lane];
+  if (row.x) st_async(row.x + in, row.y + bar, bottom);
+  if (row.z) st_async(row.z + in, row.w + bar, top);
+  if (diag.x) st_async(diag.x + in, diag.y + bar, bottom);
+  if (diag.z) st_async(diag.z + in, diag.w + bar, top);
+  if (side.x) {
+#pragma unroll
+    for (int r = 0; r < R; r++)
+      st_async(side.x + in + r * (unsigned)sizeof(typename Word::T), side.y + bar, Word::of(s.word(r, 0u)));
+  }
+}
+
+}  // namespace
+
+template <bool MASKED, class ST, int R>
+__global__ void __launch_bounds__(512, 1) k_resident_cluster(const __grid_constant__ ResArgs A) {
+  typedef ResWord<ST> Word;
+  typedef ResClusterTile<ST, R> Tile;
+  extern __shared__ __align__(16) unsigned char smem[];
+  const int warp = (int)threadIdx.x >> 5, lane = (int)threadIdx.x & 31, ctas = (int)gridDim.x;
+  Tile& C = reinterpret_cast<Tile*>(smem)[warp];
+  ResShared<ST, R>& sh = C.sh;
+  const int t = (int)cl_rank() + ctas * warp;  // this warp's tile, placed as in k_resident
+  const unsigned bar = (unsigned)__cvta_generic_to_shared(&C.bar[0]);
+  ResWarp<MASKED, ST, R> W;
+  unsigned ex = 0;
+  if (t < A.ntiles) {
+    const ResTile& T = A.tiles[t];
+    ex = W.load(sh, A, lane, t).x;
+    auto words = [&](int k, const void* field) {  // the same field of tile k's shared memory
+      const unsigned local = (unsigned)__cvta_generic_to_shared(field) + (unsigned)((k / ctas - warp) * (int)sizeof(Tile));
+      return cl_addr(local, (unsigned)(k % ctas));
+    };
+    auto there = [&](int d) { return T.nb[d] != t; };
+    const bool own = lane >= 1 && lane <= kResCols, west = lane == 1, end = west || lane == kResCols;
+    uint4 row = make_uint4(0u, 0u, 0u, 0u), diag = row;
+    uint2 side = make_uint2(0u, 0u);
+    if (own && there(1)) row.x = words(T.nb[1], &C.in[0].n[lane]), row.y = words(T.nb[1], &C.bar[0]);
+    if (own && there(0)) row.z = words(T.nb[0], &C.in[0].s[lane]), row.w = words(T.nb[0], &C.bar[0]);
+    // this tile's first column is the east halo of the tiles west of it, its last the west halo of
+    // those east of it
+    const int sw = west ? 6 : 7, nw = west ? 4 : 5, w = west ? 2 : 3, at = west ? 31 : 0;
+    if (end && there(sw)) diag.x = words(T.nb[sw], &C.in[0].n[at]), diag.y = words(T.nb[sw], &C.bar[0]);
+    if (end && there(nw)) diag.z = words(T.nb[nw], &C.in[0].s[at]), diag.w = words(T.nb[nw], &C.bar[0]);
+    if (end && there(w)) side = make_uint2(words(T.nb[w], &C.in[0].c[west ? 1 : 0][0]), words(T.nb[w], &C.bar[0]));
+    C.row[lane] = row;
+    C.diag[lane] = diag;
+    C.side[lane] = side;
+    // what no neighbour fills stays zero
+    for (int k = 0; k < 2; k++) {
+      C.in[k].n[lane] = C.in[k].s[lane] = Word::of(make_uint4(0u, 0u, 0u, 0u));
+      if (lane < 2 * R) C.in[k].c[lane / R][lane % R] = Word::of(make_uint4(0u, 0u, 0u, 0u));
+    }
+    if (lane == 0) {
+      C.bytes = (int)sizeof(typename Word::T) * (kResCols * (there(0) + there(1)) + R * (there(2) + there(3)) + there(4) +
+                                                 there(5) + there(6) + there(7));
+      for (int k = 0; k < 2; k++) {
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar + 8u * k) : "memory");
+      }
+      asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+      for (int k = 0; k < 2; k++) bar_arm(bar + 8u * k, C.bytes);
+    }
+  }
+  cl_barrier();  // every inbox is ready
+  if (t < A.ntiles) {
+    push<ST, R>(W.s, C, lane, 0);  // iteration 0's input
+    bool waiting = true;
+#pragma unroll 1
+    for (int j = 0; j < A.n; j++) {
+      const int k = j & 1;
+      for (int waits = 0; waiting && !bar_wait(bar + 8u * k, (unsigned)(j >> 1) & 1u); waits++)
+        if (waits >= kResMaxWaits) {
+          waiting = false;
+          g_res_status = 1;
+        }
+      __syncwarp();
+      const uint4 wn = Word::wide(C.in[k].n[lane]), ws = Word::wide(C.in[k].s[lane]);
+      if (lane == 0 || lane == 31) W.s.take_col(C.in[k].c[lane >> 4]);
+      __syncwarp();
+      if (lane == 0 && j + 2 < A.n) bar_arm(bar + 8u * k, C.bytes);  // for iteration j + 2
+      W.iterate(sh, A, lane, j, ex, wn, ws);
+      if (j + 1 < A.n) push<ST, R>(W.s, C, lane, j + 1);
+      if (j + 2 >= A.n) W.store(sh, A, lane, j + 1 == A.n);
+    }
+  }
+  if (!MASKED) res_fill<ST, R>(A, warp, lane);
+  cl_barrier();  // no block leaves while its neighbours may store into it
 }
 
 namespace {
@@ -1001,6 +1190,48 @@ struct Res {
     VFS_CUDA(cudaFuncSetAttribute(k_resident<MASKED, ST, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem));
     VFS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_resident<MASKED, ST, R>, kThreads, kSmem));
     return per >= 1 ? sms * res_warps<ST>(R) : 0;
+  }
+  // warps the tiles of which one cluster of `ctas` blocks holds (0: no such cluster)
+  static int cluster_capacity(int ctas) {
+    if constexpr (R == kResClusterRows) {
+      const auto k = k_resident_cluster<MASKED, ST, R>;
+      const size_t bytes = sizeof(ResClusterTile<ST, R>) * 16;
+      int dev = 0, smem = 0, n = 0;
+      VFS_CUDA(cudaGetDevice(&dev));
+      VFS_CUDA(cudaDeviceGetAttribute(&smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+      if (bytes > (size_t)smem) return 0;
+      VFS_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+      VFS_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+      cudaLaunchAttribute at[1];
+      cudaLaunchConfig_t cfg = cluster_config(ctas, 16, 0, at);
+      if (cudaOccupancyMaxActiveClusters(&n, k, &cfg) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return 0;
+      }
+      return n >= 1 ? ctas * 16 : 0;
+    }
+    return 0;
+  }
+  static cudaLaunchConfig_t cluster_config(int ctas, int warps, cudaStream_t st, cudaLaunchAttribute* at) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(ctas);
+    cfg.blockDim = dim3(32 * warps);
+    cfg.dynamicSmemBytes = sizeof(ResClusterTile<ST, R>) * warps;
+    cfg.stream = st;
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = ctas;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cfg;
+  }
+  static int launch_cluster(const ResArgs& A, cudaStream_t st) {
+    if constexpr (R == kResClusterRows) {
+      cudaLaunchAttribute at[1];
+      cudaLaunchConfig_t cfg = cluster_config(A.blocks, (A.ntiles + A.blocks - 1) / A.blocks, st, at);
+      VFS_CUDA(cudaLaunchKernelEx(&cfg, k_resident_cluster<MASKED, ST, R>, A));
+    }
+    return 0;
   }
   static int launch(const ResArgs& A, cudaStream_t st) {
     // only the warps that have a tile: blocks of other pairs' levels share the SM
@@ -1040,16 +1271,18 @@ int res_dispatch(bool masked, bool half, int rows, F&& f) {
 
 }  // namespace
 
-int res_capacity(bool masked, bool half, int rows) {
+int res_capacity(bool masked, bool half, int rows, int cluster) {
   int dev = 0;
   VFS_CUDA(cudaGetDevice(&dev));
   static std::mutex mu;
-  static std::map<std::tuple<int, bool, bool, int>, int> known;
+  static std::map<std::tuple<int, bool, bool, int, int>, int> known;
   std::lock_guard<std::mutex> lk(mu);
-  const auto key = std::make_tuple(dev, masked, half, rows);
+  const auto key = std::make_tuple(dev, masked, half, rows, cluster);
   auto it = known.find(key);
   if (it != known.end()) return it->second;
-  return known[key] = res_dispatch(masked, half, rows, [](auto k) { return decltype(k)::capacity(); });
+  return known[key] = res_dispatch(masked, half, rows, [cluster](auto k) {
+           return cluster ? decltype(k)::cluster_capacity(cluster) : decltype(k)::capacity();
+         });
 }
 
 void launch_resident(const ResArgs& A, bool masked, bool half, cudaStream_t st) {
@@ -1057,9 +1290,12 @@ void launch_resident(const ResArgs& A, bool masked, bool half, cudaStream_t st) 
   int dev = 0, sms = 0;
   VFS_CUDA(cudaGetDevice(&dev));
   VFS_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  const int per_sm = res_capacity(masked, half, A.rows) / sms;  // warps of a block
-  if (A.blocks > sms || A.ntiles > A.blocks * per_sm) throw ArgError{"resident iteration: more tiles than can be resident"};
-  res_dispatch(masked, half, A.rows, [&](auto k) { return decltype(k)::launch(A, st); });
+  const int cap = res_capacity(masked, half, A.rows, A.cluster ? A.blocks : 0);
+  if (A.cluster ? A.ntiles > cap : A.blocks > sms || A.ntiles > A.blocks * (cap / sms))
+    throw ArgError{"resident iteration: more tiles than can be resident"};
+  res_dispatch(masked, half, A.rows, [&](auto k) {
+    return A.cluster ? decltype(k)::launch_cluster(A, st) : decltype(k)::launch(A, st);
+  });
   VFS_LAUNCH_CHECK();
 }
 

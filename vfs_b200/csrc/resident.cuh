@@ -1,6 +1,6 @@
 // Register-resident form of the fused primal-dual iteration: all iterations of one warp of a
-// pyramid level in one cooperative launch, the level's state held in registers and shared
-// memory of the whole GPU (one pair per launch).
+// pyramid level in one launch, the level's state held in registers and shared memory of the
+// whole GPU or, where it is small, of one thread-block cluster (one pair per launch).
 //
 // A level is cut into tiles of 30 x R pixels, one warp each; only tiles that hold a pixel that
 // is on (or that such a pixel reads) exist.  Lane k of a warp is image column x0 - 1 + k: lanes
@@ -21,21 +21,23 @@
 // all its neighbours knows that each of them has finished k - 1, and so has read this tile's
 // words of k - 1, before it overwrites them with those of k + 1.
 //
-// The grid is launched cooperatively, so that all its blocks are resident and every wait ends;
-// a wait is bounded all the same (a warp that gives up records it, stops waiting and runs on).
+// The grid is launched cooperatively (or is one cluster), so that all its blocks are resident and
+// every wait ends; a wait is bounded all the same (a warp that gives up records it, stops waiting
+// and runs on).
 //
 // The arithmetic is that of k_fused_iter (tgv_pixel.cuh, tgv_pixel_fast.cuh) with the same
 // storage rounding, so the results are bit-identical to one launch per iteration, the values
 // that the other ping-pong buffers hold included (the state before the last iteration is
 // written there).
 //
-// What bounds it, on B200 (FP16 storage, 848 x 800, 2037 tiles of 8 rows, 4.2 us per iteration):
+// What bounds it, on B200 (FP16 storage, 848 x 800, 2037 tiles of 8 rows, 3.9 us per iteration):
 // about half of an iteration is instruction issue (1060 instructions per tile, 3.4 warps per
-// scheduler, close to one per cycle), the rest the exchange: about 1500 cycles from a
+// scheduler, close to one per cycle), the rest the exchange: 1100 to 1500 cycles from a
 // store to the load that sees it, and the wait for the slowest neighbour.  One launch per iteration
-// (k_fused_iter) takes 8.0 us there alone, bound by its loads; float storage 7.9 against 10.3 us.
-// Small levels are all latency: 53 x 50 takes 1.33 us (one launch per iteration 3.2 us, the
-// cluster-resident form 1.54 us).
+// (k_fused_iter) takes 8.0 us there alone, bound by its loads; float storage 6.2 against 10.3 us.
+// Small levels are all latency, so theirs runs in one cluster whose blocks write into each other's
+// shared memory (k_resident_cluster): 53 x 50 takes 0.90 us, through L2 1.39, one launch per
+// iteration 3.2.
 #pragma once
 #include <vector>
 
@@ -51,6 +53,14 @@ constexpr int kResMaxIters = 128;  // iterations per launch
 constexpr int kResRows[] = {2, 4, 6, 8, 12};
 constexpr int kResNumRows = 5;
 constexpr int kResMostTiles = 148 * 16;  // a bound on the tiles of a plan (one warp each)
+// The cluster form (kernels_resident.cu, k_resident_cluster): 16 blocks, tiles of two rows, for levels of
+// up to so many tiles.  Beyond, the 16 SMs have more to issue than the shorter exchange saves (us per
+// iteration, cluster / whole GPU: half storage 50 tiles 0.90 / 1.39, 128 1.02 / 1.38, 200 1.19 / 1.44,
+// 230 1.39 / 1.42; float 50 1.18 / 1.70, 128 1.46 / 1.7, 200 1.76 / 1.75, 230 2.06 / 1.75; tiles of four
+// rows, 160 of them, 1.62 / 1.42 and 2.57 / 1.75).
+constexpr int kResClusterRows = 2;
+constexpr int kResClusterCtas = 16;
+inline int res_cluster_tiles(bool half) { return half ? 208 : 128; }
 inline int res_slots(int rows) { return 64 + 2 * rows; }  // words per tile: top, bottom, left, right
 
 // What a tile's pixels ask of its iterations: none of the edge rules; the edge rules; or
@@ -87,6 +97,7 @@ struct ResArgs {
   int n;                 // iterations (1 .. kResMaxIters)
   int p_planes;          // p and q have two planes (result in plane n & 1); else one
   int rows, blocks;      // tile height, blocks of the grid
+  bool cluster;          // the grid is one thread-block cluster
   float2 minus_zero;     // -0, where the compiler does not see it
   ResStep step[kResMaxIters];
 };
@@ -94,6 +105,7 @@ struct ResArgs {
 // A level's tiles (host side).
 struct ResTiles {
   int rows = 0, blocks = 0;
+  bool cluster = false;  // the blocks are one thread-block cluster
   // Renumbers the tiles for a grid of `blocks` (tile t: warp t / blocks of block t % blocks) so that
   // those with edge rules sit on the schedulers (warp % 4) that have the fewest tiles.
   void place(int blocks);
@@ -123,6 +135,7 @@ size_t res_bytes_bound(int w, int h);
 
 // A level's plan on the device.
 struct ResPlan {
+  bool cluster = false;
   int rows = 0, blocks = 0, ntiles = 0, nfill = 0;  // ntiles = 0: the level has no plan
   const ResTile* tiles = nullptr;
   const int2* fill = nullptr;
@@ -130,8 +143,9 @@ struct ResPlan {
   ResCtl* ctl = nullptr;
 };
 
-// most tiles an instance holds with its whole grid resident (0: not available)
-int res_capacity(bool masked, bool half, int rows);
+// most tiles an instance holds with its whole grid (cluster > 0: one cluster of that many blocks)
+// resident; 0: not available
+int res_capacity(bool masked, bool half, int rows, int cluster = 0);
 void launch_resident(const ResArgs& A, bool masked, bool half, cudaStream_t st);
 // reads and clears the device status (1: a bounded wait ran out)
 int resident_status_take();

@@ -128,7 +128,7 @@ void ResTiles::place(int grid) {
   const int n = (int)tiles.size();
   // tiles per scheduler of a block that has all its warps, or one less
   auto load = [&](int t) {
-    const int b = t % grid, warps = (n - b + grid - 1) / grid, w = t / grid;
+    const int b = t % grid, warps = std::max(1, (n - b + grid - 1) / grid), w = t / grid;
     return (warps - w % 4 + 3) / 4;
   };
   std::vector<int> slot(n), tile(n), to(n);
@@ -147,7 +147,7 @@ void ResTiles::place(int grid) {
 
 // The smallest tile height whose tiles fit, since more warps with less to do each hide more of one
 // another's latency and shorten an iteration (B200, us per iteration, FP16 / float storage: 848 x 800
-// disc 8 rows 4.2 / 7.9; 640 x 480 4 rows 2.45 / 3.5, 6 rows 2.75 / 3.9, 8 rows 3.1 / 5.3; 212 x 200
+// disc 8 rows 3.9 / 6.2; 640 x 480 4 rows 2.45 / 3.5, 6 rows 2.75 / 3.9, 8 rows 3.1 / 5.3; 212 x 200
 // 2 rows 1.40 / 1.73, 4 rows 1.60 / 2.15).  Two rows are left to levels that fill at most three
 // quarters of the warps: fuller, the row above each tile, which two rows pay for as much as four,
 // costs more than it gives (424 x 400, 91 %: 2 rows 2.0, 4 rows 1.87).
@@ -157,6 +157,14 @@ bool res_choose(const uint8_t* code, int w, int h, bool masked, bool half, ResTi
   VFS_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   ResLevel L;
   if (!L.scan(code, w, h, masked)) return false;
+  out.cluster = false;
+  if (const int n = L.count(kResClusterRows);
+      n <= std::min(res_cluster_tiles(half), res_capacity(masked, half, kResClusterRows, kResClusterCtas))) {
+    L.tiles(kResClusterRows, out);
+    out.cluster = true;
+    out.place(kResClusterCtas);
+    return true;
+  }
   for (int k = 0; k < kResNumRows; k++) {
     const int rows = kResRows[k];
     const int cap = res_capacity(masked, half, rows), n = L.count(rows);

@@ -554,6 +554,7 @@ void StereoTgvImpl::ensureResident(bool masked, bool half, cudaStream_t st) {
     if (!res_choose(host_code[masked][l].data(), pW[l], pH[l], masked, half, cut[l])) continue;
     plans[l].rows = cut[l].rows;
     plans[l].blocks = cut[l].blocks;
+    plans[l].cluster = cut[l].cluster;
     plans[l].ntiles = (int)cut[l].tiles.size();
     plans[l].nfill = (int)cut[l].fill.size();
     off[l].ctl = take(sizeof(ResCtl));
