@@ -118,6 +118,18 @@ def test_zero_and_extreme_preconditioners(gpu, half):
         _same(case, params(n_levels=1, n_warp=1, n_iter=4, **kw), half, True)
 
 
+@pytest.mark.parametrize("half", [False, True], ids=["fp32", "fp16"])
+@pytest.mark.parametrize("masked", [True, False], ids=["masked", "plain"])
+def test_values_whose_squares_overflow(gpu, masked, half):
+    """Images with a patch of 1e24, infinities and NaN: dual variables whose norm overflows."""
+    i0, i1, mask, tv, cv = random_case(130, 66, seed=13)
+    for v in (1e24, np.inf, np.nan):
+        a, b = i0.astype(np.float32) / 255, i1.astype(np.float32) / 255
+        a[20:24, 40:52] = v
+        b[40:41, 80:83] = v
+        _same((a, b, mask, tv, cv), params(n_levels=1, n_warp=2, n_iter=6), half, masked)
+
+
 def test_exact_quotients_and_roots(gpu, tmp_path):
     """Every significand of a divisor and every m in [1, 4) (and scaled by 2^26), and 10^9 random
     quotients, against the device's IEEE division and square root."""

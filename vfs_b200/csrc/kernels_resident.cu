@@ -407,6 +407,12 @@ struct ResState<MASKED, float, R> {
     sh.qtop[lane] = z;
     sh.ptop[lane] = make_float2(0.f, 0.f);
   }
+  // What keeps the squared norms finite, which the exact roots ask for: a level's values are at most
+  // kMost before the first iteration, an iteration moves them by kRate at most (tau <= 1: the host
+  // sees to it), so that after kResMaxIters they are below 2^30, and a dual step adds below 2^60
+  // (sigma <= 2^14).  A pixel beyond any of it asks for the plain operators.
+  static constexpr float kMost = 0x1p24f, kMostTp = 16.0f, kRate = 0x1p20f;
+  static __device__ __forceinline__ bool beyond(float v) { return !(fabsf(v) <= kMost); }
   // in the range of the exact quotients
   static __device__ __forceinline__ bool ranged(float b) { return fabsf(b) >= 0x1p-100f && fabsf(b) <= 0x1p100f; }
   // returns whether the pixel asks for the plain operators
@@ -421,14 +427,19 @@ struct ResState<MASKED, float, R> {
     bool plain = false;
     if (in && r >= 0 && (code & kOn)) {
       const float eu = etau_math(a, b, c, P.alpha1), iu = P.Iu[pos];
-      plain = !((eu == 0.0f || ranged(eu)) && ranged(etav1_math(b, c, P.alpha0, P.alpha1)) && ranged(etav2_math(a, c, P.alpha0, P.alpha1)) &&
-                (iu == 0.0f || ranged(iu)));
+      const float e1 = etav1_math(b, c, P.alpha0, P.alpha1), e2 = etav2_math(a, c, P.alpha0, P.alpha1);
+      plain = !((eu == 0.0f || ranged(eu)) && ranged(e1) && ranged(e2) && (iu == 0.0f || ranged(iu)));
+      const float m = fmaxf(fmaxf(fabsf(a), fabsf(b)), fabsf(c)), eu1 = eu == 0.0f ? 1.0f : eu;
+      const float gv = fabsf(P.alpha1) * m + 4.0f * fabsf(P.alpha0);
+      plain = plain || !(m <= 0x1p8f && gv <= 0x1p14f && P.lambda * fabsf(iu) <= kRate * eu1 &&
+                         4.0f * fmaxf(m, kMostTp) <= kRate * eu1 && gv <= kRate * e1 && gv <= kRate * e2);
     }
     if (MASKED && in && !(code & kOn)) {
       // read by the right / lower neighbour only where that one's other side is off too
       const float2 tp = P.Tp[pos];
       a = (east & kOn) && !(east & kR) ? tp.x : 0.f;
       b = (south & kOn) && !(south & kD) ? tp.y : 0.f;
+      plain = plain || !(fabsf(a) <= kMostTp) || !(fabsf(b) <= kMostTp);
     }
     if (r < 0) {
       sh.top[lane] = make_float4(a, b, c, 0.f);
@@ -441,9 +452,11 @@ struct ResState<MASKED, float, R> {
     el(sh.ci[i][lane], 2 + k) = in ? P.Iu[pos] : 0.f;
     reinterpret_cast<float*>(&sh.iz[i][lane])[k] = in ? P.Iz[pos] : 0.f;
     float un = in ? P.u[pos] : 0.f, ubn = in ? P.u_[pos] : 0.f;
+    plain = plain || beyond(un) || beyond(ubn);
     if (MASKED && in && !(code & kOn)) {  // the other ping-pong values of a masked-out pixel
       un = P.u_s[pos];
       const float2 o = ((const float2*)P.v_s)[pos];
+      plain = plain || beyond(un) || beyond(o.x) || beyond(o.y);
       el(sh.p[i][lane], k) = o.x;
       el(sh.p[i][lane], 2 + k) = o.y;
     }
@@ -835,6 +848,15 @@ struct ResWarp {
     __syncwarp();
   }
 
+  // A tile on the plain operators marks its words, and who takes a marked word changes to them as
+  // well: values beyond the exact roots' range travel no faster than the words.
+  __device__ __forceinline__ unsigned flag(const Sh& sh) const {
+    return kPlain && sh.k.kind == kResPlain ? kResBeyond : 0u;
+  }
+  __device__ __forceinline__ void meet(Sh& sh, unsigned marks) {
+    if (marks & kResBeyond) sh.k.kind = kResPlain;
+  }
+
   // One iteration.  Returns false once a wait ran out.
   __device__ __forceinline__ bool step(Sh& sh, const ResArgs& A, int lane, int j,
                                        unsigned epoch, bool waiting) {
@@ -852,7 +874,8 @@ struct ResWarp {
       wn = ld_word(base + o.x);
       ws = ld_word(base + o.y);
       wc = ld_word(base + o.z);
-      if (__all_sync(kFull, wn.w == tag && ws.w == tag && wc.w == tag) || !waiting) break;
+      const unsigned other = (wn.w ^ tag) | (ws.w ^ tag) | (wc.w ^ tag);
+      if (__all_sync(kFull, (kPlain ? other & ~kResBeyond : other) == 0) || !waiting) break;
       if (polls >= kResMaxPolls) {
         waiting = false;
         if (lane == 0) g_res_status = 1;
@@ -861,12 +884,14 @@ struct ResWarp {
     }
     const int side = lane >> 4, row = lane & 15;
     if (row < R) s.put_col(sh, side, row, wc);
+    if (kPlain) meet(sh, wn.w | ws.w | wc.w);
     __syncwarp();
     if (lane == 0 || lane == 31) s.take_col(sh.col[side]);
     __syncwarp();
     iterate(sh, A, lane, j, o.w, wn, ws);
     if (j + 1 < A.n)
-      publish<R>(s, A.exch + (size_t)((j + 1) & (kResRing - 1)) * ring + (unsigned)(sh.k.t * kSlots), lane, tag + 1);
+      publish<R>(s, A.exch + (size_t)((j + 1) & (kResRing - 1)) * ring + (unsigned)(sh.k.t * kSlots), lane,
+                 (tag + 1) | flag(sh));
     return waiting;
   }
 
@@ -977,7 +1002,7 @@ __global__ void __launch_bounds__(32 * res_warps<ST>(R), 1) k_resident(const __g
   if (t < A.ntiles) {
     ResWarp<MASKED, ST, R> W;
     W.link(sh, A, lane, t, W.load(sh, A, lane, t));
-    publish<R>(W.s, A.exch + (size_t)t * (64 + 2 * R), lane, epoch);  // iteration 0's input
+    publish<R>(W.s, A.exch + (size_t)t * (64 + 2 * R), lane, epoch | W.flag(sh));  // iteration 0's input
     __syncwarp();
     bool waiting = true;
 #pragma unroll 1
@@ -1079,10 +1104,10 @@ __device__ __forceinline__ bool bar_wait(unsigned bar, unsigned parity) {
 
 // A tile's border after k iterations into its neighbours' inboxes.
 template <class ST, int R, class State>
-__device__ __forceinline__ void push(const State& s, const ResClusterTile<ST, R>& C, int lane, int k) {
+__device__ __forceinline__ void push(const State& s, const ResClusterTile<ST, R>& C, int lane, int k, unsigned flag) {
   typedef ResWord<ST> Word;
   const unsigned in = (k & 1) * (unsigned)sizeof(ResInbox<ST, R>), bar = (k & 1) * 8u;
-  const auto top = Word::of(s.word(0, 0u)), bottom = Word::of(s.word(R - 1, 0u));
+  const auto top = Word::of(s.word(0, flag)), bottom = Word::of(s.word(R - 1, flag));
   const uint4 row = C.row[lane], diag = C.diag[lane];
   const uint2 side = C.side[lane];
   if (row.x) st_async(row.x + in, row.y + bar, bottom);
@@ -1092,7 +1117,7 @@ __device__ __forceinline__ void push(const State& s, const ResClusterTile<ST, R>
   if (side.x) {
 #pragma unroll
     for (int r = 0; r < R; r++)
-      st_async(side.x + in + r * (unsigned)sizeof(typename Word::T), side.y + bar, Word::of(s.word(r, 0u)));
+      st_async(side.x + in + r * (unsigned)sizeof(typename Word::T), side.y + bar, Word::of(s.word(r, flag)));
   }
 }
 
@@ -1149,7 +1174,7 @@ __global__ void __launch_bounds__(512, 1) k_resident_cluster(const __grid_consta
   }
   cl_barrier();  // every inbox is ready
   if (t < A.ntiles) {
-    push<ST, R>(W.s, C, lane, 0);  // iteration 0's input
+    push<ST, R>(W.s, C, lane, 0, W.flag(sh));  // iteration 0's input
     bool waiting = true;
 #pragma unroll 1
     for (int j = 0; j < A.n; j++) {
@@ -1162,10 +1187,11 @@ __global__ void __launch_bounds__(512, 1) k_resident_cluster(const __grid_consta
       __syncwarp();
       const uint4 wn = Word::wide(C.in[k].n[lane]), ws = Word::wide(C.in[k].s[lane]);
       if (lane == 0 || lane == 31) W.s.take_col(C.in[k].c[lane >> 4]);
+      if constexpr (W.kPlain) W.meet(sh, wn.w | ws.w | C.in[k].c[lane >> 4][lane & (R - 1)].w);
       __syncwarp();
       if (lane == 0 && j + 2 < A.n) bar_arm(bar + 8u * k, C.bytes);  // for iteration j + 2
       W.iterate(sh, A, lane, j, ex, wn, ws);
-      if (j + 1 < A.n) push<ST, R>(W.s, C, lane, j + 1);
+      if (j + 1 < A.n) push<ST, R>(W.s, C, lane, j + 1, W.flag(sh));
       if (j + 2 >= A.n) W.store(sh, A, lane, j + 1 == A.n);
     }
   }

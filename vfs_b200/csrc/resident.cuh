@@ -48,7 +48,7 @@ namespace vfs {
 
 constexpr int kResCols = 30;       // owned columns per tile
 constexpr int kResRing = 2;        // iterations of exchange words kept
-constexpr int kResMaxIters = 128;  // iterations per launch
+constexpr int kResMaxIters = 128;  // iterations per launch (a tag's low seven bits)
 // tile heights the kernel is built for (float storage: those up to 8)
 constexpr int kResRows[] = {2, 4, 6, 8, 12};
 constexpr int kResNumRows = 5;
@@ -68,6 +68,7 @@ inline int res_slots(int rows) { return 64 + 2 * rows; }  // words per tile: top
 // right nor its left, or neither its lower nor its upper, neighbour).
 // kResPlain (found by the kernel): as kResKeep, with the plain division and square root.
 enum ResKind { kResInner = 0, kResEdge = 1, kResKeep = 2, kResPlain = 3 };
+constexpr unsigned kResBeyond = 0x80u;  // in a word's tag (epoch << 8 | iteration): from a kResPlain tile
 
 struct ResTile {
   int x0, y0;   // first owned column and row

@@ -531,11 +531,11 @@ void StereoTgvImpl::ensureResident(bool masked, bool half, cudaStream_t st) {
   if (!plans.empty()) return;
   plans.assign(levels(), ResPlan{});
   if (P.nSolverIters < 1 || P.nSolverIters > kResMaxIters || !(P.lambda >= 0.0f)) return;
-  // its quotients take step sizes in a range that no sane schedule leaves
+  // its quotients and roots take step sizes in a range that no sane schedule leaves
   float tau = 1.0f, sigma = 1.0f;
   for (int j = 0; j < P.nSolverIters; j++) {
     const float mu = sigma < 1000.0f ? 1.0f / std::sqrt(1 + 0.7f * tau * P.timestep_lambda) : 1.0f;
-    if (!(tau >= 0x1p-60f && tau <= 0x1p60f)) return;
+    if (!(tau >= 0x1p-60f && tau <= 1.0f && sigma <= 0x1p14f && mu > 0.0f && mu <= 1.0f)) return;
     sigma = sigma / mu;
     tau = tau * mu;
   }

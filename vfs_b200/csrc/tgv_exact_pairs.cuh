@@ -31,7 +31,7 @@ __device__ __forceinline__ x2::f2 quot(x2::f2 a, x2::f2 b, x2::f2 y) {
   const x2::f2 q = x2::mul(a, y);
   return x2::fma(x2::fma(neg(b), q, a), y, q);
 }
-// s = sqrt(m) and 1 / s for m >= 1
+// s = sqrt(m) and 1 / s for 1 <= m < infinity (a NaN stays)
 __device__ __forceinline__ void root(x2::f2 m, x2::f2& s, x2::f2& y) {
   using namespace x2;
   const float2 v = upk(m);
@@ -42,7 +42,6 @@ __device__ __forceinline__ void root(x2::f2 m, x2::f2& s, x2::f2& y) {
   s = fma(fma(neg(g1), g1, m), h1, g1);
   y = recip(s);
 }
-
 
 }  // namespace exact
 }  // namespace vfs

@@ -233,82 +233,9 @@ __device__ __forceinline__ void primal(float4 qc, float4 ql, float4 qu, float2 t
   primal_r(qc, ql, qu, tpp, etav_rcp(ev1, ev2), tau, alpha0, alpha1, mu, vb, u_new, u_bar, u_s, v_s);
 }
 
-// ---- the same steps without branches, for kernels that keep several rows of a warp in one
-// straight run of instructions (a branch per row would end every scheduling block there).
-// Each select picks the value the branch would have produced, so the bits are the same.
-
-// 1 where |.|^2 = n2 is at most 1, else 1 / |.|: multiplying by 1 is exact
+// The projection's factor without a branch, for kernels that keep several rows of a warp in one
+// straight run of instructions: 1 where |.|^2 = n2 is at most 1 (multiplying by 1 is exact), else 1 / |.|.
 __device__ __forceinline__ float unit_scale(float n2) { return n2 <= 1.0f ? 1.0f : rsqrt(n2); }
-
-__device__ __forceinline__ void project(x2::f2 pp, x2::f2 qxw, x2::f2 qzy, float2& p, float4& q) {
-  using namespace x2;
-  const float2 a = upk(pp);
-  const float rp = unit_scale(__fmaf_rn(a.x, a.x, a.y * a.y));
-  p = upk(mul(pp, pk(rp, rp)));
-  const float2 xw = upk(qxw), zy = upk(qzy);
-  const float rq = unit_scale(__fmaf_rn(xw.x, xw.x, __fmaf_rn(zy.y, zy.y, __fmaf_rn(zy.x, zy.x, xw.y * xw.y))));
-  const f2 r2 = pk(rq, rq);
-  const float2 o = upk(mul(qxw, r2)), t = upk(mul(qzy, r2));
-  q = make_float4(o.x, t.y, t.x, o.y);
-}
-
-__device__ __forceinline__ void dual_interior_flat(float u_pos, float u_xn, float u_yn, float2 vp, float2 v_xn,
-                                                   float2 v_yn, float a, float b, float c, float sp, float sq,
-                                                   float2& p, float4& q) {
-  using namespace x2;
-  const f2 vpp = pk(vp.x, vp.y);
-  const float2 u = upk(sub(sub(pk(u_xn, u_yn), pk(u_pos, u_pos)), vpp));
-  const float dtx = __fmaf_rn(a, u.x, c * u.y);
-  const float dty = __fmaf_rn(c, u.x, b * u.y);
-  const f2 s2 = pk(sq, sq);
-  project(fma(pk(sp, sp), pk(dtx, dty), pk(p.x, p.y)), fma(s2, sub(pk(v_xn.x, v_xn.y), vpp), pk(q.x, q.w)),
-          fma(s2, sub(pk(v_yn.x, v_yn.y), vpp), pk(q.z, q.y)), p, q);
-}
-
-__device__ __forceinline__ void dual_flat(bool useRight, bool useDown, float u_pos, float u_xn, float u_yn, float2 vp,
-                                          float2 v_xn, float2 v_yn, float a, float b, float c, float sp, float sq,
-                                          float2& p, float4& q) {
-  using namespace x2;
-  const float sx = useRight ? 1.0f : -1.0f;
-  const float sy = useDown ? 1.0f : -1.0f;
-  const float u_x = __fmaf_rn(sx, u_xn - u_pos, -vp.x);
-  const float u_y = __fmaf_rn(sy, u_yn - u_pos, -vp.y);
-  const float dtx = __fmaf_rn(a, u_x, c * u_y);
-  const float dty = __fmaf_rn(c, u_x, b * u_y);
-  const float qsx = sq * sx, qsy = sq * sy;  // exact: a sign change
-  const f2 vpp = pk(vp.x, vp.y);
-  project(fma(pk(sp, sp), pk(dtx, dty), pk(p.x, p.y)),
-          fma(pk(qsx, qsx), sub(pk(v_xn.x, v_xn.y), vpp), pk(q.x, q.w)),
-          fma(pk(qsy, qsy), sub(pk(v_yn.x, v_yn.y), vpp), pk(q.z, q.y)), p, q);
-}
-
-__device__ __forceinline__ float threshold_flat(float dxm, float dym, float teu, float u_bar, float upos, float Ius,
-                                                float Iz, float lambda) {
-  const float dun = __fmaf_rn(teu, dxm + dym, u_bar) - upos;
-  const float rho = __fmaf_rn(Ius, dun, Iz);
-  const float lt = lambda * teu;
-  const float upper = lt * (Ius * Ius);
-  const bool in = (rho <= upper) && (rho >= -upper), below = rho < -upper, above = rho > upper;
-  const float x = in ? -rho : below ? lt : -lt;
-  const float y = in ? rcp(Ius) : Ius;
-  float d = __fmaf_rn(x, y, dun);
-  if (in && Ius == 0.0f) d = dun;
-  return upos + ((in || below || above) ? d : 0.0f);  // a NaN residual leaves u
-}
-
-__device__ __forceinline__ void primal_flat(float4 qc, float2 qxw_l, float2 qzy_u, float2 tpp, float2 r12, float tau,
-                                            float alpha0, float alpha1, float mu, float2 vb, float u_new, float u_bar,
-                                            float& u_s, float2& v_s) {
-  using namespace x2;
-  const f2 dq = add(sub(pk(qc.x, qc.w), pk(qxw_l.x, qxw_l.y)), sub(pk(qc.z, qc.y), pk(qzy_u.x, qzy_u.y)));
-  const f2 g = fma(pk(alpha1, alpha1), pk(tpp.x, tpp.y), mul(pk(alpha0, alpha0), dq));
-  const f2 vbb = pk(vb.x, vb.y);
-  const bool zero2 = etav2_zero(r12.y);  // updatePrimalVariables.cu:103-105 writes .x again, .y keeps its value
-  const float2 w = upk(fma(pk(zero2 ? tau : tau * r12.x, tau * r12.y), g, vbb));
-  const f2 v = pk(w.x, zero2 ? vb.y : w.y);
-  u_s = __fmaf_rn(mu, u_new - u_bar, u_new);
-  v_s = upk(fma(pk(mu, mu), sub(v, vbb), v));
-}
 
 }  // namespace fast
 }  // namespace vfs
