@@ -210,7 +210,7 @@ int vfs_batch_solve_host(vfs_batch* b, const uint8_t* const* i0, const uint8_t* 
 int vfs_batch_solve_device(vfs_batch* b, const uint8_t* const* d_i0, const uint8_t* const* d_i1,
                            float* const* d_u_out, int masked);
 /* A one-pair solve (and each pair of a concurrent batch) runs every pyramid level whose state fits
- * the GPU's registers and shared memory (up to about 600,000 solved pixels with half storage,
+ * the GPU's registers and shared memory (up to about 1,050,000 solved pixels with half storage,
  * 560,000 with float) in one launch per warp, all iterations in it.  For the other levels the fused path
  * picks the tile height of its iteration kernel by timing the variants on the first solve of
  * each batch composition (on by default); the timing launches do not change results.  Off: the

@@ -94,6 +94,20 @@ def test_masks_with_isolated_pixels(gpu, half):
             _same((i0, i1, m, tv, cv), params(n_levels=1, n_warp=2, n_iter=n_iter), half, True)
 
 
+@pytest.mark.parametrize("masked", [True, False], ids=["masked", "plain"])
+@pytest.mark.parametrize("size", [(850, 702), (991, 999), (1078, 1009)])
+def test_tall_tiles(gpu, size, masked):
+    """Tiles of 12 and 16 rows (half storage): ragged right and lower edges, a disc that leaves masked-out
+    pixels and isolated ones in them, and alpha0 = 0, where eta_v2 may vanish."""
+    w, h = size
+    i0, i1, mask, tv, cv = random_case(w, h, seed=w)
+    yy, xx = np.mgrid[0:h, 0:w]
+    m = ((xx > 0) & (yy > 0) & ((xx - w / 2) ** 2 + (yy - h / 2) ** 2 < (0.62 * w) ** 2)).astype(np.float32)
+    m[np.random.default_rng(w).random((h, w)) < 0.001] = 0
+    for kw in (dict(n_iter=1), dict(n_iter=4), dict(n_iter=3, alpha0=0.0)):
+        _same((i0, i1, m, tv, cv), params(n_levels=1, n_warp=1, **kw), True, masked)
+
+
 def test_levels_it_does_not_take(gpu):
     """A masked-in pixel of column 0 without its right neighbour, more iterations than one launch
     holds, a negative lambda: the one-iteration kernels, with the same results."""

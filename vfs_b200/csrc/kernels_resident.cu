@@ -63,14 +63,37 @@ struct ResLinks {
 };
 template <class ST, int R>
 struct ResShared;
+template <int R, bool TALL = (R > 8), bool STREAM = (R > 12)>
+struct ResSharedHalf;
 template <int R>
-struct ResShared<__half, R> {
+struct ResSharedHalf<R, false, false> {
   float4 top[32];
   float4 cf[R / 2][4][32];
   float2 riu[R / 2][32];
+  uint2 p[R / 2][32];
+  uint4 q[R / 2][32];
+  uint4 pqtop[32];
   uint2 col[2][R];
   ResLinks k;
 };
+// tall tiles: (a, b), c, p, (q.x, q.y and q.z, q.w) and, up to 12 rows, (Iu, Iz); the row above's p and q
+template <int R>
+struct ResSharedHalf<R, true, true> {
+  float4 top[32];
+  float4 ab[R / 2][32];
+  float2 c[R / 2][32];
+  uint2 p[R / 2][32];
+  uint4 q[R / 2][32];
+  uint4 pqtop[32];
+  uint2 col[2][R];
+  ResLinks k;
+};
+template <int R>
+struct ResSharedHalf<R, true, false> : ResSharedHalf<R, true, true> {
+  float4 uz[R / 2][32];
+};
+template <int R>
+struct ResShared<__half, R> : ResSharedHalf<R> {};
 template <int R>
 struct ResShared<float, R> {
   float4 top[32];
@@ -97,17 +120,41 @@ struct ResState;
 // instructions, so that nearly every operation of the dual, threshold and primal steps serves
 // two pixels; only the differences along a column, whose operands straddle the pairs, the
 // comparisons and the conversions are per pixel.
+//
+// From 6 rows on p and q are in shared memory; in registers they left too few for the rest (848 x 800, 8
+// rows: 276 bytes spilled, 3.93 us per iteration; 4 bytes, 3.73).
+//
+// Tall tiles (12 and 16 rows) hold levels that 8 rows in 16 warps do not, up to 0.85 and 1.1 million
+// pixels.  The room comes from the reciprocals (formed again at every iteration, 24 instructions a
+// pair of rows) and, with 16 rows, from Iu and Iz (read again from L2, 8 bytes a pixel of the
+// one-iteration kernel's 96).  Their rows are taken four at a time by one piece of code, between whose
+// passes the registers move up: 16 rows unrolled by eight leave the instruction cache (1280 x 1024
+// disc, 2174 tiles of 16 rows: 11.6 us per iteration; by four 9.6; one launch per iteration 15.0.
+// 1000 x 900, 1883 tiles of 12: 6.1; 9.85).  Instruction issue bounds both.
 template <bool MASKED, int R>
 struct ResState<MASKED, __half, R> {
   typedef ResShared<__half, R> Sh;
   typedef x2::f2 f2;
+  static constexpr bool kTall = R > 8, kStream = R > 12;
+  static constexpr int kPasses = kTall ? R / 4 : 1, kPairs = R / 2 / kPasses;
+  static constexpr bool kSharedPQ = R > 4;
+  static constexpr int kHeld = kSharedPQ ? 0 : R;
   f2 u[R / 2], ub[R / 2];
-  unsigned v[R];                                 // v-bar
-  unsigned p[R + 1], q0[R + 1], q1[R + 1];       // rows -1 .. R-1: p, (q.x, q.y), (q.z, q.w)
+  unsigned v[R];                                             // v-bar
+  unsigned p[kHeld + 1], q0[kHeld + 1], q1[kHeld + 1];       // rows -1 .. R-1: p, (q.x, q.y), (q.z, q.w)
 
-  __device__ __forceinline__ void clear(Sh&, int) {
+  __device__ __forceinline__ void clear(Sh& sh, int lane) {
+    if constexpr (kSharedPQ) {
 #pragma unroll
-    for (int i = 0; i <= R; i++) p[i] = q0[i] = q1[i] = 0u;
+      for (int i = 0; i < R / 2; i++) {
+        sh.p[i][lane] = make_uint2(0u, 0u);
+        sh.q[i][lane] = make_uint4(0u, 0u, 0u, 0u);
+      }
+      sh.pqtop[lane] = make_uint4(0u, 0u, 0u, 0u);
+    } else {
+#pragma unroll
+      for (int i = 0; i <= R; i++) p[i] = q0[i] = q1[i] = 0u;
+    }
   }
   // east / south: edge codes of the pixel's right and lower neighbour
   __device__ __forceinline__ bool set_row(Sh& sh, int lane, const IterPair& P, int r, bool in, int pos, unsigned code,
@@ -125,20 +172,32 @@ struct ResState<MASKED, __half, R> {
       return false;
     }
     const int i = r >> 1, k = r & 1;
-    float2 rv = in ? P.rv[pos] : make_float2(1.f, 1.f);
-    // eta_v2 = 0 (updatePrimalVariables.cu:103-105): .x takes tau itself, .y keeps its value
-    if (fast::etav2_zero(rv.y)) rv = make_float2(1.f, 0.f);
-    const float iu = in ? P.Iu[pos] : 0.f;
-    const float c[8] = {ca.x, ca.y, ca.z, ca.w, iu, in ? P.Iz[pos] : 0.f, rv.x, rv.y};
+    const float iu = in ? P.Iu[pos] : 0.f, iz = in ? P.Iz[pos] : 0.f;
+    if constexpr (kTall) {
+      reinterpret_cast<float*>(&sh.ab[i][lane])[k] = ca.x;
+      reinterpret_cast<float*>(&sh.ab[i][lane])[2 + k] = ca.y;
+      reinterpret_cast<float*>(&sh.c[i][lane])[k] = ca.z;
+      if constexpr (!kStream) {
+        reinterpret_cast<float*>(&sh.uz[i][lane])[k] = iu;
+        reinterpret_cast<float*>(&sh.uz[i][lane])[2 + k] = iz;
+      }
+    } else {
+      float2 rv = in ? P.rv[pos] : make_float2(1.f, 1.f);
+      // eta_v2 = 0 (updatePrimalVariables.cu:103-105): .x takes tau itself, .y keeps its value
+      if (fast::etav2_zero(rv.y)) rv = make_float2(1.f, 0.f);
+      const float c[8] = {ca.x, ca.y, ca.z, ca.w, iu, iz, rv.x, rv.y};
 #pragma unroll
-    for (int j = 0; j < 8; j++) reinterpret_cast<float*>(&sh.cf[i][j >> 1][lane])[2 * (j & 1) + k] = c[j];
-    // the Newton step -rho / Iu of the threshold; 0 where Iu = 0 (no step there)
-    reinterpret_cast<float*>(&sh.riu[i][lane])[k] = iu == 0.0f ? 0.0f : fast::rcp(iu);
+      for (int j = 0; j < 8; j++) reinterpret_cast<float*>(&sh.cf[i][j >> 1][lane])[2 * (j & 1) + k] = c[j];
+      // the Newton step -rho / Iu of the threshold; 0 where Iu = 0 (no step there)
+      reinterpret_cast<float*>(&sh.riu[i][lane])[k] = iu == 0.0f ? 0.0f : fast::rcp(iu);
+    }
     float un = in ? P.u[pos] : 0.f, ubn = in ? P.u_[pos] : 0.f;
     v[r] = 0u;
     if (MASKED && in && !(code & kOn)) {  // the other ping-pong values of a masked-out pixel
       un = P.u_s[pos];
-      p[r + 1] = bits(((const __half2*)P.v_s)[pos]);
+      const unsigned o = bits(((const __half2*)P.v_s)[pos]);
+      if constexpr (kSharedPQ) (k ? sh.p[i][lane].y : sh.p[i][lane].x) = o;
+      else p[r + 1] = o;
     }
     u[i] = k ? x2::pk(lo(u[i]), un) : x2::pk(un, 0.f);
     ub[i] = k ? x2::pk(lo(ub[i]), ubn) : x2::pk(ubn, 0.f);
@@ -160,9 +219,51 @@ struct ResState<MASKED, __half, R> {
       v[2 * i + 1] = w.w;
     }
   }
-  __device__ __forceinline__ void store_pq(const Sh&, int, int r, void* po, void* qo, int pos) const {
-    reinterpret_cast<unsigned*>(po)[pos] = p[r + 1];
-    reinterpret_cast<uint2*>(qo)[pos] = make_uint2(q0[r + 1], q1[r + 1]);
+  __device__ __forceinline__ void store_pq(const Sh& sh, int lane, int r, void* po, void* qo, int pos) const {
+    uint2 q;
+    unsigned pv;
+    if constexpr (kSharedPQ) {
+      const uint2 pp = sh.p[r >> 1][lane];
+      const uint4 qq = sh.q[r >> 1][lane];
+      pv = r & 1 ? pp.y : pp.x;
+      q = r & 1 ? make_uint2(qq.y, qq.w) : make_uint2(qq.x, qq.z);
+    } else {
+      pv = p[r + 1];
+      q = make_uint2(q0[r + 1], q1[r + 1]);
+    }
+    reinterpret_cast<unsigned*>(po)[pos] = pv;
+    reinterpret_cast<uint2*>(qo)[pos] = q;
+  }
+  // entry i of a pass to the place of the last pass's, the others' one pass up (n entries a pair)
+  template <class T>
+  static __device__ __forceinline__ void roll(T* a, int i, int n) {
+    const T t = a[i];
+#pragma unroll
+    for (int k = 0; k + 1 < kPasses; k++) a[k * kPairs * n + i] = a[(k + 1) * kPairs * n + i];
+    a[(kPasses - 1) * kPairs * n + i] = t;
+  }
+  // the reciprocals of a pair of rows: 1 / eta_u, 1 / eta_v1 and 1 / eta_v2, 1 / Iu, as in the level's
+  // records (fast::etau_rcp, etav_rcp) and in set_row
+  static __device__ __forceinline__ void reciprocals(f2 a, f2 b, f2 c, f2 iu, const IterPair& P, f2& re, f2& rx, f2& ry,
+                                                     f2& riu) {
+    using namespace x2;
+    const f2 a1s = both(P.alpha1 * P.alpha1), a0s4 = both(4 * P.alpha0 * P.alpha0);
+    const f2 bb = mul(b, b), ac = add(a, c), bc = add(b, c), cc = mul(c, c);
+    const f2 eu = mul(fma(bc, bc, fma(ac, ac, fma(add(c, c), c, fma(a, a, bb)))), a1s);
+    const f2 e1 = fma(a1s, fma(b, b, cc), a0s4), e2 = fma(a1s, fma(a, a, cc), a0s4);
+    auto one = [](float e, float i, float x, float y, float& ro, float& xo, float& yo, float& io) {
+      ro = e == 0.0f ? 1.0f : fast::rcp(e);
+      xo = x != 0.0f && y != 0.0f ? fast::rcp(x) : 1.0f;
+      yo = y != 0.0f ? fast::rcp(y) : 0.0f;
+      io = i == 0.0f ? 0.0f : fast::rcp(i);
+    };
+    float r0, r1, x0, x1, y0, y1, i0, i1;
+    one(lo(eu), lo(iu), lo(e1), lo(e2), r0, x0, y0, i0);
+    one(hi(eu), hi(iu), hi(e1), hi(e2), r1, x1, y1, i1);
+    re = pk(r0, r1);
+    rx = pk(x0, x1);
+    ry = pk(y0, y1);
+    riu = pk(i0, i1);
   }
 
   // One iteration.  wn / ws: the words of the row above / below the tile.  KIND: ResKind of the
@@ -176,7 +277,7 @@ struct ResState<MASKED, __half, R> {
   // neighbour).  So those values are replaced by zero once, at the pixel, where it is off or
   // its right neighbour is; likewise along y.  (-0 in T p, so that 0 - x is -x.)
   template <int KIND>
-  __device__ __forceinline__ void iterate(Sh& sh, const ResArgs& A, int lane, const ResStep& S, const ResEdge& E,
+  __device__ __forceinline__ void iterate(Sh& sh, const ResArgs& A, int lane, const ResStep& S, ResEdge E,
                                           uint4 wn, uint4 ws, float2* tp_out, int s, unsigned tp_rows) {
     using namespace x2;
     constexpr bool EDGE = KIND != kResInner;
@@ -184,6 +285,21 @@ struct ResState<MASKED, __half, R> {
     const f2 sp = pk(S.sp.x, S.sp.y), sq = pk(S.sq.x, S.sq.y), tau = pk(S.tau.x, S.tau.y), mu = pk(S.mu.x, S.mu.y);
     const f2 lam = both(A.P.lambda), al0 = both(A.P.alpha0), al1 = both(A.P.alpha1);
     auto bit = [](unsigned m, int r) { return (m >> (r + 1)) & 1u; };
+    // streamed: positions of the pair's two rows and of the next pair's first, rows of the image below that
+    int a0 = 0, a1 = 0, at = 0, left = 0;
+    auto next = [&](f2& iu, f2& iz) {
+      a0 = at;
+      a1 = left > 0 ? at + s : at;
+      at = left > 1 ? a1 + s : a1;
+      left -= 2;
+      iu = pk(__ldg(A.P.Iu + a0), __ldg(A.P.Iu + a1));
+      iz = pk(__ldg(A.P.Iz + a0), __ldg(A.P.Iz + a1));
+    };
+    if constexpr (kStream) {  // (beyond the image: some pixel of it, for lanes and rows that nothing reads)
+      const ResTile& T = A.tiles[sh.k.t];
+      at = min(max(T.x0 - 1 + lane, 0), A.P.w - 1) + T.y0 * s;
+      left = A.P.h - 1 - T.y0;
+    }
     // row -1: its dual step, for T p and q of the row above row 0
     float tpy_n, qz_n, qy_n;       // T p.y, q.z and q.y of the row above
     float du_n;                    // u-bar and v-bar less those of the row above
@@ -205,6 +321,12 @@ struct ResState<MASKED, __half, R> {
         dvx = make_float2(r0 ? dvx.x : wv.x, r0 ? dvx.y : wv.y);
       }
       const float gx = dux - vp.x, gy = du_n - vp.y;
+      if constexpr (kSharedPQ) {
+        const uint4 t = sh.pqtop[lane];
+        p[0] = t.x;
+        q0[0] = t.y;
+        q1[0] = t.z;
+      }
       const float2 h0 = unpack(p[0]), h1 = unpack(q0[0]), h2 = unpack(q1[0]);
       float px = __fmaf_rn(S.sp.x, __fmaf_rn(ca.x, gx, ca.z * gy), h0.x);
       float py = __fmaf_rn(S.sp.x, __fmaf_rn(ca.z, gx, ca.y * gy), h0.y);
@@ -221,6 +343,7 @@ struct ResState<MASKED, __half, R> {
       p[0] = pack(px, py);
       q0[0] = pack(qx, qy);
       q1[0] = pack(qz, qw);
+      if constexpr (kSharedPQ) sh.pqtop[lane] = make_uint4(p[0], q0[0], q1[0], 0u);
       tpy_n = __fmaf_rn(ca.z, px, ca.y * py);
       qz_n = qz;
       qy_n = qy;
@@ -232,159 +355,214 @@ struct ResState<MASKED, __half, R> {
         qy_n = d0 ? qy : 0.f;
       }
     }
+#pragma unroll 1
+    for (int pass = 0; pass < kPasses; pass++) {
 #pragma unroll
-    for (int i = 0; i < R / 2; i++) {
-      const int r = 2 * i;
-      const f2 UB = ub[i];
-      const float ub0 = lo(UB), ub1 = hi(UB);
-      const float2 v1 = unpack(v[r + 1]);
-      const float ubd = i + 1 < R / 2 ? lo(ub[i + 1 < R / 2 ? i + 1 : 0]) : __uint_as_float(ws.x);
-      const float2 vd = unpack(i + 1 < R / 2 ? v[r + 2 < R ? r + 2 : 0] : ws.y);
-      const f2 VX = pk(vc.x, v1.x), VY = pk(vc.y, v1.y);
-      const ulonglong2 ab = *reinterpret_cast<const ulonglong2*>(&sh.cf[i][0][lane]);
-      const ulonglong2 ce = *reinterpret_cast<const ulonglong2*>(&sh.cf[i][1][lane]);
-      const ulonglong2 uz = *reinterpret_cast<const ulonglong2*>(&sh.cf[i][2][lane]);
-      const ulonglong2 rr = *reinterpret_cast<const ulonglong2*>(&sh.cf[i][3][lane]);
-      const f2 riu = *reinterpret_cast<const f2*>(&sh.riu[i][lane]);
-      // ---- differences of u-bar and v-bar to the east and to the south -----------------
-      const float2 e0 = unpack(__shfl_down_sync(kFull, v[r], 1)), e1 = unpack(__shfl_down_sync(kFull, v[r + 1], 1));
-      f2 dux = sub(pk(__shfl_down_sync(kFull, ub0, 1), __shfl_down_sync(kFull, ub1, 1)), UB);
-      f2 dxx = sub(pk(e0.x, e1.x), VX), dxy = sub(pk(e0.y, e1.y), VY);
-      const float du0 = ub1 - ub0, du1 = ubd - ub1;
-      const float2 dv0 = make_float2(v1.x - vc.x, v1.y - vc.y), dv1 = make_float2(vd.x - v1.x, vd.y - v1.y);
-      f2 duy = pk(du0, du1), dyx = pk(dv0.x, dv1.x), dyy = pk(dv0.y, dv1.y);
-      bool r0 = true, r1 = true, d0 = true, d1 = true;
-      if (EDGE) {
-        r0 = bit(E.x, r);
-        r1 = bit(E.x, r + 1);
-        d0 = bit(E.y, r);
-        d1 = bit(E.y, r + 1);
-        const float wu0 = __shfl_up_sync(kFull, lo(dux), 1), wu1 = __shfl_up_sync(kFull, hi(dux), 1);
-        const float wx0 = __shfl_up_sync(kFull, lo(dxx), 1), wx1 = __shfl_up_sync(kFull, hi(dxx), 1);
-        const float wy0 = __shfl_up_sync(kFull, lo(dxy), 1), wy1 = __shfl_up_sync(kFull, hi(dxy), 1);
-        dux = pk(r0 ? lo(dux) : wu0, r1 ? hi(dux) : wu1);
-        dxx = pk(r0 ? lo(dxx) : wx0, r1 ? hi(dxx) : wx1);
-        dxy = pk(r0 ? lo(dxy) : wy0, r1 ? hi(dxy) : wy1);
-        duy = pk(d0 ? du0 : du_n, d1 ? du1 : du0);
-        dyx = pk(d0 ? dv0.x : dv_n.x, d1 ? dv1.x : dv0.x);
-        dyy = pk(d0 ? dv0.y : dv_n.y, d1 ? dv1.y : dv0.y);
-        du_n = du1;
-        dv_n = dv1;
-      }
-      // ---- dual step ------------------------------------------------------------------
-      const f2 a = ab.x, b = ab.y, c = ce.x;
-      const f2 ux = sub(dux, VX), uy = sub(duy, VY);
-      const float2 p0 = unpack(p[r + 1]), p1 = unpack(p[r + 2]);
-      const float2 qa0 = unpack(q0[r + 1]), qa1 = unpack(q0[r + 2]), qb0 = unpack(q1[r + 1]), qb1 = unpack(q1[r + 2]);
-      f2 px = fma(sp, fma(a, ux, mul(c, uy)), pk(p0.x, p1.x));
-      f2 py = fma(sp, fma(c, ux, mul(b, uy)), pk(p0.y, p1.y));
-      const f2 n2 = fma(px, px, mul(py, py));
-      const f2 rp = pk(fast::unit_scale(lo(n2)), fast::unit_scale(hi(n2)));
-      px = mul(px, rp);
-      py = mul(py, rp);
-      f2 qx = fma(sq, dxx, pk(qa0.x, qa1.x));
-      f2 qy = fma(sq, dyy, pk(qa0.y, qa1.y));
-      f2 qz = fma(sq, dyx, pk(qb0.x, qb1.x));
-      f2 qw = fma(sq, dxy, pk(qb0.y, qb1.y));
-      const f2 m2 = fma(qx, qx, fma(qy, qy, fma(qz, qz, mul(qw, qw))));
-      const f2 rq = pk(fast::unit_scale(lo(m2)), fast::unit_scale(hi(m2)));
-      qx = mul(qx, rq);
-      qy = mul(qy, rq);
-      qz = mul(qz, rq);
-      qw = mul(qw, rq);
-      f2 tpx = fma(a, px, mul(c, py)), tpy = fma(c, px, mul(b, py));
-      unsigned pn0 = pack(lo(px), lo(py)), pn1 = pack(hi(px), hi(py));
-      q0[r + 1] = pack(lo(qx), lo(qy));
-      q1[r + 1] = pack(lo(qz), lo(qw));
-      q0[r + 2] = pack(hi(qx), hi(qy));
-      q1[r + 2] = pack(hi(qz), hi(qw));
-      if (!MASKED && EDGE) {  // outside the circle p = 0: T p = T 0
-        const float2 z = make_float2(0.f, 0.f);
-        if ((tp_rows >> r) & 1u) tp_out[r * s] = bit(E.on, r) ? make_float2(lo(tpx), lo(tpy)) : tp_math(lo(a), lo(b), lo(c), z);
-        if ((tp_rows >> (r + 1)) & 1u)
-          tp_out[(r + 1) * s] = bit(E.on, r + 1) ? make_float2(hi(tpx), hi(tpy)) : tp_math(hi(a), hi(b), hi(c), z);
-      } else {
-        if ((tp_rows >> r) & 1u) tp_out[r * s] = make_float2(lo(tpx), lo(tpy));
-        if ((tp_rows >> (r + 1)) & 1u) tp_out[(r + 1) * s] = make_float2(hi(tpx), hi(tpy));
-      }
-      // ---- threshold step -----------------------------------------------------------
-      f2 txo = tpx, tyo = tpy;  // as counted for this pixel and its right / lower neighbour
-      bool o0 = true, o1 = true;
-      if (EDGE) {
-        if (KEEP || !MASKED) {
-          o0 = bit(E.on, r);
-          o1 = bit(E.on, r + 1);
+      for (int i = 0; i < kPairs; i++) {
+        const int r = 2 * i, is = pass * kPairs + i;
+        constexpr int kNext = kTall ? kPairs : 0;  // the first pair of the next pass
+        const f2 UB = ub[i];
+        const float ub0 = lo(UB), ub1 = hi(UB);
+        const float2 v1 = unpack(v[r + 1]);
+        const bool more = kTall && pass + 1 < kPasses;
+        const int in_ = i + 1 < kPairs ? i + 1 : kNext;
+        const float ubd = i + 1 < kPairs || more ? lo(ub[in_]) : __uint_as_float(ws.x);
+        const float2 vd = unpack(i + 1 < kPairs || more ? v[2 * in_] : ws.y);
+        const f2 VX = pk(vc.x, v1.x), VY = pk(vc.y, v1.y);
+        ulonglong2 ab, ce, uz, rr;
+        f2 riu;
+        unsigned pa, pb, qa0h, qa1h, qb0h, qb1h;  // p, (q.x, q.y), (q.z, q.w) of the two rows
+        if constexpr (kTall) {
+          ab = *reinterpret_cast<const ulonglong2*>(&sh.ab[is][lane]);
+          ce.x = *reinterpret_cast<const f2*>(&sh.c[is][lane]);
+          if constexpr (kStream) {
+            next(uz.x, uz.y);
+          } else {
+            uz = *reinterpret_cast<const ulonglong2*>(&sh.uz[is][lane]);
+          }
+          reciprocals(ab.x, ab.y, ce.x, uz.x, A.P, ce.y, rr.x, rr.y, riu);
+        } else {
+          ab = *reinterpret_cast<const ulonglong2*>(&sh.cf[i][0][lane]);
+          ce = *reinterpret_cast<const ulonglong2*>(&sh.cf[i][1][lane]);
+          uz = *reinterpret_cast<const ulonglong2*>(&sh.cf[i][2][lane]);
+          rr = *reinterpret_cast<const ulonglong2*>(&sh.cf[i][3][lane]);
+          riu = *reinterpret_cast<const f2*>(&sh.riu[i][lane]);
         }
-        const float zx0 = KEEP && !o0 ? lo(a) : -0.0f, zx1 = KEEP && !o1 ? hi(a) : -0.0f;
-        const float zy0 = KEEP && !o0 ? lo(b) : -0.0f, zy1 = KEEP && !o1 ? hi(b) : -0.0f;
-        // the plain form takes the difference at the last row and column too
-        txo = pk((MASKED ? r0 : o0) ? lo(tpx) : zx0, (MASKED ? r1 : o1) ? hi(tpx) : zx1);
-        tyo = pk((MASKED ? d0 : o0) ? lo(tpy) : zy0, (MASKED ? d1 : o1) ? hi(tpy) : zy1);
-        qx = pk(r0 ? lo(qx) : 0.f, r1 ? hi(qx) : 0.f);
-        qw = pk(r0 ? lo(qw) : 0.f, r1 ? hi(qw) : 0.f);
-        qz = pk(d0 ? lo(qz) : 0.f, d1 ? hi(qz) : 0.f);
-        qy = pk(d0 ? lo(qy) : 0.f, d1 ? hi(qy) : 0.f);
-      }
-      const f2 tpw = pk(__shfl_up_sync(kFull, lo(txo), 1), __shfl_up_sync(kFull, hi(txo), 1));
-      const f2 qxw = pk(__shfl_up_sync(kFull, lo(qx), 1), __shfl_up_sync(kFull, hi(qx), 1));
-      const f2 qww = pk(__shfl_up_sync(kFull, lo(qw), 1), __shfl_up_sync(kFull, hi(qw), 1));
-      const f2 dy = pk(lo(tyo) - tpy_n, hi(tyo) - lo(tyo));
-      const f2 dqz = pk(lo(qz) - qz_n, hi(qz) - lo(qz)), dqy = pk(lo(qy) - qy_n, hi(qy) - lo(qy));
-      const f2 U = u[i], iu = uz.x;
-      const f2 teu = mul(tau, ce.y);
-      const f2 dun = sub(fma(teu, add(sub(txo, tpw), dy), UB), U);
-      const f2 rho = fma(iu, dun, uz.y);
-      const f2 lt = mul(lam, teu);
-      const f2 up = mul(lt, mul(iu, iu));
-      f2 un;
-      {
-        // |rho| <= upper: the Newton step; beyond it a step of lambda tau / eta_u against the sign of
-        // rho (lambda >= 0); a NaN residual leaves u
-        float x[2], y[2];
-        bool num[2];
+        if constexpr (kSharedPQ) {
+          const uint2 pp = sh.p[is][lane];
+          const uint4 qq = sh.q[is][lane];
+          pa = pp.x, pb = pp.y, qa0h = qq.x, qa1h = qq.y, qb0h = qq.z, qb1h = qq.w;
+        } else {
+          pa = p[r + 1], pb = p[r + 2], qa0h = q0[r + 1], qa1h = q0[r + 2], qb0h = q1[r + 1], qb1h = q1[r + 2];
+        }
+        // ---- differences of u-bar and v-bar to the east and to the south -----------------
+        const float2 e0 = unpack(__shfl_down_sync(kFull, v[r], 1)), e1 = unpack(__shfl_down_sync(kFull, v[r + 1], 1));
+        f2 dux = sub(pk(__shfl_down_sync(kFull, ub0, 1), __shfl_down_sync(kFull, ub1, 1)), UB);
+        f2 dxx = sub(pk(e0.x, e1.x), VX), dxy = sub(pk(e0.y, e1.y), VY);
+        const float du0 = ub1 - ub0, du1 = ubd - ub1;
+        const float2 dv0 = make_float2(v1.x - vc.x, v1.y - vc.y), dv1 = make_float2(vd.x - v1.x, vd.y - v1.y);
+        f2 duy = pk(du0, du1), dyx = pk(dv0.x, dv1.x), dyy = pk(dv0.y, dv1.y);
+        bool r0 = true, r1 = true, d0 = true, d1 = true;
+        if (EDGE) {
+          r0 = bit(E.x, r);
+          r1 = bit(E.x, r + 1);
+          d0 = bit(E.y, r);
+          d1 = bit(E.y, r + 1);
+          const float wu0 = __shfl_up_sync(kFull, lo(dux), 1), wu1 = __shfl_up_sync(kFull, hi(dux), 1);
+          const float wx0 = __shfl_up_sync(kFull, lo(dxx), 1), wx1 = __shfl_up_sync(kFull, hi(dxx), 1);
+          const float wy0 = __shfl_up_sync(kFull, lo(dxy), 1), wy1 = __shfl_up_sync(kFull, hi(dxy), 1);
+          dux = pk(r0 ? lo(dux) : wu0, r1 ? hi(dux) : wu1);
+          dxx = pk(r0 ? lo(dxx) : wx0, r1 ? hi(dxx) : wx1);
+          dxy = pk(r0 ? lo(dxy) : wy0, r1 ? hi(dxy) : wy1);
+          duy = pk(d0 ? du0 : du_n, d1 ? du1 : du0);
+          dyx = pk(d0 ? dv0.x : dv_n.x, d1 ? dv1.x : dv0.x);
+          dyy = pk(d0 ? dv0.y : dv_n.y, d1 ? dv1.y : dv0.y);
+          du_n = du1;
+          dv_n = dv1;
+        }
+        // ---- dual step ------------------------------------------------------------------
+        const f2 a = ab.x, b = ab.y, c = ce.x;
+        const f2 ux = sub(dux, VX), uy = sub(duy, VY);
+        const float2 p0 = unpack(pa), p1 = unpack(pb);
+        const float2 qa0 = unpack(qa0h), qa1 = unpack(qa1h), qb0 = unpack(qb0h), qb1 = unpack(qb1h);
+        f2 px = fma(sp, fma(a, ux, mul(c, uy)), pk(p0.x, p1.x));
+        f2 py = fma(sp, fma(c, ux, mul(b, uy)), pk(p0.y, p1.y));
+        const f2 n2 = fma(px, px, mul(py, py));
+        const f2 rp = pk(fast::unit_scale(lo(n2)), fast::unit_scale(hi(n2)));
+        px = mul(px, rp);
+        py = mul(py, rp);
+        f2 qx = fma(sq, dxx, pk(qa0.x, qa1.x));
+        f2 qy = fma(sq, dyy, pk(qa0.y, qa1.y));
+        f2 qz = fma(sq, dyx, pk(qb0.x, qb1.x));
+        f2 qw = fma(sq, dxy, pk(qb0.y, qb1.y));
+        const f2 m2 = fma(qx, qx, fma(qy, qy, fma(qz, qz, mul(qw, qw))));
+        const f2 rq = pk(fast::unit_scale(lo(m2)), fast::unit_scale(hi(m2)));
+        qx = mul(qx, rq);
+        qy = mul(qy, rq);
+        qz = mul(qz, rq);
+        qw = mul(qw, rq);
+        f2 tpx = fma(a, px, mul(c, py)), tpy = fma(c, px, mul(b, py));
+        unsigned pn0 = pack(lo(px), lo(py)), pn1 = pack(hi(px), hi(py));
+        if constexpr (kSharedPQ) {
+          sh.q[is][lane] =
+              make_uint4(pack(lo(qx), lo(qy)), pack(hi(qx), hi(qy)), pack(lo(qz), lo(qw)), pack(hi(qz), hi(qw)));
+        } else {
+          q0[r + 1] = pack(lo(qx), lo(qy));
+          q1[r + 1] = pack(lo(qz), lo(qw));
+          q0[r + 2] = pack(hi(qx), hi(qy));
+          q1[r + 2] = pack(hi(qz), hi(qw));
+        }
+        auto put = [&](int row, int pos, float2 t) {
+          if constexpr (kStream) A.P.Tp[pos] = t;
+          else tp_out[row * s] = t;
+        };
+        if (!MASKED && EDGE) {  // outside the circle p = 0: T p = T 0
+          const float2 z = make_float2(0.f, 0.f);
+          if ((tp_rows >> r) & 1u)
+            put(r, a0, bit(E.on, r) ? make_float2(lo(tpx), lo(tpy)) : tp_math(lo(a), lo(b), lo(c), z));
+          if ((tp_rows >> (r + 1)) & 1u)
+            put(r + 1, a1, bit(E.on, r + 1) ? make_float2(hi(tpx), hi(tpy)) : tp_math(hi(a), hi(b), hi(c), z));
+        } else {
+          if ((tp_rows >> r) & 1u) put(r, a0, make_float2(lo(tpx), lo(tpy)));
+          if ((tp_rows >> (r + 1)) & 1u) put(r + 1, a1, make_float2(hi(tpx), hi(tpy)));
+        }
+        // ---- threshold step -----------------------------------------------------------
+        f2 txo = tpx, tyo = tpy;  // as counted for this pixel and its right / lower neighbour
+        bool o0 = true, o1 = true;
+        if (EDGE) {
+          if (KEEP || !MASKED) {
+            o0 = bit(E.on, r);
+            o1 = bit(E.on, r + 1);
+          }
+          const float zx0 = KEEP && !o0 ? lo(a) : -0.0f, zx1 = KEEP && !o1 ? hi(a) : -0.0f;
+          const float zy0 = KEEP && !o0 ? lo(b) : -0.0f, zy1 = KEEP && !o1 ? hi(b) : -0.0f;
+          // the plain form takes the difference at the last row and column too
+          txo = pk((MASKED ? r0 : o0) ? lo(tpx) : zx0, (MASKED ? r1 : o1) ? hi(tpx) : zx1);
+          tyo = pk((MASKED ? d0 : o0) ? lo(tpy) : zy0, (MASKED ? d1 : o1) ? hi(tpy) : zy1);
+          qx = pk(r0 ? lo(qx) : 0.f, r1 ? hi(qx) : 0.f);
+          qw = pk(r0 ? lo(qw) : 0.f, r1 ? hi(qw) : 0.f);
+          qz = pk(d0 ? lo(qz) : 0.f, d1 ? hi(qz) : 0.f);
+          qy = pk(d0 ? lo(qy) : 0.f, d1 ? hi(qy) : 0.f);
+        }
+        const f2 tpw = pk(__shfl_up_sync(kFull, lo(txo), 1), __shfl_up_sync(kFull, hi(txo), 1));
+        const f2 qxw = pk(__shfl_up_sync(kFull, lo(qx), 1), __shfl_up_sync(kFull, hi(qx), 1));
+        const f2 qww = pk(__shfl_up_sync(kFull, lo(qw), 1), __shfl_up_sync(kFull, hi(qw), 1));
+        const f2 dy = pk(lo(tyo) - tpy_n, hi(tyo) - lo(tyo));
+        const f2 dqz = pk(lo(qz) - qz_n, hi(qz) - lo(qz)), dqy = pk(lo(qy) - qy_n, hi(qy) - lo(qy));
+        const f2 U = u[i], iu = uz.x;
+        const f2 teu = mul(tau, ce.y);
+        const f2 dun = sub(fma(teu, add(sub(txo, tpw), dy), UB), U);
+        const f2 rho = fma(iu, dun, uz.y);
+        const f2 lt = mul(lam, teu);
+        const f2 up = mul(lt, mul(iu, iu));
+        f2 un;
+        {
+          // |rho| <= upper: the Newton step; beyond it a step of lambda tau / eta_u against the sign of
+          // rho (lambda >= 0); a NaN residual leaves u
+          float x[2], y[2];
+          bool num[2];
 #pragma unroll
-        for (int k = 0; k < 2; k++) {
-          const float rh = k ? hi(rho) : lo(rho), upk_ = k ? hi(up) : lo(up), ltk = k ? hi(lt) : lo(lt);
-          const bool in = fabsf(rh) <= upk_;
-          num[k] = in || fabsf(rh) > upk_;
-          const float away = __uint_as_float(__float_as_uint(ltk) ^ (~__float_as_uint(rh) & 0x80000000u));
-          x[k] = in ? -rh : away;
-          y[k] = in ? (k ? hi(riu) : lo(riu)) : (k ? hi(iu) : lo(iu));
+          for (int k = 0; k < 2; k++) {
+            const float rh = k ? hi(rho) : lo(rho), upk_ = k ? hi(up) : lo(up), ltk = k ? hi(lt) : lo(lt);
+            const bool in = fabsf(rh) <= upk_;
+            num[k] = in || fabsf(rh) > upk_;
+            const float away = __uint_as_float(__float_as_uint(ltk) ^ (~__float_as_uint(rh) & 0x80000000u));
+            x[k] = in ? -rh : away;
+            y[k] = in ? (k ? hi(riu) : lo(riu)) : (k ? hi(iu) : lo(iu));
+          }
+          const f2 d = fma(pk(x[0], x[1]), pk(y[0], y[1]), dun);
+          un = add(U, pk(num[0] ? lo(d) : 0.0f, num[1] ? hi(d) : 0.0f));
         }
-        const f2 d = fma(pk(x[0], x[1]), pk(y[0], y[1]), dun);
-        un = add(U, pk(num[0] ? lo(d) : 0.0f, num[1] ? hi(d) : 0.0f));
+        // ---- primal step --------------------------------------------------------------
+        const f2 gx = fma(al1, tpx, mul(al0, add(sub(qx, qxw), dqz)));
+        const f2 gy = fma(al1, tpy, mul(al0, add(sub(qw, qww), dqy)));
+        const f2 vx = fma(mul(tau, rr.x), gx, VX);
+        const f2 vy = fma(mul(tau, rr.y), gy, VY);
+        f2 us = fma(mu, sub(un, UB), un);
+        const f2 vsx = fma(mu, sub(vx, VX), vx), vsy = fma(mu, sub(vy, VY), vy);
+        unsigned vn0 = pack(lo(vsx), lo(vsy)), vn1 = pack(hi(vsx), hi(vsy));
+        if (KEEP) {  // unwritten pixels alternate between the two ping-pong buffers' values
+          un = pk(o0 ? lo(un) : ub0, o1 ? hi(un) : ub1);
+          us = pk(o0 ? lo(us) : lo(U), o1 ? hi(us) : hi(U));
+          vn0 = o0 ? vn0 : pa;
+          vn1 = o1 ? vn1 : pb;
+          pn0 = o0 ? pn0 : v[r];
+          pn1 = o1 ? pn1 : v[r + 1];
+        } else if (EDGE && !MASKED) {  // outside the circle
+          un = pk(o0 ? lo(un) : 0.f, o1 ? hi(un) : 0.f);
+          us = pk(o0 ? lo(us) : 0.f, o1 ? hi(us) : 0.f);
+          vn0 = o0 ? vn0 : 0u;
+          vn1 = o1 ? vn1 : 0u;
+        }
+        u[i] = un;
+        ub[i] = us;
+        v[r] = vn0;
+        v[r + 1] = vn1;
+        if constexpr (kSharedPQ) {
+          sh.p[is][lane] = make_uint2(pn0, pn1);
+        } else {
+          p[r + 1] = pn0;
+          p[r + 2] = pn1;
+        }
+        tpy_n = hi(tyo);
+        qz_n = hi(qz);
+        qy_n = hi(qy);
+        vc = vd;
       }
-      // ---- primal step --------------------------------------------------------------
-      const f2 gx = fma(al1, tpx, mul(al0, add(sub(qx, qxw), dqz)));
-      const f2 gy = fma(al1, tpy, mul(al0, add(sub(qw, qww), dqy)));
-      const f2 vx = fma(mul(tau, rr.x), gx, VX);
-      const f2 vy = fma(mul(tau, rr.y), gy, VY);
-      f2 us = fma(mu, sub(un, UB), un);
-      const f2 vsx = fma(mu, sub(vx, VX), vx), vsy = fma(mu, sub(vy, VY), vy);
-      unsigned vn0 = pack(lo(vsx), lo(vsy)), vn1 = pack(hi(vsx), hi(vsy));
-      if (KEEP) {  // unwritten pixels alternate between the two ping-pong buffers' values
-        un = pk(o0 ? lo(un) : ub0, o1 ? hi(un) : ub1);
-        us = pk(o0 ? lo(us) : lo(U), o1 ? hi(us) : hi(U));
-        vn0 = o0 ? vn0 : p[r + 1];
-        vn1 = o1 ? vn1 : p[r + 2];
-        pn0 = o0 ? pn0 : v[r];
-        pn1 = o1 ? pn1 : v[r + 1];
-      } else if (EDGE && !MASKED) {  // outside the circle
-        un = pk(o0 ? lo(un) : 0.f, o1 ? hi(un) : 0.f);
-        us = pk(o0 ? lo(us) : 0.f, o1 ? hi(us) : 0.f);
-        vn0 = o0 ? vn0 : 0u;
-        vn1 = o1 ? vn1 : 0u;
+      if constexpr (kTall) {
+#pragma unroll
+        for (int i = 0; i < kPairs; i++) {
+          roll(u, i, 1);
+          roll(ub, i, 1);
+          roll(v, 2 * i, 2);
+          roll(v, 2 * i + 1, 2);
+        }
+        E.x >>= 2 * kPairs;
+        E.y >>= 2 * kPairs;
+        E.on >>= 2 * kPairs;
+        tp_rows >>= 2 * kPairs;
+        if (!kStream) tp_out += 2 * kPairs * s;
       }
-      u[i] = un;
-      ub[i] = us;
-      v[r] = vn0;
-      v[r + 1] = vn1;
-      p[r + 1] = pn0;
-      p[r + 2] = pn1;
-      tpy_n = hi(tyo);
-      qz_n = hi(qz);
-      qy_n = hi(qy);
-      vc = vd;
     }
   }
 };
@@ -959,7 +1137,7 @@ struct ResWarp {
 // Warps per block (one block per SM): what the registers of R rows leave.
 template <class ST>
 constexpr int res_warps(int rows) {
-  return rows <= 8 ? 16 : 12;
+  return 16;
 }
 
 // The plain form's pixels outside the circle in tiles without a pixel to solve.
@@ -1286,6 +1464,7 @@ int res_rows(int rows, F&& f) {
   if (rows == 8) return f(Res<MASKED, ST, 8>());
   if constexpr (!std::is_same<ST, float>::value) {
     if (rows == 12) return f(Res<MASKED, ST, 12>());
+    if (rows == 16) return f(Res<MASKED, ST, 16>());
   }
   return 0;
 }

@@ -5,11 +5,11 @@
 // A level is cut into tiles of 30 x R pixels, one warp each; only tiles that hold a pixel that
 // is on (or that such a pixel reads) exist.  Lane k of a warp is image column x0 - 1 + k: lanes
 // 1..30 own their column, lanes 0 and 31 hold the west and east halo.  A warp keeps u, u-bar,
-// v-bar, p and q of its rows in registers (float storage: p and q in shared memory) and the
-// level's coefficients in shared memory.  One iteration streams down the rows: the dual step of
-// row r needs u-bar and v-bar of row r + 1 (still the old values) and of the east lane; the
-// threshold and primal steps of row r need T p and q of the west lane and of row r - 1.  The
-// dual step of the west column and of the row above the tile is recomputed by the warp, so an
+// v-bar, p and q of its rows in registers and shared memory, with the level's coefficients beside
+// them.  One iteration streams down the rows: the dual step of row r needs u-bar and v-bar of row
+// r + 1 (still the old values) and of the east lane; the threshold and primal steps of row r need T p
+// and q of the west lane and of row r - 1.  The dual step of the west column and of the row above the
+// tile is recomputed by the warp, so an
 // iteration needs one exchange: u-bar and v-bar of the pixels around the tile.
 //
 // Exchange.  Every tile publishes the u-bar and v-bar of its border pixels as 16-byte words
@@ -30,11 +30,11 @@
 // that the other ping-pong buffers hold included (the state before the last iteration is
 // written there).
 //
-// What bounds it, on B200 (FP16 storage, 848 x 800, 2037 tiles of 8 rows, 3.9 us per iteration):
+// What bounds it, on B200 (FP16 storage, 848 x 800, 2037 tiles of 8 rows, 3.7 us per iteration):
 // about half of an iteration is instruction issue (1060 instructions per tile, 3.4 warps per
 // scheduler, close to one per cycle), the rest the exchange: 1100 to 1500 cycles from a
 // store to the load that sees it, and the wait for the slowest neighbour.  One launch per iteration
-// (k_fused_iter) takes 8.0 us there alone, bound by its loads; float storage 6.2 against 10.3 us.
+// (k_fused_iter) takes 8.0 us there alone, bound by its loads; float storage 6.1 against 10.3 us.
 // Small levels are all latency, so theirs runs in one cluster whose blocks write into each other's
 // shared memory (k_resident_cluster): 53 x 50 takes 0.90 us, through L2 1.39, one launch per
 // iteration 3.2.
@@ -50,8 +50,8 @@ constexpr int kResCols = 30;       // owned columns per tile
 constexpr int kResRing = 2;        // iterations of exchange words kept
 constexpr int kResMaxIters = 128;  // iterations per launch (a tag's low seven bits)
 // tile heights the kernel is built for (float storage: those up to 8)
-constexpr int kResRows[] = {2, 4, 6, 8, 12};
-constexpr int kResNumRows = 5;
+constexpr int kResRows[] = {2, 4, 6, 8, 12, 16};
+constexpr int kResNumRows = 6;
 constexpr int kResMostTiles = 148 * 16;  // a bound on the tiles of a plan (one warp each)
 // The cluster form (kernels_resident.cu, k_resident_cluster): 16 blocks, tiles of two rows, for levels of
 // up to so many tiles.  Beyond, the 16 SMs have more to issue than the shorter exchange saves (us per
