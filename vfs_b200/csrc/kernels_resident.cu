@@ -156,51 +156,65 @@ struct ResState<MASKED, __half, R> {
       for (int i = 0; i <= R; i++) p[i] = q0[i] = q1[i] = 0u;
     }
   }
+  // what a pixel has in memory (kept: masked out, with the other ping-pong buffer's values)
+  struct Pixel {
+    float4 ca;
+    float2 rv, tp;
+    float iu, iz, u, ub;
+    unsigned v;
+  };
+  static __device__ __forceinline__ Pixel fetch(const IterPair& P, int r, bool in, bool kept, int pos) {
+    Pixel x{make_float4(0.f, 0.f, 0.f, 1.f), make_float2(1.f, 1.f), make_float2(0.f, 0.f), 0.f, 0.f, 0.f, 0.f, 0u};
+    if (in) x.ca = P.abce[pos];
+    if (kept) x.tp = P.Tp[pos];
+    if (r < 0) return x;
+    if (!kTall && in) x.rv = P.rv[pos];
+    if (in) {
+      x.iu = P.Iu[pos];
+      x.iz = P.Iz[pos];
+      x.u = kept ? P.u_s[pos] : P.u[pos];
+      x.ub = P.u_[pos];
+    }
+    if (kept) x.v = bits(((const __half2*)P.v_s)[pos]);
+    return x;
+  }
   // east / south: edge codes of the pixel's right and lower neighbour
-  __device__ __forceinline__ bool set_row(Sh& sh, int lane, const IterPair& P, int r, bool in, int pos, unsigned code,
+  __device__ __forceinline__ bool set_row(Sh& sh, int lane, const IterPair&, int r, bool, bool kept, Pixel x, unsigned,
                                           unsigned east, unsigned south) {
-    float4 ca = make_float4(0.f, 0.f, 0.f, 1.f);
-    if (in) ca = P.abce[pos];
-    if (MASKED && in && !(code & kOn)) {
+    if (kept) {
       // read by the right / lower neighbour only where that one's other side is off too
-      const float2 tp = P.Tp[pos];
-      ca.x = (east & kOn) && !(east & kR) ? tp.x : 0.f;
-      ca.y = (south & kOn) && !(south & kD) ? tp.y : 0.f;
+      x.ca.x = (east & kOn) && !(east & kR) ? x.tp.x : 0.f;
+      x.ca.y = (south & kOn) && !(south & kD) ? x.tp.y : 0.f;
     }
     if (r < 0) {
-      sh.top[lane] = ca;
+      sh.top[lane] = x.ca;
       return false;
     }
     const int i = r >> 1, k = r & 1;
-    const float iu = in ? P.Iu[pos] : 0.f, iz = in ? P.Iz[pos] : 0.f;
     if constexpr (kTall) {
-      reinterpret_cast<float*>(&sh.ab[i][lane])[k] = ca.x;
-      reinterpret_cast<float*>(&sh.ab[i][lane])[2 + k] = ca.y;
-      reinterpret_cast<float*>(&sh.c[i][lane])[k] = ca.z;
+      reinterpret_cast<float*>(&sh.ab[i][lane])[k] = x.ca.x;
+      reinterpret_cast<float*>(&sh.ab[i][lane])[2 + k] = x.ca.y;
+      reinterpret_cast<float*>(&sh.c[i][lane])[k] = x.ca.z;
       if constexpr (!kStream) {
-        reinterpret_cast<float*>(&sh.uz[i][lane])[k] = iu;
-        reinterpret_cast<float*>(&sh.uz[i][lane])[2 + k] = iz;
+        reinterpret_cast<float*>(&sh.uz[i][lane])[k] = x.iu;
+        reinterpret_cast<float*>(&sh.uz[i][lane])[2 + k] = x.iz;
       }
     } else {
-      float2 rv = in ? P.rv[pos] : make_float2(1.f, 1.f);
       // eta_v2 = 0 (updatePrimalVariables.cu:103-105): .x takes tau itself, .y keeps its value
-      if (fast::etav2_zero(rv.y)) rv = make_float2(1.f, 0.f);
-      const float c[8] = {ca.x, ca.y, ca.z, ca.w, iu, iz, rv.x, rv.y};
+      if (fast::etav2_zero(x.rv.y)) x.rv = make_float2(1.f, 0.f);
+      const float c[8] = {x.ca.x, x.ca.y, x.ca.z, x.ca.w, x.iu, x.iz, x.rv.x, x.rv.y};
 #pragma unroll
       for (int j = 0; j < 8; j++) reinterpret_cast<float*>(&sh.cf[i][j >> 1][lane])[2 * (j & 1) + k] = c[j];
       // the Newton step -rho / Iu of the threshold; 0 where Iu = 0 (no step there)
-      reinterpret_cast<float*>(&sh.riu[i][lane])[k] = iu == 0.0f ? 0.0f : fast::rcp(iu);
+      reinterpret_cast<float*>(&sh.riu[i][lane])[k] = x.iu == 0.0f ? 0.0f : fast::rcp(x.iu);
     }
-    float un = in ? P.u[pos] : 0.f, ubn = in ? P.u_[pos] : 0.f;
     v[r] = 0u;
-    if (MASKED && in && !(code & kOn)) {  // the other ping-pong values of a masked-out pixel
-      un = P.u_s[pos];
-      const unsigned o = bits(((const __half2*)P.v_s)[pos]);
-      if constexpr (kSharedPQ) (k ? sh.p[i][lane].y : sh.p[i][lane].x) = o;
-      else p[r + 1] = o;
+    if (kept) {
+      if constexpr (kSharedPQ) (k ? sh.p[i][lane].y : sh.p[i][lane].x) = x.v;
+      else p[r + 1] = x.v;
     }
-    u[i] = k ? x2::pk(lo(u[i]), un) : x2::pk(un, 0.f);
-    ub[i] = k ? x2::pk(lo(ub[i]), ubn) : x2::pk(ubn, 0.f);
+    u[i] = k ? x2::pk(lo(u[i]), x.u) : x2::pk(x.u, 0.f);
+    ub[i] = k ? x2::pk(lo(ub[i]), x.ub) : x2::pk(x.ub, 0.f);
     return false;
   }
   __device__ __forceinline__ float u_of(int r) const { return r & 1 ? hi(u[r >> 1]) : lo(u[r >> 1]); }
@@ -593,53 +607,65 @@ struct ResState<MASKED, float, R> {
   static __device__ __forceinline__ bool beyond(float v) { return !(fabsf(v) <= kMost); }
   // in the range of the exact quotients
   static __device__ __forceinline__ bool ranged(float b) { return fabsf(b) >= 0x1p-100f && fabsf(b) <= 0x1p100f; }
-  // returns whether the pixel asks for the plain operators
-  __device__ __forceinline__ bool set_row(Sh& sh, int lane, const IterPair& P, int r, bool in, int pos, unsigned code,
-                                          unsigned east, unsigned south) {
-    float a = 0.f, b = 0.f, c = 0.f;
+  struct Pixel {
+    float a, b, c, iu, iz, u, ub;
+    float2 tp, v;
+  };
+  static __device__ __forceinline__ Pixel fetch(const IterPair& P, int r, bool in, bool kept, int pos) {
+    Pixel x{0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
     if (in) {
-      a = P.a[pos];
-      b = P.b[pos];
-      c = P.c[pos];
+      x.a = P.a[pos];
+      x.b = P.b[pos];
+      x.c = P.c[pos];
     }
+    if (kept) x.tp = P.Tp[pos];
+    if (r < 0) return x;
+    if (in) {
+      x.iu = P.Iu[pos];
+      x.iz = P.Iz[pos];
+      x.u = kept ? P.u_s[pos] : P.u[pos];
+      x.ub = P.u_[pos];
+    }
+    if (kept) x.v = ((const float2*)P.v_s)[pos];
+    return x;
+  }
+  // returns whether the pixel asks for the plain operators
+  __device__ __forceinline__ bool set_row(Sh& sh, int lane, const IterPair& P, int r, bool in, bool kept, Pixel x,
+                                          unsigned code, unsigned east, unsigned south) {
     bool plain = false;
     if (in && r >= 0 && (code & kOn)) {
-      const float eu = etau_math(a, b, c, P.alpha1), iu = P.Iu[pos];
-      const float e1 = etav1_math(b, c, P.alpha0, P.alpha1), e2 = etav2_math(a, c, P.alpha0, P.alpha1);
-      plain = !((eu == 0.0f || ranged(eu)) && ranged(e1) && ranged(e2) && (iu == 0.0f || ranged(iu)));
-      const float m = fmaxf(fmaxf(fabsf(a), fabsf(b)), fabsf(c)), eu1 = eu == 0.0f ? 1.0f : eu;
+      const float eu = etau_math(x.a, x.b, x.c, P.alpha1);
+      const float e1 = etav1_math(x.b, x.c, P.alpha0, P.alpha1), e2 = etav2_math(x.a, x.c, P.alpha0, P.alpha1);
+      plain = !((eu == 0.0f || ranged(eu)) && ranged(e1) && ranged(e2) && (x.iu == 0.0f || ranged(x.iu)));
+      const float m = fmaxf(fmaxf(fabsf(x.a), fabsf(x.b)), fabsf(x.c)), eu1 = eu == 0.0f ? 1.0f : eu;
       const float gv = fabsf(P.alpha1) * m + 4.0f * fabsf(P.alpha0);
-      plain = plain || !(m <= 0x1p8f && gv <= 0x1p14f && P.lambda * fabsf(iu) <= kRate * eu1 &&
+      plain = plain || !(m <= 0x1p8f && gv <= 0x1p14f && P.lambda * fabsf(x.iu) <= kRate * eu1 &&
                          4.0f * fmaxf(m, kMostTp) <= kRate * eu1 && gv <= kRate * e1 && gv <= kRate * e2);
     }
-    if (MASKED && in && !(code & kOn)) {
+    if (kept) {
       // read by the right / lower neighbour only where that one's other side is off too
-      const float2 tp = P.Tp[pos];
-      a = (east & kOn) && !(east & kR) ? tp.x : 0.f;
-      b = (south & kOn) && !(south & kD) ? tp.y : 0.f;
-      plain = plain || !(fabsf(a) <= kMostTp) || !(fabsf(b) <= kMostTp);
+      x.a = (east & kOn) && !(east & kR) ? x.tp.x : 0.f;
+      x.b = (south & kOn) && !(south & kD) ? x.tp.y : 0.f;
+      plain = plain || !(fabsf(x.a) <= kMostTp) || !(fabsf(x.b) <= kMostTp);
     }
     if (r < 0) {
-      sh.top[lane] = make_float4(a, b, c, 0.f);
+      sh.top[lane] = make_float4(x.a, x.b, x.c, 0.f);
       return plain;
     }
     const int i = r >> 1, k = r & 1;
-    el(sh.ab[i][lane], k) = a;
-    el(sh.ab[i][lane], 2 + k) = b;
-    el(sh.ci[i][lane], k) = c;
-    el(sh.ci[i][lane], 2 + k) = in ? P.Iu[pos] : 0.f;
-    reinterpret_cast<float*>(&sh.iz[i][lane])[k] = in ? P.Iz[pos] : 0.f;
-    float un = in ? P.u[pos] : 0.f, ubn = in ? P.u_[pos] : 0.f;
-    plain = plain || beyond(un) || beyond(ubn);
-    if (MASKED && in && !(code & kOn)) {  // the other ping-pong values of a masked-out pixel
-      un = P.u_s[pos];
-      const float2 o = ((const float2*)P.v_s)[pos];
-      plain = plain || beyond(un) || beyond(o.x) || beyond(o.y);
-      el(sh.p[i][lane], k) = o.x;
-      el(sh.p[i][lane], 2 + k) = o.y;
+    el(sh.ab[i][lane], k) = x.a;
+    el(sh.ab[i][lane], 2 + k) = x.b;
+    el(sh.ci[i][lane], k) = x.c;
+    el(sh.ci[i][lane], 2 + k) = x.iu;
+    reinterpret_cast<float*>(&sh.iz[i][lane])[k] = x.iz;
+    plain = plain || beyond(x.u) || beyond(x.ub);
+    if (kept) {
+      plain = plain || beyond(x.v.x) || beyond(x.v.y);
+      el(sh.p[i][lane], k) = x.v.x;
+      el(sh.p[i][lane], 2 + k) = x.v.y;
     }
-    u[i] = k ? x2::pk(lo(u[i]), un) : x2::pk(un, 0.f);
-    ub[i] = k ? x2::pk(lo(ub[i]), ubn) : x2::pk(ubn, 0.f);
+    u[i] = k ? x2::pk(lo(u[i]), x.u) : x2::pk(x.u, 0.f);
+    ub[i] = k ? x2::pk(lo(ub[i]), x.ub) : x2::pk(x.ub, 0.f);
     vx[i] = vy[i] = x2::pk(0.f, 0.f);
     return plain;
   }
@@ -969,38 +995,54 @@ struct ResWarp {
   // kind; with two kinds in turn on an SM the rarer one ran from the instruction cache's misses
   // (848 x 800: 5900 cycles a tile without edge rules, 8700 with, 7.1 us per iteration; one kind 6.16).
   static constexpr bool kInner = !kPlain || R < 8;
-  ResState<MASKED, ST, R> s;
+  static constexpr int kAtOnce = 3;  // rows fetched before the first is used
+  typedef ResState<MASKED, ST, R> State;
+  State s;
 
-  // Loads tile t: its coefficients, codes and state before the first iteration.
-  __device__ __forceinline__ ResEdge load(Sh& sh, const ResArgs& A, int lane, int t) {
+  // Loads tile t: its coefficients, codes and state before the first iteration.  All the codes are asked
+  // for at once, and the values of a few rows at a time, so that a tile waits for memory four or five
+  // times and not for every row anew (848 x 800 float: 2 us less a launch, 33 of a solve's 2230).
+  __device__ __forceinline__ ResEdge load(Sh& sh, const ResArgs& A, int lane, int t, const ResTile& T) {
     const IterPair& P = A.P;
-    const ResTile& T = A.tiles[t];
     const int x = T.x0 - 1 + lane, y0 = T.y0;
     const bool x_in = x >= 0 && x < P.w;
     ResEdge e{0u, 0u, 0u};
     bool plain = false;
+    auto inside = [&](int r) { return x_in && y0 + r >= 0 && y0 + r < P.h; };
+    unsigned codes[R + 1];
+#pragma unroll
+    for (int r = -1; r < R; r++) codes[r + 1] = inside(r) ? P.code[x + (y0 + r) * P.s] : 0u;
     s.clear(sh, lane);
 #pragma unroll
-    for (int r = -1; r < R; r++) {
-      const int y = y0 + r, pos = x + y * P.s;
-      const bool in = x_in && y >= 0 && y < P.h;
-      unsigned code = 0, east = 0, south = 0;
-      if (in) {
-        code = P.code[pos];
-        if (!MASKED) {
+    for (int first = -1; first < R; first += kAtOnce) {
+      typename State::Pixel px[kAtOnce];
+      unsigned east[kAtOnce], south[kAtOnce];
+#pragma unroll
+      for (int k = 0; k < kAtOnce; k++) {
+        const int r = first + k, pos = x + (y0 + r) * P.s;
+        if (r >= R) break;
+        unsigned& code = codes[r + 1];
+        const bool in = inside(r), kept = MASKED && in && !(code & kOn);
+        px[k] = State::fetch(P, r, in, kept, pos);
+        east[k] = kept && (code & kR) ? P.code[pos + 1] : 0u;
+        south[k] = kept && (code & kD) ? P.code[pos + P.s] : 0u;
+        if (!MASKED && in) {
           code &= kOn;
-          code |= (x + 1 < P.w ? kR : 0) | (x >= 1 ? kL : 0) | (y + 1 < P.h ? kD : 0) | (y >= 1 ? kU : 0);
-        } else if (!(code & kOn)) {
-          if (code & kR) east = P.code[pos + 1];
-          if (code & kD) south = P.code[pos + P.s];
+          code |= (x + 1 < P.w ? kR : 0) | (x >= 1 ? kL : 0) | (y0 + r + 1 < P.h ? kD : 0) | (y0 + r >= 1 ? kU : 0);
         }
       }
-      plain = s.set_row(sh, lane, P, r, in, pos, code, east, south) || plain;
-      const unsigned b = 1u << (r + 1);
-      if (code & kOn) {
-        e.on |= b;
-        if (code & kR) e.x |= b;
-        if (code & kD) e.y |= b;
+#pragma unroll
+      for (int k = 0; k < kAtOnce; k++) {
+        const int r = first + k;
+        if (r >= R) break;
+        const unsigned code = codes[r + 1], b = 1u << (r + 1);
+        const bool in = inside(r), kept = MASKED && in && !(code & kOn);
+        plain = s.set_row(sh, lane, P, r, in, kept, px[k], code, east[k], south[k]) || plain;
+        if (code & kOn) {
+          e.on |= b;
+          if (code & kR) e.x |= b;
+          if (code & kD) e.y |= b;
+        }
       }
     }
     sh.k.edge[lane] = make_uint2(e.y, e.on);
@@ -1015,8 +1057,7 @@ struct ResWarp {
   // Where this lane finds its neighbours' words.  A missing neighbour is replaced by this tile itself:
   // the tags come, the values are not used.  Lanes 0 .. R-1 fetch the west column, lanes 16 .. 16 + R-1
   // the east one.
-  __device__ __forceinline__ void link(Sh& sh, const ResArgs& A, int lane, int t, const ResEdge& e) {
-    const ResTile& T = A.tiles[t];
+  __device__ __forceinline__ void link(Sh& sh, int lane, const ResTile& T, const ResEdge& e) {
     const int tn = lane == 0 ? T.nb[4] : lane == 31 ? T.nb[5] : T.nb[0];
     const int ts = lane == 0 ? T.nb[6] : lane == 31 ? T.nb[7] : T.nb[1];
     const int col = lane == 0 ? kResCols : lane == 31 ? 1 : lane;
@@ -1179,7 +1220,8 @@ __global__ void __launch_bounds__(32 * res_warps<ST>(R), 1) k_resident(const __g
 
   if (t < A.ntiles) {
     ResWarp<MASKED, ST, R> W;
-    W.link(sh, A, lane, t, W.load(sh, A, lane, t));
+    const ResTile T = A.tiles[t];
+    W.link(sh, lane, T, W.load(sh, A, lane, t, T));
     publish<R>(W.s, A.exch + (size_t)t * (64 + 2 * R), lane, epoch | W.flag(sh));  // iteration 0's input
     __syncwarp();
     bool waiting = true;
@@ -1314,8 +1356,8 @@ __global__ void __launch_bounds__(512, 1) k_resident_cluster(const __grid_consta
   ResWarp<MASKED, ST, R> W;
   unsigned ex = 0;
   if (t < A.ntiles) {
-    const ResTile& T = A.tiles[t];
-    ex = W.load(sh, A, lane, t).x;
+    const ResTile T = A.tiles[t];
+    ex = W.load(sh, A, lane, t, T).x;
     auto words = [&](int k, const void* field) {  // the same field of tile k's shared memory
       const unsigned local = (unsigned)__cvta_generic_to_shared(field) + (unsigned)((k / ctas - warp) * (int)sizeof(Tile));
       return cl_addr(local, (unsigned)(k % ctas));
