@@ -316,7 +316,7 @@ def error_stats(us, refs, masks):
 def accuracy_report(pairs, u_timed, u64_first, half, dev):
     """Disparity error against the float64 oracle over every pair of the batch, inside the
     masks, for the timed form and the other two forms on the same inputs: the fused solve with
-    the other storage, and the plain drop-in path (one kernel per reference kernel)."""
+    the other storage, and the plain drop-in path."""
     import torch
     from vfs_b200.stereotgv import StereoBatch
     st = torch.cuda.Stream(device=dev)
@@ -353,8 +353,7 @@ def accuracy_report(pairs, u_timed, u64_first, half, dev):
 
 
 def plain_reference_run(pair, dev, flush, steps=6):
-    """The drop-in path (one kernel per reference kernel, FP32, one pair at a time) on the
-    same GPU and inputs: frames/s with device-resident inputs, L2 flushed before each frame."""
+    """The drop-in path (FP32, one pair at a time) on the same GPU and inputs: frames/s with device-resident inputs, L2 flushed before each frame."""
     import torch
     st = torch.cuda.Stream(device=dev)
     s = make_solver(pair, "plain", st)
@@ -464,10 +463,11 @@ def run_ours(args, rank, world, local):
             flush.fill_(float(k))
         device_step()
     torch.cuda.synchronize()
-    # roofline of the inner primal-dual loop: kind 0 (drop-in, one record per iteration)
+    # roofline of the inner primal-dual loop: kind 1, or 0 (drop-in path on a pair that has a level
+    # which does not fit on the chip: one record per iteration)
     # Pairs solved on concurrent streams overlap, so the time is the union of the records'
     # intervals (time during which at least one inner group ran), not their sum.
-    kind = 1 if args.path == "fused" else 0
+    kind = 1 if args.path == "fused" or any(len(s.profile_intervals(1)) for s in solvers) else 0
     iv = np.concatenate([s.profile_intervals(kind) for s in solvers])
     for s in solvers:
         s.profile(False)

@@ -42,7 +42,7 @@ void set_iter_tiles(IterArgs& A, int k, int w, int h, int rows) {
 // in flight it weighs the GPU time a variant takes from the others, and alone its latency.
 // part: 0 the whole solve; 1 the calibration warp, the pyramid and the levels above full
 // resolution (ending with the upscale to it); 2 the full-resolution level alone.  Running part 1
-// then part 2 enqueues exactly what part 0 does.
+// then part 2 does exactly what part 0 does.
 // dropin: the drop-in path (one pair, float storage, every level register-resident): p and q in the
 // pool's single planes, and the preconditioners and the last change of u left where its own kernels do.
 void fused_solve_direct(std::vector<StereoTgvImpl*>& pairs, bool masked, bool half, cudaStream_t st,
@@ -73,9 +73,11 @@ void fused_solve_direct(std::vector<StereoTgvImpl*>& pairs, bool masked, bool ha
   if (part != 2) {
   for (int k = 0; k < n; k++) {
     StereoTgvImpl* s = pairs[k];
-    launch_warp_image(s->tex1(s->pI1[0], 0), s->d_cv, s->d_i1calibrated, s->geomAt(0), st);
+    const cudaTextureObject_t i1 = s->tex1(s->pI1[0], 0);
+    if (s->warmStart()) launch_warp_image(i1, s->d_cv, s->d_i1calibrated, s->geomAt(0), st);
+    else launch_warp_image_reset(i1, s->d_cv, s->d_i1calibrated, s->d_u, s->d_u_, s->d_warpUV, s->geomAt(0), st);
     std::swap(s->pI1[0], s->d_i1calibrated);
-    s->startState(top[k], st);
+    if (s->warmStart()) s->startState(top[k], st);
   }
   for (int l = 1; l < maxL; l++) {
     DownArgs D{};
@@ -98,6 +100,43 @@ void fused_solve_direct(std::vector<StereoTgvImpl*>& pairs, bool masked, bool ha
   }
   }  // part != 2
   // ---- levels -------------------------------------------------------------------------
+  auto level_args = [&](const std::vector<StereoTgvImpl*>& on, int level) {
+    LevelArgs L{};
+    for (int k = 0; k < (int)on.size(); k++) {
+      StereoTgvImpl* s = on[k];
+      LevelPair& d = L.pr[k];
+      d.texI0 = s->tex1(s->pI0[level], level);
+      d.texSmooth = s->tex1(s->d_i0smooth, level);
+      d.mask = masked ? s->pMask[level] : nullptr;
+      d.i0smooth = s->d_i0smooth;
+      d.a = s->d_a;
+      d.b = s->d_b;
+      d.c = s->d_c;
+      d.warpUV = s->d_warpUV;
+      d.u = s->d_u;
+      d.tv = s->pTvF[level];
+      d.init_flow = level == top_of(s);
+      d.w = s->pW[level];
+      d.h = s->pH[level];
+      d.s = s->pS[level];
+      int xcov = ((d.h + s->blockWidth - 1) / s->blockWidth) * s->blockWidth;  // calcTensor.cu:81,227
+      d.xmax = std::min(d.w, xcov);
+      d.beta = s->P.beta;
+      d.gamma = s->P.gamma;
+      d.cuda_math = s->tensor_cuda_math;
+      d.abce = half ? s->f_abce : nullptr;
+      d.rv = half ? s->f_rv : nullptr;
+      d.etau = dropin ? s->d_etau : nullptr;
+      d.etav1 = s->d_etav1;
+      d.etav2 = s->d_etav2;
+      d.alpha0 = s->P.alpha0;
+      d.alpha1 = s->P.alpha1;
+      set_tiles(L, k, d.w, d.h);
+    }
+    L.npairs = (int)on.size();
+    return L;
+  };
+  bool smoothed = false;  // the level's gaussian ran with the upscale to it
   for (int level = maxL - 1; level >= 0; level--) {
     if ((part == 1 && level == 0) || (part == 2 && level > 0)) continue;
     TraceRange trace(level_range_name(level));
@@ -108,43 +147,10 @@ void fused_solve_direct(std::vector<StereoTgvImpl*>& pairs, bool masked, bool ha
     const int na = (int)act.size();
     long long px_level = 0;
     for (auto* s : act) px_level += (long long)s->pW[level] * s->pH[level];
-    {
-      LevelArgs L{};
-      for (int k = 0; k < na; k++) {
-        StereoTgvImpl* s = act[k];
-        LevelPair& d = L.pr[k];
-        d.texI0 = s->tex1(s->pI0[level], level);
-        d.texSmooth = s->tex1(s->d_i0smooth, level);
-        d.mask = masked ? s->pMask[level] : nullptr;
-        d.i0smooth = s->d_i0smooth;
-        d.a = s->d_a;
-        d.b = s->d_b;
-        d.c = s->d_c;
-        d.warpUV = s->d_warpUV;
-        d.u = s->d_u;
-        d.tv = s->pTvF[level];
-        d.init_flow = level == top_of(s);
-        d.w = s->pW[level];
-        d.h = s->pH[level];
-        d.s = s->pS[level];
-        int xcov = ((d.h + s->blockWidth - 1) / s->blockWidth) * s->blockWidth;  // calcTensor.cu:81,227
-        d.xmax = std::min(d.w, xcov);
-        d.beta = s->P.beta;
-        d.gamma = s->P.gamma;
-        d.cuda_math = s->tensor_cuda_math;
-        d.abce = half ? s->f_abce : nullptr;
-        d.rv = half ? s->f_rv : nullptr;
-        d.etau = dropin ? s->d_etau : nullptr;
-        d.etav1 = s->d_etav1;
-        d.etav2 = s->d_etav2;
-        d.alpha0 = s->P.alpha0;
-        d.alpha1 = s->P.alpha1;
-        set_tiles(L, k, d.w, d.h);
-      }
-      L.npairs = na;
-      launch_level_gaussian(L, st);
-      launch_level_tensor(L, st);
-    }
+    const LevelArgs lev = level_args(act, level);
+    if (!smoothed) launch_level_gaussian(lev, st);
+    smoothed = false;
+    if (P0.nWarpIters == 0) launch_level_tensor(lev, st);
     // the per-warp prologue's arguments (the current v-bar buffer is the one the iterations
     // left current, so the same call serves a warp's start and the previous warp's epilogue)
     // (the register-resident iteration starts from p = q = 0 by itself; the drop-in path's last
@@ -175,7 +181,7 @@ void fused_solve_direct(std::vector<StereoTgvImpl*>& pairs, bool masked, bool ha
     for (int warpIter = 0; warpIter < P0.nWarpIters; warpIter++) {
       prof->profBeginPx(kProfPrologue, px_level, 1, st);
       // later warps' prologues run in the previous warp's epilogue launch
-      if (warpIter == 0) launch_warp_start(warp_start_args(0), half, st);
+      if (warpIter == 0) launch_tensor_warp_start(lev, warp_start_args(0), half, st);
       {
         DerivArgs Dv{};
         for (int k = 0; k < na; k++) {
@@ -517,7 +523,11 @@ void fused_solve_direct(std::vector<StereoTgvImpl*>& pairs, bool masked, bool ha
         k++;
       }
       U.npairs = k;
-      launch_upscale_batched(U, st);
+      // (a solve in two parts is cut behind the upscale)
+      smoothed = part == 0;
+      for (int p = 0; p < n; p++) smoothed = smoothed && top[p] != level - 1;
+      if (smoothed) launch_upscale_gaussian(U, level_args(act, level - 1), st);
+      else launch_upscale_batched(U, st);
       for (auto* s : act) {
         std::swap(s->d_u, s->d_us);
         std::swap(s->d_u_, s->d_u_s);

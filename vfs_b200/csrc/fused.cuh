@@ -190,7 +190,6 @@ struct WarpStartArgs {
   int npairs, ntiles;
   WarpStartPair pr[kMaxPairs];
 };
-void launch_warp_start(const WarpStartArgs& A, bool half_storage, cudaStream_t st);
 
 // ---- derivatives along the translation field + u_last = u -----------------------
 struct DerivPair {
@@ -254,6 +253,8 @@ struct LevelArgs {
 };
 void launch_level_gaussian(const LevelArgs& A, cudaStream_t st);
 void launch_level_tensor(const LevelArgs& A, cudaStream_t st);
+// The level's tensor and the first warp's prologue in one launch (the same tiles).
+void launch_tensor_warp_start(const LevelArgs& A, const WarpStartArgs& B, bool half_storage, cudaStream_t st);
 
 // ---- upscale u, u-bar and warpUV to the next finer level in one pass --------------
 struct UpPair {
@@ -268,6 +269,9 @@ struct UpArgs {
   UpPair pr[kMaxPairs];
 };
 void launch_upscale_batched(const UpArgs& A, cudaStream_t st);
+// The upscale to a level and that level's gaussian in one launch (the same pairs, none of which starts
+// at that level).
+void launch_upscale_gaussian(const UpArgs& A, const LevelArgs& B, cudaStream_t st);
 
 // ---- pyramid: downscale I0 and I1 of every pair to the next coarser level --------
 struct DownPair {

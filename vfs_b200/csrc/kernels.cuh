@@ -27,6 +27,9 @@ void launch_downscale_scaled(cudaTextureObject_t fine, float* out, float scale, 
 void launch_downscale_nearest(cudaTextureObject_t fine, float* out, Geom coarse, cudaStream_t st);
 // warpImage.cu:9-23
 void launch_warp_image(cudaTextureObject_t src, const float2* warpUV, float* out, Geom g, cudaStream_t st);
+// launch_warp_image, and u, u_ and flow zero over the level's g.s x g.h
+void launch_warp_image_reset(cudaTextureObject_t src, const float2* warpUV, float* out, float* u, float* u_,
+                             float2* flow, Geom g, cudaStream_t st);
 // warpImage.cu:96-111
 void launch_find_warping_vector(cudaTextureObject_t tv, const float2* warpUV, float2* tv2, Geom g,
                                 cudaStream_t st);

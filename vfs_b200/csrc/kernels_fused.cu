@@ -424,22 +424,6 @@ __device__ __forceinline__ void warp_start_at(const WarpStartPair& P, int ix, in
   ((ST*)P.i1warp)[pos] = (ST)tex2D<float>(P.texI1, x, y);
 }
 
-template <class ST>
-__global__ void __launch_bounds__(kFTW* kFTH) k_warp_start(const __grid_constant__ WarpStartArgs A) {
-  TILE_SETUP(A)
-  if (ix >= P.w || iy >= P.h) return;
-  long long pos = ix + (long long)iy * P.s;
-  warp_start_at<ST>(P, ix, iy, pos, P.warpUV[pos]);
-}
-
-void launch_warp_start(const WarpStartArgs& A, bool half_storage, cudaStream_t st) {
-  if (A.ntiles <= 0) return;
-  dim3 blk(kFTW, kFTH);
-  if (half_storage) k_warp_start<__half><<<A.ntiles, blk, 0, st>>>(A);
-  else k_warp_start<float><<<A.ntiles, blk, 0, st>>>(A);
-  VFS_LAUNCH_CHECK();
-}
-
 // computeDerivatives.cu:89-129 and Clone(u_last, u) (stereotgv.cu:447)
 __global__ void __launch_bounds__(kFTW* kFTH) k_derivatives_b(const __grid_constant__ DerivArgs A) {
   TILE_SETUP(A)
@@ -531,10 +515,7 @@ void launch_warp_epilogue_batched(const EpiArgs& A, cudaStream_t st) {
 // calcTensor.cu:99-128 / 245-273 with the per-level zeroing of stereotgv.cu:409-415:
 // i0smooth = gaussian where computed, 0 elsewhere (level footprint); at a pair's
 // coarsest level also warpUV = u * tv (stereotgv.cu:419-421).
-__global__ void __launch_bounds__(kFTW* kFTH) k_level_gaussian(const __grid_constant__ LevelArgs A) {
-  TILE_SETUP(A)
-  if (ix >= P.w || iy >= P.h) return;
-  long long pos = ix + (long long)iy * P.s;
+__device__ __forceinline__ void level_gaussian_at(const LevelPair& P, int ix, int iy, long long pos) {
   if (P.init_flow) {
     float us = P.u[pos];
     float2 t = P.tv[pos];
@@ -559,6 +540,12 @@ __global__ void __launch_bounds__(kFTW* kFTH) k_level_gaussian(const __grid_cons
   P.i0smooth[pos] = t0;
 }
 
+__global__ void __launch_bounds__(kFTW* kFTH) k_level_gaussian(const __grid_constant__ LevelArgs A) {
+  TILE_SETUP(A)
+  if (ix >= P.w || iy >= P.h) return;
+  level_gaussian_at(P, ix, iy, ix + (long long)iy * P.s);
+}
+
 // The half-storage iteration's per-level records at one pixel: (a, b, c, 1 / eta_u) and
 // (1 / eta_v1, 1 / eta_v2), formed by the same expressions the iteration kernels use
 // (tgv_pixel_fast.cuh, a1s = alpha1^2, a0s4 = 4 alpha0^2), so reading them gives the bits of
@@ -578,10 +565,7 @@ __device__ __forceinline__ void level_etas(const LevelPair& P, long long pos, fl
 
 // calcTensor.cu:8-73 / 155-219; a = b = c = 0 where the reference does not compute
 // (masked out, or columns >= xmax of its launch grid)
-__global__ void __launch_bounds__(kFTW* kFTH) k_level_tensor(const __grid_constant__ LevelArgs A) {
-  TILE_SETUP(A)
-  if (ix >= P.w || iy >= P.h) return;
-  long long pos = ix + (long long)iy * P.s;
+__device__ __forceinline__ void level_tensor_at(const LevelPair& P, int ix, int iy, long long pos) {
   if (ix >= P.xmax || (P.mask && P.mask[pos] == 0.0f)) {
     P.a[pos] = 0.0f;
     P.b[pos] = 0.0f;
@@ -613,28 +597,77 @@ __global__ void __launch_bounds__(kFTW* kFTH) k_level_tensor(const __grid_consta
   if (P.etau) level_etas(P, pos, a, b, c, false);
 }
 
-void launch_level_gaussian(const LevelArgs& A, cudaStream_t st) {
+__global__ void __launch_bounds__(kFTW* kFTH) k_level_tensor(const __grid_constant__ LevelArgs A) {
+  TILE_SETUP(A)
+  if (ix >= P.w || iy >= P.h) return;
+  level_tensor_at(P, ix, iy, ix + (long long)iy * P.s);
+}
+
+// A level begins with the upscale to it and its gaussian, which touch different buffers, and then its
+// tensor and the first warp's prologue, which do as well: each two are one launch.  A small level's
+// kernel takes 2 to 4 us whatever it does (848 x 800 half, five levels: 1593 -> 1572 us).
+template <class ST>
+__global__ void __launch_bounds__(kFTW* kFTH) k_tensor_warp_start(const __grid_constant__ LevelArgs A,
+                                                                 const __grid_constant__ WarpStartArgs B) {
+  TILE_SETUP(A)
+  if (ix >= P.w || iy >= P.h) return;
+  const long long pos = ix + (long long)iy * P.s;
+  const WarpStartPair& W = B.pr[pi_];
+  warp_start_at<ST>(W, ix, iy, pos, W.warpUV[pos]);
+  level_tensor_at(P, ix, iy, pos);
+}
+
+void launch_tensor_warp_start(const LevelArgs& A, const WarpStartArgs& B, bool half_storage, cudaStream_t st) {
   if (A.ntiles <= 0) return;
-  k_level_gaussian<<<A.ntiles, dim3(kFTW, kFTH), 0, st>>>(A);
+  if (B.npairs != A.npairs || B.ntiles != A.ntiles) throw ArgError{"tensor and warp start tiles differ"};
+  dim3 blk(kFTW, kFTH);
+  if (half_storage) k_tensor_warp_start<__half><<<A.ntiles, blk, 0, st>>>(A, B);
+  else k_tensor_warp_start<float><<<A.ntiles, blk, 0, st>>>(A, B);
   VFS_LAUNCH_CHECK();
 }
+
 void launch_level_tensor(const LevelArgs& A, cudaStream_t st) {
   if (A.ntiles <= 0) return;
   k_level_tensor<<<A.ntiles, dim3(kFTW, kFTH), 0, st>>>(A);
   VFS_LAUNCH_CHECK();
 }
 
+void launch_level_gaussian(const LevelArgs& A, cudaStream_t st) {
+  if (A.ntiles <= 0) return;
+  k_level_gaussian<<<A.ntiles, dim3(kFTW, kFTH), 0, st>>>(A);
+  VFS_LAUNCH_CHECK();
+}
+
 // upscale.cu:8-21, 46-61 for u, u-bar and warpUV (stereotgv.cu:497-510)
-__global__ void __launch_bounds__(kFTW* kFTH) k_upscale3(const __grid_constant__ UpArgs A) {
-  TILE_SETUP(A)
-  if (ix >= P.w || iy >= P.h) return;
-  long long pos = ix + (long long)iy * P.s;
+__device__ __forceinline__ void upscale_at(const UpPair& P, int ix, int iy, long long pos) {
   float x = ((float)ix + 0.5f) / (float)P.w;
   float y = ((float)iy + 0.5f) / (float)P.h;
   P.u_out[pos] = tex2D<float>(P.texU, x, y) * P.scale;
   P.ubar_out[pos] = tex2D<float>(P.texUbar, x, y) * P.scale;
   float2 v = tex2D<float2>(P.texWarp, x, y);
   P.warp_out[pos] = make_float2(v.x * P.scale, v.y * P.scale);
+}
+
+__global__ void __launch_bounds__(kFTW* kFTH) k_upscale3(const __grid_constant__ UpArgs A) {
+  TILE_SETUP(A)
+  if (ix >= P.w || iy >= P.h) return;
+  upscale_at(P, ix, iy, ix + (long long)iy * P.s);
+}
+
+__global__ void __launch_bounds__(kFTW* kFTH) k_upscale_gaussian(const __grid_constant__ UpArgs A,
+                                                                const __grid_constant__ LevelArgs B) {
+  TILE_SETUP(A)
+  if (ix >= P.w || iy >= P.h) return;
+  const long long pos = ix + (long long)iy * P.s;
+  upscale_at(P, ix, iy, pos);
+  level_gaussian_at(B.pr[pi_], ix, iy, pos);
+}
+
+void launch_upscale_gaussian(const UpArgs& A, const LevelArgs& B, cudaStream_t st) {
+  if (A.ntiles <= 0) return;
+  if (B.npairs != A.npairs || B.ntiles != A.ntiles) throw ArgError{"upscale and gaussian tiles differ"};
+  k_upscale_gaussian<<<A.ntiles, dim3(kFTW, kFTH), 0, st>>>(A, B);
+  VFS_LAUNCH_CHECK();
 }
 
 void launch_upscale_batched(const UpArgs& A, cudaStream_t st) {

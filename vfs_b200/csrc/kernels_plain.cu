@@ -113,14 +113,32 @@ __global__ void k_downscale_nearest(cudaTextureObject_t fine, float* out, Geom g
   out[ix + iy * g.s] = tex2D<float>(fine, x, y);
 }
 
-__global__ void k_warp_image(cudaTextureObject_t src, const float2* __restrict__ warpUV, float* out, Geom g) {
-  int ix, iy;
-  if (!pixel(ix, iy, g.w, g.h)) return;
+__device__ __forceinline__ void warp_image_at(cudaTextureObject_t src, const float2* __restrict__ warpUV, float* out,
+                                             Geom g, int ix, int iy) {
   int pos = ix + iy * g.s;
   float2 wv = warpUV[pos];
   float x = ((float)ix + wv.x + 0.5f) / (float)g.w;
   float y = ((float)iy + wv.y + 0.5f) / (float)g.h;
   out[pos] = tex2D<float>(src, x, y);
+}
+
+__global__ void k_warp_image(cudaTextureObject_t src, const float2* __restrict__ warpUV, float* out, Geom g) {
+  int ix, iy;
+  if (!pixel(ix, iy, g.w, g.h)) return;
+  warp_image_at(src, warpUV, out, g, ix, iy);
+}
+
+// With the state's reset, which was three memsets of a solve's start (in a graph about 2 us each, whatever
+// their size: 96 x 64 half 182 -> 177 us, 848 x 800 half 1572 -> 1567).
+__global__ void k_warp_image_reset(cudaTextureObject_t src, const float2* __restrict__ warpUV, float* out, float* u,
+                                   float* u_, float2* flow, Geom g) {
+  int ix, iy;
+  if (!pixel(ix, iy, g.s, g.h)) return;
+  const int pos = ix + iy * g.s;
+  u[pos] = 0.0f;
+  u_[pos] = 0.0f;
+  flow[pos] = make_float2(0.0f, 0.0f);
+  if (ix < g.w) warp_image_at(src, warpUV, out, g, ix, iy);
 }
 
 __global__ void k_find_warping_vector(cudaTextureObject_t tv, const float2* __restrict__ warpUV, float2* tv2,
@@ -533,6 +551,12 @@ void launch_downscale_nearest(cudaTextureObject_t fine, float* out, Geom g, cuda
 }
 void launch_warp_image(cudaTextureObject_t src, const float2* warpUV, float* out, Geom g, cudaStream_t st) {
   k_warp_image<<<L2D(g)>>>(src, warpUV, out, g);
+  VFS_LAUNCH_CHECK();
+}
+void launch_warp_image_reset(cudaTextureObject_t src, const float2* warpUV, float* out, float* u, float* u_,
+                             float2* flow, Geom g, cudaStream_t st) {
+  const Geom all{g.s, g.h, g.s};
+  k_warp_image_reset<<<L2D(all)>>>(src, warpUV, out, u, u_, flow, g);
   VFS_LAUNCH_CHECK();
 }
 void launch_find_warping_vector(cudaTextureObject_t tv, const float2* warpUV, float2* tv2, Geom g, cudaStream_t st) {

@@ -432,7 +432,7 @@ void StereoTgvImpl::solve(bool masked) {
 
 void StereoTgvImpl::startState(int top, cudaStream_t st) {
   const size_t f = full_ * sizeof(float);
-  if (!(warm_level >= 0 && have_prev)) {  // stereotgv.cu:395-397
+  if (!warmStart()) {  // stereotgv.cu:395-397
     VFS_CUDA(cudaMemsetAsync(d_u, 0, f, st));
     VFS_CUDA(cudaMemsetAsync(d_u_, 0, f, st));
     VFS_CUDA(cudaMemsetAsync(d_warpUV, 0, 2 * f, st));

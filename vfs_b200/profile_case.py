@@ -7,14 +7,14 @@ unless --autotune 1, so the launch sequence is fixed).
                                     [--variant -1..18] [--variants 1,1,8,9,9]
 
 Launch order per frame: pyramid, then per level (coarse to fine) the level kernels and per
-warp the prologue (k_warp_start, first warp of a level only), the derivatives, the fused
-iterations and the epilogue (k_epilogue_warp_start, which also runs the next warp's prologue,
-or k_epilogue_b after a level's last warp).  With the default iteration
-variant (or --variant 0..2) each warp has 50 one-iteration launches: in the concurrent mode
-each pair's solve is enqueued in turn (pair 0 first), so k_fused_iter launches 600..749 are
-pair 0's full-resolution iterations (one pair per launch); in the one-launch mode every
-launch carries all pairs, and launches 600..749 are the full-resolution iterations of the
-batch.  With --variant 6..9 or 12..13 (K iterations per launch) each warp has 50 / K launches
+warp the prologue (with the tensor in k_tensor_warp_start, first warp of a level only), the
+derivatives, the iterations and the epilogue (k_epilogue_warp_start, which also runs the next
+warp's prologue, or k_epilogue_b after a level's last warp).  In the concurrent mode each pair's
+solve is enqueued in turn (pair 0 first), and each warp of a level that fits on the chip has one
+launch, of k_resident or, small levels, k_resident_cluster.  With --variant 0..2 (and in
+the one-launch mode) each warp has 50 one-iteration launches: k_fused_iter launches 600..749 are
+pair 0's full-resolution iterations; in the one-launch mode every launch carries all pairs, and
+launches 600..749 are the full-resolution iterations of the batch.  With --variant 6..9 or 12..13 (K iterations per launch) each warp has 50 / K launches
 of k_fused_iter_tb, coarsest level first; with --variant 14..15 each warp of a level that fits
 a cluster's shared memory has one launch of k_fused_iter_cluster.
 """

@@ -116,7 +116,7 @@ class StereoTgv:
         return n.value
 
     def set_solve_path(self, fused: bool, half_storage: bool = False) -> None:
-        """Select the drop-in path (one kernel per reference kernel) or the fused path
+        """Select the drop-in path (the reference's results bit for bit) or the fused path
         (optionally with p, q, v-bar and the warped image stored as half)."""
         check(self._h, self._L.vfs_set_solve_path(self._h, PATH_FUSED if fused else PATH_REFERENCE,
                                                   int(half_storage)))
