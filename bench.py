@@ -535,7 +535,9 @@ def run_ours(args, rank, world, local):
         achieved = (pi_l * b_alg / (ms_l / 1000.0) / 1e9) if ms_l > 0 else None
         achieved_all = (pi_all * b_alg / (ms_all / 1000.0) / 1e9) if ms_all > 0 else None
         storage = "fp16" if half else "fp32"
-        kernel_key = f"fused_inner_{storage}" if args.path == "fused" else "plain_inner_iteration"
+        # 14: the whole level in one launch, its state on the chip
+        resident = kind == 1 and (not fused or (variants and variants[0] == 14))
+        kernel_key = f"resident_{storage}" if resident else f"fused_inner_{storage}" if fused else "plain_inner_iteration"
         px_per_launch = pi_l / n_launch if n_launch else 0.0
         tr = ncu_traffic(kernel_key)
         traffic = None
@@ -557,16 +559,21 @@ def run_ours(args, rank, world, local):
             "roofline": {"bound": "latency", "peak_basis": "hbm (measured copy bandwidth)",
                          "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": (achieved / peak) if achieved else None, "traffic": traffic,
-                         "limiter": "instruction issue and short dependencies with the working sets of the pairs "
-                                    "at full resolution resident in L2 (ncu, one cold launch: DRAM 24 %, issue 53 %, "
-                                    "228 warp instructions per 32 pixels; stalls per issued instruction: long "
-                                    "scoreboard 8.4, short scoreboard 3.1, not selected 2.1); frac > 1 is an "
-                                    "algorithmic-bytes rate, not DRAM traffic",
+                         "limiter": ("instruction issue and dependent-issue latency at 3.5 warps per scheduler, and the "
+                                     "exchange between tiles; the level's state stays on the chip (ncu, half storage, one "
+                                     "launch of 50 iterations: DRAM 25 MB, issue 51 %, 1040 warp instructions per tile "
+                                     "of 240 pixels and iteration; stalls per issued instruction: long scoreboard 1.9, "
+                                     "fixed latency 1.0, not selected 0.9, math pipe 0.8); frac > 1 is an "
+                                     "algorithmic-bytes rate, not DRAM traffic") if resident else
+                                    ("instruction issue and short dependencies with the working sets of the pairs "
+                                     "at full resolution resident in L2; frac > 1 is an algorithmic-bytes rate, not "
+                                     "DRAM traffic"),
                          "frac_in_mask": (achieved * in_mask_frac / peak) if achieved else None,
                          "frac_per_launch": (pi_l * b_alg / (ms_sum / 1000.0) / 1e9 / peak) if ms_sum > 0 else None,
                          "dram_gbs_per_launch_cold": (traffic / (ms_l / 1000.0 / n_launch) / 1e9)
                          if (traffic and n_launch and ms_l > 0) else None,
-                         "kernel": ("full-resolution fused iteration (variant %s)" % (variants[0] if variants else "?"))
+                         "kernel": "full-resolution register-resident iterations, one launch per warp" if resident else
+                         ("full-resolution fused iteration (variant %s)" % (variants[0] if variants else "?"))
                          if fused else "drop-in inner iteration at full resolution",
                          "launches_measured": int(n_launch),
                          "algorithmic_bytes_per_launch": b_alg * px_per_launch,
