@@ -158,7 +158,8 @@ int vfs_debug_get_buffer(vfs_stereo* s, const char* name, int comps, float* out)
  *   VFS_PATH_REFERENCE: the reference's results to the bit.  Where every level of the solve can be
  *   held on the chip (see vfs_batch_set_autotune), the whole-level launches and the fused
  *   per-warp and per-level kernels, replayed as a CUDA graph, leave every buffer as the reference's
- *   kernels would; else one kernel per reference kernel, in the reference's order;
+ *   kernels would; else, and in a caller's stream capture, one kernel per reference kernel, in the
+ *   reference's order;
  *   VFS_PATH_FUSED: one fused kernel per primal-dual iteration plus fused per-warp and
  *   per-level kernels, replayed as a CUDA graph.  With float storage the fused path gives
  *   bit-identical results; with half storage (half_storage = 1) p, q, v-bar and the warped

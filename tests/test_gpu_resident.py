@@ -276,6 +276,41 @@ def test_dropin_solve_in_a_captured_stream(gpu):
     assert np.array_equal(out.cpu().numpy(), u)
 
 
+def test_captured_dropin_solve_after_a_new_mask(gpu):
+    """A caller's graph of the drop-in solve takes the mask that is there when it is replayed."""
+    import torch
+    case = random_case(150, 110, seed=5)
+    p = params(n_levels=2, n_warp=2, n_iter=6)
+    i0, i1 = (torch.from_numpy(x).cuda() for x in case[:2])
+    yy, xx = np.mgrid[0:110, 0:150]
+    new = ((xx > 20) & (xx < 140) & (yy > 30) & (yy < 100)).astype(np.float32)
+    outs = []
+    for capture in (False, True):
+        st = torch.cuda.Stream()
+        s = _dropin(case, p, st)
+        out = torch.zeros((110, 150), device="cuda")
+        torch.cuda.synchronize()
+
+        def frame():
+            s.copy_images_from_device(i0, i1)
+            s.solveStereoForwardMasked()
+            s.copy_1d_disparity_to_device(out)
+
+        for _ in range(2):
+            frame()
+        torch.cuda.synchronize()
+        g = torch.cuda.CUDAGraph()
+        if capture:
+            with torch.cuda.graph(g, stream=st):
+                frame()
+        s.copyMaskToDevice(new)
+        torch.cuda.synchronize()
+        g.replay() if capture else frame()
+        torch.cuda.synchronize()
+        outs.append(out.cpu().numpy())
+    assert np.array_equal(*outs)
+
+
 @pytest.mark.parametrize("half", [False, True], ids=["fp32", "fp16"])
 @pytest.mark.parametrize("masked", [True, False], ids=["masked", "plain"])
 def test_cluster_sizes(gpu, masked, half):

@@ -771,9 +771,12 @@ void FusedEngine::solve_parts(std::vector<StereoTgvImpl*>& pairs, bool masked, b
   auto in_part = [&](int l) { return !((part == 1 && l == 0) || (part == 2 && l > 0)) && l <= max_top; };
   bool need_tune = false;
   const bool one_pair = pairs.size() == 1;
-  // levels that fit the chip run the register-resident form; it is never timed against the others
-  auto resident = [&](int l) { return one_pair && !forced && pairs[0]->residentPlan(masked, half, l) != nullptr; };
-  if (one_pair && !forced) pairs[0]->ensureResident(masked, half, st);
+  // levels that fit the chip run the register-resident form; it is never timed against the others.  In a
+  // caller's stream capture nothing is timed and no plan is used: the graph may outlive it (a new mask)
+  const bool captured = stream_capturing(st);
+  const bool plans = one_pair && !forced && !captured;
+  auto resident = [&](int l) { return plans && pairs[0]->residentPlan(masked, half, l) != nullptr; };
+  if (plans) pairs[0]->ensureResident(masked, half, st);
   auto level_key = [&](int l) {
     return std::array<int, 5>{(int)masked, (int)half, concurrency > 1 ? 2 : 1, pairs[0]->pW[l], pairs[0]->pH[l]};
   };
@@ -783,7 +786,7 @@ void FusedEngine::solve_parts(std::vector<StereoTgvImpl*>& pairs, bool masked, b
     if (!all)
       for (auto* s : pairs) s->ensureSpans();
   }
-  if (autotune && !forced) {
+  if (autotune && !forced && !captured) {
     // a composition tuned before (by any engine of the process) is reused, so that every
     // pair of a batch runs the same choice and only the first tunes; a one-pair solve also
     // reuses any level tuned before in the same setting
@@ -839,8 +842,10 @@ void FusedEngine::solve_parts(std::vector<StereoTgvImpl*>& pairs, bool masked, b
     return;
   }
   std::vector<int> variants = tit->second;
-  for (int l = 0; l < maxL; l++)
+  for (int l = 0; l < maxL; l++) {
     if (resident(l)) variants[l] = kIterResident;
+    else if (variants[l] < 0 && captured) variants[l] = kIterDefaultVariant;
+  }
   if (forced_variant >= 0) variants.assign(maxL, forced_variant);
   if (!forced_levels.empty()) {
     variants.assign(maxL, kIterDefaultVariant);
@@ -860,13 +865,7 @@ void FusedEngine::solve_dropin(StereoTgvImpl* pair, bool masked, cudaStream_t st
 // The solve with the variants settled: from a graph captured in the same state, or directly.
 void FusedEngine::run(std::vector<StereoTgvImpl*>& pairs, bool masked, bool half, cudaStream_t st, int part,
                       std::vector<int>& variants, bool dropin) {
-  bool direct = !use_graph;
-  if (dropin && !direct) {  // a stream under capture takes the launches themselves
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    VFS_CUDA(cudaStreamIsCapturing(st, &cap));
-    direct = cap != cudaStreamCaptureStatusNone;
-  }
-  if (direct) {
+  if (!use_graph) {
     fused_solve_direct(pairs, masked, half, st, variants, false, concurrency, part, dropin);
     return;
   }

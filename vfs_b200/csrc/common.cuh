@@ -36,6 +36,13 @@ std::atomic<long long>& launch_counter();
     ::vfs::launch_counter().fetch_add(1, std::memory_order_relaxed);        \
   } while (0)
 
+// Whether the caller is capturing the stream.
+inline bool stream_capturing(cudaStream_t st) {
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  VFS_CUDA(cudaStreamIsCapturing(st, &cap));
+  return cap != cudaStreamCaptureStatusNone;
+}
+
 // Host-side trace ranges (NVTX) around the library's entry points and solve phases, for
 // profilers that record them (ncu --nvtx, Nsight Systems); without one attached they cost a
 // null check.  In graph replays a range covers the enqueue, not the GPU work.

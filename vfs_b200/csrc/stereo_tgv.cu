@@ -498,17 +498,12 @@ void StereoTgvImpl::ensureCodes(bool masked) {
   }
 }
 
-// Whether every level of the next solve has a plan; while the stream is being captured, whether they
-// are all there already (making one synchronises the stream).
+// Whether every level of the next solve has a plan.  Not in a caller's stream capture: the caller may
+// replay its graph after the mask has changed, and a plan belongs to one mask.
 bool StereoTgvImpl::dropinResident(bool masked) {
-  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-  VFS_CUDA(cudaStreamIsCapturing(stream_, &cap));
-  if (cap == cudaStreamCaptureStatusNone) {
-    ensureCodes(masked);
-    ensureResident(masked, false, stream_);
-  } else if (masked && !codes_valid) {
-    return false;
-  }
+  if (stream_capturing(stream_)) return false;
+  ensureCodes(masked);
+  ensureResident(masked, false, stream_);
   for (int l = 0; l <= topLevel(); l++)
     if (!residentPlan(masked, false, l)) return false;
   return true;
