@@ -45,7 +45,7 @@ __device__ __forceinline__ __half2 as_half2(unsigned b) { return *reinterpret_ca
 // the halo columns to lanes 0 and 31.  At a masked-out pixel a and b hold its stale T p instead
 // (its tensor is not used).
 // Beside them each lane's exchange offsets and pixel masks, read back at every iteration.
-// half storage: rows in pairs, each coefficient's two rows side by side for the packed
+// half storage (up to 8 rows): rows in pairs, each coefficient's two rows side by side for the packed
 // instructions: (a, b), (c, 1 / eta_u), (Iu, Iz), (1 / eta_v1, 1 / eta_v2), 1 / Iu
 // float storage: (a, b), (c, Iu), Iz, and p, (q.x, q.y), (q.z, q.w) in the same pairs
 // What a lane's edge rules need, bit r + 1 for row r: x (y): the pixel is on and takes its right
@@ -129,7 +129,7 @@ struct ResState;
 // pair of rows) and, with 16 rows, from Iu and Iz (read again from L2, 8 bytes a pixel of the
 // one-iteration kernel's 96).  Their rows are taken four at a time by one piece of code, between whose
 // passes the registers move up: 16 rows unrolled by eight leave the instruction cache (1280 x 1024
-// disc, 2174 tiles of 16 rows: 11.6 us per iteration; by four 9.6; one launch per iteration 15.0.
+// disc, 2174 tiles of 16 rows: 11.6 us per iteration; by four 9.3; one launch per iteration 15.0.
 // 1000 x 900, 1883 tiles of 12: 6.1; 9.85).  Instruction issue bounds both.
 template <bool MASKED, int R>
 struct ResState<MASKED, __half, R> {
@@ -1175,12 +1175,6 @@ struct ResWarp {
   }
 };
 
-// Warps per block (one block per SM): what the registers of R rows leave.
-template <class ST>
-constexpr int res_warps(int rows) {
-  return 16;
-}
-
 // The plain form's pixels outside the circle in tiles without a pixel to solve.
 template <class ST, int R>
 __device__ __forceinline__ void res_fill(const ResArgs& A, int warp, int lane) {
@@ -1209,7 +1203,7 @@ __device__ __forceinline__ void res_fill(const ResArgs& A, int warp, int lane) {
 }
 
 template <bool MASKED, class ST, int R>
-__global__ void __launch_bounds__(32 * res_warps<ST>(R), 1) k_resident(const __grid_constant__ ResArgs A) {
+__global__ void __launch_bounds__(32 * kResMostWarps, 1) k_resident(const __grid_constant__ ResArgs A) {
   extern __shared__ __align__(16) unsigned char smem[];
   const int warp = (int)threadIdx.x >> 5, lane = (int)threadIdx.x & 31;
   ResShared<ST, R>& sh = reinterpret_cast<ResShared<ST, R>*>(smem)[warp];
@@ -1423,8 +1417,8 @@ namespace {
 
 template <bool MASKED, class ST, int R>
 struct Res {
-  static constexpr int kThreads = 32 * res_warps<ST>(R);
-  static constexpr size_t kSmem = sizeof(ResShared<ST, R>) * res_warps<ST>(R);
+  static constexpr int kThreads = 32 * kResMostWarps;
+  static constexpr size_t kSmem = sizeof(ResShared<ST, R>) * kResMostWarps;
   // tiles that a grid of one block per SM holds, all of it resident
   static int capacity() {
     int dev = 0, sms = 0, per = 0, coop = 0, smem = 0;
@@ -1435,7 +1429,7 @@ struct Res {
     if (!coop || kSmem > (size_t)smem) return 0;
     VFS_CUDA(cudaFuncSetAttribute(k_resident<MASKED, ST, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem));
     VFS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_resident<MASKED, ST, R>, kThreads, kSmem));
-    return per >= 1 ? sms * res_warps<ST>(R) : 0;
+    return per >= 1 ? sms * kResMostWarps : 0;
   }
   // warps the tiles of which one cluster of `ctas` blocks holds (0: no such cluster)
   static int cluster_capacity(int ctas) {

@@ -52,7 +52,8 @@ constexpr int kResMaxIters = 128;  // iterations per launch (a tag's low seven b
 // tile heights the kernel is built for (float storage: those up to 8)
 constexpr int kResRows[] = {2, 4, 6, 8, 12, 16};
 constexpr int kResNumRows = 6;
-constexpr int kResMostTiles = 148 * 16;  // a bound on the tiles of a plan (one warp each)
+constexpr int kResMostWarps = 16;                   // of a block (one per SM), a tile each
+constexpr int kResMostTiles = 148 * kResMostWarps;  // a bound on the tiles of a plan
 // The cluster form (kernels_resident.cu, k_resident_cluster): 16 blocks, tiles of two rows, for levels of
 // up to so many tiles.  Beyond, the 16 SMs have more to issue than the shorter exchange saves (us per
 // iteration, cluster / whole GPU: half storage 50 tiles 0.90 / 1.39, 128 1.02 / 1.38, 200 1.19 / 1.44,

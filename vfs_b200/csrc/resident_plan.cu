@@ -188,8 +188,9 @@ bool res_choose(const uint8_t* code, int w, int h, bool masked, bool half, ResTi
   ResLevel L;
   if (!L.scan(code, w, h, masked)) return false;
   out.cluster = false;
+  // (a capacity is asked for only where the count may fit: the first question loads the kernel)
   if (const int n = L.count(kResClusterRows);
-      n <= std::min(res_cluster_tiles(half), res_capacity(masked, half, kResClusterRows, kResClusterCtas))) {
+      n <= res_cluster_tiles(half) && n <= res_capacity(masked, half, kResClusterRows, kResClusterCtas)) {
     L.tiles(kResClusterRows, out);
     out.cluster = true;
     out.place(kResClusterCtas);
@@ -197,7 +198,9 @@ bool res_choose(const uint8_t* code, int w, int h, bool masked, bool half, ResTi
   }
   for (int k = 0; k < kResNumRows; k++) {
     const int rows = kResRows[k];
-    const int cap = res_capacity(masked, half, rows), n = L.count(rows);
+    const int n = L.count(rows);
+    if (n > sms * kResMostWarps) continue;
+    const int cap = res_capacity(masked, half, rows);
     if (n > cap || (rows == kResRows[0] && 4 * (long long)n > 3 * (long long)cap)) continue;
     L.tiles(rows, out);
     out.place(std::min(sms, n));
