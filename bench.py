@@ -463,11 +463,11 @@ def run_ours(args, rank, world, local):
             flush.fill_(float(k))
         device_step()
     torch.cuda.synchronize()
-    # roofline of the inner primal-dual loop: kind 1, or 0 (drop-in path on a pair that has a level
-    # which does not fit on the chip: one record per iteration)
+    # roofline of the inner primal-dual loop: kind 0 (drop-in path: one record per warp of a level, or per
+    # iteration where a level does not fit on the chip), kind 1 (fused path)
     # Pairs solved on concurrent streams overlap, so the time is the union of the records'
     # intervals (time during which at least one inner group ran), not their sum.
-    kind = 1 if args.path == "fused" or any(len(s.profile_intervals(1)) for s in solvers) else 0
+    kind = 1 if args.path == "fused" else 0
     iv = np.concatenate([s.profile_intervals(kind) for s in solvers])
     for s in solvers:
         s.profile(False)
@@ -536,7 +536,7 @@ def run_ours(args, rank, world, local):
         achieved_all = (pi_all * b_alg / (ms_all / 1000.0) / 1e9) if ms_all > 0 else None
         storage = "fp16" if half else "fp32"
         # 14: the whole level in one launch, its state on the chip
-        resident = kind == 1 and (not fused or (variants and variants[0] == 14))
+        resident = variants[0] == 14 if fused and variants else pi_l > 1.5 * n_launch * W0 * H0
         kernel_key = f"resident_{storage}" if resident else f"fused_inner_{storage}" if fused else "plain_inner_iteration"
         px_per_launch = pi_l / n_launch if n_launch else 0.0
         tr = ncu_traffic(kernel_key)

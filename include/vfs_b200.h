@@ -298,8 +298,8 @@ int vfs_equalize_hist_u8_noalloc(const uint8_t* d_src, uint8_t* d_dst, size_t n,
  * of kernels this library has launched in the process.  With profiling on, each group of
  * inner primal-dual kernels (one iteration of the drop-in path's own kernels, else one launch of
  * one or several iterations) is bracketed by CUDA events on the handle's stream;
- * vfs_profile_read() sums the records of a group kind (0 = drop-in inner iteration,
- * 1 = fused inner launch, also the drop-in path's whole-level launches, 2 = fused per-warp prologue, 3 = fused epilogue). */
+ * vfs_profile_read() sums the records of a group kind (0 = drop-in inner iteration or whole-level
+ * launch, 1 = fused inner launch, 2 = fused per-warp prologue, 3 = fused epilogue). */
 long long vfs_launch_count(void);
 
 /* Device-side status of the current device (no counterpart in the reference): *status = 1 if
