@@ -1,0 +1,112 @@
+"""What a program sees around the solves that run whole levels in one launch: streams, captures, masks,
+first solves, errors, and the buffers that the default path leaves."""
+import subprocess
+
+import numpy as np
+import pytest
+
+from tests.helpers import params, random_case
+
+pytestmark = pytest.mark.gpu
+
+
+def _solver(case, p, stream=None, fused=False, half=False):
+    from vfs_b200.stereotgv import StereoTgv
+    i0, i1, mask, tv, cv = case
+    s = StereoTgv()
+    s.set_solve_path(fused, half)
+    h, w = i0.shape
+    s.limitRange = p["limit_range"]
+    s.initialize(w, h, p["beta"], p["gamma"], p["alpha0"], p["alpha1"], p["tsl"], p["lam"], p["n_levels"],
+                 p["f_scale"], p["n_warp"], p["n_iter"])
+    s.copyMaskToDevice(mask)
+    s.loadVectorFields(tv, cv)
+    if stream is not None:
+        s.set_stream(stream)
+    return s
+
+
+def _disparity(s, case, masked=True):
+    s.copyImagesToDevice(*case[:2])
+    (s.solveStereoForwardMasked if masked else s.solveStereoForward)()
+    return s.copy1DDisparityToHost()
+
+
+@pytest.mark.parametrize("half", [False, True], ids=["fp32", "fp16"])
+def test_first_unmasked_solve_in_a_capture(gpu, half):
+    """A handle that has only solved with its mask: its first unmasked solve goes into a caller's graph,
+    and what it solves afterwards without one is right."""
+    import torch
+    case = random_case(150, 110, seed=7)
+    p = params(n_levels=2, n_warp=2, n_iter=6)
+    want = _disparity(_solver(case, p, fused=True, half=half), case, masked=False)
+    assert want.any()
+    st = torch.cuda.Stream()
+    s = _solver(case, p, st, fused=True, half=half)
+    s.set_graph(False)
+    for _ in range(2):
+        _disparity(s, case)
+    i0, i1 = (torch.from_numpy(x).cuda() for x in case[:2])
+    out = torch.zeros((110, 150), device="cuda")
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    try:
+        with torch.cuda.graph(g, stream=st, capture_error_mode="relaxed"):
+            s.copy_images_from_device(i0, i1)
+            s.solveStereoForward()
+            s.copy_1d_disparity_to_device(out)
+        captured = True
+    except Exception:
+        captured = False
+        torch.cuda.synchronize()
+    if captured:
+        g.replay()
+        torch.cuda.synchronize()
+    assert np.array_equal(_disparity(s, case, masked=False), want)
+    assert captured and np.array_equal(out.cpu().numpy(), want)
+
+
+def test_circle_on_the_host(gpu, tmp_path):
+    """The unmasked form's circle as the host finds it, row by row, and as the kernels evaluate it."""
+    from vfs_b200.build import CSRC, NVCC_FLAGS, nvcc
+    src = tmp_path / "t.cu"
+    src.write_text(r"""
+#include <cstdio>
+#include "resident.cuh"
+#include "tgv_pixel.cuh"
+namespace vfs { int res_capacity(bool, bool, int, int) { return 0; } }
+using namespace vfs;
+__global__ void k_codes(uint8_t* c, int w, int h) {
+  const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y;
+  if (x < w) c[x + (size_t)y * w] = outside_circle(x, y, w, h) ? 0 : kOn;
+}
+int main() {
+  uint8_t* d;
+  if (cudaMalloc(&d, 1500 * 1500) != cudaSuccess) return 2;
+  int bad = 0, n = 0;
+  auto check = [&](int w, int h) {
+    std::vector<uint8_t> dev((size_t)w * h);
+    k_codes<<<dim3((w + 127) / 128, h), 128>>>(d, w, h);
+    if (cudaMemcpy(dev.data(), d, dev.size(), cudaMemcpyDeviceToHost) != cudaSuccess) return false;
+    n++;
+    if (dev != res_circle_codes(w, h)) std::printf("%d x %d\n", w, h), bad++;
+    return true;
+  };
+  for (int w = 1; w < 70; w++)
+    for (int h = 1; h < 70; h += 1 + w % 3)
+      if (!check(w, h)) return 2;
+  unsigned s = 1;
+  for (int k = 0; k < 120; k++) {
+    s = s * 1664525u + 1013904223u;
+    if (!check(70 + (s >> 8) % 1400, 70 + (s >> 20) % 1400)) return 2;
+  }
+  std::printf("%d sizes\n", n);
+  return bad != 0;
+}
+""")
+    exe = tmp_path / "t"
+    r = subprocess.run([nvcc(), *NVCC_FLAGS, f"-I{CSRC}", str(src), f"{CSRC}/resident_plan.cu", "-o", str(exe)],
+                       capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr
+    r = subprocess.run([str(exe)], capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0, r.stdout + r.stderr

@@ -641,7 +641,7 @@ void FusedEngine::prepare(std::vector<StereoTgvImpl*>& pairs, bool masked) {
   for (auto* s : pairs) {
     if (!s->initialized()) throw ArgError{"fused solve: pair not initialized"};
     s->ensureFused();
-    s->ensureCodes(masked);
+    if (masked) s->ensureMaskCodes();
   }
 }
 
@@ -660,7 +660,7 @@ void StereoTgvImpl::ensureSpans() {
   }
   for (int l = 0; l < levels(); l++) {
     const int w = pW[l], h = pH[l];
-    const std::vector<uint8_t>& code = host_code[1][l];
+    const std::vector<uint8_t>& code = mask_code[l];
     for (int y = 0; y < h; y++)
       if (code[(size_t)y * w] & kOn) {
         tma_ok[l] = 0;

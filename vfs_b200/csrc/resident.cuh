@@ -128,6 +128,9 @@ struct ResLevel {
   int count(int rows) const;  // tiles of `rows` rows
   void tiles(int rows, ResTiles& out) const;
 };
+// The plain form's codes (tight rows) on the host: kOn inside the circle.  A row's pixels inside are
+// one run about the middle (the radius grows with the distance from it, and so does its rounded value).
+std::vector<uint8_t> res_circle_codes(int w, int h);
 // Picks the tile height for the level among the instances whose grid can be resident;
 // false: no instance fits (or the form does not apply).
 bool res_choose(const uint8_t* code, int w, int h, bool masked, bool half, ResTiles& out);

@@ -3,8 +3,32 @@
 #include <cstring>
 
 #include "resident.cuh"
+#include "tgv_pixel.cuh"
 
 namespace vfs {
+
+std::vector<uint8_t> res_circle_codes(int w, int h) {
+  std::vector<uint8_t> code((size_t)w * h, 0);
+  const int mid = w / 2;  // no column is nearer to the centre
+  for (int y = 0; y < h; y++) {
+    if (mid >= w || outside_circle(mid, y, w, h)) continue;
+    int out = -1, in = mid;  // the run's first column: out is outside (or left of the image), in inside
+    while (in - out > 1) {
+      const int x = out + (in - out) / 2;
+      if (outside_circle(x, y, w, h)) out = x;
+      else in = x;
+    }
+    const int first = in;
+    in = mid, out = w;
+    while (out - in > 1) {
+      const int x = in + (out - in) / 2;
+      if (outside_circle(x, y, w, h)) out = x;
+      else in = x;
+    }
+    std::memset(&code[(size_t)y * w + first], kOn, (size_t)(in - first + 1));
+  }
+  return code;
+}
 
 // A level is mostly tiles' rows that are on or off throughout; those take three or four 8-byte looks
 // (a 1280 x 1024 disc: 2.25 ms a pixel at a time, 0.40 this way; a new mask pays it).

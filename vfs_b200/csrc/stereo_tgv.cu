@@ -131,8 +131,7 @@ void StereoTgvImpl::release() {
   tex.clear();
   dropResident(false);
   dropResident(true);
-  host_code[0].clear();
-  host_code[1].clear();
+  mask_code.clear();
   if (pool_) cudaFree(pool_);
   pool_ = nullptr;
   if (fpool_) cudaFree(fpool_);
@@ -345,6 +344,7 @@ void StereoTgvImpl::initialize(const SolverParams& p) {
     }
   VFS_CUDA(cudaMemsetAsync(pool_, 0, at, stream_));
   fillGuards(0, stream_);
+  for (int l = 0; l < levels(); l++) launch_edge_codes(nullptr, code_plain[l], pW[l], pH[l], pS[l], stream_);
   VFS_CUDA(cudaStreamSynchronize(stream_));
   initialized_ = true;
 }
@@ -479,30 +479,27 @@ void StereoTgvImpl::ensureFused() {
   fillGuards(guards_before, stream_);
 }
 
-void StereoTgvImpl::ensureCodes(bool masked) {
-  if (masked ? codes_valid : !host_code[0].empty()) return;
-  if (masked) dropResident(true);
-  std::vector<std::vector<uint8_t>>& host = host_code[masked];
-  host.assign(levels(), {});
+void StereoTgvImpl::ensureMaskCodes() {
+  if (codes_valid) return;
+  dropResident(true);
+  mask_code.assign(levels(), {});
   for (int l = 0; l < levels(); l++) {
-    uint8_t* dev = masked ? code_masked[l] : code_plain[l];
-    launch_edge_codes(masked ? pMask[l] : nullptr, dev, pW[l], pH[l], pS[l], stream_);
-    host[l].resize((size_t)pW[l] * pH[l]);
-    VFS_CUDA(cudaMemcpy2DAsync(host[l].data(), pW[l], dev, pS[l], pW[l], pH[l], cudaMemcpyDeviceToHost, stream_));
+    launch_edge_codes(pMask[l], code_masked[l], pW[l], pH[l], pS[l], stream_);
+    mask_code[l].resize((size_t)pW[l] * pH[l]);
+    VFS_CUDA(cudaMemcpy2DAsync(mask_code[l].data(), pW[l], code_masked[l], pS[l], pW[l], pH[l], cudaMemcpyDeviceToHost,
+                               stream_));
   }
   VFS_CUDA(cudaStreamSynchronize(stream_));
-  if (masked) {
-    spans_valid = false;
-    codes_valid = true;
-    generation = next_generation();  // graphs captured under the old mask are not reused
-  }
+  spans_valid = false;
+  codes_valid = true;
+  generation = next_generation();  // graphs captured under the old mask are not reused
 }
 
 // Whether every level of the next solve has a plan.  Not in a caller's stream capture: the caller may
 // replay its graph after the mask has changed, and a plan belongs to one mask.
 bool StereoTgvImpl::dropinResident(bool masked) {
   if (stream_capturing(stream_)) return false;
-  ensureCodes(masked);
+  if (masked) ensureMaskCodes();
   ensureResident(masked, false, stream_);
   for (int l = 0; l <= topLevel(); l++)
     if (!residentPlan(masked, false, l)) return false;
@@ -519,7 +516,7 @@ void StereoTgvImpl::dropResident(bool masked) {
   }
 }
 
-// Needs the host copies of the form's edge codes.  Without memory for the plans the levels
+// Needs the masked form's edge codes on the host.  Without memory for the plans the levels
 // simply have none (the solve then launches one iteration at a time).
 void StereoTgvImpl::ensureResident(bool masked, bool half, cudaStream_t st) {
   std::vector<ResPlan>& plans = res_plans_[masked][half];
@@ -546,7 +543,8 @@ void StereoTgvImpl::ensureResident(bool masked, bool half, cudaStream_t st) {
   };
   std::vector<Off> off(levels());
   for (int l = 0; l < levels(); l++) {
-    if (!res_choose(host_code[masked][l].data(), pW[l], pH[l], masked, half, cut[l])) continue;
+    const std::vector<uint8_t> circle = masked ? std::vector<uint8_t>{} : res_circle_codes(pW[l], pH[l]);
+    if (!res_choose(masked ? mask_code[l].data() : circle.data(), pW[l], pH[l], masked, half, cut[l])) continue;
     plans[l].rows = cut[l].rows;
     plans[l].blocks = cut[l].blocks;
     plans[l].cluster = cut[l].cluster;

@@ -181,11 +181,11 @@ class StereoTgvImpl {
   float2* f_rv = nullptr;
   std::vector<uint8_t*> code_masked, code_plain;
   bool codes_valid = false;
-  // the form's edge codes on the device and the host, on the handle's stream (which it synchronises
-  // when they are not there yet)
-  void ensureCodes(bool masked);
-  // host copies of the edge codes per level (tight rows), [0] plain and [1] masked
-  std::vector<std::vector<uint8_t>> host_code[2];
+  // the masked form's edge codes on the device and the host, on the handle's stream (which it
+  // synchronises when they are not there yet).  The plain form's are made with the buffers.
+  void ensureMaskCodes();
+  // host copies of the masked form's edge codes per level (tight rows)
+  std::vector<std::vector<uint8_t>> mask_code;
   // ---- register-resident iteration (resident.cuh): a plan per level, for the plain [0] and
   // masked [1] form and for float [0] and half [1] storage, made on the first solve of that
   // form with the current mask, on the solve's stream.  Its device memory (tiles and exchange words)

@@ -108,7 +108,7 @@ __device__ __forceinline__ void primal_math(float4 qc, float4 ql, float4 qu, flo
 }
 
 // updateDualVariables.cu:13-16: the plain kernels' fixed circular domain
-__device__ __forceinline__ bool outside_circle(int ix, int iy, int w, int h) {
+__host__ __device__ __forceinline__ bool outside_circle(int ix, int iy, int w, int h) {
   float desiredRadius = (float)w / 2.20f;
   float halfWidth = (float)w / 2.0f;
   float halfHeight = (float)h / 2.0f;
