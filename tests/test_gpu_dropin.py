@@ -110,3 +110,32 @@ int main() {
     assert r.returncode == 0, r.stderr
     r = subprocess.run([str(exe)], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0, r.stdout + r.stderr
+
+
+@pytest.mark.parametrize("fused,half", [(False, False), (True, False), (True, True)], ids=["dropin", "fp32", "fp16"])
+@pytest.mark.parametrize("size", [(150, 110), (640, 480)])
+def test_solves_return_after_enqueueing(gpu, size, fused, half):
+    """Behind work that keeps the stream busy for some 0.3 s: the first solve with a mask, the first
+    unmasked one and the first with another mask.  (A first handle loads the kernels.)"""
+    import torch
+    w, h = size
+    case = random_case(w, h, seed=9)
+    p = params(n_levels=3, n_warp=2, n_iter=8)
+    i0, i1 = (torch.from_numpy(x).cuda() for x in case[:2])
+    for warm in (True, False):
+        st = torch.cuda.Stream()
+        s = _solver(case, p, st, fused=fused, half=half)
+        for masked, mask in ((True, None), (False, None), (True, np.ascontiguousarray(case[2][:, ::-1]) * (case[0] > 60))):
+            if mask is not None:
+                s.copyMaskToDevice(mask)
+            s.copy_images_from_device(i0, i1)
+            torch.cuda.synchronize()
+            before = torch.cuda.Event()
+            with torch.cuda.stream(st):
+                if not warm:
+                    torch.cuda._sleep(600_000_000)
+                before.record()
+            (s.solveStereoForwardMasked if masked else s.solveStereoForward)()
+            waited = before.query()
+            torch.cuda.synchronize()
+            assert warm or not waited, (masked, mask is not None)

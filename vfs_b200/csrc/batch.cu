@@ -641,7 +641,7 @@ void FusedEngine::prepare(std::vector<StereoTgvImpl*>& pairs, bool masked) {
   for (auto* s : pairs) {
     if (!s->initialized()) throw ArgError{"fused solve: pair not initialized"};
     s->ensureFused();
-    if (masked) s->ensureMaskCodes();
+    if (masked) s->takeMask();
   }
 }
 
@@ -660,17 +660,18 @@ void StereoTgvImpl::ensureSpans() {
   }
   for (int l = 0; l < levels(); l++) {
     const int w = pW[l], h = pH[l];
-    const std::vector<uint8_t>& code = mask_code[l];
+    const uint8_t* code = maskCode(l);
+    const int s = pS[l];
     for (int y = 0; y < h; y++)
-      if (code[(size_t)y * w] & kOn) {
+      if (code[(size_t)y * s] & kOn) {
         tma_ok[l] = 0;
-        if (w == pS[l]) tb_ok[l] = 0;
+        if (w == s) tb_ok[l] = 0;
       }
     // first and last on column of every image row
     std::vector<int> xmin(h, w), xmax(h, -1);
     for (int y = 0; y < h; y++)
       for (int x = 0; x < w; x++)
-        if (code[(size_t)y * w + x] & kOn) {
+        if (code[(size_t)y * s + x] & kOn) {
           xmin[y] = std::min(xmin[y], x);
           xmax[y] = std::max(xmax[y], x);
         }
@@ -681,7 +682,7 @@ void StereoTgvImpl::ensureSpans() {
     std::vector<int> notin((size_t)h * (w + 1), 0);
     for (int y = 0; y < h; y++)
       for (int x = 0; x < w; x++)
-        notin[(size_t)y * (w + 1) + x + 1] = notin[(size_t)y * (w + 1) + x] + (code[(size_t)y * w + x] != kInterior);
+        notin[(size_t)y * (w + 1) + x + 1] = notin[(size_t)y * (w + 1) + x] + (code[(size_t)y * s + x] != kInterior);
     for (int v = 0; v < kIterVariants; v++) {
       const int slot = iter_span_slot(v);
       if (slot < 0 || !iter_variant_tiled(v)) continue;

@@ -2,6 +2,7 @@
 #include "resident.cuh"
 
 #include <algorithm>
+#include <cstring>
 #include <map>
 #include <mutex>
 #include <tuple>
@@ -1524,6 +1525,33 @@ int res_capacity(bool masked, bool half, int rows, int cluster) {
   return known[key] = res_dispatch(masked, half, rows, [cluster](auto k) {
            return cluster ? decltype(k)::cluster_capacity(cluster) : decltype(k)::capacity();
          });
+}
+
+// A plan's tables travel in kernel arguments, 28 KB a launch (848 x 800: five launches).  A copy from pageable
+// memory may wait for the stream, and the first solve with a mask then returned only when the work
+// queued before it was done.
+namespace {
+struct ResUpload {
+  unsigned* to;
+  int n;
+  unsigned w[7168];
+};
+__global__ void k_res_upload(const __grid_constant__ ResUpload U) {
+  const int i = (int)(blockIdx.x * blockDim.x + threadIdx.x);
+  if (i < U.n) U.to[i] = U.w[i];
+}
+}  // namespace
+
+void launch_res_upload(void* to, const void* from, size_t bytes, cudaStream_t st) {
+  ResUpload U;
+  for (size_t at = 0; at < bytes; at += sizeof(U.w)) {
+    const size_t b = std::min(bytes - at, sizeof(U.w));
+    U.to = (unsigned*)((char*)to + at);
+    U.n = (int)(b / 4);
+    std::memcpy(U.w, (const char*)from + at, b);
+    k_res_upload<<<(U.n + 127) / 128, 128, 0, st>>>(U);
+    VFS_LAUNCH_CHECK();
+  }
 }
 
 void launch_resident(const ResArgs& A, bool masked, bool half, cudaStream_t st) {

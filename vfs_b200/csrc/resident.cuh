@@ -114,7 +114,7 @@ struct ResTiles {
   std::vector<ResTile> tiles;
   std::vector<int2> fill;
 };
-// What the tiles of any height need of a w x h level with edge codes `code` (tight rows; masked form:
+// What the tiles of any height need of a w x h level with edge codes `code` (rows of `pitch`; masked form:
 // k_edge_codes of the mask, plain form: kOn inside the circle), found in one pass over it.
 struct ResLevel {
   int w = 0, h = 0, tx = 0;
@@ -124,7 +124,7 @@ struct ResLevel {
   // False where the form does not apply: a masked-in pixel of column 0 (row 0) without its right
   // (lower) neighbour reads outside the image, a one-pixel-wide or -high plain level has no
   // neighbour to take, or no pixel is on.
-  bool scan(const uint8_t* code, int w, int h, bool masked);
+  bool scan(const uint8_t* code, int pitch, int w, int h, bool masked);
   int count(int rows) const;  // tiles of `rows` rows
   void tiles(int rows, ResTiles& out) const;
 };
@@ -133,7 +133,7 @@ struct ResLevel {
 std::vector<uint8_t> res_circle_codes(int w, int h);
 // Picks the tile height for the level among the instances whose grid can be resident;
 // false: no instance fits (or the form does not apply).
-bool res_choose(const uint8_t* code, int w, int h, bool masked, bool half, ResTiles& out);
+bool res_choose(const uint8_t* code, int pitch, int w, int h, bool masked, bool half, ResTiles& out);
 
 // Device bytes a level's plan takes at most.
 size_t res_bytes_bound(int w, int h);
@@ -151,6 +151,8 @@ struct ResPlan {
 // most tiles an instance holds with its whole grid (cluster > 0: one cluster of that many blocks)
 // resident; 0: not available
 int res_capacity(bool masked, bool half, int rows, int cluster = 0);
+// host bytes (a multiple of four) to the device, stream-ordered; they are taken before the call returns
+void launch_res_upload(void* to, const void* from, size_t bytes, cudaStream_t st);
 void launch_resident(const ResArgs& A, bool masked, bool half, cudaStream_t st);
 // reads and clears the device status (1: a bounded wait ran out)
 int resident_status_take();

@@ -32,7 +32,7 @@ std::vector<uint8_t> res_circle_codes(int w, int h) {
 
 // A level is mostly tiles' rows that are on or off throughout; those take three or four 8-byte looks
 // (a 1280 x 1024 disc: 2.25 ms a pixel at a time, 0.40 this way; a new mask pays it).
-bool ResLevel::scan(const uint8_t* code, int w_, int h_, bool masked_) {
+bool ResLevel::scan(const uint8_t* code, int pitch, int w_, int h_, bool masked_) {
   w = w_;
   h = h_;
   masked = masked_;
@@ -53,7 +53,7 @@ bool ResLevel::scan(const uint8_t* code, int w_, int h_, bool masked_) {
   };
   bool any = false;
   for (int y = 0; y < h; y++) {
-    const uint8_t* c = code + (size_t)y * w;
+    const uint8_t* c = code + (size_t)y * pitch;
     auto mark = [&](int x, int yy) { need[(size_t)(yy / kResRows[0]) * tx + x / kResCols] = 1; };
     // per pixel: 1 on, 2 interior, 4 takes part in a read of a masked-out pixel
     auto flags = [&](int x) -> uint8_t {
@@ -77,7 +77,7 @@ bool ResLevel::scan(const uint8_t* code, int w_, int h_, bool masked_) {
           all = some = 3;
           read = false;
         } else if (!masked && (a & (kEach * kOn)) == kEach * kOn && x0 >= 1 && x1 < w && y >= 1 && y + 1 < h && (c[x1] & kOn)) {
-          bits(c + w + x0, a, o);
+          bits(c + pitch + x0, a, o);
           if ((a & (kEach * kOn)) == kEach * kOn) {
             all = some = 3;
             read = false;
@@ -103,7 +103,7 @@ bool ResLevel::scan(const uint8_t* code, int w_, int h_, bool masked_) {
           } else {
             // a pixel outside the circle that the first iteration reads
             if (x + 1 < w && !(c[x + 1] & kOn)) mark(x + 1, y);
-            if (y + 1 < h && !(c[x + w] & kOn)) mark(x, y + 1);
+            if (y + 1 < h && !(c[x + pitch] & kOn)) mark(x, y + 1);
           }
         }
       }
@@ -205,12 +205,12 @@ void ResTiles::place(int grid) {
 // quarters of the warps: fuller, the row above each tile, which two rows pay for as much as four,
 // costs more than it gives (424 x 400, 91 %: 2 rows 2.0, 4 rows 1.87).  12 and 16 rows (half storage) cost
 // more a pixel (kernels_resident.cu) and take the levels that 8 rows do not.
-bool res_choose(const uint8_t* code, int w, int h, bool masked, bool half, ResTiles& out) {
+bool res_choose(const uint8_t* code, int pitch, int w, int h, bool masked, bool half, ResTiles& out) {
   int dev = 0, sms = 0;
   VFS_CUDA(cudaGetDevice(&dev));
   VFS_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   ResLevel L;
-  if (!L.scan(code, w, h, masked)) return false;
+  if (!L.scan(code, pitch, w, h, masked)) return false;
   out.cluster = false;
   // (a capacity is asked for only where the count may fit: the first question loads the kernel)
   if (const int n = L.count(kResClusterRows);

@@ -334,10 +334,10 @@ void StereoTgvImpl::initialize(const SolverParams& p) {
   code_masked.assign(levels(), nullptr);
   code_plain.assign(levels(), nullptr);
   size_t at = pool_bytes_;
-  for (int l = 0; l < levels(); l++)
-    for (uint8_t** c : {&code_masked[l], &code_plain[l]}) {
+  for (std::vector<uint8_t*>* form : {&code_masked, &code_plain})
+    for (int l = 0; l < levels(); l++) {
       at = (at + 511) & ~(size_t)511;
-      *c = (uint8_t*)pool_ + at;
+      (*form)[l] = (uint8_t*)pool_ + at;
       at += (size_t)pS[l] * pH[l];
       guards_.push_back(pool_ + at);
       at += kGuardBytes;
@@ -346,6 +346,9 @@ void StereoTgvImpl::initialize(const SolverParams& p) {
   fillGuards(0, stream_);
   for (int l = 0; l < levels(); l++) launch_edge_codes(nullptr, code_plain[l], pW[l], pH[l], pS[l], stream_);
   VFS_CUDA(cudaStreamSynchronize(stream_));
+  // the zero mask's codes
+  mask_code.assign(code_masked.back() - code_masked[0] + (size_t)pS.back() * pH.back(), 0);
+  codes_valid = mask_taken = true;
   initialized_ = true;
 }
 
@@ -370,13 +373,13 @@ void StereoTgvImpl::loadVectorFields(const float* tv, const float* cvf) {
 void StereoTgvImpl::copyMaskToDevice(const float* mask) {
   if (!initialized_) throw ArgError{"copyMaskToDevice before initialize"};
   if (!mask) throw ArgError{"copyMaskToDevice: null mask"};
+  codes_valid = false;
   size_t row = (size_t)width * sizeof(float);
   VFS_CUDA(cudaMemsetAsync(pMask[0], 0, full_ * sizeof(float), stream_));
   VFS_CUDA(cudaMemcpy2DAsync(pMask[0], (size_t)stride * sizeof(float), mask, row, row, height, cudaMemcpyHostToDevice,
                              stream_));
   for (int l = 1; l < P.nLevels; l++) launch_downscale_nearest(t1(pMask[l - 1], l - 1, false), pMask[l], geom(l), stream_);
-  codes_valid = false;
-  VFS_CUDA(cudaStreamSynchronize(stream_));
+  makeMaskCodes();
 }
 
 // stereotgv.cu:201-213 (u8) and 215-239 (f32, u8c3)
@@ -479,27 +482,29 @@ void StereoTgvImpl::ensureFused() {
   fillGuards(guards_before, stream_);
 }
 
-void StereoTgvImpl::ensureMaskCodes() {
-  if (codes_valid) return;
-  dropResident(true);
-  mask_code.assign(levels(), {});
-  for (int l = 0; l < levels(); l++) {
-    launch_edge_codes(pMask[l], code_masked[l], pW[l], pH[l], pS[l], stream_);
-    mask_code[l].resize((size_t)pW[l] * pH[l]);
-    VFS_CUDA(cudaMemcpy2DAsync(mask_code[l].data(), pW[l], code_masked[l], pS[l], pW[l], pH[l], cudaMemcpyDeviceToHost,
-                               stream_));
-  }
+void StereoTgvImpl::makeMaskCodes() {
+  codes_valid = false;
+  const int last = levels() - 1;
+  mask_code.resize(code_masked[last] - code_masked[0] + (size_t)pS[last] * pH[last]);
+  for (int l = 0; l <= last; l++) launch_edge_codes(pMask[l], code_masked[l], pW[l], pH[l], pS[l], stream_);
+  VFS_CUDA(cudaMemcpyAsync(mask_code.data(), code_masked[0], mask_code.size(), cudaMemcpyDeviceToHost, stream_));
   VFS_CUDA(cudaStreamSynchronize(stream_));
-  spans_valid = false;
+  dropResident(true);  // (no launch uses the old plans any more)
+  spans_valid = mask_taken = false;
   codes_valid = true;
-  generation = next_generation();  // graphs captured under the old mask are not reused
+}
+
+void StereoTgvImpl::takeMask() {
+  if (!codes_valid) makeMaskCodes();
+  if (!mask_taken) generation = next_generation();  // graphs captured under the old mask are not reused
+  mask_taken = true;
 }
 
 // Whether every level of the next solve has a plan.  Not in a caller's stream capture: the caller may
 // replay its graph after the mask has changed, and a plan belongs to one mask.
 bool StereoTgvImpl::dropinResident(bool masked) {
   if (stream_capturing(stream_)) return false;
-  if (masked) ensureMaskCodes();
+  if (masked) takeMask();
   ensureResident(masked, false, stream_);
   for (int l = 0; l <= topLevel(); l++)
     if (!residentPlan(masked, false, l)) return false;
@@ -544,7 +549,8 @@ void StereoTgvImpl::ensureResident(bool masked, bool half, cudaStream_t st) {
   std::vector<Off> off(levels());
   for (int l = 0; l < levels(); l++) {
     const std::vector<uint8_t> circle = masked ? std::vector<uint8_t>{} : res_circle_codes(pW[l], pH[l]);
-    if (!res_choose(masked ? mask_code[l].data() : circle.data(), pW[l], pH[l], masked, half, cut[l])) continue;
+    if (!res_choose(masked ? maskCode(l) : circle.data(), masked ? pS[l] : pW[l], pW[l], pH[l], masked, half, cut[l]))
+      continue;
     plans[l].rows = cut[l].rows;
     plans[l].blocks = cut[l].blocks;
     plans[l].cluster = cut[l].cluster;
@@ -566,8 +572,7 @@ void StereoTgvImpl::ensureResident(bool masked, bool half, cudaStream_t st) {
     return;
   }
   res_mem_[masked][half] = m;
-  // the words' tags start at 0, which no launch waits for (epochs count from 1); the uploads are from
-  // pageable memory, staged before the calls return
+  // the words' tags start at 0, which no launch waits for (epochs count from 1)
   VFS_CUDA(cudaMemsetAsync(m, 0, bytes, st));
   for (int l = 0; l < levels(); l++) {
     ResPlan& p = plans[l];
@@ -576,11 +581,8 @@ void StereoTgvImpl::ensureResident(bool masked, bool half, cudaStream_t st) {
     p.tiles = (const ResTile*)(m + off[l].tiles);
     p.fill = (const int2*)(m + off[l].fill);
     p.exch = (uint4*)(m + off[l].exch);
-    VFS_CUDA(cudaMemcpyAsync(m + off[l].tiles, cut[l].tiles.data(), cut[l].tiles.size() * sizeof(ResTile),
-                             cudaMemcpyHostToDevice, st));
-    if (p.nfill)
-      VFS_CUDA(cudaMemcpyAsync(m + off[l].fill, cut[l].fill.data(), cut[l].fill.size() * sizeof(int2),
-                               cudaMemcpyHostToDevice, st));
+    launch_res_upload(m + off[l].tiles, cut[l].tiles.data(), cut[l].tiles.size() * sizeof(ResTile), st);
+    launch_res_upload(m + off[l].fill, cut[l].fill.data(), cut[l].fill.size() * sizeof(int2), st);
   }
 }
 
@@ -760,8 +762,8 @@ void StereoTgvImpl::importState(const void* host, size_t bytes) {
   f_parity = h.f_parity;
   have_prev = h.have_prev != 0;
   i1warp_half = h.i1warp_half != 0;
-  codes_valid = false;  // the masked edge codes and tile spans are derived again from the mask
   generation = next_generation();
+  makeMaskCodes();
 }
 
 // stereotgv.cu:517-568 outputs: level-0 views of u, warpUV, the warped image.

@@ -179,13 +179,18 @@ class StereoTgvImpl {
   // half storage: the current level's coefficient records of the iteration (IterPair::abce, rv)
   float4* f_abce = nullptr;
   float2* f_rv = nullptr;
-  std::vector<uint8_t*> code_masked, code_plain;
-  bool codes_valid = false;
-  // the masked form's edge codes on the device and the host, on the handle's stream (which it
-  // synchronises when they are not there yet).  The plain form's are made with the buffers.
-  void ensureMaskCodes();
-  // host copies of the masked form's edge codes per level (tight rows)
-  std::vector<std::vector<uint8_t>> mask_code;
+  std::vector<uint8_t*> code_masked, code_plain;  // (the masked form's levels lie together)
+  // Edge codes of the mask on the device, there and on the host.  Made with every new mask, where the
+  // stream is synchronised anyway, so that a solve never waits for the stream; the plain
+  // form's are made with the buffers.
+  void makeMaskCodes();
+  // Host side of a masked solve's start: the first with a new mask renews the generation.
+  void takeMask();
+  bool codes_valid = false;   // false: the last mask's codes could not be made
+  bool mask_taken = true;     // false: no solve has used the codes yet
+  // host copy of code_masked, all levels with their pitch and what lies between them
+  std::vector<uint8_t> mask_code;
+  const uint8_t* maskCode(int level) const { return mask_code.data() + (code_masked[level] - code_masked[0]); }
   // ---- register-resident iteration (resident.cuh): a plan per level, for the plain [0] and
   // masked [1] form and for float [0] and half [1] storage, made on the first solve of that
   // form with the current mask, on the solve's stream.  Its device memory (tiles and exchange words)
