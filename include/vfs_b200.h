@@ -97,7 +97,9 @@ int vfs_import_state(vfs_stereo* s, const void* host, size_t bytes);
 
 /* Test hook (no counterpart in the reference): with n > 0 the n-th following device-pool
  * allocation of any handle fails as if the GPU were out of memory (the call returns
- * VFS_ERR_NOMEM and leaves nothing allocated); 0 turns it off. */
+ * VFS_ERR_NOMEM and leaves nothing allocated); 0 turns it off.  The plans of the whole-level
+ * launches count one for every level and one for memory of their own; where one of those
+ * fails, the solve runs without whole-level launches. */
 int vfs_debug_fail_allocation(int n);
 /* Test hook (no counterpart in the reference): every device plane of a handle is followed by
  * a 256-byte guard zone of 0xA5 bytes, written when the plane is allocated.  *bad_zones is the

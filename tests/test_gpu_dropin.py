@@ -139,3 +139,33 @@ def test_solves_return_after_enqueueing(gpu, size, fused, half):
             waited = before.query()
             torch.cuda.synchronize()
             assert warm or not waited, (masked, mask is not None)
+
+
+@pytest.mark.parametrize("fused", [False, True], ids=["dropin", "fp32"])
+def test_plans_that_cannot_be_made(gpu, fused):
+    """Device memory runs out at each step of a form's tile plans (one a level; the second form's own
+    memory): the solve runs one iteration a launch, and the next mask has its plans."""
+    from vfs_b200._native import lib
+    from vfs_b200.stereotgv import StereoTgv
+    case = random_case(150, 110, seed=31)
+    p = params(n_levels=3, n_warp=1, n_iter=100)
+    want = {m: _disparity(_solver(case, p), case, masked=m) for m in (True, False)}
+
+    def launches(s, masked):
+        n = StereoTgv.launch_count()
+        assert np.array_equal(_disparity(s, case, masked), want[masked])
+        return StereoTgv.launch_count() - n
+
+    for failing in (1, 2, 3):
+        s = _solver(case, p, fused=fused)
+        s.set_autotune(False)
+        assert lib().vfs_debug_fail_allocation(failing + (1 if fused else 0)) == 0  # the fused buffers come first
+        assert launches(s, True) > 300
+        assert launches(s, True) > 300
+        s.copyMaskToDevice(case[2])
+        assert launches(s, True) < 100
+    assert lib().vfs_debug_fail_allocation(4) == 0  # the unmasked form's plans beside the masked form's
+    assert launches(s, False) > 300 and launches(s, False) > 300
+    assert launches(s, True) < 100
+    assert lib().vfs_debug_fail_allocation(0) == 0
+    assert s.check_guards() == 0

@@ -115,11 +115,15 @@ std::atomic<int>& alloc_failure_countdown() {
   return n;
 }
 
-static cudaError_t pool_malloc(void** p, size_t bytes) {
+static bool alloc_failure_due() {
   int n = alloc_failure_countdown().load();
   while (n > 0 && !alloc_failure_countdown().compare_exchange_weak(n, n - 1)) {
   }
-  if (n == 1) {
+  return n == 1;
+}
+
+static cudaError_t pool_malloc(void** p, size_t bytes) {
+  if (alloc_failure_due()) {
     *p = nullptr;
     return cudaErrorMemoryAllocation;
   }
@@ -514,19 +518,41 @@ bool StereoTgvImpl::dropinResident(bool masked) {
 void StereoTgvImpl::dropResident(bool masked) {
   for (int half = 0; half < 2; half++) {
     res_plans_[masked][half].clear();
-    char*& m = res_mem_[masked][half];
-    if (m && m == pool_ + resRoomAt()) res_room_used_ = false;
-    else if (m) cudaFree(m);
-    m = nullptr;
+    resFree(res_mem_[masked][half]);
+    res_mem_[masked][half] = nullptr;
   }
+}
+
+void StereoTgvImpl::resFree(char* m) {
+  if (m && m == pool_ + resRoomAt()) res_room_used_ = false;
+  else if (m) cudaFree(m);
 }
 
 // Needs the masked form's edge codes on the host.  Without memory for the plans the levels
 // simply have none (the solve then launches one iteration at a time).
 void StereoTgvImpl::ensureResident(bool masked, bool half, cudaStream_t st) {
-  std::vector<ResPlan>& plans = res_plans_[masked][half];
-  if (!plans.empty()) return;
-  plans.assign(levels(), ResPlan{});
+  if (!res_plans_[masked][half].empty()) return;
+  std::vector<ResPlan> plans(levels());
+  char* m = nullptr;
+  auto out_of_memory = [&] {
+    resFree(m);
+    m = nullptr;
+    plans.assign(levels(), ResPlan{});
+  };
+  try {
+    makePlans(masked, half, st, plans, m);
+  } catch (const CudaError& e) {  // a kernel that could not be loaded, or the plan's memory
+    out_of_memory();
+    if (e.err != cudaErrorMemoryAllocation) throw;
+    (void)cudaGetLastError();
+  } catch (const std::bad_alloc&) {
+    out_of_memory();
+  }
+  res_mem_[masked][half] = m;
+  res_plans_[masked][half] = std::move(plans);  // only now: whole, on the device, or none at all
+}
+
+void StereoTgvImpl::makePlans(bool masked, bool half, cudaStream_t st, std::vector<ResPlan>& plans, char*& m) {
   if (P.nSolverIters < 1 || P.nSolverIters > kResMaxIters || !(P.lambda >= 0.0f)) return;
   // its quotients and roots take step sizes in a range that no sane schedule leaves
   float tau = 1.0f, sigma = 1.0f;
@@ -548,6 +574,7 @@ void StereoTgvImpl::ensureResident(bool masked, bool half, cudaStream_t st) {
   };
   std::vector<Off> off(levels());
   for (int l = 0; l < levels(); l++) {
+    if (alloc_failure_due()) throw CudaError{cudaErrorMemoryAllocation, "plan of a level", __FILE__, __LINE__};
     const std::vector<uint8_t> circle = masked ? std::vector<uint8_t>{} : res_circle_codes(pW[l], pH[l]);
     if (!res_choose(masked ? maskCode(l) : circle.data(), masked ? pS[l] : pW[l], pW[l], pH[l], masked, half, cut[l]))
       continue;
@@ -562,16 +589,12 @@ void StereoTgvImpl::ensureResident(bool masked, bool half, cudaStream_t st) {
     off[l].exch = take((size_t)kResRing * plans[l].ntiles * res_slots(plans[l].rows) * sizeof(uint4));
   }
   if (bytes == 0) return;
-  char* m = nullptr;
   if (!res_room_used_ && bytes <= res_room_) {
     m = pool_ + resRoomAt();
     res_room_used_ = true;
-  } else if (cudaMalloc((void**)&m, bytes) != cudaSuccess) {
-    (void)cudaGetLastError();
-    plans.assign(levels(), ResPlan{});
-    return;
+  } else {
+    VFS_CUDA(pool_malloc((void**)&m, bytes));
   }
-  res_mem_[masked][half] = m;
   // the words' tags start at 0, which no launch waits for (epochs count from 1)
   VFS_CUDA(cudaMemsetAsync(m, 0, bytes, st));
   for (int l = 0; l < levels(); l++) {

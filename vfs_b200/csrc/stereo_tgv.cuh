@@ -300,6 +300,9 @@ class StereoTgvImpl {
   std::vector<cudaEvent_t> evpool_;
   size_t evused_ = 0;
 
+  // the plans of a form, with their device memory (m); throws with m set where that was already taken
+  void makePlans(bool masked, bool half, cudaStream_t st, std::vector<ResPlan>& plans, char*& m);
+  void resFree(char* m);
   std::vector<ResPlan> res_plans_[2][2];
   char* res_mem_[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};
   size_t res_room_ = 0;       // bytes kept for plans behind the pool's planes
