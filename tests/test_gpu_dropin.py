@@ -1,6 +1,8 @@
 """What a program sees around the solves that run whole levels in one launch: streams, captures, masks,
 first solves, errors, and the buffers that the default path leaves."""
+import ctypes
 import subprocess
+import threading
 
 import numpy as np
 import pytest
@@ -169,3 +171,55 @@ def test_plans_that_cannot_be_made(gpu, fused):
     assert launches(s, True) < 100
     assert lib().vfs_debug_fail_allocation(0) == 0
     assert s.check_guards() == 0
+
+
+@pytest.mark.parametrize("stream", [1, 2], ids=["legacy", "per-thread"])
+def test_default_path_on_the_default_streams(gpu, stream):
+    """cudaStreamLegacy and cudaStreamPerThread as the handle's stream: the first cannot be captured."""
+    case = random_case(150, 110, seed=17)
+    p = params(n_levels=2, n_warp=2, n_iter=20)
+    for masked in (True, False):
+        want = _disparity(_solver(case, p), case, masked)
+        s = _solver(case, p, stream)
+        for _ in range(8):
+            assert np.array_equal(_disparity(s, case, masked), want)
+
+
+def test_default_path_beside_work_on_the_legacy_stream(gpu):
+    """The handle on a stream that synchronises with the legacy default stream, on which another
+    thread keeps working: both go on undisturbed."""
+    import torch
+    rt = ctypes.CDLL("libcudart.so.12")
+    st = ctypes.c_void_p()
+    assert rt.cudaStreamCreate(ctypes.byref(st)) == 0
+    case = random_case(150, 110, seed=19)
+    p = params(n_levels=3, n_warp=2, n_iter=20)
+    want = _disparity(_solver(case, p), case)
+    s = _solver(case, p, st.value)
+    x = torch.zeros(1024, device="cuda")
+    torch.cuda.synchronize()
+    stop, errors, calls = threading.Event(), [], [0]
+
+    def work():
+        while not stop.is_set():
+            e = rt.cudaMemsetAsync(ctypes.c_void_p(x.data_ptr()), 0, ctypes.c_size_t(4096), ctypes.c_void_p(1))
+            if e:
+                errors.append(e)
+            calls[0] += 1
+            if calls[0] % 64 == 0:
+                rt.cudaStreamSynchronize(ctypes.c_void_p(1))
+
+    t = threading.Thread(target=work)
+    t.start()
+    try:
+        for k in range(12):
+            s.copyMaskToDevice(case[2])  # the graphs of the last mask go
+            for _ in range(5):
+                assert np.array_equal(_disparity(s, case), want)
+    finally:
+        stop.set()
+        t.join()
+        s.close()
+        rt.cudaStreamDestroy(st)
+    assert not errors, errors[:3]
+    assert calls[0] > 100

@@ -863,6 +863,26 @@ void FusedEngine::solve_dropin(StereoTgvImpl* pair, bool masked, cudaStream_t st
   pair->i1warp_half = false;
 }
 
+namespace {
+// The stream a graph is recorded on.  For the drop-in path one of its own, of the solve's priority: the
+// caller's may be the legacy default stream, which cannot be captured, or a stream that synchronises
+// with it, where another thread's work on the default stream would break the capture (and fail).
+struct RecordStream {
+  cudaStream_t st;
+  const bool own;
+  RecordStream(cudaStream_t solve, bool separate) : st(solve), own(separate) {
+    if (!own) return;
+    int priority = 0;
+    VFS_CUDA(cudaStreamGetPriority(solve, &priority));
+    VFS_CUDA(cudaStreamCreateWithPriority(&st, cudaStreamNonBlocking, priority));
+  }
+  RecordStream(const RecordStream&) = delete;
+  ~RecordStream() {
+    if (own) cudaStreamDestroy(st);
+  }
+};
+}  // namespace
+
 // The solve with the variants settled: from a graph captured in the same state, or directly.
 void FusedEngine::run(std::vector<StereoTgvImpl*>& pairs, bool masked, bool half, cudaStream_t st, int part,
                       std::vector<int>& variants, bool dropin) {
@@ -893,18 +913,19 @@ void FusedEngine::run(std::vector<StereoTgvImpl*>& pairs, bool masked, bool half
     evict(pairs);
     Entry e;
     for (auto* s : pairs) e.owners.emplace_back(s, s->generation);
+    const RecordStream rec(st, dropin);
+    cudaGraph_t g = nullptr;
+    VFS_CUDA(cudaStreamBeginCapture(rec.st, cudaStreamCaptureModeRelaxed));
     std::vector<ProfRec> saved = prof->profRecords();
     prof->profReset();
     prof->capture_events = &e.events;
-    cudaGraph_t g = nullptr;
     long long launches0 = launch_counter().load();
-    VFS_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeRelaxed));
     try {
-      fused_solve_direct(pairs, masked, half, st, variants, false, concurrency, part, dropin);
+      fused_solve_direct(pairs, masked, half, rec.st, variants, false, concurrency, part, dropin);
     } catch (...) {
       prof->capture_events = nullptr;
       cudaGraph_t junk = nullptr;
-      cudaStreamEndCapture(st, &junk);
+      cudaStreamEndCapture(rec.st, &junk);
       if (junk) cudaGraphDestroy(junk);
       for (auto ev : e.events) cudaEventDestroy(ev);
       for (size_t k = 0; k < pairs.size(); k++) set_ptrs(pairs[k], before[k]);
@@ -913,7 +934,7 @@ void FusedEngine::run(std::vector<StereoTgvImpl*>& pairs, bool masked, bool half
     prof->capture_events = nullptr;
     e.kernels = launch_counter().load() - launches0;
     launch_counter().fetch_sub(e.kernels);  // captured, not launched: counted when replayed
-    VFS_CUDA(cudaStreamEndCapture(st, &g));
+    VFS_CUDA(cudaStreamEndCapture(rec.st, &g));
     cudaError_t ie = cudaGraphInstantiate(&e.exec, g, 0);
     cudaGraphDestroy(g);
     if (ie != cudaSuccess) throw CudaError{ie, "cudaGraphInstantiate", __FILE__, __LINE__};
