@@ -223,3 +223,45 @@ def test_default_path_beside_work_on_the_legacy_stream(gpu):
         rt.cudaStreamDestroy(st)
     assert not errors, errors[:3]
     assert calls[0] > 100
+
+
+def test_states_that_come_once(gpu):
+    """A new mask or limit for every frame: nothing is recorded that is not replayed, and a short solve
+    makes its plans only when its mask comes a second time."""
+    from vfs_b200._native import lib
+    from vfs_b200.stereotgv import StereoTgv
+    case = random_case(150, 110, seed=41)
+    other = np.ascontiguousarray(case[2][:, ::-1])
+
+    def pair(p):  # and the same frames through the one-iteration kernels
+        s, t = _solver(case, p), _solver(case, p, fused=True)
+        t.set_iteration_variant(1)
+        return s, t
+
+    def frame(st, mask=None, limit=None):
+        u = []
+        for s in st:
+            if mask is not None:
+                s.copyMaskToDevice(mask)
+            if limit is not None:
+                s.limitRange = limit
+            n = StereoTgv.launch_count()
+            u.append(_disparity(s, case))
+            if s is st[0]:
+                launches = StereoTgv.launch_count() - n
+        assert np.array_equal(*u)
+        return launches
+
+    short, usual = params(n_levels=2, n_warp=1, n_iter=5), params(n_levels=2, n_warp=1, n_iter=6)
+    st = pair(short)
+    per_operation = frame(st)
+    assert frame(st) < per_operation  # the mask's second solve
+    for mask in (other, case[2]):
+        assert frame(st, mask) == per_operation
+    st = pair(usual)
+    for k in range(6):
+        assert frame(st, case[2], 0.1 + 0.01 * k) < per_operation
+    assert lib().vfs_cached_graphs(st[0].handle) == 0
+    for k in range(6):
+        frame(st)
+    assert lib().vfs_cached_graphs(st[0].handle) > 0

@@ -909,10 +909,21 @@ void FusedEngine::run(std::vector<StereoTgvImpl*>& pairs, bool masked, bool half
     key.push_back(lr);
   }
   auto it = cache_.find(key);
-  if (it == cache_.end()) {
+  Entry e;
+  for (auto* s : pairs) e.owners.emplace_back(s, s->generation);
+  if (it == cache_.end() && dropin) {
+    // The drop-in path records a state when it meets it again: a program that changes its mask or limit
+    // every frame never does, and recording takes longer than launching once.
     evict(pairs);
-    Entry e;
-    for (auto* s : pairs) e.owners.emplace_back(s, s->generation);
+    e.last_use = ++use_clock_;
+    cache_.emplace(key, std::move(e));
+    if (prof->profiling) prof->profReset();  // the records describe the last solve
+    fused_solve_direct(pairs, masked, half, st, variants, false, concurrency, part, dropin);
+    return;
+  }
+  if (it == cache_.end() || !it->second.exec) {
+    if (it == cache_.end()) evict(pairs);
+    else cache_.erase(it);
     const RecordStream rec(st, dropin);
     cudaGraph_t g = nullptr;
     VFS_CUDA(cudaStreamBeginCapture(rec.st, cudaStreamCaptureModeRelaxed));

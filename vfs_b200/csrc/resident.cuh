@@ -62,6 +62,11 @@ constexpr int kResMostTiles = 148 * kResMostWarps;  // a bound on the tiles of a
 constexpr int kResClusterRows = 2;
 constexpr int kResClusterCtas = 16;
 inline int res_cluster_tiles(bool half) { return half ? 208 : 128; }
+// The drop-in path makes its plans at a mask's first solve where that runs at least so many iterations a
+// level (all warps), else at its second: a plan takes the host longer than a short solve saves.  B200, ms from a new
+// mask to the disparity on the host, 1 warp: 848 x 800 with plans 1.70 + 0.008 an iteration, a kernel per operation
+// 1.27 + 0.09; 424 x 400 0.77 + 0.003, 0.70 + 0.065; 64 x 48 0.23, 0.29 + 0.03.
+constexpr int kResPlanIters = 6;
 inline int res_slots(int rows) { return 64 + 2 * rows; }  // words per tile: top, bottom, left, right
 
 // What a tile's pixels ask of its iterations: none of the edge rules; the edge rules; or

@@ -147,7 +147,7 @@ void StereoTgvImpl::release() {
   code_plain.clear();
   codes_valid = spans_valid = false;
   pool_bytes_ = pool_used_ = res_room_ = 0;
-  res_room_used_ = false;
+  res_room_used_ = res_asked_[0] = res_asked_[1] = false;
   guards_.clear();
   initialized_ = false;
 }
@@ -494,7 +494,7 @@ void StereoTgvImpl::makeMaskCodes() {
   VFS_CUDA(cudaMemcpyAsync(mask_code.data(), code_masked[0], mask_code.size(), cudaMemcpyDeviceToHost, stream_));
   VFS_CUDA(cudaStreamSynchronize(stream_));
   dropResident(true);  // (no launch uses the old plans any more)
-  spans_valid = mask_taken = false;
+  spans_valid = mask_taken = res_asked_[1] = false;
   codes_valid = true;
 }
 
@@ -509,6 +509,10 @@ void StereoTgvImpl::takeMask() {
 bool StereoTgvImpl::dropinResident(bool masked) {
   if (stream_capturing(stream_)) return false;
   if (masked) takeMask();
+  if (P.nWarpIters * P.nSolverIters < kResPlanIters && res_plans_[masked][0].empty() && !res_asked_[masked]) {
+    res_asked_[masked] = true;
+    return false;
+  }
   ensureResident(masked, false, stream_);
   for (int l = 0; l <= topLevel(); l++)
     if (!residentPlan(masked, false, l)) return false;

@@ -64,14 +64,18 @@ class FusedEngine {
  public:
   // allocate fused buffers and refresh edge codes, each on the pair's own stream
   static void prepare(std::vector<StereoTgvImpl*>& pairs, bool masked);
-  size_t graphs() const { return cache_.size(); }
+  size_t graphs() const {
+    size_t n = 0;
+    for (const auto& kv : cache_) n += kv.second.exec != nullptr;
+    return n;
+  }
   // iteration-kernel variant per pyramid level (finest first) of the last solve
   std::vector<int> last_variants;
   void note_variants(std::vector<int> v, int part);
 
  private:
   struct Entry {
-    cudaGraphExec_t exec = nullptr;
+    cudaGraphExec_t exec = nullptr;  // null: met once, run directly
     long long kernels = 0;  // kernel launches recorded in the graph (added to the launch count per replay)
     std::vector<PairPtrs> after;
     std::vector<ProfRec> prof;
@@ -304,6 +308,7 @@ class StereoTgvImpl {
   void makePlans(bool masked, bool half, cudaStream_t st, std::vector<ResPlan>& plans, char*& m);
   void resFree(char* m);
   std::vector<ResPlan> res_plans_[2][2];
+  bool res_asked_[2] = {false, false};  // a short solve of the form has passed its plans by (dropinResident)
   char* res_mem_[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};
   size_t res_room_ = 0;       // bytes kept for plans behind the pool's planes
   bool res_room_used_ = false;
