@@ -471,6 +471,7 @@ def run_ours(args, rank, world, local):
     iv = np.concatenate([s.profile_intervals(kind) for s in solvers])
     for s in solvers:
         s.profile(False)
+        s.check_solve()  # no wait on the device ran out
     # all levels, and the dominant kernel alone: the iteration kernel at full resolution (the
     # records with the largest pixel count)
     pi_all = float(iv[:, 2].sum()) if len(iv) else 0.0

@@ -304,11 +304,20 @@ int vfs_equalize_hist_u8_noalloc(const uint8_t* d_src, uint8_t* d_dst, size_t n,
  * launch, 1 = fused inner launch, 2 = fused per-warp prologue, 3 = fused epilogue). */
 long long vfs_launch_count(void);
 
+/* The tiles of a whole-level launch wait on the device for one another's values, each wait with a limit
+ * (about a second).  When one runs out, the solve ends all the same and its results are undefined:
+ * vfs_synchronize, vfs_copy_*_to_host (except the debug ones) and vfs_batch_solve_host then return
+ * VFS_ERR_TIMEOUT instead of VFS_OK until the handle's next solve (vfs_batch_solve_host for every
+ * pair).  Programs that leave results on the device ask vfs_solve_status, which does not wait
+ * (VFS_OK or VFS_ERR_TIMEOUT), once the solve has completed.  (No counterpart in the reference.) */
+int vfs_solve_status(vfs_stereo* s);
+/* Test hook: whole-level launches enqueued while it is on leave out their first tile's first values, so
+ * that its neighbours' waits run out (on = 0: as usual). */
+int vfs_debug_mute_tile(int on);
 /* Device-side status of the current device (no counterpart in the reference): *status = 1 if
  * a kernel of the TMA-staged iteration variant gave up a bounded wait for its copies (its block
- * then wrote nothing), or one of the whole-level launches a wait for a neighbour's values (the
- * solve's results are then undefined), since the last call, else 0; the flag is cleared.
- * Synchronous. */
+ * then wrote nothing), or one of the whole-level launches of any handle a wait for a neighbour's
+ * values, since the last call, else 0; the flag is cleared.  Synchronous. */
 int vfs_device_status(int* status);
 /* Process-wide: launch the fused iteration kernels with programmatic dependent launch
  * (on = 1, the default), so that each launch is scheduled while the previous one drains;

@@ -265,3 +265,64 @@ def test_states_that_come_once(gpu):
     for k in range(6):
         frame(st)
     assert lib().vfs_cached_graphs(st[0].handle) > 0
+
+
+@pytest.fixture
+def muted(gpu):
+    """Whole-level launches leave out a tile's first values: its neighbours' waits run out."""
+    from vfs_b200._native import lib
+    st = ctypes.c_int()
+    lib().vfs_device_status(ctypes.byref(st))
+    assert lib().vfs_debug_mute_tile(1) == 0
+    yield lib()
+    assert lib().vfs_debug_mute_tile(0) == 0
+    lib().vfs_device_status(ctypes.byref(st))
+
+
+# in one cluster and on the whole GPU
+@pytest.mark.parametrize("size", [(60, 50), (300, 280)])
+@pytest.mark.parametrize("fused,half", [(False, False), (True, True)], ids=["dropin", "fp16"])
+def test_a_wait_that_runs_out_is_an_error(muted, size, fused, half):
+    from vfs_b200._native import VfsError
+    w, h = size
+    case = random_case(w, h, seed=w)
+    p = params(n_levels=1, n_warp=1, n_iter=40)
+    s = _solver(case, p, fused=fused, half=half)
+    s.check_solve()
+    for call in (lambda: _disparity(s, case), s.copyDisparityToHost, s.synchronize, s.check_solve):
+        with pytest.raises(VfsError) as e:  # the solve's copy, and every later question
+            call()
+        assert e.value.status == -6
+    st = ctypes.c_int()
+    assert muted.vfs_device_status(ctypes.byref(st)) == 0 and st.value == 1
+    muted.vfs_debug_mute_tile(0)
+    want = _disparity(_solver(case, p, fused=fused, half=half), case)
+    s.copyMaskToDevice(case[2])  # (recorded launches stay muted)
+    got = _disparity(s, case)
+    from scipy.ndimage import binary_erosion
+    on = binary_erosion(case[2] > 0, iterations=4)  # beyond the median's reach of masked-out pixels, which keep theirs
+    assert on.any() and np.array_equal(got[on], want[on])
+    s.check_solve()
+    assert s.check_guards() == 0
+
+
+def test_a_wait_that_runs_out_in_a_batch_and_a_server(muted):
+    from vfs_b200._native import VfsError
+    from vfs_b200.serving import StereoServer
+    from vfs_b200.stereotgv import StereoBatch
+    cases = [random_case(160, 120, seed=k) for k in range(2)]
+    p = params(n_levels=1, n_warp=1, n_iter=40)
+    b = StereoBatch(half_storage=True)
+    for c in cases:
+        b.add(_solver(c, p, fused=True, half=True))
+    with pytest.raises(VfsError) as e:
+        b.solve_host([c[:2] for c in cases])
+    assert e.value.status == -6 and "pair 0" in str(e.value)
+    for m in b.members:
+        with pytest.raises(VfsError):
+            m.check_solve()
+    srv = StereoServer(lanes=1)
+    srv.open_stream(0, 160, 120, cases[0][2], cases[0][3], cases[0][4], 1, dict(nWarpIters=1))
+    bad = srv.submit(0, *cases[0][:2])
+    srv.run_until_idle()
+    assert bad.u is None and "-6" in bad.error and srv.stats()["failed"] == 1

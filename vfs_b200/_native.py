@@ -41,6 +41,8 @@ SIGNATURES = {
     "vfs_destroy": [_vp],
     "vfs_set_stream": [_vp, _vp],
     "vfs_synchronize": [_vp],
+    "vfs_solve_status": [_vp],
+    "vfs_debug_mute_tile": [_i],
     "vfs_initialize": [_vp, _i, _i, _f, _f, _f, _f, _f, _f, _i, _f, _i, _i],
     "vfs_set_limit_range": [_vp, _f],
     "vfs_set_camera": [_vp, _f, _f],

@@ -428,6 +428,8 @@ void fused_solve_direct(std::vector<StereoTgvImpl*>& pairs, bool masked, bool ha
           A.rows = res->rows;
           A.blocks = res->blocks;
           A.cluster = res->cluster;
+          A.mute = res_muted().load(std::memory_order_relaxed) ? 0 : -1;
+          A.gave_up = act[0]->wait_word;
           A.minus_zero = make_float2(-0.0f, -0.0f);
           for (int j = 0; j < n_it; j++) {
             const float mu = sigma < 1000.0f ? 1.0f / std::sqrt(1 + 0.7f * tau * P0.timestep_lambda) : 1.0f;
@@ -640,6 +642,7 @@ void FusedEngine::evict(const std::vector<StereoTgvImpl*>& pairs) {
 void FusedEngine::prepare(std::vector<StereoTgvImpl*>& pairs, bool masked) {
   for (auto* s : pairs) {
     if (!s->initialized()) throw ArgError{"fused solve: pair not initialized"};
+    s->wait_failed = false;
     s->ensureFused();
     if (masked) s->takeMask();
   }

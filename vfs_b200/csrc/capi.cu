@@ -81,6 +81,9 @@ int guarded(H* s, F&& f) {
   } catch (const vfs::ArgError& e) {
     s->err = e.msg;
     return VFS_ERR_ARG;
+  } catch (const vfs::WaitError& e) {
+    s->err = e.msg;
+    return VFS_ERR_TIMEOUT;
   } catch (const std::bad_alloc&) {
     s->err = "host allocation failed";
     return VFS_ERR_NOMEM;
@@ -144,7 +147,19 @@ int vfs_set_stream(vfs_stereo* s, void* st) {
 }
 
 int vfs_synchronize(vfs_stereo* s) {
-  return guarded(s, [&] { VFS_CUDA(cudaStreamSynchronize(s->impl.stream())); });
+  return guarded(s, [&] {
+    VFS_CUDA(cudaStreamSynchronize(s->impl.stream()));
+    s->impl.checkWaits();
+  });
+}
+
+int vfs_solve_status(vfs_stereo* s) {
+  return guarded(s, [&] { s->impl.checkWaits(); });
+}
+
+int vfs_debug_mute_tile(int on) {
+  vfs::res_muted().store(on != 0);
+  return VFS_OK;
 }
 
 int vfs_initialize(vfs_stereo* s, int width, int height, float beta, float gamma, float alpha0, float alpha1,
@@ -301,6 +316,7 @@ int vfs_copy_stereo_to_host(vfs_stereo* s, float* depth, float* X, float fx, flo
     if (depth) s->impl.copyOut("depth", depth, true);
     if (X) s->impl.copyOut("X", X, true);
     VFS_CUDA(cudaStreamSynchronize(s->impl.stream()));
+    s->impl.checkWaits();
   });
 }
 
@@ -648,7 +664,16 @@ void batch_solve(vfs_batch* b, int masked, const BatchHostIO* io) {
   VFS_CUDA(cudaEventRecord(b->done, b->stream));
   for (auto* p : pairs)
     if (p->stream() != b->stream) VFS_CUDA(cudaStreamWaitEvent(p->stream(), b->done, 0));
-  if (io && !io->device) VFS_CUDA(cudaStreamSynchronize(b->stream));
+  if (io && !io->device) {
+    VFS_CUDA(cudaStreamSynchronize(b->stream));
+    for (size_t k = 0; k < pairs.size(); k++) {
+      try {
+        pairs[k]->checkWaits();
+      } catch (const vfs::WaitError& e) {
+        throw vfs::WaitError{"pair " + std::to_string(k) + ": " + e.msg};
+      }
+    }
+  }
 }
 
 }  // namespace
@@ -866,6 +891,7 @@ void SolveStereo(vfs_stereo* s, unsigned char* fs1, unsigned char* fs2, unsigned
       }
     } else {
       VFS_CUDA(cudaStreamSynchronize(st));
+      I.checkWaits();
     }
   });
 }

@@ -69,6 +69,9 @@ enum ProfTag { kProfInner = 0, kProfFused = 1, kProfPrologue = 2, kProfEpilogue 
 struct ArgError {
   std::string msg;
 };
+struct WaitError {  // a solve's results are undefined: a wait on the device ran out
+  std::string msg;
+};
 
 // Programmatic dependent launch of the fused iteration kernels.  With it on, the next launch
 // on a stream may be scheduled while the previous one drains; every kernel launched this way

@@ -19,9 +19,14 @@ namespace x2 = fast::x2;
 namespace {
 
 constexpr unsigned kFull = 0xffffffffu;
-constexpr int kResMaxPolls = 1 << 20;
+constexpr int kResLooks = 1 << 20;  // after which a wait gives up: some 0.5 to 1 s
 
 __device__ int g_res_status;  // 1 = a wait for a neighbour's words ran out
+
+__device__ __forceinline__ void give_up(const ResArgs& A) {
+  g_res_status = 1;
+  *(volatile unsigned*)A.gave_up = 1u;
+}
 
 // one exchange word as a single 128-bit memory operation at L2
 __device__ __forceinline__ void st_word(uint4* p, uint4 v) {
@@ -1096,9 +1101,9 @@ struct ResWarp {
       wc = ld_word(base + o.z);
       const unsigned other = (wn.w ^ tag) | (ws.w ^ tag) | (wc.w ^ tag);
       if (__all_sync(kFull, (kPlain ? other & ~kResBeyond : other) == 0) || !waiting) break;
-      if (polls >= kResMaxPolls) {
+      if (polls >= kResLooks) {
         waiting = false;
-        if (lane == 0) g_res_status = 1;
+        if (lane == 0) atomicAdd(&A.ctl->done, kResGaveUp);
         break;
       }
     }
@@ -1217,7 +1222,8 @@ __global__ void __launch_bounds__(32 * kResMostWarps, 1) k_resident(const __grid
     ResWarp<MASKED, ST, R> W;
     const ResTile T = A.tiles[t];
     W.link(sh, lane, T, W.load(sh, A, lane, t, T));
-    publish<R>(W.s, A.exch + (size_t)t * (64 + 2 * R), lane, epoch | W.flag(sh));  // iteration 0's input
+    if (t != A.mute)  // iteration 0's input
+      publish<R>(W.s, A.exch + (size_t)t * (64 + 2 * R), lane, epoch | W.flag(sh));
     __syncwarp();
     bool waiting = true;
 #pragma unroll 1
@@ -1231,9 +1237,11 @@ __global__ void __launch_bounds__(32 * kResMostWarps, 1) k_resident(const __grid
   __syncthreads();
   if (threadIdx.x == 0) {
     __threadfence();
-    if (atomicAdd(&A.ctl->done, 1u) == gridDim.x - 1) {
+    const unsigned done = atomicAdd(&A.ctl->done, 1u);
+    if ((done & (kResGaveUp - 1u)) == gridDim.x - 1) {
       A.ctl->done = 0;
       A.ctl->epoch += 1;
+      if (done >= kResGaveUp) give_up(A);
     }
   }
 }
@@ -1247,7 +1255,7 @@ __global__ void __launch_bounds__(32 * kResMostWarps, 1) k_resident(const __grid
 // iteration, for the reason the ring has two.
 namespace {
 
-constexpr int kResMaxWaits = 1 << 20;
+constexpr int kResWaits = 1 << 16;  // after which a wait gives up: some 0.8 s
 
 template <class ST>
 struct ResWord;  // u-bar and v-bar of a border pixel
@@ -1389,26 +1397,25 @@ __global__ void __launch_bounds__(512, 1) k_resident_cluster(const __grid_consta
   }
   cl_barrier();  // every inbox is ready
   if (t < A.ntiles) {
-    push<ST, R>(W.s, C, lane, 0, W.flag(sh));  // iteration 0's input
+    if (t != A.mute) push<ST, R>(W.s, C, lane, 0, W.flag(sh));  // iteration 0's input
     bool waiting = true;
 #pragma unroll 1
     for (int j = 0; j < A.n; j++) {
       const int k = j & 1;
       for (int waits = 0; waiting && !bar_wait(bar + 8u * k, (unsigned)(j >> 1) & 1u); waits++)
-        if (waits >= kResMaxWaits) {
-          waiting = false;
-          g_res_status = 1;
-        }
+        if (waits >= kResWaits) waiting = false;
       __syncwarp();
       const uint4 wn = Word::wide(C.in[k].n[lane]), ws = Word::wide(C.in[k].s[lane]);
       if (lane == 0 || lane == 31) W.s.take_col(C.in[k].c[lane >> 4]);
       if constexpr (W.kPlain) W.meet(sh, wn.w | ws.w | C.in[k].c[lane >> 4][lane & (R - 1)].w);
       __syncwarp();
-      if (lane == 0 && j + 2 < A.n) bar_arm(bar + 8u * k, C.bytes);  // for iteration j + 2
+      // for iteration j + 2 (not once the barrier may still be armed for this one)
+      if (lane == 0 && waiting && j + 2 < A.n) bar_arm(bar + 8u * k, C.bytes);
       W.iterate(sh, A, lane, j, ex, wn, ws);
       if (j + 1 < A.n) push<ST, R>(W.s, C, lane, j + 1, W.flag(sh));
       if (j + 2 >= A.n) W.store(sh, A, lane, j + 1 == A.n);
     }
+    if (!waiting && lane == 0) give_up(A);
   }
   if (!MASKED) res_fill<ST, R>(A, warp, lane);
   cl_barrier();  // no block leaves while its neighbours may store into it
@@ -1566,6 +1573,11 @@ void launch_resident(const ResArgs& A, bool masked, bool half, cudaStream_t st) 
     return A.cluster ? decltype(k)::launch_cluster(A, st) : decltype(k)::launch(A, st);
   });
   VFS_LAUNCH_CHECK();
+}
+
+std::atomic<bool>& res_muted() {
+  static std::atomic<bool> on{false};
+  return on;
 }
 
 int resident_status_take() {

@@ -22,8 +22,8 @@
 // words of k - 1, before it overwrites them with those of k + 1.
 //
 // The grid is launched cooperatively (or is one cluster), so that all its blocks are resident and
-// every wait ends; a wait is bounded all the same (a warp that gives up records it, stops waiting
-// and runs on).
+// every wait ends; a wait is bounded all the same.  A warp that gives up records it in its handle's word
+// (StereoTgvImpl::checkWaits), stops waiting and runs on.
 //
 // The arithmetic is that of k_fused_iter (tgv_pixel.cuh, tgv_pixel_fast.cuh) with the same
 // storage rounding, so the results are bit-identical to one launch per iteration, the values
@@ -39,6 +39,7 @@
 // shared memory (k_resident_cluster): 53 x 50 takes 0.90 us, through L2 1.39, one launch per
 // iteration 3.2.
 #pragma once
+#include <atomic>
 #include <vector>
 
 #include "common.cuh"
@@ -85,8 +86,9 @@ struct ResTile {
 
 struct ResCtl {   // per level plan, in device memory
   unsigned epoch; // launches completed
-  unsigned done;  // blocks of the running launch that have ended
+  unsigned done;  // of the running launch: blocks that have ended, and kResGaveUp for each warp that gave up a wait
 };
+constexpr unsigned kResGaveUp = 1u << 16;
 
 // One iteration's step sizes (evaluated on the host), each twice for the packed instructions.
 struct ResStep {
@@ -105,6 +107,8 @@ struct ResArgs {
   int p_planes;          // p and q have two planes (result in plane n & 1); else one
   int rows, blocks;      // tile height, blocks of the grid
   bool cluster;          // the grid is one thread-block cluster
+  int mute;              // tests: a tile that leaves out its first words (-1: none)
+  unsigned* gave_up;     // host memory: 1 once a wait ran out
   float2 minus_zero;     // -0, where the compiler does not see it
   ResStep step[kResMaxIters];
 };
@@ -159,6 +163,8 @@ int res_capacity(bool masked, bool half, int rows, int cluster = 0);
 // host bytes (a multiple of four) to the device, stream-ordered; they are taken before the call returns
 void launch_res_upload(void* to, const void* from, size_t bytes, cudaStream_t st);
 void launch_resident(const ResArgs& A, bool masked, bool half, cudaStream_t st);
+// test hook: launches leave out the first words of their first tile
+std::atomic<bool>& res_muted();
 // reads and clears the device status (1: a bounded wait ran out)
 int resident_status_take();
 

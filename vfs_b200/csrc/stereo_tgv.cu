@@ -2,6 +2,7 @@
 // solver (stereotgv/stereotgv.cu:44-598), on one CUDA stream.
 #include <cmath>
 #include <cstring>
+#include <mutex>
 
 #include "stereo_tgv.cuh"
 
@@ -11,8 +12,51 @@ namespace vfs {
 
 StereoTgvImpl::StereoTgvImpl(int bw, int bh, int sa) : blockWidth(bw), blockHeight(bh), strideAlignment(sa) {}
 
+namespace {
+// The words that the whole-level kernels report to, one a handle: the host reads them after any wait for
+// the device, without a copy.  Page-locking takes 2 ms, so they come from a slab of the process, which
+// takes words back and is left to it; handles beyond the slab share its last word.
+class WaitWords {
+ public:
+  static WaitWords& get() {
+    static WaitWords* w = new WaitWords;  // (handles may outlive the statics)
+    return *w;
+  }
+  unsigned* take() {
+    std::lock_guard<std::mutex> lk(mu_);
+    cudaPointerAttributes at{};
+    if (slab_ && (cudaPointerGetAttributes(&at, slab_) != cudaSuccess || at.type != cudaMemoryTypeHost)) {
+      (void)cudaGetLastError();  // gone with its context (cudaDeviceReset)
+      slab_ = nullptr;
+      free_.clear();
+    }
+    if (!slab_) {
+      VFS_CUDA(cudaHostAlloc((void**)&slab_, kWords * sizeof(unsigned), cudaHostAllocPortable | cudaHostAllocMapped));
+      std::memset(slab_, 0, kWords * sizeof(unsigned));
+      for (int k = 0; k < kWords - 1; k++) free_.push_back(kWords - 2 - k);
+    }
+    if (free_.empty()) return slab_ + kWords - 1;
+    unsigned* w = slab_ + free_.back();
+    free_.pop_back();
+    *w = 0;
+    return w;
+  }
+  void give(unsigned* w) {
+    std::lock_guard<std::mutex> lk(mu_);
+    if (w && slab_ && w >= slab_ && w < slab_ + kWords - 1) free_.push_back((int)(w - slab_));
+  }
+
+ private:
+  static constexpr int kWords = 1024;
+  std::mutex mu_;
+  unsigned* slab_ = nullptr;
+  std::vector<int> free_;
+};
+}  // namespace
+
 StereoTgvImpl::~StereoTgvImpl() {
   release();
+  WaitWords::get().give(wait_word);
   for (auto e : evpool_) cudaEventDestroy(e);
   if (own_stream_) cudaStreamDestroy(own_stream_);
 }
@@ -128,6 +172,17 @@ static cudaError_t pool_malloc(void** p, size_t bytes) {
     return cudaErrorMemoryAllocation;
   }
   return cudaMalloc(p, bytes);
+}
+
+void StereoTgvImpl::checkWaits() {
+  volatile unsigned* w = wait_word;
+  if (w && *w) {
+    *w = 0;
+    wait_failed = true;
+  }
+  if (wait_failed)
+    throw WaitError{"a wait on the device ran out: the results of the last solve, and of those before it that have "
+                    "not been read, are undefined"};
 }
 
 void StereoTgvImpl::release() {
@@ -279,6 +334,8 @@ void StereoTgvImpl::initialize(const SolverParams& p) {
   res_room_used_ = false;
   const size_t code_bytes = code_bytes_for(pS, pH);
   code_bytes_ = code_bytes;
+  if (!wait_word) wait_word = WaitWords::get().take();
+  wait_failed = false;
   cudaError_t e = pool_malloc((void**)&pool_, resRoomAt() + res_room_);
   if (e != cudaSuccess) {
     pool_ = nullptr;
@@ -427,6 +484,7 @@ void StereoTgvImpl::copyImagesU8C3(const uint8_t* i0, const uint8_t* i1) {
 
 void StereoTgvImpl::solve(bool masked) {
   if (!initialized_) throw ArgError{"solve before initialize"};
+  wait_failed = false;
   if (path == SolvePath::kFused) {
     std::vector<StereoTgvImpl*> one{this};
     engine.solve(one, masked, half_storage, stream_);
@@ -796,7 +854,10 @@ void StereoTgvImpl::importState(const void* host, size_t bytes) {
 // stereotgv.cu:517-568 outputs: level-0 views of u, warpUV, the warped image.
 void StereoTgvImpl::copyOut(const char* what, float* dst, bool to_host) {
   copyOutOn(what, dst, to_host ? cudaMemcpyDeviceToHost : cudaMemcpyDeviceToDevice, stream_);
-  if (to_host) VFS_CUDA(cudaStreamSynchronize(stream_));
+  if (to_host) {
+    VFS_CUDA(cudaStreamSynchronize(stream_));
+    checkWaits();
+  }
 }
 
 void StereoTgvImpl::copyOutOn(const char* what, float* dst, cudaMemcpyKind kind, cudaStream_t st) {

@@ -206,6 +206,10 @@ class StereoTgvImpl {
     const std::vector<ResPlan>& v = res_plans_[masked][half];
     return level < (int)v.size() && v[level].ntiles > 0 ? &v[level] : nullptr;
   }
+  // Throws when a wait ran out in a solve whose end the host has waited for; until the next solve.
+  void checkWaits();
+  unsigned* wait_word = nullptr;  // page-locked: set by the kernel (WaitWords)
+  bool wait_failed = false;
   // What the kernels that launch one or a few iterations at a time ask of the mask, derived when
   // a masked solve first runs one of them.
   void ensureSpans();

@@ -9,7 +9,8 @@ each with its own CUDA stream.  Whenever a slot is free it takes up to ``max_bat
 requests, at most one per camera (a camera's frames are solved in order), and launches them as
 one batched fused solve that overlaps the batches already on the GPU.  Finished slots are
 detected by event, their disparities copied back, and their requests' latencies recorded.  A
-request therefore joins the next free slot without waiting for the batches in flight.
+request therefore joins the next free slot without waiting for the batches in flight.  A solve that
+failed on the device (vfs_solve_status) finishes its request with ``error`` set and no disparity.
 
 Admission by free device memory happens per request, as slots and memory free up:
 * a request is launched only when the device memory it still needs fits in the free memory
@@ -35,7 +36,7 @@ from typing import Deque, Dict, List, Optional
 
 import numpy as np
 
-from ._native import lib
+from ._native import VfsError, lib
 from .stereotgv import StereoBatch, StereoTgv
 
 
@@ -54,6 +55,7 @@ class Request:
     t_done: float = 0.0
     u: Optional[np.ndarray] = None
     cancelled: bool = False
+    error: Optional[str] = None  # the solve failed on the device: no disparity
 
     @property
     def latency_ms(self) -> float:
@@ -307,9 +309,15 @@ class StereoServer:
             if lane.busy and lane.event.query():
                 now = time.perf_counter()
                 for r, h in zip(lane.requests, lane.hosts):
-                    r.u = h.numpy().copy()
-                    r.t_done = now
                     cam = self.cameras.get(r.stream_id)
+                    try:
+                        if cam is not None:
+                            cam.solver.check_solve()
+                        r.u = h.numpy().copy()
+                    except VfsError as e:
+                        r.error = str(e)
+                        self.counters["failed"] += 1
+                    r.t_done = now
                     if cam is not None:
                         cam.busy = False
                         cam.frames += 1

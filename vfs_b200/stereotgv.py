@@ -108,6 +108,11 @@ class StereoTgv:
     def synchronize(self) -> None:
         check(self._h, self._L.vfs_synchronize(self._h))
 
+    def check_solve(self) -> None:
+        """Raise if a wait on the device ran out in a solve that has completed (its results are then
+        undefined); does not wait.  The copies to the host and synchronize() do the same."""
+        check(self._h, self._L.vfs_solve_status(self._h))
+
     def check_guards(self) -> int:
         """Number of the guard zones after the handle's device planes that a kernel has
         stored into (0: every store stayed in bounds)."""
