@@ -326,3 +326,23 @@ def test_a_wait_that_runs_out_in_a_batch_and_a_server(muted):
     bad = srv.submit(0, *cases[0][:2])
     srv.run_until_idle()
     assert bad.u is None and "-6" in bad.error and srv.stats()["failed"] == 1
+
+
+def test_default_path_after_a_device_reset(gpu):
+    """A program that resets the device between two handles (in a process of its own)."""
+    import os
+    import sys
+    code = """
+import ctypes, gc
+import numpy as np
+from tests.helpers import params, random_case, run_gpu
+case, p = random_case(150, 110, seed=3), params(n_levels=2, n_warp=2, n_iter=20)
+want = run_gpu(*case, p).copy1DDisparityToHost()
+gc.collect()
+assert ctypes.CDLL("libcudart.so.12").cudaDeviceReset() == 0
+for _ in range(2):
+    assert np.array_equal(run_gpu(*case, p).copy1DDisparityToHost(), want)
+"""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", code], cwd=root, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]

@@ -1427,6 +1427,20 @@ template <bool MASKED, class ST, int R>
 struct Res {
   static constexpr int kThreads = 32 * kResMostWarps;
   static constexpr size_t kSmem = sizeof(ResShared<ST, R>) * kResMostWarps;
+  static constexpr size_t kClusterSmem = sizeof(ResClusterTile<ST, R>) * 16;
+  // What the launches ask of the kernel, set with every plan: a device that has been reset forgets it.
+  static int use(bool cluster) {
+    if (!cluster)
+      VFS_CUDA(cudaFuncSetAttribute(k_resident<MASKED, ST, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem));
+    if constexpr (R == kResClusterRows) {
+      if (cluster) {
+        const auto k = k_resident_cluster<MASKED, ST, R>;
+        VFS_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kClusterSmem));
+        VFS_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+      }
+    }
+    return 0;
+  }
   // tiles that a grid of one block per SM holds, all of it resident
   static int capacity() {
     int dev = 0, sms = 0, per = 0, coop = 0, smem = 0;
@@ -1435,7 +1449,7 @@ struct Res {
     VFS_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
     VFS_CUDA(cudaDeviceGetAttribute(&smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
     if (!coop || kSmem > (size_t)smem) return 0;
-    VFS_CUDA(cudaFuncSetAttribute(k_resident<MASKED, ST, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem));
+    use(false);
     VFS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_resident<MASKED, ST, R>, kThreads, kSmem));
     return per >= 1 ? sms * kResMostWarps : 0;
   }
@@ -1443,13 +1457,11 @@ struct Res {
   static int cluster_capacity(int ctas) {
     if constexpr (R == kResClusterRows) {
       const auto k = k_resident_cluster<MASKED, ST, R>;
-      const size_t bytes = sizeof(ResClusterTile<ST, R>) * 16;
       int dev = 0, smem = 0, n = 0;
       VFS_CUDA(cudaGetDevice(&dev));
       VFS_CUDA(cudaDeviceGetAttribute(&smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-      if (bytes > (size_t)smem) return 0;
-      VFS_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
-      VFS_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+      if (kClusterSmem > (size_t)smem) return 0;
+      use(true);
       cudaLaunchAttribute at[1];
       cudaLaunchConfig_t cfg = cluster_config(ctas, 16, 0, at);
       if (cudaOccupancyMaxActiveClusters(&n, k, &cfg) != cudaSuccess) {
@@ -1548,6 +1560,10 @@ __global__ void k_res_upload(const __grid_constant__ ResUpload U) {
   if (i < U.n) U.to[i] = U.w[i];
 }
 }  // namespace
+
+void res_use(bool masked, bool half, int rows, bool cluster) {
+  res_dispatch(masked, half, rows, [cluster](auto k) { return decltype(k)::use(cluster); });
+}
 
 void launch_res_upload(void* to, const void* from, size_t bytes, cudaStream_t st) {
   ResUpload U;

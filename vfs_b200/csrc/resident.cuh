@@ -160,6 +160,8 @@ struct ResPlan {
 // most tiles an instance holds with its whole grid (cluster > 0: one cluster of that many blocks)
 // resident; 0: not available
 int res_capacity(bool masked, bool half, int rows, int cluster = 0);
+// readies an instance for launches (once a plan has chosen it)
+void res_use(bool masked, bool half, int rows, bool cluster);
 // host bytes (a multiple of four) to the device, stream-ordered; they are taken before the call returns
 void launch_res_upload(void* to, const void* from, size_t bytes, cudaStream_t st);
 void launch_resident(const ResArgs& A, bool masked, bool half, cudaStream_t st);

@@ -640,6 +640,7 @@ void StereoTgvImpl::makePlans(bool masked, bool half, cudaStream_t st, std::vect
     const std::vector<uint8_t> circle = masked ? std::vector<uint8_t>{} : res_circle_codes(pW[l], pH[l]);
     if (!res_choose(masked ? maskCode(l) : circle.data(), masked ? pS[l] : pW[l], pW[l], pH[l], masked, half, cut[l]))
       continue;
+    res_use(masked, half, cut[l].rows, cut[l].cluster);
     plans[l].rows = cut[l].rows;
     plans[l].blocks = cut[l].blocks;
     plans[l].cluster = cut[l].cluster;
