@@ -482,6 +482,7 @@ def run_ours(args, rank, world, local):
     ms_l = union_ms(top[:, :2]) if len(top) else 0.0
     ms_sum = float((top[:, 1] - top[:, 0]).sum()) if len(top) else 0.0
     variants = solvers[0].iteration_variants() if fused else []
+    whole_level = solvers[0].level_launches()[0][0] > 0
     n_variant_sets = len({tuple(s.iteration_variants()) for s in solvers}) if fused else 0
     # job-wide: frames of all replicas over the slowest replica's time
     from vfs_b200.replicas import job_rate
@@ -536,8 +537,7 @@ def run_ours(args, rank, world, local):
         achieved = (pi_l * b_alg / (ms_l / 1000.0) / 1e9) if ms_l > 0 else None
         achieved_all = (pi_all * b_alg / (ms_all / 1000.0) / 1e9) if ms_all > 0 else None
         storage = "fp16" if half else "fp32"
-        # 14: the whole level in one launch, its state on the chip
-        resident = variants[0] == 14 if fused and variants else pi_l > 1.5 * n_launch * W0 * H0
+        resident = whole_level  # full resolution in one launch per warp, its state on the chip
         kernel_key = f"resident_{storage}" if resident else f"fused_inner_{storage}" if fused else "plain_inner_iteration"
         px_per_launch = pi_l / n_launch if n_launch else 0.0
         tr = ncu_traffic(kernel_key)

@@ -263,13 +263,20 @@ int vfs_set_autotune(vfs_stereo* s, int on);
 #define VFS_ITER_VARIANTS 20
 int vfs_set_iteration_variant(vfs_stereo* s, int variant);
 /* Force one variant per pyramid level (finest first; levels beyond n_levels use variant 1),
- * e.g. to pin a tuned choice; n_levels = 0 clears it. */
+ * e.g. to pin the choice that vfs_get_iteration_variants has reported; n_levels = 0 clears it.  14 in the
+ * list is a whole-level launch where the level has one (vfs_get_level_launches), else the cluster kernel
+ * that vfs_set_iteration_variant(s, 14) forces at every level. */
 int vfs_set_iteration_variants(vfs_stereo* s, const int* variants, int n_levels);
 int vfs_batch_set_iteration_variants(vfs_batch* b, const int* variants, int n_levels);
 /* The variant each pyramid level (finest first) used in the handle's last fused solve
- * (tuned, default or forced); *count receives the number of levels.  A level held on the chip by
- * the whole GPU (unforced, see vfs_batch_set_autotune) is reported as 14. */
+ * (tuned, default or forced); *count receives the number of levels.  A level run by whole-level
+ * launches (see vfs_batch_set_autotune) is reported as 14, as is variant 14's kernel. */
 int vfs_get_iteration_variants(vfs_stereo* s, int* variants, int max_levels, int* count);
+/* How the handle's last solve, of either path, ran each pyramid level (finest first).  rows[l] > 0: one
+ * launch per warp for the whole level, of tiles[l] tiles of 30 x rows[l] pixels, in one thread-block
+ * cluster (cluster[l] = 1) or over the whole GPU (0).  rows[l] = 0: several launches a warp, or a
+ * level that a warm start skips.  *count receives the number of levels (0 before the first solve). */
+int vfs_get_level_launches(vfs_stereo* s, int* rows, int* tiles, int* cluster, int max_levels, int* count);
 int vfs_batch_set_iteration_variant(vfs_batch* b, int variant);
 
 /* Histogram equalisation of n 8-bit pixels in device memory (d_dst may equal d_src), as

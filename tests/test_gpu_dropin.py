@@ -346,3 +346,39 @@ for _ in range(2):
     root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
     r = subprocess.run([sys.executable, "-c", code], cwd=root, capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stderr[-2000:]
+
+
+# The form a level takes: 30-column tiles of the least rows that leave them at most 2,368 (two rows: three
+# quarters of that), one cluster up to 208 tiles of two rows with half storage and 128 with float
+@pytest.mark.parametrize("half,w,h,rows,cluster", [
+    (True, 118, 104, 2, True), (True, 119, 106, 2, False), (False, 115, 64, 2, True), (False, 118, 66, 2, False),
+    (True, 640, 100, 2, False), (False, 424, 400, 4, False), (True, 600, 520, 6, False), (False, 760, 480, 6, False),
+    (True, 830, 560, 8, False), (False, 850, 560, 8, False), (True, 810, 760, 12, False), (True, 1078, 1009, 16, False),
+    (False, 850, 760, 0, False), (True, 1200, 1100, 0, False)])
+def test_the_form_of_a_level_and_pinning_it(gpu, half, w, h, rows, cluster):
+    case = list(random_case(w, h, seed=w + h, circle=False))
+    case[2][0] = case[2][:, 0] = 0
+    p = params(n_levels=1, n_warp=1, n_iter=6)
+    tiles = -(-w // 30) * -(-h // rows) if rows else 0
+    want = [(rows, tiles, cluster)]
+    s = _solver(case, p, fused=True, half=half)
+    s.set_autotune(False)
+    u = _disparity(s, case)
+    assert s.level_launches() == want
+    assert s.iteration_variants() == [14 if rows else 1]
+    t = _solver(case, p, fused=True, half=half)
+    t.set_iteration_variants(s.iteration_variants())  # pinned from the report
+    assert np.array_equal(_disparity(t, case), u)
+    assert t.level_launches() == want and t.iteration_variants() == s.iteration_variants()
+    t.set_iteration_variants([])
+    t.set_iteration_variant(14 if rows == 2 else 1)  # another kernel, the same bits
+    t.copyMaskToDevice(case[2])
+    f = _solver(case, p, fused=True, half=half)
+    f.set_iteration_variant(1)
+    assert np.array_equal(_disparity(f, case), u)
+    _disparity(t, case)
+    assert t.level_launches() == [(0, 0, False)] == f.level_launches()
+    if not half:
+        d = _solver(case, p)
+        assert np.array_equal(_disparity(d, case), u)
+        assert d.level_launches() == want

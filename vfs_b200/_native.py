@@ -94,6 +94,7 @@ SIGNATURES = {
     "vfs_set_autotune": [_vp, _i],
     "vfs_set_iteration_variant": [_vp, _i],
     "vfs_get_iteration_variants": [_vp, _vp, _i, ctypes.POINTER(_i)],
+    "vfs_get_level_launches": [_vp, _vp, _vp, _vp, _i, ctypes.POINTER(_i)],
     "vfs_set_iteration_variants": [_vp, _vp, _i],
     "vfs_batch_set_iteration_variants": [_vp, _vp, _i],
     "vfs_batch_set_iteration_variant": [_vp, _i],

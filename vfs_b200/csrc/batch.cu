@@ -776,14 +776,27 @@ void FusedEngine::solve_parts(std::vector<StereoTgvImpl*>& pairs, bool masked, b
   bool need_tune = false;
   const bool one_pair = pairs.size() == 1;
   // levels that fit the chip run the register-resident form; it is never timed against the others.  In a
-  // caller's stream capture nothing is timed and no plan is used: the graph may outlive it (a new mask)
+  // caller's stream capture nothing is timed and no plan is used: the graph may outlive it (a new mask).
+  // A list of variants pins it where it says 14, as the solve it was read from reported it.
   const bool captured = stream_capturing(st);
-  const bool plans = one_pair && !forced && !captured;
-  auto resident = [&](int l) { return plans && pairs[0]->residentPlan(masked, half, l) != nullptr; };
+  auto on_chip = [&](int l) {
+    if (forced_levels.empty()) return forced_variant < 0;
+    return l < (int)forced_levels.size() && forced_levels[l] == kIterFirstClusterVariant;
+  };
+  bool plans = false;
+  for (int l = 0; l < maxL; l++) plans = plans || (one_pair && !captured && on_chip(l));
+  auto resident = [&](int l) { return plans && on_chip(l) && pairs[0]->residentPlan(masked, half, l) != nullptr; };
   if (plans) pairs[0]->ensureResident(masked, half, st);
   auto level_key = [&](int l) {
     return std::array<int, 5>{(int)masked, (int)half, concurrency > 1 ? 2 : 1, pairs[0]->pW[l], pairs[0]->pH[l]};
   };
+  for (auto* s : pairs) {
+    s->solved_by.resize(s->levels());
+    for (int l = 0; l < s->levels(); l++) {
+      if (in_part(l)) s->solved_by[l] = resident(l) ? *s->residentPlan(masked, half, l) : ResPlan{};
+      else if (l > max_top) s->solved_by[l] = ResPlan{};
+    }
+  }
   if (masked) {
     bool all = true;
     for (int l = 0; l < maxL; l++) all = all && (!in_part(l) || resident(l));
@@ -846,15 +859,15 @@ void FusedEngine::solve_parts(std::vector<StereoTgvImpl*>& pairs, bool masked, b
     return;
   }
   std::vector<int> variants = tit->second;
-  for (int l = 0; l < maxL; l++) {
-    if (resident(l)) variants[l] = kIterResident;
-    else if (variants[l] < 0 && captured) variants[l] = kIterDefaultVariant;
-  }
+  for (int l = 0; l < maxL; l++)
+    if (variants[l] < 0 && captured) variants[l] = kIterDefaultVariant;
   if (forced_variant >= 0) variants.assign(maxL, forced_variant);
   if (!forced_levels.empty()) {
     variants.assign(maxL, kIterDefaultVariant);
     for (int l = 0; l < maxL && l < (int)forced_levels.size(); l++) variants[l] = forced_levels[l];
   }
+  for (int l = 0; l < maxL; l++)
+    if (resident(l)) variants[l] = kIterResident;
   note_variants(variants, part);
   run(pairs, masked, half, st, part, variants, false);
 }
@@ -862,6 +875,7 @@ void FusedEngine::solve_parts(std::vector<StereoTgvImpl*>& pairs, bool masked, b
 void FusedEngine::solve_dropin(StereoTgvImpl* pair, bool masked, cudaStream_t st) {
   std::vector<StereoTgvImpl*> one{pair};
   std::vector<int> variants(pair->levels(), kIterResident);
+  for (int l = 0; l <= pair->topLevel(); l++) pair->solved_by[l] = *pair->residentPlan(masked, false, l);
   run(one, masked, false, st, 0, variants, true);
   pair->i1warp_half = false;
 }

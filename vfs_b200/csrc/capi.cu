@@ -458,6 +458,18 @@ int vfs_get_iteration_variants(vfs_stereo* s, int* variants, int max_levels, int
   });
 }
 
+int vfs_get_level_launches(vfs_stereo* s, int* rows, int* tiles, int* cluster, int max_levels, int* count) {
+  return guarded(s, [&] {
+    const std::vector<vfs::ResPlan>& v = s->impl.solved_by;
+    if (count) *count = (int)v.size();
+    for (int l = 0; l < max_levels && l < (int)v.size(); l++) {
+      if (rows) rows[l] = v[l].ntiles > 0 ? v[l].rows : 0;
+      if (tiles) tiles[l] = v[l].ntiles;
+      if (cluster) cluster[l] = v[l].ntiles > 0 && v[l].cluster;
+    }
+  });
+}
+
 int vfs_batch_set_iteration_variant(vfs_batch* b, int variant) {
   return guarded(b, [&] {
     if (variant != -1 && !vfs::iter_variant_valid(variant)) throw vfs::ArgError{"iteration variant out of range or retired"};

@@ -191,6 +191,7 @@ void StereoTgvImpl::release() {
   dropResident(false);
   dropResident(true);
   mask_code.clear();
+  solved_by.clear();
   if (pool_) cudaFree(pool_);
   pool_ = nullptr;
   if (fpool_) cudaFree(fpool_);
@@ -489,6 +490,7 @@ void StereoTgvImpl::solve(bool masked) {
     std::vector<StereoTgvImpl*> one{this};
     engine.solve(one, masked, half_storage, stream_);
   } else {
+    solved_by.assign(levels(), ResPlan{});
     if (dropinResident(masked)) engine.solve_dropin(this, masked, stream_);
     else solveReference(masked);
     have_prev = true;

@@ -210,6 +210,8 @@ class StereoTgvImpl {
   void checkWaits();
   unsigned* wait_word = nullptr;  // page-locked: set by the kernel (WaitWords)
   bool wait_failed = false;
+  // per level, the plan (its sizes) by which the last solve ran it; no tiles: without one, or not at all
+  std::vector<ResPlan> solved_by;
   // What the kernels that launch one or a few iterations at a time ask of the mask, derived when
   // a masked solve first runs one of them.
   void ensureSpans();

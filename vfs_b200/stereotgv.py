@@ -149,6 +149,14 @@ class StereoTgv:
         check(self._h, self._L.vfs_get_iteration_variants(self._h, out, 16, ctypes.byref(n)))
         return [out[i] for i in range(min(n.value, 16))]
 
+    def level_launches(self):
+        """(tile rows, tiles, in one cluster) per pyramid level (finest first) that the last solve ran in
+        one launch per warp, (0, 0, False) for the other levels."""
+        out = [(ctypes.c_int * 16)() for _ in range(3)]
+        n = ctypes.c_int()
+        check(self._h, self._L.vfs_get_level_launches(self._h, *out, 16, ctypes.byref(n)))
+        return [(out[0][l], out[1][l], bool(out[2][l])) for l in range(min(n.value, 16))]
+
     # ---- reference methods -------------------------------------------------
     def initialize(self, width, height, beta, gamma, alpha0, alpha1, timestep_lambda, lambda_,
                    nLevels, fScale, nWarpIters, nSolverIters) -> int:
