@@ -359,7 +359,7 @@ def plain_reference_run(pair, dev, flush, steps=6):
     s = make_solver(pair, "plain", st)
     a = torch.from_numpy(pair["i0"]).to(dev)
     b = torch.from_numpy(pair["i1"]).to(dev)
-    for _ in range(2):
+    for _ in range(4):  # the first solve is launched, the next two record the two states' graphs
         s.copy_images_from_device(a, b)
         s.solveStereoForwardMasked()
     torch.cuda.synchronize()

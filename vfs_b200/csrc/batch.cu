@@ -926,21 +926,18 @@ void FusedEngine::run(std::vector<StereoTgvImpl*>& pairs, bool masked, bool half
     key.push_back(lr);
   }
   auto it = cache_.find(key);
-  Entry e;
-  for (auto* s : pairs) e.owners.emplace_back(s, s->generation);
-  if (it == cache_.end() && dropin) {
-    // The drop-in path records a state when it meets it again: a program that changes its mask or limit
-    // every frame never does, and recording takes longer than launching once.
+  if (it == cache_.end()) {
     evict(pairs);
-    e.last_use = ++use_clock_;
-    cache_.emplace(key, std::move(e));
-    if (prof->profiling) prof->profReset();  // the records describe the last solve
-    fused_solve_direct(pairs, masked, half, st, variants, false, concurrency, part, dropin);
-    return;
-  }
-  if (it == cache_.end() || !it->second.exec) {
-    if (it == cache_.end()) evict(pairs);
-    else cache_.erase(it);
+    if (dropin && launched_generation_ != prof->generation) {
+      // The drop-in path launches the first solve after a change: a program that changes its mask or limit
+      // every frame never meets a state again, and recording takes longer than launching once.
+      launched_generation_ = prof->generation;
+      if (prof->profiling) prof->profReset();  // the records describe the last solve
+      fused_solve_direct(pairs, masked, half, st, variants, false, concurrency, part, dropin);
+      return;
+    }
+    Entry e;
+    for (auto* s : pairs) e.owners.emplace_back(s, s->generation);
     const RecordStream rec(st, dropin);
     cudaGraph_t g = nullptr;
     VFS_CUDA(cudaStreamBeginCapture(rec.st, cudaStreamCaptureModeRelaxed));

@@ -64,18 +64,14 @@ class FusedEngine {
  public:
   // allocate fused buffers and refresh edge codes, each on the pair's own stream
   static void prepare(std::vector<StereoTgvImpl*>& pairs, bool masked);
-  size_t graphs() const {
-    size_t n = 0;
-    for (const auto& kv : cache_) n += kv.second.exec != nullptr;
-    return n;
-  }
+  size_t graphs() const { return cache_.size(); }
   // iteration-kernel variant per pyramid level (finest first) of the last solve
   std::vector<int> last_variants;
   void note_variants(std::vector<int> v, int part);
 
  private:
   struct Entry {
-    cudaGraphExec_t exec = nullptr;  // null: met once, run directly
+    cudaGraphExec_t exec = nullptr;
     long long kernels = 0;  // kernel launches recorded in the graph (added to the launch count per replay)
     std::vector<PairPtrs> after;
     std::vector<ProfRec> prof;
@@ -91,6 +87,7 @@ class FusedEngine {
   void evict(const std::vector<StereoTgvImpl*>& pairs);
   void drop(std::map<std::vector<uintptr_t>, Entry>::iterator it);
   uint64_t use_clock_ = 0;
+  uint64_t launched_generation_ = 0;  // the last one whose first drop-in solve was launched without a graph
   std::map<std::vector<uintptr_t>, Entry> cache_;
   std::map<std::vector<int>, std::vector<int>> tuned_;
 };
