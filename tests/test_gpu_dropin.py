@@ -386,3 +386,39 @@ def test_the_form_of_a_level_and_pinning_it(gpu, half, w, h, rows, cluster):
         d = _solver(case, p)
         assert np.array_equal(_disparity(d, case), u)
         assert d.level_launches() == want
+
+
+def test_exported_state_holds_the_edge_codes(gpu):
+    """Where the fused buffers held them: a library that reads them from a state finds those of the
+    mask and of the circle, level after level, with their guard zones."""
+    w, h = 150, 110
+    case = random_case(w, h, seed=61)
+    s = _solver(case, params(n_levels=2, n_warp=1, n_iter=6), fused=True)
+    _disparity(s, case)
+    state = s.export_state()
+    sizes = s.level_sizes()
+    n = sizes[0][1] * sizes[0][2]
+
+    def place(at, b):
+        at = -(-at // 512) * 512
+        return at, at + b + 256
+
+    at = 0
+    for b in (16 * n, 32 * n, 4 * n, 4 * n, 16 * n, 8 * n):  # the planes before them
+        _, at = place(at, b)
+    pool = int.from_bytes(state[48:56].tobytes(), "little")
+    f = state[160 + pool:]
+    for l, (lw, lh, ls) in enumerate(sizes):
+        for masked in (True, False):
+            lo, at = place(at, ls * lh)
+            on = f[lo:lo + ls * lh].reshape(lh, ls)[:, :lw] & 1
+            assert (f[lo + ls * lh:at] == 0xA5).all()
+            yy, xx = np.mgrid[0:lh, 0:lw].astype(np.float32)
+            r = np.sqrt((yy - np.float32(lh) / 2) ** 2 + (xx - np.float32(lw) / 2) ** 2)
+            if not masked:
+                assert np.array_equal(on, r < np.float32(lw) / np.float32(2.2))
+            elif l == 0:
+                assert np.array_equal(on, case[2] > 0)
+    t = _solver(case, params(n_levels=2, n_warp=1, n_iter=6), fused=True)
+    t.import_state(state)
+    assert np.array_equal(_disparity(t, case, False), _disparity(s, case, False))

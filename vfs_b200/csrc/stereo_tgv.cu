@@ -253,8 +253,7 @@ static size_t pool_bytes_for(const std::vector<int>& pS, const std::vector<int>&
 }
 
 // p, q two planes each (float: 8 + 16 bytes per pixel and plane), half v-bar pair, the
-// coefficient records, and two bytes per pixel and level that exported states carry (the edge
-// codes' former place).
+// coefficient records, and two bytes per pixel and level that exported states carry (exportState).
 static size_t fused_bytes_for(const std::vector<int>& pS, const std::vector<int>& pH, size_t full) {
   size_t bytes = full * 2 * 8 + full * 2 * 16 + full * 4 * 2 + full * 16 + full * 8 + 8 * 512 +
                  8 * StereoTgvImpl::kGuardBytes;
@@ -542,6 +541,7 @@ void StereoTgvImpl::ensureFused() {
   f_vhs = take(n * 4);
   f_abce = (float4*)take(n * 16);
   f_rv = (float2*)take(n * 8);
+  f_codes_at_ = off;
   VFS_CUDA(cudaMemsetAsync(fpool_, 0, bytes, stream_));
   fillGuards(guards_before, stream_);
 }
@@ -804,7 +804,20 @@ void StereoTgvImpl::exportState(void* host, size_t bytes) {
   char* out = (char*)host;
   std::memcpy(out, &h, sizeof(h));
   VFS_CUDA(cudaMemcpy(out + sizeof(h), pool_, pool_bytes_, cudaMemcpyDeviceToHost));
-  if (fbytes) VFS_CUDA(cudaMemcpy(out + sizeof(h) + pool_bytes_, fpool_, fbytes, cudaMemcpyDeviceToHost));
+  if (!fbytes) return;
+  char* f = out + sizeof(h) + pool_bytes_;
+  VFS_CUDA(cudaMemcpy(f, fpool_, fbytes, cudaMemcpyDeviceToHost));
+  // The edge codes had their place here before they moved behind the pool, and a library of that time takes
+  // the plain form's from the state (and the guard zones with them).
+  size_t at = f_codes_at_;
+  for (int l = 0; l < levels(); l++)
+    for (const uint8_t* code : {code_masked[l], code_plain[l]}) {
+      const size_t b = (size_t)pS[l] * pH[l];
+      at = (at + 511) & ~(size_t)511;
+      VFS_CUDA(cudaMemcpy(f + at, code, b, cudaMemcpyDeviceToHost));
+      std::memset(f + at + b, kGuardByte, kGuardBytes);
+      at += b + kGuardBytes;
+    }
 }
 
 void StereoTgvImpl::importState(const void* host, size_t bytes) {

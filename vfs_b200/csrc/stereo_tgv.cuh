@@ -323,6 +323,7 @@ class StereoTgvImpl {
   cudaStream_t own_stream_ = nullptr;
   cudaStream_t stream_ = 0;
   char* fpool_ = nullptr;
+  size_t f_codes_at_ = 0;  // where its planes end
   char* pool_ = nullptr;
   size_t pool_bytes_ = 0, pool_used_ = 0;
   size_t full_ = 0;  // elements of a full-resolution pitched plane
