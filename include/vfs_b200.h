@@ -162,8 +162,10 @@ int vfs_debug_get_buffer(vfs_stereo* s, const char* name, int comps, float* out)
  *   per-warp and per-level kernels, replayed as a CUDA graph, leave every buffer as the reference's
  *   kernels would; else, and in a caller's stream capture, one kernel per reference kernel, in the
  *   reference's order;
- *   VFS_PATH_FUSED: one fused kernel per primal-dual iteration plus fused per-warp and
- *   per-level kernels, replayed as a CUDA graph.  With float storage the fused path gives
+ *   VFS_PATH_FUSED: whole-level launches, or one fused kernel per primal-dual iteration, plus fused
+ *   per-warp and per-level kernels, replayed as a CUDA graph.  A caller's stream capture takes them, one
+ *   iteration a launch, with the handle's own graphs off (vfs_set_graph(s, 0)); with them on it is
+ *   refused.  With float storage the fused path gives
  *   bit-identical results; with half storage (half_storage = 1) p, q, v-bar and the warped
  *   image are kept as IEEE half in memory (all arithmetic stays float; the warped image is
  *   widened to float when it is copied out). */

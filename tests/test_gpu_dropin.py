@@ -422,3 +422,91 @@ def test_exported_state_holds_the_edge_codes(gpu):
     t = _solver(case, params(n_levels=2, n_warp=1, n_iter=6), fused=True)
     t.import_state(state)
     assert np.array_equal(_disparity(t, case, False), _disparity(s, case, False))
+
+
+BUFFERS = (("u", 1), ("u_", 1), ("warpUV", 2), ("a", 1), ("b", 1), ("c", 1), ("etau", 1), ("etav1", 1), ("etav2", 1),
+           ("Iu", 1), ("Iz", 1), ("i1warp", 1), ("tv2", 2), ("i0smooth", 1), ("p", 2), ("q", 4), ("v_", 2), ("Tp", 2),
+           ("us", 1), ("u_s", 1), ("v_s", 2), ("du", 1), ("u_last", 1), ("warpUVs", 2), ("i1calibrated", 1))
+
+
+@pytest.mark.parametrize("masked", [True, False], ids=["masked", "plain"])
+@pytest.mark.parametrize("w,h,levels,warps,iters,kw", [
+    (64, 48, 2, 1, 2, {}), (64, 48, 2, 2, 5, {}), (64, 48, 2, 0, 3, {}), (97, 53, 2, 2, 3, {}), (53, 97, 2, 2, 4, {}),
+    (130, 60, 1, 1, 6, dict(alpha0=0.0)), (300, 280, 3, 2, 7, {}), (640, 480, 4, 1, 9, {})])
+def test_default_path_leaves_every_buffer_as_a_kernel_per_operation_does(gpu, w, h, levels, warps, iters, kw, masked):
+    """The same frames on two handles, the last ones of the second in a caller's capture, where the
+    default path takes a kernel per operation: every buffer's bits, over a new mask in between."""
+    import torch
+    case = random_case(w, h, seed=w + h, circle=w != 64)
+    case[2][0] = case[2][:, 0] = 0
+    new = case[2].copy()
+    new[h // 3:h // 2, w // 4:w // 2] = 0
+    p = params(n_levels=levels, n_warp=warps, n_iter=iters, **kw)
+    i0, i1 = (torch.from_numpy(x).cuda() for x in case[:2])
+    out = []
+    for captured in (False, True):
+        st = torch.cuda.Stream()
+        s = _solver(case, p, st)
+        solve = s.solveStereoForwardMasked if masked else s.solveStereoForward
+        frames = []
+        for k in range(10):  # the first eight make the texture objects of every pointer state
+            if k == 9:
+                s.copyMaskToDevice(new)
+            s.copy_images_from_device(i0, i1)
+            torch.cuda.synchronize()
+            if captured and k >= 8:
+                g = torch.cuda.CUDAGraph()
+                with torch.cuda.graph(g, stream=st):
+                    solve()
+                assert not any(r for r, _, _ in s.level_launches())
+                g.replay()
+            else:
+                solve()
+                assert k < 6 or warps == 0 or k == 9 or all(r for r, _, _ in s.level_launches())
+            torch.cuda.synchronize()
+            if k >= 8:
+                frames.append({n: s.debug_buffer(n, c) for n, c in BUFFERS})
+        out.append(frames)
+    for a, b in zip(*out):
+        for n, _ in BUFFERS:
+            assert np.array_equal(a[n], b[n], equal_nan=True), n
+            assert np.array_equal(np.signbit(a[n]), np.signbit(b[n])), n
+
+
+def test_fused_solve_in_a_captured_stream(gpu):
+    """With the handle's own graphs off its launches go into the caller's graph, one iteration a launch;
+    with them on the capture is refused, and the handle solves as before."""
+    import torch
+    from vfs_b200._native import VfsError
+    case = random_case(150, 110, seed=23)
+    p = params(n_levels=2, n_warp=2, n_iter=8)
+    want = _disparity(_solver(case, p, fused=True, half=True), case)
+    i0, i1 = (torch.from_numpy(x).cuda() for x in case[:2])
+    st = torch.cuda.Stream()
+    s = _solver(case, p, st, fused=True, half=True)
+    out = torch.zeros((110, 150), device="cuda")
+
+    def frame():
+        s.copy_images_from_device(i0, i1)
+        s.solveStereoForwardMasked()
+        s.copy_1d_disparity_to_device(out)
+
+    for _ in range(2):
+        frame()
+    torch.cuda.synchronize()
+    with pytest.raises((VfsError, RuntimeError)):
+        with torch.cuda.graph(torch.cuda.CUDAGraph(), stream=st, capture_error_mode="relaxed"):
+            frame()
+    torch.cuda.synchronize()
+    assert np.array_equal(_disparity(s, case), want)
+    assert all(r for r, _, _ in s.level_launches())
+    s.set_graph(False)
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=st, capture_error_mode="relaxed"):
+        frame()
+    assert not any(r for r, _, _ in s.level_launches())
+    out.zero_()
+    g.replay()
+    torch.cuda.synchronize()
+    assert np.array_equal(out.cpu().numpy(), want)
+    assert np.array_equal(_disparity(s, case), want)
