@@ -510,3 +510,104 @@ def test_fused_solve_in_a_captured_stream(gpu):
     torch.cuda.synchronize()
     assert np.array_equal(out.cpu().numpy(), want)
     assert np.array_equal(_disparity(s, case), want)
+
+
+def _spreading_case(w, h, rows, seed):
+    """Two equal images but for a strip near an end of the longer side: the disparity spreads from there by
+    a pixel an iteration, each time smaller, down to zero.  rows: the images differ in the upper half too,
+    alike in every column, so that a large vertical step stands beside the horizontal one that spreads."""
+    rng = np.random.default_rng(seed)
+    i0 = rng.uniform(0.2, 0.8, (h, w)).astype(np.float32)
+    tv = np.zeros((h, w, 2), np.float32)
+    tv[..., 0] = -1.0
+    if rows:
+        i0[:] = np.linspace(0.1, 0.9, h, dtype=np.float32)[:, None] ** 2
+        tv[:] = (0.0, 1.0)
+    i1 = i0.copy()
+    if rows:
+        i1[:h // 2] += np.float32(0.3)
+    if w >= h:
+        i1[2:h - 2, w // 8:w // 8 + 4] += np.float32(0.2)
+    else:
+        i1[h // 8:h // 8 + 4, 2:w - 2] += np.float32(0.2)
+    mask = np.ones((h, w), np.float32)
+    mask[0] = mask[:, 0] = 0
+    return i0, i1, mask, tv, np.zeros((h, w, 2), np.float32)
+
+
+# (30 x 240: in one cluster; the unmasked form's circle is too small for the values to shrink there)
+@pytest.mark.parametrize("w,h,rows,masked", [(30, 240, False, True)] + [
+    (w, h, rows, masked) for w, h in ((160, 160), (500, 400), (848, 640)) for rows in (False, True)
+    for masked in (True, False)])
+def test_values_down_to_the_smallest(gpu, w, h, rows, masked):
+    """Disparities and dual variables that shrink to subnormal numbers, some beside a norm above 1: their
+    quotients are the plain division's too."""
+    case = _spreading_case(w, h, rows, w)
+    p = params(n_levels=1, n_warp=2, n_iter=60, alpha0=1.0, lam=50.0)
+    out = []
+    for variant in (1, None):
+        s = _solver(case, p, fused=True)
+        if variant is not None:
+            s.set_iteration_variant(variant)
+        _disparity(s, case, masked)
+        out.append({n: s.debug_buffer(n, c) for n, c in (("u", 1), ("u_", 1), ("us", 1), ("u_s", 1), ("v_", 2),
+                                                         ("v_s", 2), ("Tp", 2))})
+    assert s.level_launches()[0][0] > 0
+    a = np.abs(out[0]["us"])
+    assert ((a > 0) & (a < 2.0 ** -102)).any() and ((a > 0) & (a < 2.0 ** -126)).any()
+    for n in out[0]:
+        same = out[0][n].view(np.int32) == out[1][n].view(np.int32)
+        assert same.all(), (n, int((~same).sum()), same.size)
+
+
+def test_exact_quotients_of_any_dividend(gpu, tmp_path):
+    """10^9 quotients by divisors from 2^-64 to 2^64, dividends from the smallest subnormal on (half of
+    them below 2^-100), against the device's division.  Left out, as the header says: quotients exactly
+    halfway between two subnormals, which take an integer divisor (a few in 10^9 here), and the sign of
+    a zero divided by a negative number."""
+    from vfs_b200.build import ARCH, CSRC, nvcc
+    src = tmp_path / "t.cu"
+    src.write_text(r"""
+#include <cstdio>
+#include "tgv_exact_pairs.cuh"
+using namespace vfs;
+namespace x2 = fast::x2;
+__device__ unsigned long long bad, tiny, halfway;
+__global__ void k_quot(int n) {
+  unsigned long long s = 0x9E3779B97F4A7C15ull * (blockIdx.x * blockDim.x + threadIdx.x + 1);
+  for (int i = 0; i < n; i++) {
+    s ^= s << 13; s ^= s >> 7; s ^= s << 17;
+    // exponents of b - 127: 0 .. 15 (as a norm's), or -64 .. 63; of a: 0 .. 31, or 0 .. 191
+    const unsigned eb = (s >> 40) & 1 ? 127 + ((s >> 41) & 15) : 63 + ((s >> 41) & 127);
+    const unsigned ea = (s >> 48) & 1 ? (s >> 49) & 31 : ((s >> 49) % 192);
+    const float a = __uint_as_float((unsigned)(s >> 63) << 31 | ea << 23 | ((unsigned)s & 0x7fffff));
+    const float b = __uint_as_float(eb << 23 | (unsigned)((s * 0xD1342543DE82EF95ull) >> 41));
+    const float q = a / b;
+    if (!(fabsf(q) <= 0x1p120f)) continue;
+    const x2::f2 B = x2::pk(b, -b), Q = exact::quot(x2::pk(a, a), exact::Divisor(B, exact::recip(B)));
+    if (fabsf(q) <= 0x1p-126f && fmod(fabs((double)a / (double)b) * 0x1p150, 2.0) == 1.0) {
+      atomicAdd(&halfway, 1ull);
+      if (b != rint(b)) atomicAdd(&bad, 1ull);
+      continue;
+    }
+    if (__float_as_uint(x2::upk(Q).x) != __float_as_uint(q) ||
+        (a != 0.0f && __float_as_uint(x2::upk(Q).y) != __float_as_uint(-q)))
+      atomicAdd(&bad, 1ull);
+    if (fabsf(q) < 0x1p-126f && q != 0.0f) atomicAdd(&tiny, 1ull);
+  }
+}
+int main() {
+  k_quot<<<1024, 256>>>(4000);
+  unsigned long long h[3];
+  if (cudaMemcpyFromSymbol(h, bad, 8) != cudaSuccess || cudaMemcpyFromSymbol(h + 1, tiny, 8) != cudaSuccess ||
+      cudaMemcpyFromSymbol(h + 2, halfway, 8) != cudaSuccess) return 2;
+  std::printf("%llu wrong, %llu subnormal, %llu halfway\n", h[0], h[1], h[2]);
+  return h[0] != 0 || h[1] < 1000000 || h[2] > 1000;
+}
+""")
+    exe = tmp_path / "t"
+    r = subprocess.run([nvcc(), *ARCH, "-O3", "-std=c++17", "-fmad=false", f"-I{CSRC}", str(src), "-o", str(exe)],
+                       capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr
+    r = subprocess.run([str(exe)], capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0, r.stdout + r.stderr

@@ -611,7 +611,8 @@ struct ResState<MASKED, float, R> {
   // (sigma <= 2^14).  A pixel beyond any of it asks for the plain operators.
   static constexpr float kMost = 0x1p24f, kMostTp = 16.0f, kRate = 0x1p20f;
   static __device__ __forceinline__ bool beyond(float v) { return !(fabsf(v) <= kMost); }
-  // in the range of the exact quotients
+  // in the range of the exact quotients (Iu, whose dividends are of any size: 2^-64 to 2^32; a residual that
+  // takes the Newton step is then below 2^52, since lambda |Iu| <= kRate eta_u)
   static __device__ __forceinline__ bool ranged(float b) { return fabsf(b) >= 0x1p-100f && fabsf(b) <= 0x1p100f; }
   struct Pixel {
     float a, b, c, iu, iz, u, ub;
@@ -642,7 +643,8 @@ struct ResState<MASKED, float, R> {
     if (in && r >= 0 && (code & kOn)) {
       const float eu = etau_math(x.a, x.b, x.c, P.alpha1);
       const float e1 = etav1_math(x.b, x.c, P.alpha0, P.alpha1), e2 = etav2_math(x.a, x.c, P.alpha0, P.alpha1);
-      plain = !((eu == 0.0f || ranged(eu)) && ranged(e1) && ranged(e2) && (x.iu == 0.0f || ranged(x.iu)));
+      plain = !((eu == 0.0f || ranged(eu)) && ranged(e1) && ranged(e2) &&
+                (x.iu == 0.0f || (fabsf(x.iu) >= 0x1p-64f && fabsf(x.iu) <= 0x1p32f)));
       const float m = fmaxf(fmaxf(fabsf(x.a), fabsf(x.b)), fabsf(x.c)), eu1 = eu == 0.0f ? 1.0f : eu;
       const float gv = fabsf(P.alpha1) * m + 4.0f * fabsf(P.alpha0);
       plain = plain || !(m <= 0x1p8f && gv <= 0x1p14f && P.lambda * fabsf(x.iu) <= kRate * eu1 &&
@@ -712,8 +714,9 @@ struct ResState<MASKED, float, R> {
     } else {
       f2 s, y;
       exact::root(pk(max1(lo(n2)), max1(hi(n2))), s, y);
-      a = exact::quot(a, s, y);
-      b = exact::quot(b, s, y);
+      const exact::Divisor d(s, y);
+      a = exact::quot(a, d);
+      b = exact::quot(b, d);
     }
   }
   // max(v, 1); a NaN stays
@@ -738,10 +741,11 @@ struct ResState<MASKED, float, R> {
     } else {
       f2 s, y;
       exact::root(pk(max1(lo(m2)), max1(hi(m2))), s, y);
-      x = exact::quot(x, s, y);
-      y_ = exact::quot(y_, s, y);
-      z = exact::quot(z, s, y);
-      w = exact::quot(w, s, y);
+      const exact::Divisor d(s, y);
+      x = exact::quot(x, d);
+      y_ = exact::quot(y_, d);
+      z = exact::quot(z, d);
+      w = exact::quot(w, d);
     }
   }
   // tau / eta; eta = 0 takes tau itself
@@ -805,9 +809,11 @@ struct ResState<MASKED, float, R> {
       } else {
         f2 sr, y;
         exact::root(pk(max1(n2), max1(m2)), sr, y);
-        pp = exact::quot(pp, both(lo(sr)), both(lo(y)));
-        qa = exact::quot(qa, both(hi(sr)), both(hi(y)));
-        qb = exact::quot(qb, both(hi(sr)), both(hi(y)));
+        const exact::Divisor d(sr, y);
+        const exact::Divisor dp = d.low(), dq = d.high();
+        pp = exact::quot(pp, dp);
+        qa = exact::quot(qa, dq);
+        qb = exact::quot(qb, dq);
       }
       p = upk(pp);
       sh.ptop[lane] = p;
@@ -917,7 +923,7 @@ struct ResState<MASKED, float, R> {
       const f2 up = prod(lt, prod(iu, iu)), far = prod(lt, iu);
       f2 newton;
       if (PLAIN) newton = pk(lo(rho) / lo(iu), hi(rho) / hi(iu));
-      else newton = exact::quot(rho, iu, exact::recip(iu));
+      else newton = exact::quot(rho, exact::Divisor(iu, exact::recip(iu)));
       f2 un;
       {
         // |rho| <= upper: the Newton step (none where Iu = 0); beyond it a step of lambda tau Iu / eta_u
