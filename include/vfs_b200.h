@@ -234,9 +234,10 @@ int vfs_batch_set_mode(vfs_batch* b, int mode);
  * limit; -1, the default: as many full-resolution working sets as fit in three quarters of
  * the L2 cache, and no limit when that is fewer than 2).  Each pair's solve is then two graphs: all pairs' coarser levels
  * start together, and pair k's full-resolution level follows pair k - max_pairs's, so that the
- * full-resolution working sets in flight stay in L2 (on B200, 8 pairs of 848 x 800 with FP16
- * storage: 15.3 ms per batch with 2 at a time against 17.2 ms without a limit).  Results are
- * unchanged. */
+ * full-resolution working sets in flight stay in L2.  That is worth most for levels that run one
+ * launch per iteration; where the full-resolution level is one launch per warp, those take the GPU in
+ * turn and the limit changes little (on B200, 8 pairs of 848 x 800 with FP16 storage: 7.89 ms per
+ * batch with 2 at a time, 7.94 without a limit).  Results are unchanged. */
 int vfs_batch_set_fine_concurrency(vfs_batch* b, int max_pairs);
 /* With a full-resolution limit: stagger_coarse = 1 also runs the coarser levels max_pairs
  * pairs at a time (pair k's after pair k - max_pairs's); priority = 1 runs the

@@ -566,7 +566,12 @@ void batch_solve(vfs_batch* b, int masked, const BatchHostIO* io) {
     int S = b->fine_limit;
     if (S < 0) {
       // auto: as many full-resolution working sets as fit in three quarters of L2, at least
-      // two (per pixel: the iteration's reads and the other ping-pong planes it writes)
+      // two (per pixel: the iteration's reads and the other ping-pong planes it writes).  The line was drawn for one
+      // launch per iteration (8 x 848x800 half: 15.3 ms with two pairs at once, 17.2 without a limit).  Whole-level
+      // launches hold their state on the chip and take the GPU in turn, and the limit matters little (B200, ms a
+      // batch with 1, 2, 4 at once and no limit: 8 x 848x800 half 7.94, 7.89, 7.88, 7.94, automatic 2; float 12.29,
+      // 12.26, 12.18, 12.16, automatic none; 16 float pairs of three sizes 18.4, 17.7, 17.5, 17.9, automatic none;
+      // 4 x 1280x1024 float, one launch per iteration at full resolution: 19.3, 17.4, 17.5, 17.6, automatic none)
       int dev = 0, l2 = 0;
       VFS_CUDA(cudaGetDevice(&dev));
       VFS_CUDA(cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, dev));
