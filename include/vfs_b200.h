@@ -216,7 +216,9 @@ int vfs_batch_solve_device(vfs_batch* b, const uint8_t* const* d_i0, const uint8
                            float* const* d_u_out, int masked);
 /* A one-pair solve (and each pair of a concurrent batch) runs every pyramid level whose state fits
  * the GPU's registers and shared memory (up to about 1,050,000 solved pixels with half storage,
- * 560,000 with float) in one launch per warp, all iterations in it.  For the other levels the fused path
+ * 560,000 with float) in one launch per warp, all iterations in it.  The blocks of such a launch wait for
+ * one another, so it starts when the GPU has room for all of them at once: a kernel of the caller's that
+ * keeps an SM's shared memory or registers holds it up.  For the other levels the fused path
  * picks the tile height of its iteration kernel by timing the variants on the first solve of
  * each batch composition (on by default); the timing launches do not change results.  Off: the
  * default 31 x 8 tiles there. */

@@ -31,10 +31,10 @@
 // written there).
 //
 // What bounds it, on B200 (FP16 storage, 848 x 800, 2037 tiles of 8 rows, 3.7 us per iteration):
-// about half of an iteration is instruction issue (1060 instructions per tile, 3.4 warps per
+// about half of an iteration is instruction issue (1040 instructions per tile, 3.4 warps per
 // scheduler, close to one per cycle), the rest the exchange: 1100 to 1500 cycles from a
 // store to the load that sees it, and the wait for the slowest neighbour.  One launch per iteration
-// (k_fused_iter) takes 8.0 us there alone, bound by its loads; float storage 6.1 against 10.3 us.
+// (k_fused_iter) takes 8.0 us there alone, bound by its loads; float storage 6.3 against 10.3 us.
 // Small levels are all latency, so theirs runs in one cluster whose blocks write into each other's
 // shared memory (k_resident_cluster): 53 x 50 takes 0.90 us, through L2 1.39, one launch per
 // iteration 3.2.

@@ -200,7 +200,7 @@ void ResTiles::place(int grid) {
 
 // The smallest tile height whose tiles fit, since more warps with less to do each hide more of one
 // another's latency and shorten an iteration (B200, us per iteration, FP16 / float storage: 848 x 800
-// disc 8 rows 3.7 / 6.1; 640 x 480 4 rows 2.45 / 3.5, 6 rows 2.75 / 3.9, 8 rows 3.1 / 5.3; 212 x 200
+// disc 8 rows 3.7 / 6.3; 640 x 480 4 rows 2.45 / 3.6, 6 rows 2.75 / 3.9, 8 rows 3.1 / 5.3; 212 x 200
 // 2 rows 1.40 / 1.73, 4 rows 1.60 / 2.15).  Two rows are left to levels that fill at most three
 // quarters of the warps: fuller, the row above each tile, which two rows pay for as much as four,
 // costs more than it gives (424 x 400, 91 %: 2 rows 2.0, 4 rows 1.87).  12 and 16 rows (half storage) cost

@@ -27,8 +27,10 @@ __device__ __forceinline__ float rsqrt(float x) {
 }
 
 // Pairs of floats on the packed FP32 instructions of sm_100 (add / sub / mul / fma .rn.f32x2,
-// no flush to zero): each lane is the IEEE single-precision operation of the scalar form, so
-// a packed step gives the bits of the two scalar steps it replaces.
+// no flush to zero): each lane is the IEEE single-precision operation of the scalar form.  ptxas (CUDA 12.9)
+// contracts a packed mul whose result is added into one fma, -fmad=false notwithstanding, so a packed
+// step gives the bits of the two scalar steps it replaces where those are fma's already, as in this file,
+// or where products are rounded by an fma of -0 (kernels_resident.cu, the float form).
 namespace x2 {
 typedef unsigned long long f2;
 __device__ __forceinline__ f2 pk(float x, float y) {
