@@ -1402,6 +1402,7 @@ __global__ void __launch_bounds__(512, 1) k_resident_cluster(const __grid_consta
     }
   }
   cl_barrier();  // every inbox is ready
+  bool gave_up = false;
   if (t < A.ntiles) {
     if (t != A.mute) push<ST, R>(W.s, C, lane, 0, W.flag(sh));  // iteration 0's input
     bool waiting = true;
@@ -1421,10 +1422,16 @@ __global__ void __launch_bounds__(512, 1) k_resident_cluster(const __grid_consta
       if (j + 1 < A.n) push<ST, R>(W.s, C, lane, j + 1, W.flag(sh));
       if (j + 2 >= A.n) W.store(sh, A, lane, j + 1 == A.n);
     }
-    if (!waiting && lane == 0) give_up(A);
+    gave_up = !__all_sync(kFull, waiting);
+    if (gave_up && lane == 0) give_up(A);
   }
   if (!MASKED) res_fill<ST, R>(A, warp, lane);
   cl_barrier();  // no block leaves while its neighbours may store into it
+  // Words that a tile has not waited for may still be on their way when all of them have been sent; its
+  // block stays until they are in (a word takes 600 cycles).
+  if (gave_up)
+    for (const long long c = clock64(); clock64() - c < 200000ll;) {
+    }
 }
 
 namespace {
